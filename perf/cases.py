@@ -136,24 +136,52 @@ def _mxfp4(w: torch.Tensor):
     return nib.cpu().numpy(), (exp + 127.0).to(torch.uint8).cpu().numpy()
 
 
-def _matrix(fmt: int, O: int, K: int, gen: torch.Generator) -> backend.CudaTensor:
+def _packed(fmt: int, O: int, K: int, gen: torch.Generator):
+    """One matrix in its container's form: (codes, scales, tensor scale)."""
     w = torch.randn((O, K), generator=gen, device="cuda") * WEIGHT_STD
     if fmt == FMT_NVFP4:
-        nib, scales, g = backend.quantize_nvfp4_dev(w)
-        return backend.CudaTensor.from_device(fmt, nib, scales, g, K, O)
+        return backend.quantize_nvfp4_dev(w)
     if fmt == FMT_FP8_B128:
-        codes, scales = backend.quantize_fp8_b128_dev(w)
-        return backend.CudaTensor.from_device(fmt, codes, scales, 1.0, K, O)
+        return (*backend.quantize_fp8_b128_dev(w), 1.0)
     if fmt == FMT_E4M3_ROW:
         scales = w.abs().amax(1) / 448.0
-        codes = (w / scales[:, None]).to(torch.float8_e4m3fn).view(torch.uint8)
-        return backend.CudaTensor.from_device(fmt, codes, scales, 1.0, K, O)
-    nib, scales = _mxfp4(w)
-    return backend.CudaTensor.wrap_mxfp4(nib, scales, 1.0, K, O)
+        return (w / scales[:, None]).to(torch.float8_e4m3fn).view(torch.uint8), scales, 1.0
+    return (*_mxfp4(w), 1.0)
+
+
+def _matrix(fmt: int, O: int, K: int, gen: torch.Generator) -> backend.CudaTensor:
+    codes, scales, g = _packed(fmt, O, K, gen)
+    if fmt == FMT_MXFP4:
+        return backend.CudaTensor.wrap_mxfp4(codes, scales, g, K, O)
+    return backend.CudaTensor.from_device(fmt, codes, scales, g, K, O)
 
 
 def _expert(s: MoeShape, gen: torch.Generator) -> Expert:
     return Expert(_matrix(s.fmt, s.I, s.H, gen), _matrix(s.fmt, s.I, s.H, gen), _matrix(s.fmt, s.H, s.I, gen))
+
+
+def _host_rows(s: MoeShape, seed: int, gen: torch.Generator):
+    # every seed has the same ragged counts, spread over the experts in another order
+    rng = np.random.default_rng(seed)
+    rows = [int(v) for v in rng.permutation(1 + np.random.default_rng(s.E).integers(0, s.T, s.E))]
+    return rows, torch.randn((sum(rows), s.H), generator=gen, device="cuda").cpu().numpy()
+
+
+def _router(s: MoeShape, seed: int, gen: torch.Generator):
+    """(weights bf16 [E,H], selection bias or None, logit bias or None)"""
+    rng = np.random.default_rng(seed)
+    router = (torch.randn((s.E, s.H), generator=gen, device="cuda") / math.sqrt(s.H)).to(torch.bfloat16)
+    popularity = -s.zipf_s * np.log(rng.permutation(s.E) + 1.0)
+    return (router, (rng.standard_normal(s.E) * s.select_bias_std).astype(np.float32) if s.select_bias_std else None,
+            (popularity - popularity.mean()).astype(np.float32) if s.zipf_s else None)
+
+
+def _tokens(case: dict, s: MoeShape, gen: torch.Generator):
+    """bf16 rows, or (f32 residual stream, norm weights) of a layer step"""
+    x = torch.randn((s.T, s.H), generator=gen, device="cuda")
+    if case["path"] == "layer_step":
+        return x * 4.0, 1.0 + 0.1 * torch.randn(s.H, generator=gen, device="cuda")
+    return x.to(torch.bfloat16)
 
 
 def prepare(case: dict, seed: int) -> dict:
@@ -161,26 +189,19 @@ def prepare(case: dict, seed: int) -> dict:
     s = _shape(case)
     gen = torch.Generator(device="cuda")
     gen.manual_seed(seed)
-    rng = np.random.default_rng(seed)
     experts = [_expert(s, gen) for _ in range(s.E)]
     state = dict(path=case["path"], T=s.T)
     if case["path"] == "experts":
-        # every seed has the same ragged counts, spread over the experts in another order
-        rows = [int(v) for v in rng.permutation(1 + np.random.default_rng(s.E).integers(0, s.T, s.E))]
-        x = torch.randn((sum(rows), s.H), generator=gen, device="cuda").cpu().numpy()
+        rows, x = _host_rows(s, seed, gen)
         return dict(state, gates=[e.gate for e in experts], ups=[e.up for e in experts], downs=[e.down for e in experts],
                     rows=rows, x=x)
-    router = (torch.randn((s.E, s.H), generator=gen, device="cuda") / math.sqrt(s.H)).to(torch.bfloat16)
-    popularity = -s.zipf_s * np.log(rng.permutation(s.E) + 1.0)
-    layer = Layer(router=router.view(torch.int16).cpu().numpy().view(np.uint16), experts=experts,
-                  router_bias=(rng.standard_normal(s.E) * s.select_bias_std).astype(np.float32) if s.select_bias_std else None,
-                  logit_bias=(popularity - popularity.mean()).astype(np.float32) if s.zipf_s else None,
-                  shared=_expert(s, gen) if s.shared else None)
+    router, select_bias, logit_bias = _router(s, seed, gen)
+    layer = Layer(router=router.view(torch.int16).cpu().numpy().view(np.uint16), experts=experts, router_bias=select_bias,
+                  logit_bias=logit_bias, shared=_expert(s, gen) if s.shared else None)
     state["block"] = MoeBlock(Config.from_shape(s), layer, case["max_tokens"])
-    x = torch.randn((s.T, s.H), generator=gen, device="cuda")
+    x = _tokens(case, s, gen)
     if case["path"] == "layer_step":
-        return dict(state, resid=x * 4.0, ln=1.0 + 0.1 * torch.randn(s.H, generator=gen, device="cuda"))
-    x = x.to(torch.bfloat16)
+        return dict(state, resid=x[0], ln=x[1])
     if case["path"] == "host_block":
         return dict(state, x=x.cpu().pin_memory(), out=torch.empty((s.T, s.H), dtype=torch.bfloat16).pin_memory())
     return dict(state, x=x)
@@ -223,3 +244,76 @@ def tolerance(case: dict) -> dict:
     if case["path"] == "layer_step":
         return {"rel": 4e-3, "max": 0.06}
     return {"rel": 1e-2, "max": 0.06}
+
+
+# ---- the same results in 64 bits -------------------------------------------------------------------------
+_E2M1 = [0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0, -0.0, -0.5, -1.0, -1.5, -2.0, -3.0, -4.0, -6.0]
+
+
+def _dense(fmt: int, packed, O: int, K: int) -> torch.Tensor:
+    """The f64 [O,K] weights that a packed matrix stands for."""
+    codes, scales, g = packed
+    if fmt in (FMT_FP8_B128, FMT_E4M3_ROW):
+        w = codes.view(torch.float8_e4m3fn).double()
+        if fmt == FMT_E4M3_ROW:
+            return w * scales.double()[:, None]
+        return w * scales.double().repeat_interleave(128, 0)[:O].repeat_interleave(128, 1)[:, :K]
+    codes, scales = torch.as_tensor(codes, device="cuda").long(), torch.as_tensor(scales, device="cuda")
+    table = torch.tensor(_E2M1, dtype=torch.float64, device="cuda")
+    w = torch.stack((table[codes & 15], table[codes >> 4]), 2).reshape(O, -1)[:, :K]
+    if fmt == FMT_NVFP4:
+        return w * (scales.view(torch.float8_e4m3fn).double() * g).repeat_interleave(16, 1)[:, :K]
+    return w * (torch.exp2(scales.double() - 127.0) * g).repeat_interleave(32, 1)[:, :K]
+
+
+def _ffn(s: MoeShape, packed, x: torch.Tensor) -> torch.Tensor:
+    gate, up, down = (_dense(s.fmt, m, *((s.H, s.I) if i == 2 else (s.I, s.H))) for i, m in enumerate(packed))
+    return (torch.nn.functional.silu(x @ gate.T) * (x @ up.T)) @ down.T
+
+
+def _route(s: MoeShape, x: torch.Tensor, router, select_bias, logit_bias):
+    """(experts, weights) of every row: moe.rs:1047-1132 with the group limit and the logit bias"""
+    z = x @ router.double().T
+    if logit_bias is not None:
+        z = z + torch.as_tensor(logit_bias, device="cuda").double()
+    score = torch.sigmoid(z) if s.score == SCORE_SIGMOID else torch.softmax(z, 1)
+    choice = score if select_bias is None else score + torch.as_tensor(select_bias, device="cuda").double()
+    if s.n_group > 1:
+        best = choice.view(s.T, s.n_group, -1).topk(2, dim=2).values.sum(2).topk(s.topk_group, dim=1).indices
+        allowed = torch.zeros((s.T, s.n_group), dtype=torch.bool, device="cuda").scatter_(1, best, True)
+        choice = choice.masked_fill(~allowed.repeat_interleave(s.E // s.n_group, 1), -math.inf)
+    idx = choice.topk(s.k, dim=1).indices
+    w = score.gather(1, idx)
+    if s.norm_topk:
+        w = w / w.sum(1, keepdim=True)
+    return idx, w * s.routed_scale
+
+
+def exact(case: dict, seed: int):
+    backend.init([0])
+    s = _shape(case)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(seed)
+    shapes = ((s.I, s.H), (s.I, s.H), (s.H, s.I))
+    experts = [[_packed(s.fmt, O, K, gen) for O, K in shapes] for _ in range(s.E)]
+    if case["path"] == "experts":
+        rows, x = _host_rows(s, seed, gen)
+        parts = torch.as_tensor(x, device="cuda").double().split(rows)
+        return torch.cat([_ffn(s, e, part) for e, part in zip(experts, parts)]).cpu().numpy()
+    routing = _router(s, seed, gen)
+    shared = [_packed(s.fmt, O, K, gen) for O, K in shapes] if s.shared else None
+    x = resid = _tokens(case, s, gen)
+    if case["path"] == "layer_step":
+        resid = x[0].double()
+        normed = resid * torch.rsqrt(resid.pow(2).mean(1, keepdim=True) + 1e-6) * x[1].double()
+        x = normed.to(torch.bfloat16)  # what the router and the experts are given
+    x = x.double()
+    idx, w = _route(s, x, *routing)
+    out = _ffn(s, shared, x) if s.shared else torch.zeros_like(x)
+    for e, packed in enumerate(experts):
+        token, kk = (idx == e).nonzero(as_tuple=True)
+        if len(token):
+            out.index_add_(0, token, _ffn(s, packed, x[token]) * w[token, kk, None])
+    if case["path"] == "layer_step":
+        return out + resid
+    return out.cpu() if case["path"] == "host_block" else out
