@@ -14,7 +14,7 @@
 //     CF_* round-to-nearest intrinsics;
 //   * the arg-max of each round is the largest value with the lowest index, which is what the
 //     ascending strict-`>` scan returns; a round with no candidate above -inf returns 0.
-#include <cstdlib>
+#include <cmath>
 
 #include "internal.cuh"
 
@@ -84,9 +84,7 @@ __global__ void __launch_bounds__(256) k_router_gemm(RouteParams p) {
 // Router GEMM, batched shapes: BM tokens x 64 experts per CTA of NT threads, (BM*16/NT) x 4
 // outputs per thread, k-chunks of 32 staged with 16-byte loads and stored transposed as f32, so
 // the inner loop is a few 128-bit shared loads per block of FMAs.  Same arithmetic as above: each
-// output is one thread's k-ascending fmaf chain.  Needs H % 8 == 0.  The chain makes the kernel
-// issue-bound with a fixed time per CTA, so the variants trade work per thread against the number
-// of CTAs: the launcher takes the largest tile that still covers the SMs.
+// output is one thread's k-ascending fmaf chain.  Needs H % 8 == 0.
 // Two independent f32 FMAs in one instruction (sm_100): c.x = fma(a.x, b, c.x), c.y = fma(a.y, b, c.y),
 // each rounded as a scalar fmaf, so an output's k-ascending chain is unchanged.  It halves the FMA
 // instructions of k_router_gemm_big (0.51 -> 0.475 ms at 4096 tokens x 256 experts x 7168); the 8 x 8
@@ -335,6 +333,147 @@ __global__ void __launch_bounds__(NT) k_router_rt(RouteParams p) {
     }
 }
 
+// Router GEMM for the batches below those of the two kernels above (H % 8 == 0): every thread owns
+// TM x TN outputs, each one k-ascending fmaf chain; a warp covers 4 TM tokens x 8 TN experts, a CTA
+// WM x WN warps.  Token and expert rows travel as bf16, in k-blocks of BK through a ring of STAGES
+// cp.async stages, so the loads of the next stages are in flight while one is multiplied; rows are
+// padded by 16 bytes, which puts eight consecutive rows of a quarter-warp's 128-bit loads into
+// different banks.
+// What bounds it: the chain of H dependent FMAs (4.3 cycles each, measured) with few outputs per SM,
+// the issue slots otherwise: for 8 k a thread issues 8 TM TN FMAs, 8 (TM + TN) operations that widen
+// bf16 to f32 (at half the FMA rate) and TM + TN shared loads.  A small tile spreads few outputs over
+// all SMs, a large one spends fewer slots per FMA: pick_router_tile weighs the two.
+// Measured with the top-k behind it, before (the kernels above, or a CTA of 16 tokens x 64 experts)
+// and now: 48 tokens x 128 experts x 2048 63.8 -> 19.7 us, 24 x 256 x 7168 202 -> 47, 512 x 128 x 2048
+// 65 -> 30, 709 x 256 x 7168 320 -> 151, 2048 x 256 x 7168 320 -> 277.  Staging the operands as f32 by
+// warps of their own was built and is slower from 200 tokens on (shared-memory reads).
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16u : 0u) : "memory");
+}
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+template <int TM_, int TN_, int WM_, int WN_, int BK_, int STAGES_>
+struct RouterTile {
+  static constexpr int TM = TM_, TN = TN_, WM = WM_, WN = WN_, BK = BK_, STAGES = STAGES_;
+  static constexpr int BM = 4 * TM * WM, BN = 8 * TN * WN, NT = 32 * WM * WN;
+  static constexpr int RS = BK * 2 + 16;  // row stride in bytes: an odd multiple of 16
+  static constexpr int CH = BK / 8;       // 16-byte chunks of a row
+  static constexpr int STAGE_BYTES = (BM + BN) * RS;
+  static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES;
+  static_assert((RS / 16) % 2 == 1 && (BM + BN) * CH % NT == 0, "row padding / staging split");
+};
+template <class C>
+__global__ void __launch_bounds__(C::NT) k_router_chain(RouteParams p) {
+  constexpr int TM = C::TM, TN = C::TN, RS = C::RS, CH = C::CH, BM = C::BM, BN = C::BN;
+  constexpr bool SMALL = TM * TN <= 8;  // the next chunk's operands are loaded ahead of this one's FMAs
+  constexpr bool PAIRED = TM % 2 == 0;  // two tokens per FMA instruction (3 to 6 % at every tile that can)
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const uint32_t smem = (uint32_t)__cvta_generic_to_shared(smem_raw);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+  const int xrow = (warp / C::WN) * 4 * TM + (lane >> 3), wrow = (warp % C::WN) * 8 * TN + (lane & 7);
+  const int nkb = (p.H + C::BK - 1) / C::BK;
+
+  auto fetch = [&](int kb) {  // rows of k-block kb; beyond T, E or H they are zeros
+    const uint32_t dst = smem + (uint32_t)(kb % C::STAGES) * C::STAGE_BYTES;
+#pragma unroll
+    for (int i = 0; i < (BM + BN) * CH / C::NT; ++i) {
+      const int idx = i * C::NT + (int)threadIdx.x;
+      const int r = idx / CH, c = idx % CH, k = kb * C::BK + c * 8;
+      const int row = r < BM ? m0 + r : n0 + r - BM;
+      const bool valid = row < (r < BM ? p.T : p.E) && k < p.H;
+      const __nv_bfloat16 *src = r < BM ? p.x : p.router_w;
+      cp_async16(dst + (uint32_t)(r * RS + c * 16), valid ? src + (size_t)row * p.H + k : src, valid);
+    }
+  };
+#pragma unroll
+  for (int s = 0; s < C::STAGES - 1; ++s) {
+    if (s < nkb) fetch(s);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  float acc[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
+  float2 acc2[(TM + 1) / 2][TN];
+#pragma unroll
+  for (int i = 0; i < (TM + 1) / 2; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc2[i][j] = make_float2(0.0f, 0.0f);
+
+  for (int kb = 0; kb < nkb; ++kb) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(C::STAGES - 2) : "memory");
+    __syncthreads();  // block kb has arrived for every thread, and its predecessor's slot is free
+    if (kb + C::STAGES - 1 < nkb) fetch(kb + C::STAGES - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const uint32_t xs = smem + (uint32_t)(kb % C::STAGES) * C::STAGE_BYTES + (uint32_t)(xrow * RS);
+    const uint32_t ws = smem + (uint32_t)(kb % C::STAGES) * C::STAGE_BYTES + (uint32_t)((BM + wrow) * RS);
+    uint4 xv[TM], wv[TN];
+    auto load = [&](uint4 (&xv)[TM], uint4 (&wv)[TN], int c) {
+#pragma unroll
+      for (int i = 0; i < TM; ++i) xv[i] = lds128(xs + (uint32_t)(i * 4 * RS + c * 16));
+#pragma unroll
+      for (int j = 0; j < TN; ++j) wv[j] = lds128(ws + (uint32_t)(j * 8 * RS + c * 16));
+    };
+    // element q of a chunk: the low or the high half of word q / 2
+    auto widen = [](const uint4 &v, int q) {
+      const uint32_t w = (&v.x)[q >> 1];
+      return __uint_as_float((q & 1) ? w & 0xffff0000u : w << 16);
+    };
+#pragma unroll(SMALL ? CH : 1)
+    for (int c = 0; c < CH; ++c) {
+      if (c == 0 || !SMALL) load(xv, wv, c);
+      uint4 xc[TM], wc[TN];
+#pragma unroll
+      for (int i = 0; i < TM; ++i) xc[i] = xv[i];
+#pragma unroll
+      for (int j = 0; j < TN; ++j) wc[j] = wv[j];
+      if (SMALL && c + 1 < CH) load(xv, wv, c + 1);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        float a[TM], b[TN];
+#pragma unroll
+        for (int i = 0; i < TM; ++i) a[i] = widen(xc[i], q);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) b[j] = widen(wc[j], q);
+        if constexpr (PAIRED) {
+#pragma unroll
+          for (int i = 0; i < TM; i += 2)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) coli_ffma2(acc2[i / 2][j], make_float2(a[i], a[i + 1]), b[j]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j] = __fmaf_rn(a[i], b[j], acc[i][j]);
+        }
+      }
+    }
+  }
+  if constexpr (PAIRED) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) acc[i][j] = (i & 1) ? acc2[i / 2][j].y : acc2[i / 2][j].x;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int m = m0 + xrow + 4 * i, n = n0 + wrow + 8 * j;
+      if (m < p.T && n < p.E) {
+        float v = acc[i][j];
+        if (p.logit_bias) v = __fadd_rn(v, p.logit_bias[n]);
+        p.logits[(size_t)m * p.E + n] = v;
+      }
+    }
+}
+
 // Decode shape (T <= 8): one thread per (token, expert) walking its own k chain; the block's 8
 // expert rows and all token rows are staged in shared memory as bf16 with coalesced 16-byte
 // loads first.  The chain of H dependent FMAs is the latency floor of bit-exact routing.
@@ -388,10 +527,6 @@ __device__ __forceinline__ void router_decode_block(const RouteParams &p, unsign
   }
   if (p.logit_bias) acc = __fadd_rn(acc, p.logit_bias[e0 + el]);
   p.logits[(size_t)t * p.E + e0 + el] = acc;
-}
-__global__ void __launch_bounds__(256) k_router_decode(RouteParams p) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  router_decode_block(p, smem_raw);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -563,33 +698,30 @@ static bool launch_router_rt(const RouteParams &p, cudaStream_t st) {
   k_router_rt<TM, TN, NT><<<grid, NT, smem, st>>>(p);
   return true;
 }
-// The register-tiled variants, largest tile first; `force` (1-based, from COLI_ROUTER_TILE, a
-// measurement aid) picks one regardless of the batch.  Returns -1 when none applies.
-static int launch_router_tiled(const RouteParams &p, cudaStream_t st) {
-  if (p.H % 8 != 0 || p.E < 64) return -1;
-  const char *fe = getenv("COLI_ROUTER_TILE");
-  const int force = fe ? atoi(fe) : 0;
-  auto ctas = [&](int bm, int bn) { return (long)((p.T + bm - 1) / bm) * ((p.E + bn - 1) / bn); };
-  int pick = force;
-  if (pick <= 0) {
-    // Measured on B200 (H = 7168 / 6144): the 8 x 8 tile pays once a batch gives every SM well over one
-    // 128 x 128 CTA (T = 16384, E = 384: 1.92 ms against 2.17); below that the narrower tiles of
-    // k_router_gemm_big, which keep two warps per scheduler, are as fast or faster.
-    if (p.E >= 128 && ctas(128, 128) >= 240) pick = 7;
-    else return -1;
-  }
-  bool ok = false;
-  switch (pick) {
-    case 1: ok = launch_router_rt<8, 8, 128>(p, st); break;   // 64 tokens x 128 experts
-    case 2: ok = launch_router_rt<4, 8, 128>(p, st); break;   // 32 x 128
-    case 3: ok = launch_router_rt<4, 4, 128>(p, st); break;   // 32 x 64
-    case 4: ok = launch_router_rt<4, 4, 64>(p, st); break;    // 16 x 64, two warps
-    case 5: ok = launch_router_rt<2, 4, 64>(p, st); break;    // 8 x 64
-    case 6: ok = launch_router_rt<8, 4, 128>(p, st); break;   // 64 x 64
-    case 7: ok = launch_router_rt<8, 8, 256>(p, st); break;   // 128 x 128
-    default: return -1;
-  }
-  return ok ? 1 : 0;
+// The tiles of k_router_chain.
+//                              TM TN WM WN  BK  stages
+using RouterTile8x8 = RouterTile<1, 1, 2, 1, 128, 8>;
+using RouterTile16x32 = RouterTile<2, 2, 2, 2, 64, 8>;
+using RouterTile64x64 = RouterTile<8, 4, 2, 2, 64, 6>;
+template <class C>
+static bool launch_router_chain(const RouteParams &p, cudaStream_t st) {
+  static ColiPerDeviceOnce attr_once;
+  if (C::SMEM > 48 * 1024 && !coli_set_smem_limit(attr_once, k_router_chain<C>, C::SMEM, "router shared-memory attribute")) return false;
+  k_router_chain<C><<<dim3((p.T + C::BM - 1) / C::BM, (p.E + C::BN - 1) / C::BN), C::NT, C::SMEM, st>>>(p);
+  return true;
+}
+// The kernel and tile of a batch: 0 = 8 x 8, 1 = 16 x 32, 2 = 64 x 64 tokens x experts of k_router_chain,
+// 3 = 128 x 64 of k_router_gemm_big, 4 = 128 x 128 of k_router_rt.  The time of one k is a function of
+// n, the CTAs of the fullest SM; the figures are nanoseconds measured on B200 between 21 and 16384
+// tokens (5.3 and 10 are the chain's latency, with its loads and conversions, when an SM has little else).
+static int pick_router_tile(const RouteParams &p) {
+  auto n = [&](int bm, int bn) { return (float)(((long)((p.T + bm - 1) / bm) * ((p.E + bn - 1) / bn) + 147) / 148); };
+  const float ns[5] = {fmaxf(5.3f, 1.6f * n(8, 8)), fmaxf(10.0f, 3.0f + 5.6f * n(16, 32)), 3.0f + 33.0f * n(64, 64),
+                       63.0f * n(128, 64), 103.0f * n(128, 128)};
+  int best = 0;
+  for (int i = 1; i < 5; ++i)
+    if (ns[i] < ns[best]) best = i;
+  return best;
 }
 
 int launch_router(const RouteParams &p, cudaStream_t st) {
@@ -606,40 +738,24 @@ int launch_router(const RouteParams &p, cudaStream_t st) {
     coli_set_error("router: k=%d exceeds the experts of the %d groups a token may use", p.k, p.topk_group);
     return 0;
   }
-  const size_t dec_smem = (size_t)(p.T + 8) * (p.H + 8) * sizeof(__nv_bfloat16);
-  if (p.T <= 8 && p.H % 8 == 0 && dec_smem <= 200 * 1024) {
-    static ColiPerDeviceOnce attr_once;
-    if (!coli_set_smem_limit(attr_once, k_router_decode, 200 * 1024, "decode router shared-memory attribute")) return 0;
-    k_router_decode<<<(p.E + 7) / 8, 256, dec_smem, st>>>(p);  // 256 threads stage the rows, T*8 of them walk the chains
-    coli_count_launch(1);
-  } else if (const int tiled = launch_router_tiled(p, st); tiled >= 0) {
-    if (tiled == 0) return 0;
-    coli_count_launch(1);
-  } else {
-    // the largest tile that still covers the SMs; every variant has identical arithmetic
-    auto blocks = [&](int bm, int bn) { return (long)((p.T + bm - 1) / bm) * ((p.E + bn - 1) / bn); };
-    const long want = 120;
-    if (p.H % 8 == 0 && blocks(128, 64) >= want) {
-      dim3 grid((p.E + 63) / 64, (p.T + 127) / 128);
-      if (!launch_router_big<128, 256>(p, grid, st)) return 0;
-    } else if (p.H % 8 == 0 && blocks(64, 64) >= want) {
-      dim3 grid((p.E + 63) / 64, (p.T + 63) / 64);
-      if (!launch_router_big<64, 256>(p, grid, st)) return 0;
-    } else if (p.H % 8 == 0 && blocks(32, 64) >= want) {
-      dim3 grid((p.E + 63) / 64, (p.T + 31) / 32);
-      if (!launch_router_big<32, 128>(p, grid, st)) return 0;
-    } else if (p.H % 8 == 0 && p.T >= 16) {
-      dim3 grid((p.E + 63) / 64, (p.T + 15) / 16);
-      if (!launch_router_big<16, 128>(p, grid, st)) return 0;
-    } else if (blocks(32, 32) >= 96) {
-      dim3 grid((p.E + 31) / 32, (p.T + 31) / 32);
-      k_router_gemm<2, 2><<<grid, 256, 0, st>>>(p);
-    } else {
-      dim3 grid((p.E + 15) / 16, (p.T + 15) / 16);
-      k_router_gemm<1, 1><<<grid, 256, 0, st>>>(p);
+  // the batched kernels copy 16-byte chunks of rows; anything else takes the element-wise kernel
+  const bool rows16 = p.H % 8 == 0 && ((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.router_w)) & 15) == 0;
+  if (rows16) {
+    bool ok = false;
+    switch (pick_router_tile(p)) {
+      case 0: ok = launch_router_chain<RouterTile8x8>(p, st); break;
+      case 1: ok = launch_router_chain<RouterTile16x32>(p, st); break;
+      case 2: ok = launch_router_chain<RouterTile64x64>(p, st); break;
+      case 3: ok = launch_router_big<128, 256>(p, dim3((p.E + 63) / 64, (p.T + 127) / 128), st); break;
+      case 4: ok = launch_router_rt<8, 8, 256>(p, st); break;
     }
-    coli_count_launch(1);
+    if (!ok) return 0;
+  } else if ((long)((p.T + 31) / 32) * ((p.E + 31) / 32) >= 96) {
+    k_router_gemm<2, 2><<<dim3((p.E + 31) / 32, (p.T + 31) / 32), 256, 0, st>>>(p);
+  } else {
+    k_router_gemm<1, 1><<<dim3((p.E + 15) / 16, (p.T + 15) / 16), 256, 0, st>>>(p);
   }
+  coli_count_launch(1);
   const size_t sm = (size_t)4 * 2 * p.E * sizeof(float);
   k_route_topk<<<(p.T + 3) / 4, 128, sm, st>>>(p);
   coli_count_launch(1);
