@@ -85,18 +85,21 @@ template <int FMT>
 __device__ __forceinline__ void load_a(AFrag<FMT> &f, const WeightRef &w, int Op, int r0, int kt, int lane) {
   if (FMT == COLI_FMT_NVFP4) {
     const uint8_t *slab = w.q + ((size_t)kt * Op + r0) * 64;
-    f.lo[0] = ldg_nc_v4(slab + lane * 16);
-    f.hi[0] = ldg_nc_v4(slab + 512 + lane * 16);
+    // chunk t of rows g and g + 8 (r0 is a multiple of 16, so both are permuted alike)
+    const int off = (lane >> 2) * 64 + coli_fp4_chunk(lane >> 2, lane & 3) * 16;
+    f.lo[0] = ldg_nc_v4(slab + off);
+    f.hi[0] = ldg_nc_v4(slab + 512 + off);
     const uint8_t *ss = w.s + ((size_t)kt * Op + r0) * 8;
     const uint32_t s0 = *reinterpret_cast<const uint16_t *>(ss + lane * 2);
     const uint32_t s1 = *reinterpret_cast<const uint16_t *>(ss + 64 + lane * 2);
     f.sc = s0 | (s1 << 16);
   } else {
     const uint8_t *slab = w.q + ((size_t)kt * Op + r0) * 128;
-    f.lo[0] = ldg_nc_v4(slab + lane * 32);
-    f.lo[1] = ldg_nc_v4(slab + lane * 32 + 16);
-    f.hi[0] = ldg_nc_v4(slab + 1024 + lane * 32);
-    f.hi[1] = ldg_nc_v4(slab + 1024 + lane * 32 + 16);
+    const int g = lane >> 2, off0 = g * 128 + coli_fp8_chunk(g, 2 * (lane & 3)) * 16, off1 = off0 ^ 16;
+    f.lo[0] = ldg_nc_v4(slab + off0);
+    f.lo[1] = ldg_nc_v4(slab + off1);
+    f.hi[0] = ldg_nc_v4(slab + 1024 + off0);
+    f.hi[1] = ldg_nc_v4(slab + 1024 + off1);
     f.sc = 0;
   }
 }

@@ -56,13 +56,13 @@ __device__ __forceinline__ TcPackedKT tc_load_kt(const WeightRef &w, int Op, int
   r.sc = make_uint2(0, 0);
   if (row < Op) {
     const size_t base = (size_t)kt * Op + row;
-    const uint8_t *qp = w.q + base * 64 + c * 16;
+    const uint8_t *qp = w.q + base * 64 + coli_fp4_chunk(row, c) * 16;
     asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r.q0.x), "=r"(r.q0.y), "=r"(r.q0.z), "=r"(r.q0.w)
                  : "l"(qp));
     asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r.q1.x), "=r"(r.q1.y), "=r"(r.q1.z), "=r"(r.q1.w)
-                 : "l"(qp + 32));
+                 : "l"(w.q + base * 64 + coli_fp4_chunk(row, c + 2) * 16));
     asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(r.sc.x), "=r"(r.sc.y) : "l"(w.s + base * 8));
   }
   return r;
@@ -166,9 +166,8 @@ __global__ void __launch_bounds__(TcCfg<GATED>::THREADS, 1) k_ffn_tc(const __gri
     }
   } else if (warp == 1) {
     // ---------------- MMA issue ----------------
-    // (one issuing thread: with both operands in shared memory this kernel is bound by that
-    // memory's bandwidth, and a second issuing thread, which helps expert_tc_tmem.cu, measured
-    // no faster here)
+    // (with both operands in shared memory this kernel is bound by that memory's bandwidth; a second
+    // issuing thread measured no faster)
     if (lane == 0) {
       uint32_t it = 0, small_units = 0;
       uint32_t waits[2] = {0u, 0u};  // completed waits on each buffer's "drained" barrier

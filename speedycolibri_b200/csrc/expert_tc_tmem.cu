@@ -3,26 +3,37 @@
 //
 // Same formulation as expert_tc.cu (features on the MMA's M = 128, the ragged token count on its
 // N), but the decoded weights never pass through shared memory:
-// * A operand: 16 producer warps stream the packed NVFP4 or FP8 bytes from HBM with 256-bit loads
-//   (one thread = one weight row = one TMEM lane), convert them to f16 in registers and write 64 k
-//   per stage straight into a ring of 32-column TMEM slots with tcgen05.st.  A stage holds two
-//   weight tiles (gate + up of the same 128 features, or two adjacent 128-feature tiles of down);
-//   the ring is three stages deep beside 160-column accumulators, six beside 64-column ones.
+// * A operand: two loading warps copy the packed NVFP4 or FP8 bytes from HBM into a shared-memory
+//   ring of k-tiles (cp.async, 3 to 9 slots of 18 or 32 KB); 16 producer warps read them (one thread
+//   = one weight row = one TMEM lane), convert them to f16 in registers and write 64 k per stage
+//   into a ring of 32-column TMEM slots with tcgen05.st.  A stage holds two weight tiles (gate + up
+//   of the same 128 features, or two adjacent 128-feature tiles of down); the ring is three stages
+//   deep beside 160-column accumulators, six beside 64-column ones.
 // * B operand: up to 160 token rows x 64 k of f16 activations per stage, copied by TMA as ONE box
 //   (cp.async.bulk.tensor, 128-byte swizzle, no multicast; one tensor map per box height) into a
 //   6-deep shared-memory ring and shared by both weight tiles of the stage.
-// * tcgen05.mma kind::f16 with A from tensor memory and B through a shared-memory descriptor,
-//   two accumulators of 160 columns, each fed by its own issuing thread (the instruction stream
-//   of a single issuing thread, not the tensor core, bounded the first version of this kernel);
-//   the epilogue forms act(g, u) or writes the two down tiles.
+// * tcgen05.mma kind::f16 with A from tensor memory and B through a shared-memory descriptor, two
+//   accumulators of 160 columns fed by one issuing warp, two stages per barrier wait; the epilogue
+//   forms act(g, u) or writes the two down tiles.
 // Why: with both operands in shared memory an MMA of 128 x 128 x 16 fetches 8 KB per 64 cycles,
 // the whole shared-memory bandwidth of an SM, before a single decoded weight is stored there
 // (expert_tc.cu tops out near half of the tensor peak at 128 tokens per expert).  Here shared
-// memory carries only the token tiles: 16-20 KB written + twice that read per stage.
+// memory carries the token tiles (16-20 KB written + twice that read per stage) and the packed
+// weights (9 or 16 KB each way).
 // TMEM budget: 2 x 160 accumulator columns + 6 x 32 weight columns = 512, which is why this
 // kernel takes tiles of at most 160 tokens (a layer with 128 rows per expert on average has
 // nearly all of its segments under that); wider segments are cut into several work items.
 // Layers with short segments run a second instantiation with 2 x 64 + 12 x 32 columns.
+//
+// What bounds it, measured with clock stamps.  An MMA takes N / 2 cycles from 16 tokens up when it is
+// issued back to back; the wait for a stage costs the issuing warp about 190 cycles on top, which long
+// tiles hide.  With one branch on the lane index per thread of issue, a wait and a commit per stage and
+// accumulator, a stage took 830 cycles whatever its tokens (256 of MMA at 64); with weights loaded into
+// the producers' registers it stayed there, and with bulk copies in place of cp.async at 728 (the copy
+// engine).  Gate+up and down, before and now: 709 tokens on H 7168, I 2048, 256 experts 1461 + 771 us
+// -> 1100 + 573 (4.2 GB of weights: 650 + 325 at the copy rate); 4096 tokens 2153 + 1170 -> 2020 + 1047
+// (1320 + 660 at the tensor rate); FP8, 512 tokens, H 2048, I 768, 128 experts 130 + 77 -> 97 + 57;
+// NVFP4, 1024 tokens on the same sizes 123 + 71 -> 97 + 56.
 //
 // Roles are warp-specialised and synchronise through mbarriers only; the kernel is persistent.
 // Every barrier wait is bounded: on a time-out the CTA raises a status word, stops issuing work,
@@ -61,46 +72,33 @@ struct TtBudget {
   // number of stage barriers (a ring twice as deep was measured and changed nothing)
   static constexpr int B_BYTES = ACC * TC_BK * 2;
   static constexpr int B_STAGES = 6;
-  static constexpr int NBARS = 2 * B_STAGES + 2;
+  static constexpr int NBARS = 2 * B_STAGES + 2 + 2 * 9;  // stages, accumulators, at most 9 weight slots
   static_assert(B_STAGES % A_STAGES == 0 && B_BYTES % 1024 == 0, "a stage barrier serves both rings");
 };
 // The token tile of a stage arrives as ONE box of N rows: the copy engine of an SM takes about 64
 // cycles per box plus 4 per 128-byte row (measured: 21 B/clk with 32-row boxes, 31 B/clk with
 // 160-row ones, on 8 SMs as on 148), and at 21 B/clk the 20 KB tile of a 160-token stage takes
-// longer than the stage's MMAs.  One tensor map per box height (32, 64, ... rows).
+// longer than the stage's MMAs.  One tensor map per box height (16, 32, ... rows).
+template <int ACC>
 struct TtMaps {
-  CUtensorMap m[TCT_MAX_TOKENS / TC_BOXN];
+  CUtensorMap m[ACC / TC_BOXN];
 };
 constexpr int TT_PROD_WARPS = 16;
-constexpr int TT_MMA2_WARP = 2 + TC_EPI_WARPS + TT_PROD_WARPS;       // the second MMA-issuing warp
-constexpr int TT_THREADS = 32 * (TT_MMA2_WARP + 1);                  // 736
+constexpr int TT_LOAD_WARP0 = 2 + TC_EPI_WARPS + TT_PROD_WARPS;      // the two warps that copy weight slabs
+constexpr int TT_LOAD_THREADS = 64;
+constexpr int TT_THREADS = 32 * TT_LOAD_WARP0 + TT_LOAD_THREADS;     // 768
 
-// The MMAs of one 64-k stage into ONE accumulator and the commit that releases the stage's
+// The MMAs of one 64-k stage into both accumulators and the commit that releases the stage's
 // operands, as one instruction sequence: four k steps of 16 (8 TMEM columns of f16 weights, 32
-// bytes = 2 descriptor units of tokens per step).
-__device__ __forceinline__ void tt_issue_stage(uint32_t acc, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate_first,
-                                               uint32_t bar) {
-  asm volatile(
-      "{\n"
-      ".reg .pred pf, pt;\n"
-      ".reg .b64 bd;\n"
-      ".reg .b32 a;\n"
-      "setp.ne.b32 pf, %4, 0;\n"
-      "setp.eq.b32 pt, %4, %4;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, pf;\n"
-      "add.s64 bd, %2, 2;\n"
-      "add.u32 a, %1, 8;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %3, pt;\n"
-      "add.s64 bd, %2, 4;\n"
-      "add.u32 a, %1, 16;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %3, pt;\n"
-      "add.s64 bd, %2, 6;\n"
-      "add.u32 a, %1, 24;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %3, pt;\n"
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n"
-      "}\n"
-      ::"r"(acc), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate_first), "r"(bar)
-      : "memory");
+// bytes = 2 descriptor units of tokens per step); the second tile's weights are 32 columns on.
+__device__ __forceinline__ void tt_issue_stage(uint32_t acc0, uint32_t acc1, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
+                                               uint32_t accumulate_first, uint32_t bar) {
+#pragma unroll
+  for (int k4 = 0; k4 < TC_BK / 16; ++k4) {
+    umma_f16_ts(acc0, a_tmem + 8 * k4, bdesc + 2 * k4, idesc, k4 ? 1u : accumulate_first);
+    umma_f16_ts(acc1, a_tmem + 32 + 8 * k4, bdesc + 2 * k4, idesc, k4 ? 1u : accumulate_first);
+  }
+  umma_commit(bar);
 }
 // 32 consecutive columns of this thread's lane
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -120,20 +118,18 @@ struct TtPacked {
   uint4 q0, q1;
   uint32_t sc;
 };
-__device__ __forceinline__ TtPacked tt_load_packed(const WeightRef &w, int Op, int row, int kb) {
+__device__ __forceinline__ uint4 tt_lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+// `slab` = shared-memory address of the 128-row slab of one k-tile: 64 B of codes per row, then 8 B
+// of scales per row; `half` = which 64 of its 128 k.
+__device__ __forceinline__ TtPacked tt_read_packed(uint32_t slab, int row, int half) {
   TtPacked r;
-  r.q0 = make_uint4(0, 0, 0, 0);
-  r.q1 = r.q0;
-  r.sc = 0;
-  if (row < Op) {
-    const size_t base = (size_t)(kb >> 1) * Op + row;
-    const uint8_t *qp = w.q + base * 64 + (kb & 1) * 32;
-    // one 256-bit load: the 32-byte sector of this row and stage is requested from L2 once
-    asm volatile("ld.global.nc.L1::no_allocate.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r.q0.x), "=r"(r.q0.y), "=r"(r.q0.z), "=r"(r.q0.w), "=r"(r.q1.x), "=r"(r.q1.y), "=r"(r.q1.z), "=r"(r.q1.w)
-                 : "l"(qp));
-    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(r.sc) : "l"(w.s + base * 8 + (kb & 1) * 4));
-  }
+  r.q0 = tt_lds128(slab + row * 64 + coli_fp4_chunk(row, 2 * half) * 16);
+  r.q1 = tt_lds128(slab + row * 64 + coli_fp4_chunk(row, 2 * half + 1) * 16);
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r.sc) : "r"(slab + TC_BM * 64 + row * 8 + half * 4) : "memory");
   return r;
 }
 // Convert one stage of one row and hand it to the tensor core through 32 TMEM columns.
@@ -171,29 +167,11 @@ __device__ __forceinline__ uint32_t tt_f16x2_both(float v) {
   const __half2 h = __float2half2_rn(v);
   return *reinterpret_cast<const uint32_t *>(&h);
 }
-__device__ __forceinline__ TtPacked8 tt_zero_packed8() {
+__device__ __forceinline__ TtPacked8 tt_read_packed8(uint32_t slab, int row, int half, uint32_t mult) {
   TtPacked8 r;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) r.q[j] = make_uint4(0, 0, 0, 0);
-  r.mult = 0;
-  return r;
-}
-// `norm` = TT_FP8_HEADROOM / max scale of the row block (block-scaled form), `srow` = that block's
-// row of the scale grid; both unused for per-row scales.
-template <int FMT>
-__device__ __forceinline__ TtPacked8 tt_load_packed8(const WeightRef &w, int Op, int row, int kb, const float *srow, float norm) {
-  TtPacked8 r = tt_zero_packed8();
-  if (row < Op) {
-    const uint8_t *qp = w.q + ((size_t)(kb >> 1) * Op + row) * 128 + (kb & 1) * 64;
-    // 256-bit loads: each 32-byte sector of this row and stage is requested from L2 once
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-      asm volatile("ld.global.nc.L1::no_allocate.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                   : "=r"(r.q[2 * j].x), "=r"(r.q[2 * j].y), "=r"(r.q[2 * j].z), "=r"(r.q[2 * j].w), "=r"(r.q[2 * j + 1].x),
-                     "=r"(r.q[2 * j + 1].y), "=r"(r.q[2 * j + 1].z), "=r"(r.q[2 * j + 1].w)
-                   : "l"(qp + 32 * j));
-    r.mult = FMT == COLI_FMT_FP8_B128 ? tt_f16x2_both(__ldg(srow + (kb >> 1)) * norm) : 0x3c003c00u /* 1.0 */;
-  }
+  for (int j = 0; j < 4; ++j) r.q[j] = tt_lds128(slab + row * 128 + coli_fp8_chunk(row, 4 * half + j) * 16);
+  r.mult = mult;
   return r;
 }
 __device__ __forceinline__ void tt_cvt_e4m3x4(uint32_t w, uint32_t &p0, uint32_t &p1) {
@@ -220,29 +198,50 @@ __device__ __forceinline__ void tt_convert8(const TtPacked8 &pk, uint32_t (&r)[3
     }
   }
 }
-// Largest scale of one row block over all k-tiles (every thread of a tile computes the same value).
-__device__ __forceinline__ float tt_block_scale_max(const float *srow, int KT) {
+// Largest scale of one row block over all k-tiles; a warp's lanes share the block and the loads.
+__device__ __forceinline__ float tt_block_scale_max(const float *srow, int KT, int lane) {
   float m = 0.0f;
-  for (int kt = 0; kt < KT; ++kt) m = fmaxf(m, __ldg(srow + kt));
+  for (int kt = lane; kt < KT; kt += 32) m = fmaxf(m, __ldg(srow + kt));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   return m;
+}
+
+// Shared memory: the ring of token tiles, then a ring of packed weight slabs -- both tiles of a stage,
+// one k-tile of 128 k (two stages) per slot -- that two warps fill with 16-byte cp.async copies, far
+// ahead of the producer warps.  A slab is one contiguous run of bytes in HBM.  (Bulk copies were
+// measured too: the copy engine that brings the token tiles then moves 17 KB per stage of 64 tokens
+// at about 23 bytes per clock and is what the kernel waits for.)
+template <int FMT, int ACC>
+struct TtWeightRing {
+  static constexpr int SLAB = FMT == COLI_FMT_NVFP4 ? TC_BM * (64 + 8) : TC_BM * 128;
+  static constexpr int SLOT = 2 * SLAB;
+  static constexpr int SLOTS = FMT == COLI_FMT_NVFP4 ? (ACC <= 64 ? 9 : 5) : (ACC <= 64 ? 5 : 3);
+  static constexpr int BYTES = SLOT * SLOTS;
+};
+__device__ __forceinline__ void tt_cp_async16(uint32_t dst, const void *src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16u : 0u) : "memory");
 }
 
 // GATED: the two weight tiles of a stage are gate and up of the same 128 features, result
 // h = act(g, u).  Otherwise: two adjacent 128-feature tiles of the down projection, result y.
 template <bool GATED, int FMT, int ACC>
-__global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant__ TtMaps maps, TcParams p) {
+__global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant__ TtMaps<ACC> maps, TcParams p) {
   constexpr int TT_A_STAGES = TtBudget<ACC>::A_STAGES, TT_A_COL0 = TtBudget<ACC>::A_COL0, TT_ACC_COLS = ACC;
   constexpr int TT_B_STAGES = TtBudget<ACC>::B_STAGES, TT_B_BYTES = TtBudget<ACC>::B_BYTES, TT_NBARS = TtBudget<ACC>::NBARS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + TT_B_STAGES * TT_B_BYTES);
-  // One "filled" and one "drained" barrier per stage of the token ring serve both operands: the
-  // issuing threads then pay one wait and one commit per stage.  filled[s]: 8 producer warps + the
-  // TMA thread's expect_tx arrival.  drained[s]: the commits of the two issuing threads.  The
-  // weight ring is half as deep, so a producer about to fill stage `it` waits for drained of
-  // stage it - TT_A_STAGES.
+  using Ring = TtWeightRing<FMT, ACC>;
+  const uint32_t wring = smem_u32(smem + TT_B_STAGES * TT_B_BYTES);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + TT_B_STAGES * TT_B_BYTES + Ring::BYTES);
+  // filled[s], s even: both operands of stages s and s + 1 (a k-tile), 8 producer warps + the TMA
+  // thread's expect_tx arrival; the issuing warp pays one wait for the two.  drained[s]: the commit
+  // behind stage s.  The tensor-memory ring is shallower, so a producer about to fill stage `it`
+  // waits for drained of stage it - TT_A_STAGES.
   const uint32_t full_s = smem_u32(bars), empty_s = smem_u32(bars + TT_B_STAGES);
   const uint32_t acc_full = smem_u32(bars + TT_NBARS - 2), acc_empty = smem_u32(bars + TT_NBARS - 1);
+  // weight slots: filled by the copies of the loading warps, read by the eight producer warps of their k-tile
+  const uint32_t wfull = smem_u32(bars + 2 * TT_B_STAGES), wempty = smem_u32(bars + 2 * TT_B_STAGES + Ring::SLOTS);
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + TT_NBARS);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
@@ -257,9 +256,13 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
   if (threadIdx.x == 0) {
     for (int s = 0; s < TT_B_STAGES; ++s) {
       mbar_init(full_s + 8 * s, 9);
-      mbar_init(empty_s + 8 * s, 2);
+      mbar_init(empty_s + 8 * s, 1);
     }
-    mbar_init(acc_full, 2);
+    for (int s = 0; s < Ring::SLOTS; ++s) {
+      mbar_init(wfull + 8 * s, TT_LOAD_THREADS);
+      mbar_init(wempty + 8 * s, TT_PROD_WARPS / 2);
+    }
+    mbar_init(acc_full, 1);
     mbar_init(acc_empty, TC_EPI_WARPS);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -291,8 +294,9 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
           }
           TT_TRACE(it, 6);
           const uint32_t dst = smem_u32(smem + s * TT_B_BYTES);
-          mbar_expect_tx(full_s + 8 * s, (uint32_t)N * TC_BK * 2);
-          tma_load_2d(dst, tmap, kb * TC_BK, row0, full_s + 8 * s);
+          const uint32_t full = full_s + 8 * (s & ~1u);  // (both rings of stages and k are even)
+          if (!(kb & 1)) mbar_expect_tx(full, (uint32_t)N * TC_BK * 4);
+          tma_load_2d(dst, tmap, kb * TC_BK, row0, full);
         }
       }
       if (!alive) {
@@ -300,47 +304,98 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
         for (int i = 0; i < 2000; ++i) __nanosleep(1000);
       }
     }
-  } else if (warp == 1 || warp == TT_MMA2_WARP) {
-    // ---------------- MMA issue: warp 1 feeds accumulator 0, the extra warp accumulator 1 ----------------
-    // One thread per accumulator keeps the order of its additions fixed, so results repeat bit for
-    // bit from run to run.  (Two threads per accumulator taking alternate stages were measured: the
-    // additions then interleave differently each run and the time per stage does not change.)
-    if (lane == 0) {
-      const uint32_t which = warp == 1 ? 0u : 1u;
-      uint32_t tix = 0;
-      bool alive = true;
-      const uint64_t bdesc_ring = umma_smem_desc(smem_u32(smem));  // token-tile stage 0; stages are TT_B_BYTES apart
-      const uint32_t acc = tmem_base + which * TT_ACC_COLS;
-      const uint32_t a_ring = tmem_base + TT_A_COL0 + which * 32;
-      // ring positions as counters: this thread's instruction stream is on the critical path of the
-      // kernel, so no division or modulo per stage
-      uint32_t sa = 0, sb = 0, phb = 0;
-      for (int w = blockIdx.x; w < n_work && alive; w += gridDim.x, ++tix) {
-        const int item = w / n_ftiles;
-        const int nrows = p.item_nrows[item];
-        const int N = (nrows + TC_BOXN - 1) / TC_BOXN * TC_BOXN;
-        const uint32_t idesc = umma_idesc(N);
-        if (!mbar_wait(acc_empty, (tix & 1u) ^ 1u, abort_flag, p.status, TC_ERR_MMA_WAIT, 1)) break;
-        tc_fence_after();
-        for (int kb = 0; kb < KB; ++kb) {
-          if (which == 0) TT_TRACE(tix * KB + kb, 0);
-          if (!mbar_wait(full_s + 8 * sb, phb, abort_flag, p.status, TC_ERR_MMA_WAIT, 1)) {
-            alive = false;
-            break;
+  } else if (warp >= TT_LOAD_WARP0) {
+    // ---------------- packed weight slabs: HBM -> shared memory ----------------
+    const int tid = (int)threadIdx.x - TT_LOAD_WARP0 * 32;
+    constexpr int QB = FMT == COLI_FMT_NVFP4 ? 64 : 128;        // code bytes of a row
+    constexpr int SB = FMT == COLI_FMT_NVFP4 ? 8 : 0;           // scale bytes of a row
+    constexpr int QI = TC_BM * QB / 16 / TT_LOAD_THREADS;       // chunks per thread: the codes of one tile
+    constexpr int SI = TC_BM * SB / 16 / TT_LOAD_THREADS;       // ... and its scales
+    static_assert(2 * (QI + SI) * TT_LOAD_THREADS * 16 == Ring::SLOT, "slab split");
+    uint32_t slot = 0, ph = 0;
+    bool alive = true;
+    for (int w = blockIdx.x; w < n_work && alive; w += gridDim.x) {
+      const int item = w / n_ftiles, ft = w % n_ftiles;
+      const int seg = p.item_seg[item];
+      const int ex = p.seg_expert ? p.seg_expert[seg] : seg;
+      const WeightRef wt[2] = {GATED ? p.gate[ex] : p.down[ex], GATED ? p.up[ex] : p.down[ex]};
+      for (int kt = 0; kt < (KB >> 1); ++kt) {
+        if (!__all_sync(0xffffffffu, mbar_wait(wempty + 8 * slot, ph ^ 1u, abort_flag, p.status, TC_ERR_TMA_WAIT, 1))) {
+          alive = false;
+          break;
+        }
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          const int row0 = ft * FT + (GATED ? 0 : m * TC_BM);
+          const int n = min(TC_BM, Op - row0);  // rows of this tile that exist; the rest are zeros
+          const size_t r = (size_t)kt * Op + row0;
+          const uint32_t dst = wring + slot * Ring::SLOT + m * Ring::SLAB;
+#pragma unroll
+          for (int i = 0; i < QI; ++i) {
+            const int c = (i * TT_LOAD_THREADS + tid) * 16;
+            tt_cp_async16(dst + c, c < n * QB ? wt[m].q + r * QB + c : wt[m].q, c < n * QB);
           }
-          if (which == 0) TT_TRACE(tix * KB + kb, 1);
-          tc_fence_after();
-          // both issuers commit: the rings are refilled once both accumulators have read them
-          tt_issue_stage(acc, a_ring + sa * 64, bdesc_ring + (uint64_t)(sb * (TT_B_BYTES >> 4)), idesc, kb ? 1u : 0u, empty_s + 8 * sb);
-          if (which == 0) TT_TRACE(tix * KB + kb, 2);
-          if (++sa == TT_A_STAGES) sa = 0;
-          if (++sb == TT_B_STAGES) {
-            sb = 0;
-            phb ^= 1u;
+#pragma unroll
+          for (int i = 0; i < SI; ++i) {
+            const int c = (i * TT_LOAD_THREADS + tid) * 16;
+            tt_cp_async16(dst + TC_BM * QB + c, c < n * SB ? wt[m].s + r * SB + c : wt[m].s, c < n * SB);
           }
         }
-        if (alive) umma_commit(acc_full);
+        // arrives when this thread's copies up to here have landed
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(wfull + 8 * slot) : "memory");
+        if (++slot == Ring::SLOTS) {
+          slot = 0;
+          ph ^= 1u;
+        }
       }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");  // nothing is in flight when this thread leaves
+  } else if (warp == 1) {
+    // ---------------- MMA issue ----------------
+    // The whole warp walks the loop and one elected lane issues, and every operand is a value the
+    // compiler knows to be the same in all lanes (constants, loop counters, warp reductions): an MMA
+    // takes its descriptors and addresses from uniform registers, and moving them there one by one
+    // under a branch on the lane index cost as much of this instruction stream as the MMAs themselves.
+    // Measured alone, with a barrier wait and a commit per stage: 317 cycles for the eight MMAs of 32
+    // tokens, 373 for 64, 640 (the tensor pipe's N / 2 each) for 160, the wait being about 190 of them
+    // that only the longer MMAs hide; two warps with an accumulator each take 435, 435 and 640.
+    const uint32_t tmem_u = __reduce_max_sync(0xffffffffu, tmem_base);
+    const uint64_t bdesc_ring = umma_smem_desc(smem_u32(smem));  // token-tile stage 0; stages are TT_B_BYTES apart
+    const uint32_t a_ring = tmem_u + TT_A_COL0;
+    uint32_t tix = 0;
+    bool alive = true;
+    // ring positions as counters: no division or modulo per stage
+    uint32_t sa = 0, sb = 0, phb = 0;
+    for (int w = blockIdx.x; w < n_work && alive; w += gridDim.x, ++tix) {
+      const int item = w / n_ftiles;
+      const int nrows = __reduce_max_sync(0xffffffffu, p.item_nrows[item]);
+      const int N = (nrows + TC_BOXN - 1) / TC_BOXN * TC_BOXN;
+      const uint32_t idesc = umma_idesc(N);
+      alive = __all_sync(0xffffffffu, mbar_wait(acc_empty, (tix & 1u) ^ 1u, abort_flag, p.status, TC_ERR_MMA_WAIT, 1));
+      if (!alive) break;
+      tc_fence_after();
+      for (int kb = 0; kb < KB; kb += 2) {
+        if (lane == 0) TT_TRACE(tix * KB + kb, 0);
+        alive = __all_sync(0xffffffffu, mbar_wait(full_s + 8 * sb, phb, abort_flag, p.status, TC_ERR_MMA_WAIT, 1));
+        if (!alive) break;
+        if (lane == 0) TT_TRACE(tix * KB + kb, 1);
+        tc_fence_after();
+        const uint32_t sa1 = sa + 1 == TT_A_STAGES ? 0u : sa + 1;
+        if (elect_one()) {
+          const uint64_t bd = bdesc_ring + (uint64_t)(sb * (TT_B_BYTES >> 4));
+          tt_issue_stage(tmem_u, tmem_u + TT_ACC_COLS, a_ring + sa * 64, bd, idesc, kb ? 1u : 0u, empty_s + 8 * sb);
+          tt_issue_stage(tmem_u, tmem_u + TT_ACC_COLS, a_ring + sa1 * 64, bd + (TT_B_BYTES >> 4), idesc, 1u, empty_s + 8 * (sb + 1));
+        }
+        __syncwarp();
+        if (lane == 0) TT_TRACE(tix * KB + kb, 2);
+        sa = sa1 + 1 == TT_A_STAGES ? 0u : sa1 + 1;
+        if ((sb += 2) == TT_B_STAGES) {
+          sb = 0;
+          phb ^= 1u;
+        }
+      }
+      if (alive && elect_one()) umma_commit(acc_full);
+      __syncwarp();
     }
   } else if (warp < 2 + TC_EPI_WARPS) {
     // ---------------- epilogue: TMEM -> registers -> global ----------------
@@ -358,8 +413,8 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
         // undo the per-tile normalisation of the producers (both tiles of a stage are 128-row aligned)
         const int KT = KB >> 1;
         const int rb0 = (ft * FT) >> 7, rb1 = GATED ? rb0 : rb0 + 1, nrb = (Oout + 127) >> 7;
-        s0 = tt_block_scale_max(reinterpret_cast<const float *>(w0.s) + (size_t)rb0 * KT, KT) * (1.0f / TT_FP8_HEADROOM);
-        s1 = rb1 < nrb ? tt_block_scale_max(reinterpret_cast<const float *>(w1.s) + (size_t)rb1 * KT, KT) * (1.0f / TT_FP8_HEADROOM) : 0.0f;
+        s0 = tt_block_scale_max(reinterpret_cast<const float *>(w0.s) + (size_t)rb0 * KT, KT, lane) * (1.0f / TT_FP8_HEADROOM);
+        s1 = rb1 < nrb ? tt_block_scale_max(reinterpret_cast<const float *>(w1.s) + (size_t)rb1 * KT, KT, lane) * (1.0f / TT_FP8_HEADROOM) : 0.0f;
       } else if (FMT == COLI_FMT_E4M3_ROW) {
         const int f1 = GATED ? f : f + TC_BM;
         s0 = f < Oout ? __ldg(reinterpret_cast<const float *>(w0.s) + f) : 0.0f;
@@ -416,89 +471,79 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
       if (lane == 0) mbar_arrive(acc_empty);
     }
   } else {
-    // ---------------- weight producers: HBM -> registers -> f16 -> tensor memory ----------------
-    // four groups of four warps (128 lanes = 128 weight rows each): group g fills weight tile
-    // (g & 1) of the stages whose index has parity (g >> 1)
+    // ---------------- weight producers: shared memory -> registers -> f16 -> tensor memory ----------------
+    // four groups of four warps (128 lanes = 128 weight rows each): group g converts weight tile
+    // (g & 1) of the k-tiles whose running index has parity (g >> 1), two stages each
     const int grp = (warp - 2 - TC_EPI_WARPS) >> 2;
     const int mtx = grp & 1, par = grp >> 1;
     const int quarter = warp & 3;  // TMEM lane quarter this warp may write
     const int row = quarter * 32 + lane;
     const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + TT_A_COL0 + mtx * 32;
-    uint32_t it0 = 0;
+    const int KT = KB >> 1;
+    uint32_t g = par;  // running index of this group's next k-tile
+    uint32_t g0 = 0;   // ... and of the tile's first
+    uint32_t wslot = par, wph = 0;
     bool alive = true;
-    // The conversion runs BEFORE the wait for the slot, so that only the store stands between the
-    // slot's release and the barrier that hands it to the issuing threads.
-    auto stage = [&](const auto &pk, uint32_t it) -> bool {
-      uint32_t r[32];
-      if constexpr (FMT == COLI_FMT_NVFP4)
-        tt_convert(pk, r);
-      else
-        tt_convert8<FMT>(pk, r);
-      const uint32_t sa = it % TT_A_STAGES;
-      bool ok = true;
-      if (mtx == 0 && quarter == 0 && lane == 0) TT_TRACE(it, 3);
-      if (it >= (uint32_t)TT_A_STAGES) {  // the weight slot was last read by stage it - TT_A_STAGES
-        const uint32_t u = it - TT_A_STAGES;
-        if (lane == 0) ok = mbar_wait(empty_s + 8 * (u % TT_B_STAGES), (u / TT_B_STAGES) & 1u, abort_flag, p.status, TC_ERR_PROD_WAIT, 1);
-        ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-        if (!ok) return false;
-        tc_fence_after();
+    for (int w = blockIdx.x; w < n_work && alive; w += gridDim.x, g0 += KT) {
+      const float *srow = nullptr;
+      float norm = 0.0f, scale = 0.0f;
+      int kt = (int)(g - g0);
+      if constexpr (FMT == COLI_FMT_FP8_B128) {
+        const int item = w / n_ftiles, ft = w % n_ftiles, seg = p.item_seg[item];
+        const int ex = p.seg_expert ? p.seg_expert[seg] : seg;
+        const WeightRef wr = GATED ? (mtx ? p.up[ex] : p.gate[ex]) : p.down[ex];
+        // (a second tile past the end has no scale row; its codes are zeros)
+        const int rb = min(GATED ? ft : 2 * ft + mtx, (Oout - 1) >> 7);
+        srow = reinterpret_cast<const float *>(wr.s) + (size_t)rb * KT;
+        // a row block whose scales are all zero (an all-zero or padded weight block: the encoder
+        // writes scale = amax / 448 = 0) decodes to zeros, as code x 0 does in convert.rs:731-741
+        const float mx = tt_block_scale_max(srow, KT, lane);
+        norm = mx > 0.0f ? TT_FP8_HEADROOM / mx : 0.0f;
+        scale = kt < KT ? __ldg(srow + kt) : 0.0f;
       }
-      if (mtx == 0 && quarter == 0 && lane == 0) TT_TRACE(it, 4);
-      tmem_st32(taddr + sa * 64, r);
-      tmem_st_wait();
-      if (mtx == 0 && quarter == 0 && lane == 0) TT_TRACE(it, 5);
-      tc_fence_before();
-      __syncwarp();
-#ifdef COLI_TT_TRACE
-      if (GATED && blockIdx.x == 0 && lane == 0 && it < 256u) atomicMax((unsigned long long *)&g_tt_trace[it * 8 + 7], (unsigned long long)clock64());
-#endif
-      if (lane == 0) mbar_arrive(full_s + 8 * (it % TT_B_STAGES));
-      return true;
-    };
-    for (int w = blockIdx.x; w < n_work && alive; w += gridDim.x, it0 += KB) {
-      const int item = w / n_ftiles, ft = w % n_ftiles;
-      const int seg = p.item_seg[item];
-      const int ex = p.seg_expert ? p.seg_expert[seg] : seg;
-      const WeightRef wr = GATED ? (mtx ? p.up[ex] : p.gate[ex]) : p.down[ex];
-      const int grow = GATED ? ft * TC_BM + row : ft * FT + mtx * TC_BM + row;
-      // this group's k blocks of the tile: those whose global stage index it0 + kb has parity `par`
-      const int kb0 = (int)((par - it0) & 1u);
-      // two register sets alternate (kb, kb+2 | kb+4, kb+6 | ...): the bytes of the next two stages
-      // of this group are in flight while one is converted, and no set is refilled before it is used
-      if constexpr (FMT == COLI_FMT_NVFP4) {
-        TtPacked pa, pb;
-        pa.q0 = make_uint4(0, 0, 0, 0);
-        pa.q1 = pa.q0;
-        pa.sc = 0;
-        pb = pa;
-        if (kb0 < KB) pa = tt_load_packed(wr, Op, grow, kb0);
-        if (kb0 + 2 < KB) pb = tt_load_packed(wr, Op, grow, kb0 + 2);
-        for (int kb = kb0; kb < KB && alive; kb += 4) {
-          alive = stage(pa, it0 + kb);
-          if (kb + 4 < KB) pa = tt_load_packed(wr, Op, grow, kb + 4);
-          if (alive && kb + 2 < KB) alive = stage(pb, it0 + kb + 2);
-          if (kb + 6 < KB) pb = tt_load_packed(wr, Op, grow, kb + 6);
+      for (; kt < KT && alive; kt += 2, g += 2) {
+        if (!__all_sync(0xffffffffu, mbar_wait(wfull + 8 * wslot, wph, abort_flag, p.status, TC_ERR_PROD_WAIT, 1))) {
+          alive = false;
+          break;
         }
-      } else {
-        const float *srow = nullptr;
-        float norm = 0.0f;
-        if (FMT == COLI_FMT_FP8_B128 && grow < Op) {
-          const int KT = KB >> 1;
-          srow = reinterpret_cast<const float *>(wr.s) + (size_t)(grow >> 7) * KT;
-          // a row block whose scales are all zero (an all-zero or padded weight block: the encoder
-          // writes scale = amax / 448 = 0) decodes to zeros, as code x 0 does in convert.rs:731-741
-          const float mx = tt_block_scale_max(srow, KT);
-          norm = mx > 0.0f ? TT_FP8_HEADROOM / mx : 0.0f;
+        const uint32_t slab = wring + wslot * Ring::SLOT + mtx * Ring::SLAB;
+        const uint32_t mult = FMT == COLI_FMT_FP8_B128 ? tt_f16x2_both(scale * norm) : 0x3c003c00u /* 1.0 */;
+        if (FMT == COLI_FMT_FP8_B128 && kt + 2 < KT) scale = __ldg(srow + kt + 2);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          // The conversion runs BEFORE the wait for the tensor-memory slot, so that only the store stands
+          // between the slot's release and the barrier that hands it to the issuing warp.
+          uint32_t r[32];
+          if constexpr (FMT == COLI_FMT_NVFP4)
+            tt_convert(tt_read_packed(slab, row, half), r);
+          else
+            tt_convert8<FMT>(tt_read_packed8(slab, row, half, mult), r);
+          if (half == 1) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(wempty + 8 * wslot);
+          }
+          const uint32_t it = 2 * g + half;
+          const uint32_t sa = it % TT_A_STAGES;
+          if (mtx == 0 && quarter == 0 && lane == 0) TT_TRACE(it, 3);
+          if (it >= (uint32_t)TT_A_STAGES) {  // the weight slot was last read by stage it - TT_A_STAGES
+            const uint32_t u = it - TT_A_STAGES;
+            if (!__all_sync(0xffffffffu, mbar_wait(empty_s + 8 * (u % TT_B_STAGES), (u / TT_B_STAGES) & 1u, abort_flag, p.status, TC_ERR_PROD_WAIT, 1))) {
+              alive = false;
+              break;
+            }
+            tc_fence_after();
+          }
+          if (mtx == 0 && quarter == 0 && lane == 0) TT_TRACE(it, 4);
+          tmem_st32(taddr + sa * 64, r);
+          tmem_st_wait();
+          if (mtx == 0 && quarter == 0 && lane == 0) TT_TRACE(it, 5);
+          tc_fence_before();
+          __syncwarp();
+          if (half == 1 && lane == 0) mbar_arrive(full_s + 8 * ((it - 1) % TT_B_STAGES));
         }
-        TtPacked8 pa = tt_zero_packed8(), pb = pa;
-        if (kb0 < KB) pa = tt_load_packed8<FMT>(wr, Op, grow, kb0, srow, norm);
-        if (kb0 + 2 < KB) pb = tt_load_packed8<FMT>(wr, Op, grow, kb0 + 2, srow, norm);
-        for (int kb = kb0; kb < KB && alive; kb += 4) {
-          alive = stage(pa, it0 + kb);
-          if (kb + 4 < KB) pa = tt_load_packed8<FMT>(wr, Op, grow, kb + 4, srow, norm);
-          if (alive && kb + 2 < KB) alive = stage(pb, it0 + kb + 2);
-          if (kb + 6 < KB) pb = tt_load_packed8<FMT>(wr, Op, grow, kb + 6, srow, norm);
+        if ((wslot += 2) >= (uint32_t)Ring::SLOTS) {
+          wslot -= Ring::SLOTS;
+          wph ^= 1u;
         }
       }
     }
@@ -514,11 +559,11 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
 
 template <bool GATED, int FMT, int ACC>
 static int launch_tct(const TcParams &p, const void *rows_base, int rows_cap, int sm_count, cudaStream_t st) {
-  const size_t smem = (size_t)TtBudget<ACC>::B_STAGES * TtBudget<ACC>::B_BYTES + 1024 /*align*/ + 8 * TtBudget<ACC>::NBARS + 16 + 64;
+  const size_t smem = (size_t)TtBudget<ACC>::B_STAGES * TtBudget<ACC>::B_BYTES + TtWeightRing<FMT, ACC>::BYTES + 1024 /*align*/ + 8 * TtBudget<ACC>::NBARS + 16 + 64;
   static ColiPerDeviceOnce attr_once;
   if (!coli_set_smem_limit(attr_once, k_ffn_tct<GATED, FMT, ACC>, smem, "tcgen05 kernel shared-memory attribute")) return 0;
-  TtMaps maps;
-  for (int j = 0; j < TCT_MAX_TOKENS / TC_BOXN; ++j)
+  TtMaps<ACC> maps;
+  for (int j = 0; j < ACC / TC_BOXN; ++j)
     if (!make_rows_map(&maps.m[j], rows_base, rows_cap, GATED ? p.H : p.I, (j + 1) * TC_BOXN)) return 0;
   const int FT = GATED ? TC_BM : 2 * TC_BM;
   const int n_ftiles = ((GATED ? p.I : p.H) + FT - 1) / FT;

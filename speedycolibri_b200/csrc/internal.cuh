@@ -26,6 +26,9 @@
 //             expert kernel reads it unchanged; `s_src` keeps the container's own scale bytes for
 //             the export call.  The handle's fmt stays 6; kernels are given coli_kernel_fmt(fmt).
 // Op = O rounded up to 16, Kp = I rounded up to 128; padding bytes are zero (decode to 0.0).
+// Inside a row's 64 or 128 bytes of q the 16-byte chunks are permuted by the row (coli_fp4_chunk,
+// coli_fp8_chunk): a slab copied to shared memory as it is can then be read by a thread per row,
+// 16 bytes at a time, without bank conflicts.
 //
 // Arithmetic type of the expert GEMMs: f16 x f16 -> f32.  FP4/FP8 codes convert to f16 with one
 // hardware cvt per pair, a decoded weight (code x block scale, at most 6 significant bits, between
@@ -53,6 +56,10 @@ struct WeightRef {
   float g;
   int pad;
 };
+
+// Where chunk c of row `row` is stored among the row's chunks; each is its own inverse.
+__host__ __device__ static inline int coli_fp4_chunk(int row, int c) { return c ^ ((row >> 1) & 3); }
+__host__ __device__ static inline int coli_fp8_chunk(int row, int c) { return c ^ (row & 7); }
 
 static inline int round_up(int a, int b) { return (a + b - 1) / b * b; }
 // Upper bound of the work items `rows` rows in at most `nseg` segments cut into: a segment of n

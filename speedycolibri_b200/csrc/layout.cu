@@ -13,16 +13,17 @@ __device__ __forceinline__ uint32_t nib_at(const uint8_t *nib, int rb, int row, 
   return (k & 1) ? (uint32_t)(b >> 4) : (uint32_t)(b & 0x0f);
 }
 
-// one thread per 32-bit word of the packed array: (kt, row, word j) covers k = kt*128 + 8j .. +7,
+// one thread per 32-bit word of the packed array: the word that holds k = kt*128 + 8j .. +7 of a row,
 // k ascending from the least significant nibble (the container's own order: byte = two
 // consecutive k, low nibble first, which is what cvt.rn.f16x2.e2m1x2 consumes)
 __global__ void k_pack_nvfp4_q(const uint8_t *nib, uint32_t *q, int O, int I, int Op, int KT) {
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t total = (size_t)KT * Op * 16;
   if (idx >= total) return;
-  const int j = (int)(idx % 16);
+  const int pos = (int)(idx % 16);
   const int row = (int)((idx / 16) % Op);
   const int kt = (int)(idx / 16 / Op);
+  const int j = coli_fp4_chunk(row, pos >> 2) * 4 + (pos & 3);
   const int rb = (I + 1) / 2;
   const int k0 = kt * 128 + j * 8;
   uint32_t w = 0;
@@ -51,7 +52,7 @@ __global__ void k_unpack_nvfp4_q(const uint32_t *q, uint8_t *nib, int O, int I, 
     const int k = byte * 2 + h;
     if (k >= I) break;
     const int kt = k >> 7, j = (k & 127) >> 3, el = k & 7;
-    const uint32_t w = q[((size_t)kt * Op + row) * 16 + j];
+    const uint32_t w = q[((size_t)kt * Op + row) * 16 + coli_fp4_chunk(row, j >> 2) * 4 + (j & 3)];
     out |= ((w >> (4 * el)) & 0xfu) << (4 * h);
   }
   nib[idx] = (uint8_t)out;
@@ -65,14 +66,15 @@ __global__ void k_unpack_nvfp4_s(const uint8_t *s, uint8_t *bs, int O, int I, in
 }
 
 // ---- FP8 ---------------------------------------------------------------------------------------
-// bytes stay in k order: a 16-bit half word is one (k, k+1) pair for cvt.rn.f16x2.e4m3x2
+// bytes of a chunk stay in k order: a 16-bit half word is one (k, k+1) pair for cvt.rn.f16x2.e4m3x2
 __global__ void k_pack_fp8(const uint8_t *codes, uint8_t *q, int O, int I, int Op, int KT) {
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t total = (size_t)KT * Op * 128;
   if (idx >= total) return;
-  const int j = (int)(idx % 128);
+  const int pos = (int)(idx % 128);
   const int row = (int)((idx / 128) % Op);
   const int kt = (int)(idx / 128 / Op);
+  const int j = coli_fp8_chunk(row, pos >> 4) * 16 + (pos & 15);
   const int k = kt * 128 + j;
   const uint8_t v = (row < O && k < I) ? codes[(size_t)row * I + k] : (uint8_t)0;
   q[idx] = v;
@@ -82,7 +84,7 @@ __global__ void k_unpack_fp8(const uint8_t *q, uint8_t *codes, int O, int I, int
   if (idx >= (size_t)O * I) return;
   const int row = (int)(idx / I), k = (int)(idx % I);
   const int kt = k >> 7, j = k & 127;
-  codes[idx] = q[((size_t)kt * Op + row) * 128 + j];
+  codes[idx] = q[((size_t)kt * Op + row) * 128 + coli_fp8_chunk(row, j >> 4) * 16 + (j & 15)];
 }
 
 static inline unsigned nblk(size_t n, int b) { return (unsigned)((n + b - 1) / b); }
