@@ -75,11 +75,9 @@ CF_HD double cf_bits_f64(uint64_t u) {
 // exp(x) for f32 x, evaluated in f64 and rounded once.  n = rint(x*log2e); r = x - n*ln2 in
 // two fma steps (hi/lo split of ln2); Taylor polynomial of degree 13 by Horner with fma
 // (|r| <= 0.3466, truncation error 1.7e-16); scale by 2^n built from exponent bits.
+// Branch-free, so that a thread's several evaluations overlap.
 CF_HD float coli_expf(float xf) {
-  if (xf != xf) return xf;
-  if (xf > 88.8f) return cf_bits_f32(0x7f800000u);  // +inf; the f64->f32 round gives inf above 88.7228
-  if (xf < -104.0f) return 0.0f;                    // below half the smallest f32 subnormal
-  const double x = (double)xf;
+  const double x = (double)fminf(fmaxf(xf, -104.0f), 88.8f);
   const double n = rint(CF_DMUL(x, 1.4426950408889634074));
   double r = CF_DFMA(n, -6.93147180369123816490e-01, x);
   r = CF_DFMA(n, -1.90821492927058770002e-10, r);
@@ -99,7 +97,10 @@ CF_HD float coli_expf(float xf) {
   p = CF_DFMA(p, r, 1.0);
   const int64_t ni = (int64_t)n;  // |n| <= 151, 2^n is a normal f64
   const double s = cf_bits_f64((uint64_t)(ni + 1023) << 52);
-  return (float)CF_DMUL(p, s);
+  float e = (float)CF_DMUL(p, s);
+  if (xf > 88.8f) e = cf_bits_f32(0x7f800000u);  // +inf; the f64->f32 round gives inf above 88.7228
+  if (xf < -104.0f) e = 0.0f;                    // below half the smallest f32 subnormal
+  return xf != xf ? xf : e;
 }
 
 // 1/(1+exp(-x)) — crates/colibri-engine/src/math.rs:122-125.

@@ -128,31 +128,53 @@ int launch_finish(const float *partial, const __nv_bfloat16 *shared_y, __nv_bflo
   return coli_cuda_check(cudaGetLastError(), "finish launch") ? 1 : 0;
 }
 
-// One warp per token row.  Lane partial sums in f64, combined by a shuffle tree: not the
-// reference's left-to-right order, but 53-bit partials of 24-bit squares differ from it by less
-// than the f32 rounding of the mean in all but ~1e-9 of rows.
+// One CTA per token row: thread partial sums in f64, combined by a shuffle tree and over the warps: not
+// the reference's left-to-right order, but 53-bit partials of 24-bit squares differ from it by less
+// than the f32 rounding of the mean in all but ~1e-9 of rows.  The kernel is latency: a warp per row
+// read the row twice in 2 x H / 128 dependent steps, 12 us for 48 rows of 2048.
 __global__ void __launch_bounds__(256) k_rmsnorm_bf16(const float *x, const float *w, float eps, __nv_bfloat16 *out, int T, int H) {
-  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (row >= T) return;
-  const float4 *xr = reinterpret_cast<const float4 *>(x + (size_t)row * H);
+  __shared__ double part[8];
+  coli_grid_dependency_sync();
+  const int lane = threadIdx.x & 31;
+  const float4 *xr = reinterpret_cast<const float4 *>(x + (size_t)blockIdx.x * H);
   const float4 *wr = reinterpret_cast<const float4 *>(w);
+  constexpr int KEEP = 8;  // the part of a row (8192 elements) that stays in registers between the passes
+  float4 keep[KEEP];
   double ms = 0.0;
-  for (int i = lane; i < H / 4; i += 32) {
-    const float4 v = xr[i];
+  auto square = [&](const float4 &v) {
     ms += (double)v.x * (double)v.x + (double)v.y * (double)v.y + (double)v.z * (double)v.z + (double)v.w * (double)v.w;
+  };
+#pragma unroll
+  for (int j = 0; j < KEEP; ++j) {
+    const int i = (int)threadIdx.x + 256 * j;
+    keep[j] = i < H / 4 ? xr[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
 #pragma unroll
+  for (int j = 0; j < KEEP; ++j) square(keep[j]);
+  for (int i = (int)threadIdx.x + 256 * KEEP; i < H / 4; i += 256) square(xr[i]);
+#pragma unroll
   for (int off = 16; off > 0; off >>= 1) ms += __shfl_xor_sync(0xffffffffu, ms, off);
+  if (lane == 0) part[threadIdx.x >> 5] = ms;
+  __syncthreads();
+  ms = part[0];
+#pragma unroll
+  for (int i = 1; i < 8; ++i) ms += part[i];
   const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn((float)(ms / (double)H), eps)));
-  uint2 *o = reinterpret_cast<uint2 *>(out + (size_t)row * H);
-  for (int i = lane; i < H / 4; i += 32) {
-    const float4 v = xr[i], g = wr[i];
+  uint2 *o = reinterpret_cast<uint2 *>(out + (size_t)blockIdx.x * H);
+  auto store = [&](int i, const float4 &v) {
+    const float4 g = wr[i];
     const uint32_t a = __bfloat16_as_ushort(__float2bfloat16_rn(__fmul_rn(__fmul_rn(v.x, r), g.x)));
     const uint32_t b = __bfloat16_as_ushort(__float2bfloat16_rn(__fmul_rn(__fmul_rn(v.y, r), g.y)));
     const uint32_t c = __bfloat16_as_ushort(__float2bfloat16_rn(__fmul_rn(__fmul_rn(v.z, r), g.z)));
     const uint32_t d = __bfloat16_as_ushort(__float2bfloat16_rn(__fmul_rn(__fmul_rn(v.w, r), g.w)));
     o[i] = make_uint2(a | (b << 16), c | (d << 16));
+  };
+#pragma unroll
+  for (int j = 0; j < KEEP; ++j) {
+    const int i = (int)threadIdx.x + 256 * j;
+    if (i < H / 4) store(i, keep[j]);
   }
+  for (int i = (int)threadIdx.x + 256 * KEEP; i < H / 4; i += 256) store(i, xr[i]);
 }
 int launch_rmsnorm_bf16(const float *x, const float *w, float eps, __nv_bfloat16 *out, int T, int H, cudaStream_t st) {
   if (T <= 0) return 1;
@@ -160,9 +182,8 @@ int launch_rmsnorm_bf16(const float *x, const float *w, float eps, __nv_bfloat16
     coli_set_error("rmsnorm: H=%d must be a multiple of 4", H);
     return 0;
   }
-  k_rmsnorm_bf16<<<(T + 7) / 8, 256, 0, st>>>(x, w, eps, out, T, H);
   coli_count_launch(1);
-  return coli_cuda_check(cudaGetLastError(), "rmsnorm launch") ? 1 : 0;
+  return coli_cuda_check(launch_dependent(k_rmsnorm_bf16, dim3(T), dim3(256), 0, st, x, w, eps, out, T, H), "rmsnorm launch") ? 1 : 0;
 }
 
 __global__ void k_f32_to_bf16(const float *src, __nv_bfloat16 *dst, size_t n) {
