@@ -251,7 +251,6 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
   const int KB = ((K + 127) >> 7) * 2;      // 64-wide k blocks, covering the zero-padded k tiles
   const int FT = GATED ? TC_BM : 2 * TC_BM;  // output features per tile
   const int n_ftiles = (Oout + FT - 1) / FT;
-  const int n_work = *p.n_items * n_ftiles;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < TT_B_STAGES; ++s) {
@@ -275,6 +274,8 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  coli_grid_dependency_sync();  // (the set-up above overlaps the predecessor's end)
+  const int n_work = *p.n_items * n_ftiles;
 
   if (warp == 0) {
     // ---------------- TMA: token tiles ----------------
@@ -570,9 +571,8 @@ static int launch_tct(const TcParams &p, const void *rows_base, int rows_cap, in
   const long max_work = (long)p.max_items * n_ftiles;
   const int grid = (int)(max_work < sm_count ? max_work : sm_count);
   if (grid <= 0) return 1;
-  k_ffn_tct<GATED, FMT, ACC><<<grid, TT_THREADS, smem, st>>>(maps, p);
   coli_count_launch(1);
-  return coli_cuda_check(cudaGetLastError(), "tcgen05 expert ffn launch") ? 1 : 0;
+  return coli_cuda_check(launch_dependent(k_ffn_tct<GATED, FMT, ACC>, dim3(grid), dim3(TT_THREADS), smem, st, maps, p), "tcgen05 expert ffn launch") ? 1 : 0;
 }
 template <bool GATED, int FMT>
 static int launch_tct_acc(const TcParams &p, const void *rows_base, int rows_cap, int sm_count, cudaStream_t st) {

@@ -268,15 +268,22 @@ int launch_bf16_to_f32(const __nv_bfloat16 *src, float *dst, size_t n, cudaStrea
 // (crates/colibri-engine/src/linear.rs:199-220).
 int launch_matmul_f32_seq(const float *x, const float *w, float *y, int S, int I, int O, cudaStream_t st);
 
-// Programmatic dependent launch.  The kernels of the decode step are a few microseconds each, so
-// the launch latency between them is a visible share of the step: launched with this helper, a
-// kernel may be scheduled while its predecessor in the stream is still running; it must then
-// execute coli_grid_dependency_sync() before its first global-memory access, which returns once
-// the predecessor has completed and its writes are visible.  Launched the ordinary way (as the
-// profiled path does, with an event between kernels) the two device calls are no-ops.
+// Programmatic dependent launch.  Most kernels of a call are a few microseconds each, so the launch
+// latency between them is a visible share: launched with launch_dependent, a kernel may be scheduled
+// while its predecessor in the stream is still running; it must then execute coli_grid_dependency_sync()
+// (or coli_grid_wait()) before its first global-memory access, which returns once the predecessor has
+// completed and its writes are visible.  Launched the ordinary way (as the profiled path does, with an
+// event between kernels) the device calls are no-ops.
+// Where it is not used, or not early: a kernel whose CTAs must spread evenly over the SMs, several
+// fitting on one, packs onto the SMs that happen to be free while its predecessor still runs (the
+// router of 4096 tokens took 1180 us instead of 445 that way).  The router GEMMs, first in a call, are
+// therefore launched the ordinary way, and the one-CTA permutation lets its successor, the register-
+// level expert kernel, start only when it is done.
+__device__ __forceinline__ void coli_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void coli_grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void coli_grid_dependency_sync() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // let the successor be scheduled early too
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  coli_grid_trigger();  // let the successor be scheduled early too
+  coli_grid_wait();
 }
 template <typename... KArgs, typename... Args>
 static inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {

@@ -26,6 +26,7 @@ namespace colib {
 // ---------------------------------------------------------------------------------------------
 template <int TM, int TN>
 __global__ void __launch_bounds__(256) k_router_gemm(RouteParams p) {
+  coli_grid_trigger();  // the top-k may be scheduled; it waits for this grid
   constexpr int BM = 16 * TM, BN = 16 * TN, BK = 32;
   __shared__ float xs[BK][BM + 4];
   __shared__ float ws[BK][BN + 4];
@@ -100,6 +101,7 @@ __device__ __forceinline__ void coli_ffma2(float2 &c, const float2 a, const floa
 
 template <int BM, int NT>
 __global__ void __launch_bounds__(NT) k_router_gemm_big(RouteParams p) {
+  coli_grid_trigger();  // the top-k may be scheduled; it waits for this grid
   constexpr int TMR = BM * 16 / NT;  // token rows per thread
   constexpr int BN = 64, BK = 32, LDX = BM + 4, LDW = BN + 4;
   constexpr int SR = NT / 4;                  // rows staged per pass (4 chunks of 8 k each)
@@ -221,6 +223,7 @@ __global__ void __launch_bounds__(NT) k_router_gemm_big(RouteParams p) {
 // Needs H % 8 == 0.
 template <int TM, int TN, int NT>
 __global__ void __launch_bounds__(NT) k_router_rt(RouteParams p) {
+  coli_grid_trigger();  // the top-k may be scheduled; it waits for this grid
   static_assert(TN % 4 == 0 && (TM % 4 == 0 || TM == 2), "tile shape");
   constexpr int BM = (NT / 16) * TM, BN = 16 * TN, BK = 32, LDX = BM + 4, LDW = BN + 4;
   constexpr int SR = NT / 4;  // rows staged per pass (4 chunks of 8 k each)
@@ -367,6 +370,7 @@ struct RouterTile {
 };
 template <class C>
 __global__ void __launch_bounds__(C::NT) k_router_chain(RouteParams p) {
+  coli_grid_trigger();  // the top-k may be scheduled; it waits for this grid
   constexpr int TM = C::TM, TN = C::TN, RS = C::RS, CH = C::CH, BM = C::BM, BN = C::BN;
   constexpr bool SMALL = TM * TN <= 8;  // the next chunk's operands are loaded ahead of this one's FMAs
   constexpr bool PAIRED = TM % 2 == 0;  // two tokens per FMA instruction (3 to 6 % at every tile that can)
@@ -733,6 +737,7 @@ __device__ __forceinline__ void route_topk_token(const RouteParams &p, int t, fl
 }
 
 __global__ void __launch_bounds__(128) k_route_topk(RouteParams p) {
+  coli_grid_dependency_sync();
   extern __shared__ __align__(16) float sm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + warp;
@@ -768,7 +773,8 @@ template <class C>
 static bool launch_router_chain(const RouteParams &p, cudaStream_t st) {
   static ColiPerDeviceOnce attr_once;
   if (C::SMEM > 48 * 1024 && !coli_set_smem_limit(attr_once, k_router_chain<C>, C::SMEM, "router shared-memory attribute")) return false;
-  k_router_chain<C><<<dim3((p.T + C::BM - 1) / C::BM, (p.E + C::BN - 1) / C::BN), C::NT, C::SMEM, st>>>(p);
+  const dim3 grid((p.T + C::BM - 1) / C::BM, (p.E + C::BN - 1) / C::BN);
+  k_router_chain<C><<<grid, C::NT, C::SMEM, st>>>(p);
   return true;
 }
 // The kernel and tile of a batch: 0 = 8 x 8, 1 = 16 x 32, 2 = 64 x 64 tokens x experts of k_router_chain,
@@ -818,9 +824,9 @@ int launch_router(const RouteParams &p, cudaStream_t st) {
   }
   coli_count_launch(1);
   const size_t sm = (size_t)4 * topk_row_floats(p.E) * sizeof(float);
-  k_route_topk<<<(p.T + 3) / 4, 128, sm, st>>>(p);
+  if (!coli_cuda_check(cudaGetLastError(), "router launch")) return 0;
   coli_count_launch(1);
-  return coli_cuda_check(cudaGetLastError(), "router launch") ? 1 : 0;
+  return coli_cuda_check(launch_dependent(k_route_topk, dim3((p.T + 3) / 4), dim3(128), sm, st, p), "top-k launch") ? 1 : 0;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -850,6 +856,7 @@ __device__ __forceinline__ int rank_before(const int *ids, int i) {
   return n;
 }
 __global__ void __launch_bounds__(256) k_seg_count(PermuteParams p, int nchunk) {
+  coli_grid_dependency_sync();
   extern __shared__ __align__(16) int cnt_sm[];  // 32 k ids of the chunk, then E counters
   int *ids = cnt_sm, *cnt = cnt_sm + 32 * p.k;
   const int chunk = blockIdx.x;
@@ -931,6 +938,7 @@ __device__ __forceinline__ void build_work_list(const PermuteParams &p, const in
 }
 
 __global__ void __launch_bounds__(1024) k_seg_scan(PermuteParams p, int nchunk, int max_items) {
+  coli_grid_dependency_sync();
   __shared__ int seg_cnt[1024 + 1];
   __shared__ int seg_off[1024 + 2];
   __shared__ int seg_ibase[1024 + 2];
@@ -976,6 +984,7 @@ __global__ void __launch_bounds__(1024) k_seg_scan(PermuteParams p, int nchunk, 
 }
 
 __global__ void __launch_bounds__(256) k_permute(PermuteParams p) {
+  coli_grid_dependency_sync();
   // one warp per (t, kk) row; rows T*k .. T*k+T-1 are the shared expert's identity rows; when a
   // token-order f16 copy of x is wanted, T more warps write it
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -1092,6 +1101,7 @@ __device__ __forceinline__ void permute_small_body(const PermuteParams &p, int m
 }
 
 __global__ void __launch_bounds__(1024) k_permute_small(PermuteParams p, int max_items) {
+  coli_grid_wait();
   __shared__ PermuteSmallSmem sm;
   if (blockIdx.x > 0) {  // the extra CTAs only write the token-order f16 copy of x
     const size_t n = (size_t)p.T * p.H / 8;
@@ -1175,18 +1185,16 @@ int launch_permute(const PermuteParams &p, cudaStream_t st) {
       conv = (int)((n + 1023) / 1024);
       if (conv > 64) conv = 64;
     }
-    k_permute_small<<<1 + conv, 1024, 0, st>>>(p, max_items);
     coli_count_launch(1);
-    return coli_cuda_check(cudaGetLastError(), "permute launch") ? 1 : 0;
+    return coli_cuda_check(launch_dependent(k_permute_small, dim3(1 + conv), dim3(1024), 0, st, p, max_items), "permute launch") ? 1 : 0;
   }
-  k_seg_count<<<nchunk, 256, (size_t)(32 * p.k + p.E) * sizeof(int), st>>>(p, nchunk);
-  coli_count_launch(1);
-  k_seg_scan<<<1, 1024, 0, st>>>(p, nchunk, max_items);
-  coli_count_launch(1);
   const int total = p.T * p.k + (p.has_shared ? p.T : 0) + (p.x16 ? p.T : 0);
-  k_permute<<<(total + 7) / 8, 256, 0, st>>>(p);
-  coli_count_launch(1);
-  return coli_cuda_check(cudaGetLastError(), "permute launch") ? 1 : 0;
+  coli_count_launch(3);
+  return coli_cuda_check(launch_dependent(k_seg_count, dim3(nchunk), dim3(256), (size_t)(32 * p.k + p.E) * sizeof(int), st, p, nchunk), "permute launch") &&
+                 coli_cuda_check(launch_dependent(k_seg_scan, dim3(1), dim3(1024), 0, st, p, nchunk, max_items), "permute launch") &&
+                 coli_cuda_check(launch_dependent(k_permute, dim3((total + 7) / 8), dim3(256), 0, st, p), "permute launch")
+             ? 1
+             : 0;
 }
 
 __global__ void k_items_from_counts(const int32_t *seg_count, int nseg, int rows_per_item, int32_t *seg_off,
