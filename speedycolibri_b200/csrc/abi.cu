@@ -494,32 +494,30 @@ extern "C" int coli_b200_moe_phase_ms(ColiMoe *m, float *ms, int *calls) {
 }
 extern "C" void *coli_b200_moe_stream(ColiMoe *m) { return m ? (void *)m->ctx->stream : nullptr; }
 
-// The tcgen05 path takes over from 8 rows per segment on average: below that the register-level
-// kernel re-reads so few token rows per weight tile that it wins; a pure function of (rows,
-// segments, format) so that kernel selection never depends on data or addresses.
-// Which tcgen05 kernel: the one with the weight operand in tensor memory takes tiles of at most
-// 160 tokens and wins while segments are about that long; longer NVFP4 segments amortise the
-// shared-memory weight tiles of the other kernel over 256 tokens.  The FP8 formats exist in the
-// tensor-memory kernel only (longer segments are cut into several of its tiles).
-bool coli_use_tct(int fmt, int rows, int nseg) {
-  return fmt != COLI_FMT_NVFP4 || rows <= 160 * (nseg > 0 ? nseg : 1);
-}
-// Tile width of the tensor-memory kernel: short tiles (and a weight ring twice as deep) while the
-// average segment fits one of them with room to spare, the full width otherwise.
+// Tile width of the tcgen05 kernel: short tiles (and a weight ring twice as deep) while the average
+// segment fits one of them with room to spare, the full width otherwise.
 int coli_tct_tile_tokens(int rows, int nseg) {
   return rows <= 48 * (nseg > 0 ? nseg : 1) ? colib::TCT_SHORT_TOKENS : colib::TCT_MAX_TOKENS;
 }
-bool coli_use_tc_path(int fmt, int rows, int nseg) {
-  return (fmt == COLI_FMT_NVFP4 || fmt == COLI_FMT_FP8_B128 || fmt == COLI_FMT_E4M3_ROW) && nseg > 0 && rows / nseg >= 8;
+// The tcgen05 path takes over from 8 rows per segment on average: below that the register-level
+// kernel re-reads so few token rows per weight tile that it wins.  It cuts segments into items of 8
+// rows there and reads their weights once per item, so on a layer too large for L2 the line lies at 6
+// rows, as long as the tcgen05 kernel's tiles (128 features of an expert) divide well over the SMs.
+// Measured (register-level / tcgen05, us a call): H 7168, I 2048, 256 experts at 4.5 rows 1443 / 1452,
+// 7.0 2300 / 1496; H 2048, I 768, 128 experts at 6.7 136 / 147, 8.0 150 / 148, FP8 6.7 167 / 179, 8.0
+// 182 / 180.  A pure function of shapes, so that kernel selection never depends on data or addresses.
+bool coli_use_tc_path(int fmt, int rows, int nseg, int I) {
+  if ((fmt != COLI_FMT_NVFP4 && fmt != COLI_FMT_FP8_B128 && fmt != COLI_FMT_E4M3_ROW) || nseg <= 0) return false;
+  const bool many_tiles = (long)nseg * ((I + 127) / 128) >= 148L * 12;
+  return (long)rows >= (many_tiles ? 6L : 8L) * nseg;
 }
 
 int coli_rows_per_item_for(int rows, int nseg) {
   const int avg = (rows + nseg - 1) / (nseg > 0 ? nseg : 1);
   return avg <= 8 ? 8 : avg <= 16 ? 16 : 32;
 }
-static bool use_tct(int fmt, int rows, int nseg) { return coli_use_tct(fmt, rows, nseg); }
 static int tct_tile_tokens(int rows, int nseg) { return coli_tct_tile_tokens(rows, nseg); }
-static bool use_tc_path(int fmt, int rows, int nseg) { return coli_use_tc_path(fmt, rows, nseg); }
+static bool use_tc_path(int fmt, int rows, int nseg, int I) { return coli_use_tc_path(fmt, rows, nseg, I); }
 static int rows_per_item_for(const ColiMoeLayer &, int rows, int nseg) { return coli_rows_per_item_for(rows, nseg); }
 
 extern "C" int coli_b200_moe_create(ColiMoe **out, const ColiMoeLayer *L, int max_tokens) {
@@ -660,7 +658,7 @@ extern "C" int coli_b200_moe_create(ColiMoe **out, const ColiMoeLayer *L, int ma
   ok = ok && ws_alloc(m, &m->status, 1) && coli_cuda_check(cudaMemset(m->status, 0, sizeof(int)), "status clear");
   m->ticket = nullptr;
   ok = ok && ws_alloc(m, &m->ticket, 1) && coli_cuda_check(cudaMemset(m->ticket, 0, sizeof(unsigned int)), "ticket clear");
-  if (ok && use_tc_path(coli_kernel_fmt(L->fmt), (int)rows, m->nseg)) ok = ws_alloc(m, &m->xg, rows * H);
+  if (ok && use_tc_path(coli_kernel_fmt(L->fmt), (int)rows, m->nseg, L->I)) ok = ws_alloc(m, &m->xg, rows * H);
   m->select_bias = nullptr;
   m->logit_bias = nullptr;
   if (ok && L->select_bias) ok = ws_alloc(m, &m->select_bias, E);
@@ -796,9 +794,8 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
   cudaStream_t st = pick_stream(m, stream);
   const int k = m->L.k;
   const int rows = T * k + (m->has_shared ? T : 0);
-  const bool tc = use_tc_path(m->L.fmt, rows, m->nseg) && m->xg != nullptr;
-  const bool tct = tc && use_tct(m->L.fmt, rows, m->nseg);
-  const int rpi = tc ? (tct ? tct_tile_tokens(rows, m->nseg) : colib::TC_MAX_TOKENS) : rows_per_item_for(m->L, rows, m->nseg);
+  const bool tc = use_tc_path(m->L.fmt, rows, m->nseg, m->L.I) && m->xg != nullptr;
+  const int rpi = tc ? tct_tile_tokens(rows, m->nseg) : rows_per_item_for(m->L, rows, m->nseg);
   const int max_items = max_work_items(rows, m->nseg, rpi);
   const bool prof = m->profiling;
 #define COLI_MARK(i)                                                         \
@@ -838,10 +835,9 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
     tp.y = m->y;
     tp.status = m->status;
     tp.act = m->act;
-    if (!(tct ? colib::launch_gate_up_tct(tp, m->xg, rows, m->sm_count, st) : colib::launch_gate_up_tc(tp, m->xg, rows, m->sm_count, st)))
-      return 0;
+    if (!colib::launch_gate_up_tct(tp, m->xg, rows, m->sm_count, st)) return 0;
     COLI_MARK(3);
-    if (!(tct ? colib::launch_down_tct(tp, rows, m->sm_count, st) : colib::launch_down_tc(tp, rows, m->sm_count, st))) return 0;
+    if (!colib::launch_down_tct(tp, rows, m->sm_count, st)) return 0;
   } else {
     colib::FfnParams fp;
     fp.fmt = m->L.fmt;
@@ -1006,7 +1002,7 @@ extern "C" int coli_b200_moe_gather_local_dev(ColiMoe *m, const void *x_dev, con
   }
   cudaStream_t st = pick_stream(m, stream);
   if (T == 0) return coli_cuda_check(cudaMemsetAsync(seg_count_dev, 0, sizeof(int32_t) * m->n_local_seg, st), "count clear") ? 1 : 0;
-  colib::PermuteParams pp = permute_params(m, x_dev, T, false, colib::TC_MAX_TOKENS, rows_dev, seg_count_dev, slot_dev);
+  colib::PermuteParams pp = permute_params(m, x_dev, T, false, colib::TCT_MAX_TOKENS, rows_dev, seg_count_dev, slot_dev);
   pp.topk_idx = topk_idx_dev;
   pp.expert_slot = m->local_slot;
   pp.nseg_routed = m->n_local_seg;
@@ -1044,9 +1040,8 @@ int coli_run_segments(ColiMoe *m, SegScratch &sc, const WeightRef *g, const Weig
                       const int32_t *seg_expert_dev, const void *rows_dev, const int32_t *seg_count_dev, int n_seg,
                       int rows_cap, int rows_expected, void *y_dev, cudaStream_t st) {
   if (rows_cap == 0 || n_seg == 0) return 1;
-  const bool tc = use_tc_path(m->L.fmt, rows_expected, n_seg);
-  const bool tct = tc && use_tct(m->L.fmt, rows_expected, n_seg);
-  const int rpi = tc ? (tct ? tct_tile_tokens(rows_expected, n_seg) : colib::TC_MAX_TOKENS) : rows_per_item_for(m->L, rows_expected, n_seg);
+  const bool tc = use_tc_path(m->L.fmt, rows_expected, n_seg, m->L.I);
+  const int rpi = tc ? tct_tile_tokens(rows_expected, n_seg) : rows_per_item_for(m->L, rows_expected, n_seg);
   const int max_items = max_work_items(rows_cap, n_seg, rpi);
   if (!ensure_h(m, sc, (size_t)rows_cap) || !ensure_items(m, sc, max_items, n_seg)) return 0;
   if (!colib::launch_items_from_counts(seg_count_dev, n_seg, rpi, sc.seg_off, sc.item_seg, sc.item_row0, sc.item_nrows,
@@ -1071,8 +1066,7 @@ int coli_run_segments(ColiMoe *m, SegScratch &sc, const WeightRef *g, const Weig
     tp.y = (__nv_bfloat16 *)y_dev;
     tp.status = m->status;
     tp.act = m->act;
-    if (tct) return colib::launch_gate_up_tct(tp, rows_dev, rows_cap, m->sm_count, st) && colib::launch_down_tct(tp, rows_cap, m->sm_count, st);
-    return colib::launch_gate_up_tc(tp, rows_dev, rows_cap, m->sm_count, st) && colib::launch_down_tc(tp, rows_cap, m->sm_count, st);
+    return colib::launch_gate_up_tct(tp, rows_dev, rows_cap, m->sm_count, st) && colib::launch_down_tct(tp, rows_cap, m->sm_count, st);
   }
   colib::FfnParams fp;
   fp.fmt = m->L.fmt;
@@ -1244,10 +1238,9 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
   std::lock_guard<std::mutex> lk(ctx->mu);
   cudaStream_t st = ctx->stream;
   const int kfmt = coli_kernel_fmt(fmt);
-  const bool tc = use_tc_path(kfmt, (int)total, count);
-  const bool tct = tc && use_tct(kfmt, (int)total, count);
+  const bool tc = use_tc_path(kfmt, (int)total, count, I);
   const int avg = (int)((total + count - 1) / count);
-  const int rpi = tc ? (tct ? tct_tile_tokens((int)total, count) : colib::TC_MAX_TOKENS) : (avg <= 8 ? 8 : avg <= 16 ? 16 : 32);
+  const int rpi = tc ? tct_tile_tokens((int)total, count) : (avg <= 8 ? 8 : avg <= 16 ? 16 : 32);
   const int max_items = max_work_items((int)total, count, rpi);
   const size_t xb = (size_t)total * D;
   // slots: 0 x f32 / y f32, 1 x f16, 2 h f16, 3 tables + counts + work list + status word, 4 y bf16 (tcgen05 path)
@@ -1301,8 +1294,7 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
     tp.status = d_status;
     tp.act = current_activation();
     const int sms = ctx->sm_count;
-    const int ok = tct ? colib::launch_gate_up_tct(tp, ctx->buf[1], (int)total, sms, st) && colib::launch_down_tct(tp, (int)total, sms, st)
-                       : colib::launch_gate_up_tc(tp, ctx->buf[1], (int)total, sms, st) && colib::launch_down_tc(tp, (int)total, sms, st);
+    const int ok = colib::launch_gate_up_tct(tp, ctx->buf[1], (int)total, sms, st) && colib::launch_down_tct(tp, (int)total, sms, st);
     if (!ok || !colib::launch_bf16_to_f32((const __nv_bfloat16 *)ctx->buf[4], (float *)ctx->buf[0], xb, st)) return 0;
   } else {
     colib::FfnParams fp;

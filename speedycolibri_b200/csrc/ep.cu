@@ -729,7 +729,7 @@ int ep_phase_b(ColiMoe *m, const EpCounts &c, cudaStream_t st) {
   const int k = m->L.k, H = m->L.H;
   EP_MARK(4);
   if (c.R > 0) {
-    colib::PermuteParams pp = coli_permute_params(m, ep->recv_x, c.R, false, colib::TC_MAX_TOKENS, ep->rows, ep->seg_count, ep->recv_slot);
+    colib::PermuteParams pp = coli_permute_params(m, ep->recv_x, c.R, false, colib::TCT_MAX_TOKENS, ep->rows, ep->seg_count, ep->recv_slot);
     pp.topk_idx = ep->recv_meta;
     pp.expert_slot = m->local_slot;
     pp.nseg_routed = m->n_local_seg;
@@ -791,7 +791,7 @@ int ep_direct_phase_b(ColiMoe *m, cudaStream_t st) {
   colib::k_ep_recv_layout<<<1, 32, 0, st>>>(reinterpret_cast<const int32_t *>(ep->slab + ep->table_off), ep->world, ep->rank, ep->tl_cap, ep->info);
   coli_count_launch(1);
   EP_MARK(4);
-  colib::PermuteParams pp = coli_permute_params(m, ep->slab + ep->x_off, cap_tok, false, colib::TC_MAX_TOKENS, ep->rows, ep->seg_count, ep->recv_slot);
+  colib::PermuteParams pp = coli_permute_params(m, ep->slab + ep->x_off, cap_tok, false, colib::TCT_MAX_TOKENS, ep->rows, ep->seg_count, ep->recv_slot);
   pp.topk_idx = reinterpret_cast<const int32_t *>(ep->slab + ep->meta_off);
   pp.expert_slot = m->local_slot;
   pp.nseg_routed = m->n_local_seg;

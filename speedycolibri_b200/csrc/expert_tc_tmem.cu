@@ -1,8 +1,12 @@
-// Expert FFN for segments of up to 160 rows per tile on the 5th-generation tensor cores, with the
-// weight operand in TENSOR MEMORY.
+// Expert FFN for prefill-sized segments on the 5th-generation tensor cores, with the weight operand
+// in TENSOR MEMORY; tiles of up to 160 token rows, longer segments are shared out over several.
 //
-// Same formulation as expert_tc.cu (features on the MMA's M = 128, the ragged token count on its
-// N), but the decoded weights never pass through shared memory:
+// Formulation (operands swapped so that the ragged token count lands on the MMA's N, which has a
+// granularity of 16, and the always-full feature axis on its M = 128):
+//     D[feature, token] = W[feature, :] . X[token, :]^T          per expert segment
+// It replaces the reference's dequant-to-half + wmma kernels nvfp4_matmul / nvfp4_gate_up
+// (crates/colibri-backend/cuda/backend_cuda.cu:1355-1430) and its separate silu_mul launch
+// (backend_cuda.cu:3785-3787).
 // * A operand: two loading warps copy the packed NVFP4 or FP8 bytes from HBM into a shared-memory
 //   ring of k-tiles (cp.async, 3 to 9 slots of 18 or 32 KB); 16 producer warps read them (one thread
 //   = one weight row = one TMEM lane), convert them to f16 in registers and write 64 k per stage
@@ -16,10 +20,11 @@
 //   accumulators of 160 columns fed by one issuing warp, two stages per barrier wait; the epilogue
 //   forms act(g, u) or writes the two down tiles.
 // Why: with both operands in shared memory an MMA of 128 x 128 x 16 fetches 8 KB per 64 cycles,
-// the whole shared-memory bandwidth of an SM, before a single decoded weight is stored there
-// (expert_tc.cu tops out near half of the tensor peak at 128 tokens per expert).  Here shared
-// memory carries the token tiles (16-20 KB written + twice that read per stage) and the packed
-// weights (9 or 16 KB each way).
+// the whole shared-memory bandwidth of an SM, before a single decoded weight is stored there; a kernel
+// of that form with tiles of 256 tokens was kept for long segments until this one passed it (16384
+// tokens with skewed experts, H 6144, I 2048: 6092 + 3241 us against 5205 + 2704).  Here shared memory
+// carries the token tiles (16-20 KB written + twice that read per stage) and the packed weights (9 or
+// 16 KB each way).
 // TMEM budget: 2 x 160 accumulator columns + 6 x 32 weight columns = 512, which is why this
 // kernel takes tiles of at most 160 tokens (a layer with 128 rows per expert on average has
 // nearly all of its segments under that); wider segments are cut into several work items.
@@ -38,6 +43,8 @@
 // Roles are warp-specialised and synchronise through mbarriers only; the kernel is persistent.
 // Every barrier wait is bounded: on a time-out the CTA raises a status word, stops issuing work,
 // waits for its own copies and frees its TMEM before returning.
+#include <type_traits>
+
 #include "tc_common.cuh"
 
 #ifdef COLI_TT_TRACE
@@ -73,7 +80,7 @@ struct TtBudget {
   static constexpr int B_BYTES = ACC * TC_BK * 2;
   static constexpr int B_STAGES = 6;
   static constexpr int NBARS = 2 * B_STAGES + 2 + 2 * 9;  // stages, accumulators, at most 9 weight slots
-  static_assert(B_STAGES % A_STAGES == 0 && B_BYTES % 1024 == 0, "a stage barrier serves both rings");
+  static_assert(B_STAGES == 6 && B_STAGES % A_STAGES == 0 && B_BYTES % 1024 == 0, "a stage barrier serves both rings");
 };
 // The token tile of a stage arrives as ONE box of N rows: the copy engine of an SM takes about 64
 // cycles per box plus 4 per 128-byte row (measured: 21 B/clk with 32-row boxes, 31 B/clk with
@@ -366,7 +373,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
     uint32_t tix = 0;
     bool alive = true;
     // ring positions as counters: no division or modulo per stage
-    uint32_t sa = 0, sb = 0, phb = 0;
+    uint32_t sb = 0, phb = 0;
     for (int w = blockIdx.x; w < n_work && alive; w += gridDim.x, ++tix) {
       const int item = w / n_ftiles;
       const int nrows = __reduce_max_sync(0xffffffffu, p.item_nrows[item]);
@@ -381,15 +388,24 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
         if (!alive) break;
         if (lane == 0) TT_TRACE(tix * KB + kb, 1);
         tc_fence_after();
-        const uint32_t sa1 = sa + 1 == TT_A_STAGES ? 0u : sa + 1;
         if (elect_one()) {
-          const uint64_t bd = bdesc_ring + (uint64_t)(sb * (TT_B_BYTES >> 4));
-          tt_issue_stage(tmem_u, tmem_u + TT_ACC_COLS, a_ring + sa * 64, bd, idesc, kb ? 1u : 0u, empty_s + 8 * sb);
-          tt_issue_stage(tmem_u, tmem_u + TT_ACC_COLS, a_ring + sa1 * 64, bd + (TT_B_BYTES >> 4), idesc, 1u, empty_s + 8 * (sb + 1));
+          // one copy of the code per ring position: every address is then a constant offset
+          auto issue = [&](auto pos) {
+            constexpr uint32_t b = 2 * decltype(pos)::value, a0 = b % TT_A_STAGES, a1 = (b + 1) % TT_A_STAGES;
+            tt_issue_stage(tmem_u, tmem_u + TT_ACC_COLS, a_ring + a0 * 64, bdesc_ring + (uint64_t)(b * (TT_B_BYTES >> 4)), idesc,
+                           kb ? 1u : 0u, empty_s + 8 * b);
+            tt_issue_stage(tmem_u, tmem_u + TT_ACC_COLS, a_ring + a1 * 64, bdesc_ring + (uint64_t)((b + 1) * (TT_B_BYTES >> 4)), idesc,
+                           1u, empty_s + 8 * (b + 1));
+          };
+          if (sb == 0)
+            issue(std::integral_constant<uint32_t, 0>());
+          else if (sb == 2)
+            issue(std::integral_constant<uint32_t, 1>());
+          else
+            issue(std::integral_constant<uint32_t, 2>());
         }
         __syncwarp();
         if (lane == 0) TT_TRACE(tix * KB + kb, 2);
-        sa = sa1 + 1 == TT_A_STAGES ? 0u : sa1 + 1;
         if ((sb += 2) == TT_B_STAGES) {
           sb = 0;
           phb ^= 1u;

@@ -87,9 +87,8 @@ static inline bool ws_alloc(ColiMoe *m, T **p, size_t count) {
 
 
 // kernel-family selection: pure functions of (format, rows, segments)
-bool coli_use_tct(int fmt, int rows, int nseg);
 int coli_tct_tile_tokens(int rows, int nseg);
-bool coli_use_tc_path(int fmt, int rows, int nseg);
+bool coli_use_tc_path(int fmt, int rows, int nseg, int I);
 int coli_rows_per_item_for(int rows, int nseg);
 
 bool coli_check_T(ColiMoe *m, int T, const char *who);

@@ -65,6 +65,7 @@ static inline int round_up(int a, int b) { return (a + b - 1) / b * b; }
 // Upper bound of the work items `rows` rows in at most `nseg` segments cut into: a segment of n
 // rows gives ceil(n / rpi) <= n / rpi + 1 items and at most min(nseg, rows) segments hold a row.
 // Kernel grids are sized from this bound, so a loose one costs idle CTAs on every decode step.
+// (Items of the tcgen05 kernel share a segment's rows evenly: work_item_rows.)
 static inline int max_work_items(int rows, int nseg, int rpi) { return rows / rpi + (rows < nseg ? rows : nseg); }
 
 // ---- error reporting -------------------------------------------------------------------------
@@ -212,30 +213,26 @@ int launch_gate_up_small(const FfnParams &p, cudaStream_t st);  // h = silu(gate
 int launch_down_small(const FfnParams &p, cudaStream_t st);     // y = down h
 int launch_ffn_small(const FfnParams &p, cudaStream_t st);      // both
 
-// expert_tc.cu — tcgen05 path for prefill-sized segments
-constexpr int TC_MAX_TOKENS = 256;  // token rows per tile = rows per work item on this path
+// expert_tc_tmem.cu — tcgen05 path for prefill-sized segments.  Token rows per work item = per tile:
+constexpr int TCT_MAX_TOKENS = 160;
+// ... or this many for layers whose segments are short: narrower accumulators leave tensor memory for
+// a weight ring twice as deep (TcParams::tile_tokens says which)
+constexpr int TCT_SHORT_TOKENS = 64;
+constexpr int TCT_ROW_GRAIN = 16;  // rows a tile is padded to a multiple of
 struct TcParams {
-  int fmt;  // COLI_FMT_NVFP4 (both kernels); COLI_FMT_FP8_B128 / COLI_FMT_E4M3_ROW (tensor-memory kernel only)
+  int fmt;  // COLI_FMT_NVFP4, COLI_FMT_FP8_B128 or COLI_FMT_E4M3_ROW
   int H, I;
   const WeightRef *gate, *up, *down;
   const int32_t *seg_expert;
   const int32_t *item_seg, *item_row0, *item_nrows, *n_items;
   int max_items;
-  int tile_tokens;   // rows per item the work list was cut with: TC_MAX_TOKENS, TCT_MAX_TOKENS or TCT_SHORT_TOKENS
+  int tile_tokens;   // rows per item the work list was cut with: TCT_MAX_TOKENS or TCT_SHORT_TOKENS
   __half *h;         // [rows, I]
   __nv_bfloat16 *y;  // [rows, H]
   int *status;       // device word: 0, or the code of the first bounded wait that gave up
   ActParams act;
 };
 // x_rows: f16 [rows_cap, H] expert-contiguous rows (row index = position in the work list)
-int launch_gate_up_tc(const TcParams &p, const void *x_rows, int rows_cap, int sm_count, cudaStream_t st);
-int launch_down_tc(const TcParams &p, int rows_cap, int sm_count, cudaStream_t st);
-// expert_tc_tmem.cu — the same two stages with the weight operand in tensor memory; tiles of at
-// most TCT_MAX_TOKENS rows (the work list must be cut with that many rows per item)
-constexpr int TCT_MAX_TOKENS = 160;
-// ... or with TCT_SHORT_TOKENS rows per item, for layers whose segments are short: narrower
-// accumulators leave tensor memory for a weight ring twice as deep (TcParams::tile_tokens says which)
-constexpr int TCT_SHORT_TOKENS = 64;
 int launch_gate_up_tct(const TcParams &p, const void *x_rows, int rows_cap, int sm_count, cudaStream_t st);
 int launch_down_tct(const TcParams &p, int rows_cap, int sm_count, cudaStream_t st);
 

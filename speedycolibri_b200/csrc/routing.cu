@@ -879,6 +879,14 @@ __global__ void __launch_bounds__(256) k_seg_count(PermuteParams p, int nchunk) 
   for (int e = threadIdx.x; e < p.E; e += blockDim.x) p.chunk_cnt[(size_t)chunk * p.E + e] = cnt[e];
 }
 
+// Rows per item of a segment of n rows cut into items of at most rpi: items of the tcgen05 kernel
+// (rpi >= 64) take equal shares, because a tile of few rows still decodes all of its weights -- 170 rows
+// as 96 + 74 and not 160 + 10; the number of items is the same.
+__device__ __forceinline__ int work_item_rows(int n, int rpi) {
+  if (rpi < 64 || n <= rpi) return rpi;
+  const int items = (n + rpi - 1) / rpi;
+  return ((n + items - 1) / items + TCT_ROW_GRAIN - 1) / TCT_ROW_GRAIN * TCT_ROW_GRAIN;
+}
 // Segment offsets and the work list from per-segment row counts in shared memory, by the whole
 // CTA: a shuffle scan per warp and a pass over the warps' sums (row offsets and item bases at once),
 // then one thread per segment writes that segment's items.  off and ibase hold nseg + 1 entries.
@@ -925,12 +933,13 @@ __device__ __forceinline__ void build_work_list(const PermuteParams &p, const in
   __syncthreads();
   for (int s = threadIdx.x; s < nseg; s += blockDim.x) {
     const int n = cnt[s], r0 = off[s];
+    const int share = work_item_rows(n, rpi);
     int it = ibase[s];
-    for (int r = 0; r < n; r += rpi, ++it) {
+    for (int r = 0; r < n; r += share, ++it) {
       if (it < max_items) {
         p.item_seg[it] = s;
         p.item_row0[it] = r0 + r;
-        p.item_nrows[it] = min(rpi, n - r);
+        p.item_nrows[it] = min(share, n - r);
       }
     }
   }
@@ -1197,33 +1206,63 @@ int launch_permute(const PermuteParams &p, cudaStream_t st) {
              : 0;
 }
 
-__global__ void k_items_from_counts(const int32_t *seg_count, int nseg, int rows_per_item, int32_t *seg_off,
-                                    int32_t *item_seg, int32_t *item_row0, int32_t *item_nrows,
-                                    int32_t *n_items) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int run = 0, items = 0;
-  for (int s = 0; s < nseg; ++s) {
-    seg_off[s] = run;
-    const int n = seg_count[s];
-    for (int r = 0; r < n; r += rows_per_item) {
-      item_seg[items] = s;
-      item_row0[items] = run + r;
-      item_nrows[items] = min(rows_per_item, n - r);
-      ++items;
+// The same for rows that are already expert-contiguous: counts on the device, any number of segments,
+// one CTA.  (One thread walking the segments took 12 us for 24 of them.)
+__global__ void __launch_bounds__(1024) k_items_from_counts(const int32_t *seg_count, int nseg, int rows_per_item, int32_t *seg_off,
+                                                            int32_t *item_seg, int32_t *item_row0, int32_t *item_nrows, int32_t *n_items) {
+  __shared__ int2 warp_sum[32];
+  coli_grid_dependency_sync();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5, rpi = rows_per_item;
+  int2 run = make_int2(0, 0);  // rows and items of the segments before `base`
+  for (int base = 0; base < nseg; base += (int)blockDim.x) {
+    const int s = base + (int)threadIdx.x;
+    const int n = s < nseg ? seg_count[s] : 0;
+    const int ni = (n + rpi - 1) / rpi;
+    int a = n, b = ni;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int ua = __shfl_up_sync(0xffffffffu, a, o), ub = __shfl_up_sync(0xffffffffu, b, o);
+      if (lane >= o) {
+        a += ua;
+        b += ub;
+      }
     }
-    run += n;
+    if (lane == 31) warp_sum[warp] = make_int2(a, b);
+    __syncthreads();
+    int2 before = run;
+    for (int w = 0; w < nwarp; ++w) {
+      const int2 v = warp_sum[w];
+      if (w < warp) before.x += v.x, before.y += v.y;
+      run.x += v.x, run.y += v.y;
+    }
+    if (s < nseg) {
+      const int row0 = before.x + a - n, share = work_item_rows(n, rpi);
+      int it = before.y + b - ni;
+      seg_off[s] = row0;
+      for (int r = 0; r < n; r += share, ++it) {
+        item_seg[it] = s;
+        item_row0[it] = row0 + r;
+        item_nrows[it] = min(share, n - r);
+      }
+    }
+    __syncthreads();
   }
-  seg_off[nseg] = run;
-  *n_items = items;
+  if (threadIdx.x == 0) {
+    seg_off[nseg] = run.x;
+    *n_items = run.y;
+  }
 }
 
 int launch_items_from_counts(const int32_t *seg_count, int nseg, int rows_per_item, int32_t *seg_off,
                              int32_t *item_seg, int32_t *item_row0, int32_t *item_nrows, int32_t *n_items,
                              cudaStream_t st) {
-  k_items_from_counts<<<1, 32, 0, st>>>(seg_count, nseg, rows_per_item, seg_off, item_seg, item_row0,
-                                        item_nrows, n_items);
+  const int threads = nseg >= 1024 ? 1024 : (nseg + 31) / 32 * 32;
   coli_count_launch(1);
-  return coli_cuda_check(cudaGetLastError(), "work list launch") ? 1 : 0;
+  return coli_cuda_check(launch_dependent(k_items_from_counts, dim3(1), dim3(threads > 0 ? threads : 32), 0, st, seg_count, nseg, rows_per_item,
+                                          seg_off, item_seg, item_row0, item_nrows, n_items),
+                         "work list launch")
+             ? 1
+             : 0;
 }
 
 }  // namespace colib

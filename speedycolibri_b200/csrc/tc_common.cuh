@@ -1,4 +1,4 @@
-// Pieces shared by the tcgen05 expert kernels: PTX wrappers (mbarrier, TMA, tcgen05), bounded waits,
+// Pieces of the tcgen05 expert kernel: PTX wrappers (mbarrier, TMA, tcgen05), bounded waits,
 // UMMA descriptors, the NVFP4 -> f16 conversion, and the host-side tensor map for token rows.
 #pragma once
 #include <cuda.h>
@@ -64,6 +64,7 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
 // tenth of an instruction per cycle, the MMA-issuing threads lost ~500 cycles per stage).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status, int code,
                                           uint32_t sleep_ns = 0) {
+  if (mbar_test_wait(bar, parity)) return true;
   const uint32_t hint = sleep_ns > 1000u ? sleep_ns : 1000u;
   const uint32_t limit = sleep_ns ? (TC_SPIN_LIMIT >> 4) : TC_SPIN_LIMIT;  // at most ~0.3 s of suspended polls
   for (uint32_t i = 0; i < limit; ++i) {
