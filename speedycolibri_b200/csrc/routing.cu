@@ -82,14 +82,10 @@ __global__ void __launch_bounds__(256) k_router_gemm(RouteParams p) {
     }
 }
 
-// Router GEMM, batched shapes: BM tokens x 64 experts per CTA of NT threads, (BM*16/NT) x 4
-// outputs per thread, k-chunks of 32 staged with 16-byte loads and stored transposed as f32, so
-// the inner loop is a few 128-bit shared loads per block of FMAs.  Same arithmetic as above: each
-// output is one thread's k-ascending fmaf chain.  Needs H % 8 == 0.
 // Two independent f32 FMAs in one instruction (sm_100): c.x = fma(a.x, b, c.x), c.y = fma(a.y, b, c.y),
-// each rounded as a scalar fmaf, so an output's k-ascending chain is unchanged.  It halves the FMA
-// instructions of k_router_gemm_big (0.51 -> 0.475 ms at 4096 tokens x 256 experts x 7168); the 8 x 8
-// register-tiled kernel below measured the same with and without it and keeps scalar FMAs.
+// each rounded as a scalar fmaf, so an output's k-ascending chain is unchanged.  Fed from shared memory,
+// an 8 x 8 register tile reaches 110 FMAs per clock and SM with it and 94 without (two warps per
+// scheduler; 87 and 75 with one).
 __device__ __forceinline__ void coli_ffma2(float2 &c, const float2 a, const float b) {
   unsigned long long cc, aa, bb;
   asm("mov.b64 %0, {%1, %2};" : "=l"(cc) : "f"(c.x), "f"(c.y));
@@ -99,244 +95,121 @@ __device__ __forceinline__ void coli_ffma2(float2 &c, const float2 a, const floa
   asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(cc));
 }
 
-template <int BM, int NT>
-__global__ void __launch_bounds__(NT) k_router_gemm_big(RouteParams p) {
+// Router GEMM of the large batches (H % 8 == 0): every thread owns TM x TN outputs, each one k-ascending
+// fmaf chain, two tokens per FMA instruction; a warp covers 4 TM tokens x 8 TN experts, a CTA WM x WN
+// warps.  Operands are staged as f32, k-major, two buffers of 32 k, with 16-byte loads one block ahead;
+// a warp's lanes take consecutive rows, so the transposed stores fall into different banks.  CW warps of
+// their own do the staging, or (CW = 0) the computing warps between blocks: with one computing warp per
+// scheduler, the 8 x 8 tile, staging in between costs 10 % (443 against 403 us with the top-k, 4096
+// tokens x 256 experts x 7168), with the 16 x 8 tile and three CTAs per SM the extra warps cost 4 %.
+// Bound by FMA issue and the operand reads between them: 16384 x 384 x 6144 1894 -> 1617 us, 103 FMAs
+// per clock and SM of the SM's 128 while its last CTAs keep it full.
+template <int TM_, int TN_, int WM_, int WN_, int CW_>
+struct RouterPairTile {
+  static constexpr int TM = TM_, TN = TN_, WM = WM_, WN = WN_, CW = CW_, BK = 32;
+  static constexpr int BM = 4 * TM * WM, BN = 8 * TN * WN, ROWS = BM + BN;
+  static constexpr int COMPUTE = 32 * WM * WN, NT = COMPUTE + 32 * CW, STAGING = CW ? 32 * CW : COMPUTE;
+  static constexpr int LD = ROWS + 4;              // floats per k: tokens, then experts, then padding
+  static constexpr int CPT = ROWS * (BK / 8) / STAGING;  // 16-byte chunks a thread stages per block
+  static constexpr size_t SMEM = (size_t)2 * BK * LD * 4;
+  static_assert(ROWS * (BK / 8) % STAGING == 0 && ROWS % 32 == 0 && TM % 4 == 0 && TN % 4 == 0, "tile shape");
+};
+template <class C>
+__global__ void __launch_bounds__(C::NT) k_router_pair(RouteParams p) {
   coli_grid_trigger();  // the top-k may be scheduled; it waits for this grid
-  constexpr int TMR = BM * 16 / NT;  // token rows per thread
-  constexpr int BN = 64, BK = 32, LDX = BM + 4, LDW = BN + 4;
-  constexpr int SR = NT / 4;                  // rows staged per pass (4 chunks of 8 k each)
-  constexpr int XP = (BM + SR - 1) / SR, WP = BN / SR;
-  static_assert(TMR >= 1 && BN % SR == 0, "tile / thread-count mismatch");
-  // two buffers of each staged tile: chunk i+1 is written while chunk i is multiplied, so one
-  // barrier per chunk suffices
+  constexpr int TM = C::TM, TN = C::TN, BK = C::BK, LD = C::LD, BM = C::BM;
   extern __shared__ __align__(16) float rsm[];
-  float(*xs)[BK][LDX] = reinterpret_cast<float(*)[BK][LDX]>(rsm);                  // [2][BK][LDX]
-  float(*ws)[BK][LDW] = reinterpret_cast<float(*)[BK][LDW]>(rsm + 2 * BK * LDX);   // [2][BK][LDW]
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // tx -> 4 experts, ty -> TMR tokens
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  static_assert(TMR % 2 == 0, "token rows are accumulated in pairs");
-  float2 acc[TMR / 2][4];  // .x = token row 2i, .y = row 2i + 1
+  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * C::BN;
+  const int nkb = (p.H + BK - 1) / BK;
+  // staging: by the warps behind the computing ones, or by all
+  const int tid = C::CW ? (int)threadIdx.x - C::COMPUTE : (int)threadIdx.x;
+  uint4 v[C::CPT];
+  auto fetch = [&](int kb) {
 #pragma unroll
-  for (int i = 0; i < TMR / 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
-  // staging assignment: the threads of a warp take consecutive rows of one 8-k chunk, so their
-  // transposed stores fall into consecutive banks
-  const int sr = threadIdx.x % SR, sc = threadIdx.x / SR;
-  uint4 xv[XP], wv[WP];
-  auto fetch = [&](int k0) {  // global -> registers; issued one chunk ahead of its use
-    const int k = k0 + sc * 8;
-#pragma unroll
-    for (int h = 0; h < XP; ++h) {
-      const int m = m0 + sr + SR * h;
-      xv[h] = make_uint4(0, 0, 0, 0);
-      if (sr + SR * h < BM && m < p.T && k < p.H) xv[h] = *reinterpret_cast<const uint4 *>(p.x + (size_t)m * p.H + k);
-    }
-#pragma unroll
-    for (int h = 0; h < WP; ++h) {
-      const int n = n0 + sr + SR * h;
-      wv[h] = make_uint4(0, 0, 0, 0);
-      if (n < p.E && k < p.H) wv[h] = *reinterpret_cast<const uint4 *>(p.router_w + (size_t)n * p.H + k);
+    for (int i = 0; i < C::CPT; ++i) {
+      const int idx = i * C::STAGING + tid, r = idx % C::ROWS, k = kb * BK + idx / C::ROWS * 8;
+      const int row = r < BM ? m0 + r : n0 + r - BM;
+      v[i] = make_uint4(0, 0, 0, 0);
+      if (row < (r < BM ? p.T : p.E) && k < p.H)
+        v[i] = *reinterpret_cast<const uint4 *>((r < BM ? p.x : p.router_w) + (size_t)row * p.H + k);
     }
   };
-  auto stage = [&](int buf) {  // registers -> shared memory, bf16 -> f32, transposed
+  auto stage = [&](int kb) {
+    float *dst = rsm + (kb & 1) * (BK * LD);
 #pragma unroll
-    for (int h = 0; h < XP; ++h) {
-      if (sr + SR * h >= BM) break;
-      const uint32_t u[4] = {xv[h].x, xv[h].y, xv[h].z, xv[h].w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        xs[buf][sc * 8 + 2 * j][sr + SR * h] = __uint_as_float(u[j] << 16);
-        xs[buf][sc * 8 + 2 * j + 1][sr + SR * h] = __uint_as_float(u[j] & 0xffff0000u);
-      }
-    }
-#pragma unroll
-    for (int h = 0; h < WP; ++h) {
-      const uint32_t u[4] = {wv[h].x, wv[h].y, wv[h].z, wv[h].w};
+    for (int i = 0; i < C::CPT; ++i) {
+      const int idx = i * C::STAGING + tid, r = idx % C::ROWS, k = idx / C::ROWS * 8;
+      const uint32_t u[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        ws[buf][sc * 8 + 2 * j][sr + SR * h] = __uint_as_float(u[j] << 16);
-        ws[buf][sc * 8 + 2 * j + 1][sr + SR * h] = __uint_as_float(u[j] & 0xffff0000u);
+        dst[(k + 2 * j) * LD + r] = __uint_as_float(u[j] << 16);
+        dst[(k + 2 * j + 1) * LD + r] = __uint_as_float(u[j] & 0xffff0000u);
       }
     }
   };
-  fetch(0);
-  stage(0);
-  __syncthreads();
-  if (BK < p.H) fetch(BK);
-  int buf = 0;
-  for (int k0 = 0; k0 < p.H; k0 += BK, buf ^= 1) {
-#pragma unroll 8
-    for (int kk = 0; kk < BK; ++kk) {
-      float a[TMR];
-      if (TMR >= 4) {
-#pragma unroll
-        for (int q = 0; q < TMR / 4; ++q) {
-          const float4 v = *reinterpret_cast<const float4 *>(&xs[buf][kk][ty * TMR + 4 * q]);
-          a[4 * q] = v.x;
-          a[4 * q + 1] = v.y;
-          a[4 * q + 2] = v.z;
-          a[4 * q + 3] = v.w;
-        }
-      } else if (TMR == 2) {
-        const float2 v = *reinterpret_cast<const float2 *>(&xs[buf][kk][ty * 2]);
-        a[0] = v.x;
-        a[TMR - 1] = v.y;
-      } else {
-#pragma unroll
-        for (int i = 0; i < TMR; ++i) a[i] = xs[buf][kk][ty * TMR + i];
+  if (C::CW && threadIdx.x >= C::COMPUTE) {  // block kb + 1 is stored while block kb is multiplied
+    fetch(0);
+    stage(0);
+    if (nkb > 1) fetch(1);
+    for (int kb = 0; kb < nkb; ++kb) {
+      __syncthreads();
+      if (kb + 1 < nkb) {
+        stage(kb + 1);  // that buffer was last read one barrier ago
+        if (kb + 2 < nkb) fetch(kb + 2);
       }
-      const float4 b = *reinterpret_cast<const float4 *>(&ws[buf][kk][tx * 4]);
-      const float bb[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-      for (int i = 0; i < TMR / 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) coli_ffma2(acc[i][j], make_float2(a[2 * i], a[2 * i + 1]), bb[j]);
     }
-    if (k0 + BK < p.H) {
-      stage(buf ^ 1);  // chunk k0 + BK, fetched while this one was multiplied; that buffer was last read one barrier ago
-      if (k0 + 2 * BK < p.H) fetch(k0 + 2 * BK);
-    }
-    __syncthreads();
+    return;
   }
+  // ---------------- computing warps ----------------
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int mt = (warp / C::WN) * 4 * TM + (lane >> 3) * TM;         // this thread's first token of the tile
+  const int nt = (warp % C::WN) * 8 * TN + (lane & 7) * 4;           // and first expert; the others 32 q + j on
+  if (!C::CW) {
+    fetch(0);
+    stage(0);
+    if (nkb > 1) fetch(1);
+  }
+  float2 acc[TM / 2][TN];  // .x = token 2 i, .y = token 2 i + 1
 #pragma unroll
-  for (int i = 0; i < TMR; ++i)
+  for (int i = 0; i < TM / 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int m = m0 + ty * TMR + i, n = n0 + tx * 4 + j;
-      if (m < p.T && n < p.E) {
-        float v = (i & 1) ? acc[i >> 1][j].y : acc[i >> 1][j].x;
-        if (p.logit_bias) v = __fadd_rn(v, p.logit_bias[n]);
-        p.logits[(size_t)m * p.E + n] = v;
-      }
-    }
-}
-
-// Router GEMM, register-tiled: every thread owns TM tokens x TN experts (TM*TN independent
-// k-ascending fmaf chains), a CTA of NT threads covers (NT/16)*TM tokens x 16*TN experts.  The
-// kernel is bound by the shared-memory operand traffic per FMA, (TM + TN) / (TM * TN) words: an
-// 8 x 8 tile needs a quarter of what a 2 x 4 tile does, so large batches take the largest tile and
-// small ones the largest tile that still gives every SM a CTA.  Operands are staged as f32,
-// transposed (k-major), two buffers, 16-byte loads one chunk ahead; a thread's experts are
-// {tx*4 + j} in each 64-wide group, so the 16 lanes of a row read consecutive 16-byte words.
-// Same arithmetic as the other router kernels: the tile shape never changes an output's k order.
-// Needs H % 8 == 0.
-template <int TM, int TN, int NT>
-__global__ void __launch_bounds__(NT) k_router_rt(RouteParams p) {
-  coli_grid_trigger();  // the top-k may be scheduled; it waits for this grid
-  static_assert(TN % 4 == 0 && (TM % 4 == 0 || TM == 2), "tile shape");
-  constexpr int BM = (NT / 16) * TM, BN = 16 * TN, BK = 32, LDX = BM + 4, LDW = BN + 4;
-  constexpr int SR = NT / 4;  // rows staged per pass (4 chunks of 8 k each)
-  constexpr int XP = (BM + SR - 1) / SR, WP = (BN + SR - 1) / SR;
-  extern __shared__ __align__(16) float rsm[];
-  float(*xs)[BK][LDX] = reinterpret_cast<float(*)[BK][LDX]>(rsm);
-  float(*ws)[BK][LDW] = reinterpret_cast<float(*)[BK][LDW]>(rsm + 2 * BK * LDX);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  float acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
-  const int sr = threadIdx.x % SR, sc = threadIdx.x / SR;
-  uint4 xv[XP], wv[WP];
-  auto fetch = [&](int k0) {
-    const int k = k0 + sc * 8;
-#pragma unroll
-    for (int h = 0; h < XP; ++h) {
-      const int r = sr + SR * h, m = m0 + r;
-      xv[h] = make_uint4(0, 0, 0, 0);
-      if (r < BM && m < p.T && k < p.H) xv[h] = *reinterpret_cast<const uint4 *>(p.x + (size_t)m * p.H + k);
-    }
-#pragma unroll
-    for (int h = 0; h < WP; ++h) {
-      const int r = sr + SR * h, n = n0 + r;
-      wv[h] = make_uint4(0, 0, 0, 0);
-      if (r < BN && n < p.E && k < p.H) wv[h] = *reinterpret_cast<const uint4 *>(p.router_w + (size_t)n * p.H + k);
-    }
-  };
-  auto stage = [&](int buf) {
-#pragma unroll
-    for (int h = 0; h < XP; ++h) {
-      const int r = sr + SR * h;
-      if (r < BM) {
-        const uint32_t u[4] = {xv[h].x, xv[h].y, xv[h].z, xv[h].w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          xs[buf][sc * 8 + 2 * j][r] = __uint_as_float(u[j] << 16);
-          xs[buf][sc * 8 + 2 * j + 1][r] = __uint_as_float(u[j] & 0xffff0000u);
-        }
-      }
-    }
-#pragma unroll
-    for (int h = 0; h < WP; ++h) {
-      const int r = sr + SR * h;
-      if (r < BN) {
-        const uint32_t u[4] = {wv[h].x, wv[h].y, wv[h].z, wv[h].w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          ws[buf][sc * 8 + 2 * j][r] = __uint_as_float(u[j] << 16);
-          ws[buf][sc * 8 + 2 * j + 1][r] = __uint_as_float(u[j] & 0xffff0000u);
-        }
-      }
-    }
-  };
-  fetch(0);
-  stage(0);
-  __syncthreads();
-  if (BK < p.H) fetch(BK);
-  int buf = 0;
-  for (int k0 = 0; k0 < p.H; k0 += BK, buf ^= 1) {
+    for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+  for (int kb = 0; kb < nkb; ++kb) {
+    __syncthreads();  // block kb is staged
+    const float *buf = rsm + (kb & 1) * (BK * LD);
 #pragma unroll 4
     for (int kk = 0; kk < BK; ++kk) {
-      float a[TM], b[TN];
-      if (TM == 2) {
-        const float2 v = *reinterpret_cast<const float2 *>(&xs[buf][kk][ty * 2]);
-        a[0] = v.x;
-        a[TM - 1] = v.y;
-      } else {
+      float4 a[TM / 4], b[TN / 4];
 #pragma unroll
-        for (int q = 0; q < TM / 4; ++q) {
-          const float4 v = *reinterpret_cast<const float4 *>(&xs[buf][kk][ty * TM + 4 * q]);
-          a[4 * q] = v.x;
-          a[4 * q + 1] = v.y;
-          a[4 * q + 2] = v.z;
-          a[4 * q + 3] = v.w;
-        }
+      for (int q = 0; q < TM / 4; ++q) a[q] = *reinterpret_cast<const float4 *>(buf + kk * LD + mt + 4 * q);
+#pragma unroll
+      for (int q = 0; q < TN / 4; ++q) b[q] = *reinterpret_cast<const float4 *>(buf + kk * LD + BM + nt + 32 * q);
+#pragma unroll
+      for (int i = 0; i < TM / 2; ++i) {
+        const float2 ai = (i & 1) ? make_float2(a[i >> 1].z, a[i >> 1].w) : make_float2(a[i >> 1].x, a[i >> 1].y);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) coli_ffma2(acc[i][j], ai, (&b[j >> 2].x)[j & 3]);
       }
-#pragma unroll
-      for (int q = 0; q < TN / 4; ++q) {
-        const float4 v = *reinterpret_cast<const float4 *>(&ws[buf][kk][q * 64 + tx * 4]);
-        b[4 * q] = v.x;
-        b[4 * q + 1] = v.y;
-        b[4 * q + 2] = v.z;
-        b[4 * q + 3] = v.w;
-      }
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = __fmaf_rn(a[i], b[j], acc[i][j]);
     }
-    if (k0 + BK < p.H) {
-      stage(buf ^ 1);
-      if (k0 + 2 * BK < p.H) fetch(k0 + 2 * BK);
+    if (!C::CW && kb + 1 < nkb) {
+      stage(kb + 1);  // fetched while this block was multiplied; that buffer was last read one barrier ago
+      if (kb + 2 < nkb) fetch(kb + 2);
     }
-    __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
-      const int m = m0 + ty * TM + i, n = n0 + (j >> 2) * 64 + tx * 4 + (j & 3);
+      const int m = m0 + mt + i, n = n0 + nt + (j >> 2) * 32 + (j & 3);
       if (m < p.T && n < p.E) {
-        float v = acc[i][j];
-        if (p.logit_bias) v = __fadd_rn(v, p.logit_bias[n]);
-        p.logits[(size_t)m * p.E + n] = v;
+        float o = (i & 1) ? acc[i >> 1][j].y : acc[i >> 1][j].x;
+        if (p.logit_bias) o = __fadd_rn(o, p.logit_bias[n]);
+        p.logits[(size_t)m * p.E + n] = o;
       }
     }
 }
 
-// Router GEMM for the batches below those of the two kernels above (H % 8 == 0): every thread owns
+// Router GEMM for the batches below those of the kernel above (H % 8 == 0): every thread owns
 // TM x TN outputs, each one k-ascending fmaf chain; a warp covers 4 TM tokens x 8 TN experts, a CTA
 // WM x WN warps.  Token and expert rows travel as bf16, in k-blocks of BK through a ring of STAGES
 // cp.async stages, so the loads of the next stages are in flight while one is multiplied; rows are
@@ -346,8 +219,7 @@ __global__ void __launch_bounds__(NT) k_router_rt(RouteParams p) {
 // the issue slots otherwise: for 8 k a thread issues 8 TM TN FMAs, 8 (TM + TN) operations that widen
 // bf16 to f32 (at half the FMA rate) and TM + TN shared loads.  A small tile spreads few outputs over
 // all SMs, a large one spends fewer slots per FMA: pick_router_tile weighs the two.
-// Measured with the top-k behind it, before (the kernels above, or a CTA of 16 tokens x 64 experts)
-// and now: 48 tokens x 128 experts x 2048 63.8 -> 19.7 us, 24 x 256 x 7168 202 -> 47, 512 x 128 x 2048
+// Measured with the top-k behind it, against a kernel of 16 to 128 tokens x 64 experts per CTA: 48 tokens x 128 experts x 2048 63.8 -> 19.7 us, 24 x 256 x 7168 202 -> 47, 512 x 128 x 2048
 // 65 -> 30, 709 x 256 x 7168 320 -> 151, 2048 x 256 x 7168 320 -> 277.  Staging the operands as f32 by
 // warps of their own was built and is slower from 200 tokens on (shared-memory reads).
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool valid) {
@@ -745,30 +617,14 @@ __global__ void __launch_bounds__(128) k_route_topk(RouteParams p) {
   route_topk_token(p, t, sm + (size_t)warp * topk_row_floats(p.E), lane);
 }
 
-template <int BM, int NT>
-static bool launch_router_big(const RouteParams &p, dim3 grid, cudaStream_t st) {
-  constexpr size_t smem = (size_t)2 * 32 * ((BM + 4) + (64 + 4)) * sizeof(float);
-  static ColiPerDeviceOnce attr_once;
-  if (smem > 48 * 1024 && !coli_set_smem_limit(attr_once, k_router_gemm_big<BM, NT>, smem, "router shared-memory attribute")) return false;
-  k_router_gemm_big<BM, NT><<<grid, NT, smem, st>>>(p);
-  return true;
-}
-
-template <int TM, int TN, int NT>
-static bool launch_router_rt(const RouteParams &p, cudaStream_t st) {
-  constexpr int BM = (NT / 16) * TM, BN = 16 * TN;
-  constexpr size_t smem = (size_t)2 * 32 * ((BM + 4) + (BN + 4)) * sizeof(float);
-  static ColiPerDeviceOnce attr_once;
-  if (smem > 48 * 1024 && !coli_set_smem_limit(attr_once, k_router_rt<TM, TN, NT>, smem, "router shared-memory attribute")) return false;
-  dim3 grid((p.E + BN - 1) / BN, (p.T + BM - 1) / BM);
-  k_router_rt<TM, TN, NT><<<grid, NT, smem, st>>>(p);
-  return true;
-}
 // The tiles of k_router_chain.
 //                              TM TN WM WN  BK  stages
 using RouterTile8x8 = RouterTile<1, 1, 2, 1, 128, 8>;
 using RouterTile16x32 = RouterTile<2, 2, 2, 2, 64, 8>;
 using RouterTile64x64 = RouterTile<8, 4, 2, 2, 64, 6>;
+// ... and of k_router_pair:             TM TN WM WN CW
+using RouterTile128x64 = RouterPairTile<8, 8, 4, 1, 2>;
+using RouterTile128x128 = RouterPairTile<16, 8, 2, 2, 0>;
 template <class C>
 static bool launch_router_chain(const RouteParams &p, cudaStream_t st) {
   static ColiPerDeviceOnce attr_once;
@@ -777,14 +633,21 @@ static bool launch_router_chain(const RouteParams &p, cudaStream_t st) {
   k_router_chain<C><<<grid, C::NT, C::SMEM, st>>>(p);
   return true;
 }
-// The kernel and tile of a batch: 0 = 8 x 8, 1 = 16 x 32, 2 = 64 x 64 tokens x experts of k_router_chain,
-// 3 = 128 x 64 of k_router_gemm_big, 4 = 128 x 128 of k_router_rt.  The time of one k is a function of
-// n, the CTAs of the fullest SM; the figures are nanoseconds measured on B200 between 21 and 16384
-// tokens (5.3 and 10 are the chain's latency, with its loads and conversions, when an SM has little else).
+template <class C>
+static bool launch_router_pair(const RouteParams &p, cudaStream_t st) {
+  static ColiPerDeviceOnce attr_once;
+  if (C::SMEM > 48 * 1024 && !coli_set_smem_limit(attr_once, k_router_pair<C>, C::SMEM, "router shared-memory attribute")) return false;
+  k_router_pair<C><<<dim3((p.T + C::BM - 1) / C::BM, (p.E + C::BN - 1) / C::BN), C::NT, C::SMEM, st>>>(p);
+  return true;
+}
+// The tile of a batch: 0 = 8 x 8, 1 = 16 x 32, 2 = 64 x 64, 3 = 128 x 64, 4 = 128 x 128 tokens x experts.
+// The time of one k is a function of n, the CTAs of the fullest SM; the figures are nanoseconds measured
+// on B200 between 21 and 16384 tokens (5.3 and 10 are the chain's latency, with its loads and
+// conversions, when an SM has little else).
 static int pick_router_tile(const RouteParams &p) {
   auto n = [&](int bm, int bn) { return (float)(((long)((p.T + bm - 1) / bm) * ((p.E + bn - 1) / bn) + 147) / 148); };
   const float ns[5] = {fmaxf(5.3f, 1.6f * n(8, 8)), fmaxf(10.0f, 3.0f + 5.6f * n(16, 32)), 3.0f + 33.0f * n(64, 64),
-                       63.0f * n(128, 64), 103.0f * n(128, 128)};
+                       5.0f + 46.5f * n(128, 64), 8.0f + 81.0f * n(128, 128)};
   int best = 0;
   for (int i = 1; i < 5; ++i)
     if (ns[i] < ns[best]) best = i;
@@ -813,8 +676,8 @@ int launch_router(const RouteParams &p, cudaStream_t st) {
       case 0: ok = launch_router_chain<RouterTile8x8>(p, st); break;
       case 1: ok = launch_router_chain<RouterTile16x32>(p, st); break;
       case 2: ok = launch_router_chain<RouterTile64x64>(p, st); break;
-      case 3: ok = launch_router_big<128, 256>(p, dim3((p.E + 63) / 64, (p.T + 127) / 128), st); break;
-      case 4: ok = launch_router_rt<8, 8, 256>(p, st); break;
+      case 3: ok = launch_router_pair<RouterTile128x64>(p, st); break;
+      case 4: ok = launch_router_pair<RouterTile128x128>(p, st); break;
     }
     if (!ok) return 0;
   } else if ((long)((p.T + 31) / 32) * ((p.E + 31) / 32) >= 96) {
