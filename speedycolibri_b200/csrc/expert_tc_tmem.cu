@@ -80,7 +80,7 @@ struct TtBudget {
   static constexpr int B_BYTES = ACC * TC_BK * 2;
   static constexpr int B_STAGES = 6;
   static constexpr int NBARS = 2 * B_STAGES + 2 + 2 * 9;  // stages, accumulators, at most 9 weight slots
-  static_assert(B_STAGES == 6 && B_STAGES % A_STAGES == 0 && B_BYTES % 1024 == 0, "a stage barrier serves both rings");
+  static_assert(B_STAGES == 6 && (A_STAGES == 3 || A_STAGES == 6) && B_BYTES % 1024 == 0, "a stage barrier serves both rings");
 };
 // The token tile of a stage arrives as ONE box of N rows: the copy engine of an SM takes about 64
 // cycles per box plus 4 per 128-byte row (measured: 21 B/clk with 32-row boxes, 31 B/clk with
@@ -120,6 +120,15 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// One FP8 word -> two f16x2 (also: four ue4m3 block scales)
+__device__ __forceinline__ void tt_cvt_e4m3x4(uint32_t w, uint32_t &p0, uint32_t &p1) {
+  asm("{ .reg .b16 h0, h1;\n"
+      "  mov.b32 {h0, h1}, %2;\n"
+      "  cvt.rn.f16x2.e4m3x2 %0, h0;\n"
+      "  cvt.rn.f16x2.e4m3x2 %1, h1; }\n"
+      : "=r"(p0), "=r"(p1)
+      : "r"(w));
+}
 // The 64 weights (32 packed bytes) and 4 block-scale bytes of one row for one 64-k stage.
 struct TtPacked {
   uint4 q0, q1;
@@ -130,29 +139,41 @@ __device__ __forceinline__ uint4 tt_lds128(uint32_t addr) {
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
   return v;
 }
-// `slab` = shared-memory address of the 128-row slab of one k-tile: 64 B of codes per row, then 8 B
-// of scales per row; `half` = which 64 of its 128 k.
-__device__ __forceinline__ TtPacked tt_read_packed(uint32_t slab, int row, int half) {
+// `codes` = address of the row's chunk 0 (chunks are permuted by XOR, so chunk j is at codes ^ 16 j),
+// `scales` = address of its scale bytes; `half` = which 64 of the k-tile's 128 k.
+__device__ __forceinline__ TtPacked tt_read_packed(uint32_t codes, uint32_t scales, int half) {
   TtPacked r;
-  r.q0 = tt_lds128(slab + row * 64 + coli_fp4_chunk(row, 2 * half) * 16);
-  r.q1 = tt_lds128(slab + row * 64 + coli_fp4_chunk(row, 2 * half + 1) * 16);
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r.sc) : "r"(slab + TC_BM * 64 + row * 8 + half * 4) : "memory");
+  const uint32_t a = codes ^ (uint32_t)(half << 5);
+  r.q0 = tt_lds128(a);
+  r.q1 = tt_lds128(a ^ 16u);
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r.sc) : "r"(scales + half * 4) : "memory");
   return r;
 }
-// Convert one stage of one row and hand it to the tensor core through 32 TMEM columns.
+// Convert one stage of one row: one conversion and one multiply per pair of weights (the multiply takes
+// either half of the scale pair as its operand, so the scales need no spreading).
 __device__ __forceinline__ void tt_convert(const TtPacked &pk, uint32_t (&r)[32]) {
-  uint32_t m0, m1, m2, m3;
-  tc_scales(pk.sc, m0, m1);
-  tc_scales(pk.sc >> 16, m2, m3);
   const uint32_t w[8] = {pk.q0.x, pk.q0.y, pk.q0.z, pk.q0.w, pk.q1.x, pk.q1.y, pk.q1.z, pk.q1.w};
-  const uint32_t m[4] = {m0, m1, m2, m3};
+  uint32_t s01, s23;
+  tt_cvt_e4m3x4(pk.sc, s01, s23);
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const uint4 o = tc_dequant_word(w[j], m[j >> 1]);
-    r[4 * j] = o.x;
-    r[4 * j + 1] = o.y;
-    r[4 * j + 2] = o.z;
-    r[4 * j + 3] = o.w;
+    const __half2 pair = *reinterpret_cast<const __half2 *>(j < 4 ? &s01 : &s23);
+    const __half2 m = (j & 2) ? __high2half2(pair) : __low2half2(pair);
+    uint4 o;
+    asm("{ .reg .b8 b0, b1, b2, b3;\n"
+        "  mov.b32 {b0, b1, b2, b3}, %4;\n"
+        "  cvt.rn.f16x2.e2m1x2 %0, b0;\n"
+        "  cvt.rn.f16x2.e2m1x2 %1, b1;\n"
+        "  cvt.rn.f16x2.e2m1x2 %2, b2;\n"
+        "  cvt.rn.f16x2.e2m1x2 %3, b3; }\n"
+        : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w)
+        : "r"(w[j]));
+    const uint32_t v[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const __half2 z = __hmul2_rn(*reinterpret_cast<const __half2 *>(&v[q]), m);
+      r[4 * j + q] = *reinterpret_cast<const uint32_t *>(&z);
+    }
   }
 }
 
@@ -174,20 +195,12 @@ __device__ __forceinline__ uint32_t tt_f16x2_both(float v) {
   const __half2 h = __float2half2_rn(v);
   return *reinterpret_cast<const uint32_t *>(&h);
 }
-__device__ __forceinline__ TtPacked8 tt_read_packed8(uint32_t slab, int row, int half, uint32_t mult) {
+__device__ __forceinline__ TtPacked8 tt_read_packed8(uint32_t codes, int half, uint32_t mult) {
   TtPacked8 r;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) r.q[j] = tt_lds128(slab + row * 128 + coli_fp8_chunk(row, 4 * half + j) * 16);
+  for (int j = 0; j < 4; ++j) r.q[j] = tt_lds128(codes ^ (uint32_t)((half << 6) | (j << 4)));
   r.mult = mult;
   return r;
-}
-__device__ __forceinline__ void tt_cvt_e4m3x4(uint32_t w, uint32_t &p0, uint32_t &p1) {
-  asm("{ .reg .b16 h0, h1;\n"
-      "  mov.b32 {h0, h1}, %2;\n"
-      "  cvt.rn.f16x2.e4m3x2 %0, h0;\n"
-      "  cvt.rn.f16x2.e4m3x2 %1, h1; }\n"
-      : "=r"(p0), "=r"(p1)
-      : "r"(w));
 }
 template <int FMT>
 __device__ __forceinline__ void tt_convert8(const TtPacked8 &pk, uint32_t (&r)[32]) {
@@ -226,8 +239,18 @@ struct TtWeightRing {
   static constexpr int SLOTS = FMT == COLI_FMT_NVFP4 ? (ACC <= 64 ? 9 : 5) : (ACC <= 64 ? 5 : 3);
   static constexpr int BYTES = SLOT * SLOTS;
 };
+__device__ __forceinline__ void tt_cp_async16(uint32_t dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
 __device__ __forceinline__ void tt_cp_async16(uint32_t dst, const void *src, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16u : 0u) : "memory");
+}
+
+// Whole-warp wait: the common case, a phase that has completed, costs a test and a vote.  (Kept inline:
+// with the rest behind a call the producers' registers no longer fit and 160-row tiles lost 8 %.)
+__device__ __forceinline__ bool tt_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status, int code) {
+  return __all_sync(0xffffffffu, mbar_test_wait(bar, parity)) ||
+         __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code, 1));
 }
 
 // GATED: the two weight tiles of a stage are gate and up of the same 128 features, result
@@ -327,27 +350,53 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
       const int seg = p.item_seg[item];
       const int ex = p.seg_expert ? p.seg_expert[seg] : seg;
       const WeightRef wt[2] = {GATED ? p.gate[ex] : p.down[ex], GATED ? p.up[ex] : p.down[ex]};
+      // this thread's first chunk of each tile's codes and scales; the next k-tile is Op rows on
+      const uint8_t *qsrc[2], *ssrc[2];
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const size_t row0 = (size_t)ft * FT + (GATED ? 0 : m * TC_BM);
+        qsrc[m] = wt[m].q + row0 * QB + tid * 16;
+        ssrc[m] = wt[m].s + row0 * SB + tid * 16;
+      }
+      const bool whole = ft * FT + FT <= Op;
       for (int kt = 0; kt < (KB >> 1); ++kt) {
-        if (!__all_sync(0xffffffffu, mbar_wait(wempty + 8 * slot, ph ^ 1u, abort_flag, p.status, TC_ERR_TMA_WAIT, 1))) {
+        if (!tt_wait(wempty + 8 * slot, ph ^ 1u, abort_flag, p.status, TC_ERR_TMA_WAIT)) {
           alive = false;
           break;
         }
+        const uint32_t dst = wring + slot * Ring::SLOT + tid * 16;
+        if (whole) {
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+#pragma unroll
+            for (int i = 0; i < QI; ++i)
+              tt_cp_async16(dst + m * Ring::SLAB + i * TT_LOAD_THREADS * 16, qsrc[m] + i * TT_LOAD_THREADS * 16);
+#pragma unroll
+            for (int i = 0; i < SI; ++i)
+              tt_cp_async16(dst + m * Ring::SLAB + TC_BM * QB + i * TT_LOAD_THREADS * 16, ssrc[m] + i * TT_LOAD_THREADS * 16);
+          }
+        } else {  // rows past the end of the matrix are zeros
+#pragma unroll 1
+          for (int m = 0; m < 2; ++m) {
+            const int n = max(0, min(TC_BM, Op - (ft * FT + (GATED ? 0 : m * TC_BM))));
+#pragma unroll 1
+            for (int i = 0; i < QI; ++i) {
+              const int c = i * TT_LOAD_THREADS * 16;
+              const bool in = c + tid * 16 < n * QB;
+              tt_cp_async16(dst + m * Ring::SLAB + c, in ? qsrc[m] + c : wt[m].q, in);
+            }
+#pragma unroll 1
+            for (int i = 0; i < SI; ++i) {
+              const int c = i * TT_LOAD_THREADS * 16;
+              const bool in = c + tid * 16 < n * SB;
+              tt_cp_async16(dst + m * Ring::SLAB + TC_BM * QB + c, in ? ssrc[m] + c : wt[m].s, in);
+            }
+          }
+        }
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
-          const int row0 = ft * FT + (GATED ? 0 : m * TC_BM);
-          const int n = min(TC_BM, Op - row0);  // rows of this tile that exist; the rest are zeros
-          const size_t r = (size_t)kt * Op + row0;
-          const uint32_t dst = wring + slot * Ring::SLOT + m * Ring::SLAB;
-#pragma unroll
-          for (int i = 0; i < QI; ++i) {
-            const int c = (i * TT_LOAD_THREADS + tid) * 16;
-            tt_cp_async16(dst + c, c < n * QB ? wt[m].q + r * QB + c : wt[m].q, c < n * QB);
-          }
-#pragma unroll
-          for (int i = 0; i < SI; ++i) {
-            const int c = (i * TT_LOAD_THREADS + tid) * 16;
-            tt_cp_async16(dst + TC_BM * QB + c, c < n * SB ? wt[m].s + r * SB + c : wt[m].s, c < n * SB);
-          }
+          qsrc[m] += (size_t)Op * QB;
+          ssrc[m] += (size_t)Op * SB;
         }
         // arrives when this thread's copies up to here have landed
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(wfull + 8 * slot) : "memory");
@@ -379,12 +428,12 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
       const int nrows = __reduce_max_sync(0xffffffffu, p.item_nrows[item]);
       const int N = (nrows + TC_BOXN - 1) / TC_BOXN * TC_BOXN;
       const uint32_t idesc = umma_idesc(N);
-      alive = __all_sync(0xffffffffu, mbar_wait(acc_empty, (tix & 1u) ^ 1u, abort_flag, p.status, TC_ERR_MMA_WAIT, 1));
+      alive = tt_wait(acc_empty, (tix & 1u) ^ 1u, abort_flag, p.status, TC_ERR_MMA_WAIT);
       if (!alive) break;
       tc_fence_after();
       for (int kb = 0; kb < KB; kb += 2) {
         if (lane == 0) TT_TRACE(tix * KB + kb, 0);
-        alive = __all_sync(0xffffffffu, mbar_wait(full_s + 8 * sb, phb, abort_flag, p.status, TC_ERR_MMA_WAIT, 1));
+        alive = tt_wait(full_s + 8 * sb, phb, abort_flag, p.status, TC_ERR_MMA_WAIT);
         if (!alive) break;
         if (lane == 0) TT_TRACE(tix * KB + kb, 1);
         tc_fence_after();
@@ -497,14 +546,16 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
     const int row = quarter * 32 + lane;
     const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + TT_A_COL0 + mtx * 32;
     const int KT = KB >> 1;
-    uint32_t g = par;  // running index of this group's next k-tile
-    uint32_t g0 = 0;   // ... and of the tile's first
+    const uint32_t code_off = FMT == COLI_FMT_NVFP4 ? row * 64 + coli_fp4_chunk(row, 0) * 16 : row * 128 + coli_fp8_chunk(row, 0) * 16;
+    int ahead = par;   // k-tiles from the start of the tile to this group's next one
     uint32_t wslot = par, wph = 0;
+    // stage barrier of the group's next stage (0, 2 or 4 of 6) and the phase of that round
+    uint32_t sb = 2 * par, ph = 0;
     bool alive = true;
-    for (int w = blockIdx.x; w < n_work && alive; w += gridDim.x, g0 += KT) {
+    for (int w = blockIdx.x; w < n_work && alive; w += gridDim.x) {
       const float *srow = nullptr;
       float norm = 0.0f, scale = 0.0f;
-      int kt = (int)(g - g0);
+      int kt = ahead;
       if constexpr (FMT == COLI_FMT_FP8_B128) {
         const int item = w / n_ftiles, ft = w % n_ftiles, seg = p.item_seg[item];
         const int ex = p.seg_expert ? p.seg_expert[seg] : seg;
@@ -518,51 +569,56 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
         norm = mx > 0.0f ? TT_FP8_HEADROOM / mx : 0.0f;
         scale = kt < KT ? __ldg(srow + kt) : 0.0f;
       }
-      for (; kt < KT && alive; kt += 2, g += 2) {
-        if (!__all_sync(0xffffffffu, mbar_wait(wfull + 8 * wslot, wph, abort_flag, p.status, TC_ERR_PROD_WAIT, 1))) {
+      for (; kt < KT; kt += 2) {
+        if (!tt_wait(wfull + 8 * wslot, wph, abort_flag, p.status, TC_ERR_PROD_WAIT)) {
           alive = false;
           break;
         }
         const uint32_t slab = wring + wslot * Ring::SLOT + mtx * Ring::SLAB;
+        const uint32_t codes = slab + code_off;
         const uint32_t mult = FMT == COLI_FMT_FP8_B128 ? tt_f16x2_both(scale * norm) : 0x3c003c00u /* 1.0 */;
         if (FMT == COLI_FMT_FP8_B128 && kt + 2 < KT) scale = __ldg(srow + kt + 2);
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
+        for (uint32_t half = 0; half < 2; ++half) {
           // The conversion runs BEFORE the wait for the tensor-memory slot, so that only the store stands
           // between the slot's release and the barrier that hands it to the issuing warp.
           uint32_t r[32];
           if constexpr (FMT == COLI_FMT_NVFP4)
-            tt_convert(tt_read_packed(slab, row, half), r);
+            tt_convert(tt_read_packed(codes, slab + TC_BM * 64 + row * 8, half), r);
           else
-            tt_convert8<FMT>(tt_read_packed8(slab, row, half, mult), r);
-          if (half == 1) {
+            tt_convert8<FMT>(tt_read_packed8(codes, half, mult), r);
+          if (half == 1) {  // the slab has been read
             __syncwarp();
             if (lane == 0) mbar_arrive(wempty + 8 * wslot);
           }
-          const uint32_t it = 2 * g + half;
-          const uint32_t sa = it % TT_A_STAGES;
-          if (mtx == 0 && quarter == 0 && lane == 0) TT_TRACE(it, 3);
-          if (it >= (uint32_t)TT_A_STAGES) {  // the weight slot was last read by stage it - TT_A_STAGES
-            const uint32_t u = it - TT_A_STAGES;
-            if (!__all_sync(0xffffffffu, mbar_wait(empty_s + 8 * (u % TT_B_STAGES), (u / TT_B_STAGES) & 1u, abort_flag, p.status, TC_ERR_PROD_WAIT, 1))) {
-              alive = false;
-              break;
-            }
-            tc_fence_after();
+          // The slot was last read by the stage TT_A_STAGES earlier: the same barrier one round ago with six
+          // slots, the one three on (of this round for the later three) with three.  A wait for the round
+          // before the first returns at once.
+          const uint32_t st = sb + half;
+          const uint32_t eb = TT_A_STAGES == 6 ? st : (st >= 3 ? st - 3 : st + 3);
+          const uint32_t ep = TT_A_STAGES == 6 || st < 3 ? ph ^ 1u : ph;
+          if (!tt_wait(empty_s + 8 * eb, ep, abort_flag, p.status, TC_ERR_PROD_WAIT)) {
+            alive = false;
+            break;
           }
-          if (mtx == 0 && quarter == 0 && lane == 0) TT_TRACE(it, 4);
-          tmem_st32(taddr + sa * 64, r);
-          tmem_st_wait();
-          if (mtx == 0 && quarter == 0 && lane == 0) TT_TRACE(it, 5);
-          tc_fence_before();
-          __syncwarp();
-          if (half == 1 && lane == 0) mbar_arrive(full_s + 8 * ((it - 1) % TT_B_STAGES));
+          tc_fence_after();
+          tmem_st32(taddr + (TT_A_STAGES == 6 ? st : (st >= 3 ? st - 3 : st)) * 64, r);
         }
+        if (!alive) break;
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full_s + 8 * sb);
         if ((wslot += 2) >= (uint32_t)Ring::SLOTS) {
           wslot -= Ring::SLOTS;
           wph ^= 1u;
         }
+        if ((sb += 4) >= (uint32_t)TT_B_STAGES) {
+          sb -= TT_B_STAGES;
+          ph ^= 1u;
+        }
       }
+      ahead = kt - KT;
     }
   }
 
