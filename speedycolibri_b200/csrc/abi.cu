@@ -824,7 +824,7 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
     tp.gate = m->gate;
     tp.up = m->up;
     tp.down = m->down;
-    tp.seg_expert = m->seg_expert;
+    tp.seg_expert = nullptr;  // every expert is resident: segment order is expert order, the shared expert last
     tp.item_seg = m->item_seg;
     tp.item_row0 = m->item_row0;
     tp.item_nrows = m->item_nrows;
@@ -846,7 +846,7 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
     fp.gate = m->gate;
     fp.up = m->up;
     fp.down = m->down;
-    fp.seg_expert = m->seg_expert;
+    fp.seg_expert = nullptr;  // every expert is resident: segment order is expert order, the shared expert last
     fp.item_seg = m->item_seg;
     fp.item_row0 = m->item_row0;
     fp.item_nrows = m->item_nrows;
@@ -1271,9 +1271,14 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
   CK(cudaMemcpyAsync(d_cnt, rows, sizeof(int32_t) * count, cudaMemcpyHostToDevice, st), "row count upload");
   CK(cudaMemsetAsync(d_status, 0, sizeof(int32_t), st), "status clear");
   CK(cudaEventRecord(ctx->ev[1], st), "phase event");
-  CK(cudaStreamSynchronize(st), "expert upload sync");  // tbl is a local; rows/x belong to the caller
-  if (!colib::launch_f32_to_f16((const float *)ctx->buf[0], (__half *)ctx->buf[1], xb, st)) return 0;
-  if (!colib::launch_items_from_counts(d_cnt, count, rpi, d_off, d_iseg, d_irow, d_inr, d_nit, st)) return 0;
+  // The call waits for the stream before it returns, on every path: the copies above may still be reading
+  // tbl, rows and x.  (Waiting here as well put 10 us between the copies and the kernels.)
+  const auto fail = [&]() {
+    cudaStreamSynchronize(st);
+    return 0;
+  };
+  if (!colib::launch_f32_to_f16((const float *)ctx->buf[0], (__half *)ctx->buf[1], xb, st)) return fail();
+  if (!colib::launch_items_from_counts(d_cnt, count, rpi, d_off, d_iseg, d_irow, d_inr, d_nit, st)) return fail();
   if (tc) {
     colib::TcParams tp;
     tp.fmt = kfmt;
@@ -1295,7 +1300,7 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
     tp.act = current_activation();
     const int sms = ctx->sm_count;
     const int ok = colib::launch_gate_up_tct(tp, ctx->buf[1], (int)total, sms, st) && colib::launch_down_tct(tp, (int)total, sms, st);
-    if (!ok || !colib::launch_bf16_to_f32((const __nv_bfloat16 *)ctx->buf[4], (float *)ctx->buf[0], xb, st)) return 0;
+    if (!ok || !colib::launch_bf16_to_f32((const __nv_bfloat16 *)ctx->buf[4], (float *)ctx->buf[0], xb, st)) return fail();
   } else {
     colib::FfnParams fp;
     fp.fmt = kfmt;
@@ -1319,7 +1324,7 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
     fp.y32 = (float *)ctx->buf[0];  // x f32 is dead once converted
     fp.relu2_out = nullptr;
     fp.act = current_activation();
-    if (!colib::launch_ffn_small(fp, st)) return 0;
+    if (!colib::launch_ffn_small(fp, st)) return fail();
   }
   CK(cudaEventRecord(ctx->ev[2], st), "phase event");
   int32_t kst = 0;

@@ -903,7 +903,15 @@ __global__ void __launch_bounds__(256) k_permute(PermuteParams p) {
     const int vec = p.H / 8;
     const uint4 *src = reinterpret_cast<const uint4 *>(p.x + (size_t)trow * p.H);
     uint4 *dst = reinterpret_cast<uint4 *>(p.xg + (size_t)pos * p.H);
-    for (int c = lane; c < vec; c += 32) dst[c] = coli_bf16x8_to_f16x8(src[c]);
+    int c = lane;
+    for (; c + 96 < vec; c += 128) {  // four loads in flight per lane
+      uint4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = src[c + 32 * u];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) dst[c + 32 * u] = coli_bf16x8_to_f16x8(v[u]);
+    }
+    for (; c < vec; c += 32) dst[c] = coli_bf16x8_to_f16x8(src[c]);
   }
 }
 

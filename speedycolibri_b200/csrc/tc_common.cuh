@@ -1,5 +1,5 @@
 // Pieces of the tcgen05 expert kernel: PTX wrappers (mbarrier, TMA, tcgen05), bounded waits,
-// UMMA descriptors, the NVFP4 -> f16 conversion, and the host-side tensor map for token rows.
+// UMMA descriptors, the epilogue's stores, and the host-side tensor map for token rows.
 #pragma once
 #include <cuda.h>
 
@@ -26,15 +26,6 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
 }
 // try_wait with a suspend-time hint: the thread stays suspended in hardware (taking no issue slots)
 // until the phase completes or about `ns` nanoseconds have passed
@@ -75,7 +66,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   atomicCAS(status, TC_OK, code);
   return false;
 }
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
@@ -84,13 +74,7 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
       ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// the same with A in tensor memory
+// D += A . B^T with A in tensor memory and B in shared memory; issued by one lane
 __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
@@ -135,36 +119,6 @@ __device__ __forceinline__ uint32_t tc_hmul2(uint32_t a, uint32_t b) {
   asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
-// One NVFP4 word (8 consecutive k, two per byte, low nibble first) -> 8 f16 (four f16x2, k
-// ascending) times the block scale held in both halves of `mult`.
-__device__ __forceinline__ uint4 tc_dequant_word(uint32_t w, uint32_t mult) {
-  uint4 o;
-  asm("{ .reg .b8 b0, b1, b2, b3;\n"
-      "  mov.b32 {b0, b1, b2, b3}, %4;\n"
-      "  cvt.rn.f16x2.e2m1x2 %0, b0;\n"
-      "  cvt.rn.f16x2.e2m1x2 %1, b1;\n"
-      "  cvt.rn.f16x2.e2m1x2 %2, b2;\n"
-      "  cvt.rn.f16x2.e2m1x2 %3, b3; }\n"
-      : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w)
-      : "r"(w));
-  o.x = tc_hmul2(o.x, mult);
-  o.y = tc_hmul2(o.y, mult);
-  o.z = tc_hmul2(o.z, mult);
-  o.w = tc_hmul2(o.w, mult);
-  return o;
-}
-// two ue4m3 block scales (low 16 bits of sc) -> each as f16 in both halves of a word
-__device__ __forceinline__ void tc_scales(uint32_t sc, uint32_t &m0, uint32_t &m1) {
-  uint32_t v;
-  asm("{ .reg .b16 h0, h1;\n"
-      "  mov.b32 {h0, h1}, %1;\n"
-      "  cvt.rn.f16x2.e4m3x2 %0, h0; }\n"
-      : "=r"(v)
-      : "r"(sc));
-  m0 = __byte_perm(v, v, 0x1010);
-  m1 = __byte_perm(v, v, 0x3232);
-}
-
 // ---- epilogue stores ------------------------------------------------------------------------------------
 // An epilogue lane owns ONE feature (its TMEM lane) and 16 token columns of it, while the result
 // matrices are token-major: written lane by lane, every value is a 2-byte store of its own, and
