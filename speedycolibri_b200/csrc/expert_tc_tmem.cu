@@ -22,7 +22,7 @@
 // Why: with both operands in shared memory an MMA of 128 x 128 x 16 fetches 8 KB per 64 cycles,
 // the whole shared-memory bandwidth of an SM, before a single decoded weight is stored there; a kernel
 // of that form with tiles of 256 tokens was kept for long segments until this one passed it (16384
-// tokens with skewed experts, H 6144, I 2048: 6092 + 3241 us against 5205 + 2704).  Here shared memory
+// tokens with skewed experts, H 6144, I 2048: 6092 + 3241 us against 4990 + 2570).  Here shared memory
 // carries the token tiles (16-20 KB written + twice that read per stage) and the packed weights (9 or
 // 16 KB each way).
 // TMEM budget: 2 x 160 accumulator columns + 6 x 32 weight columns = 512, which is why this
@@ -35,10 +35,11 @@
 // tiles hide.  With one branch on the lane index per thread of issue, a wait and a commit per stage and
 // accumulator, a stage took 830 cycles whatever its tokens (256 of MMA at 64); with weights loaded into
 // the producers' registers it stayed there, and with bulk copies in place of cp.async at 728 (the copy
-// engine).  Gate+up and down, before and now: 709 tokens on H 7168, I 2048, 256 experts 1461 + 771 us
-// -> 1100 + 573 (4.2 GB of weights: 650 + 325 at the copy rate); 4096 tokens 2153 + 1170 -> 2020 + 1047
-// (1320 + 660 at the tensor rate); FP8, 512 tokens, H 2048, I 768, 128 experts 130 + 77 -> 97 + 57;
-// NVFP4, 1024 tokens on the same sizes 123 + 71 -> 97 + 56.
+// engine).  Then the producers' instructions: 2700 per k-tile,
+// 1100 of them conversions; slot and phase are counters and a wait is a test and a vote since.  Gate+up and down, before and now: 709 tokens
+// on H 7168, I 2048, 256 experts 1461 + 771 us -> 1035 + 535 (4.2 GB of weights: 650 + 325 at the copy
+// rate); 4096 tokens 2153 + 1170 -> 1900 + 1000 (1320 + 660 at the tensor rate); FP8, 512 tokens, H 2048,
+// I 768, 128 experts 130 + 77 -> 92 + 56; NVFP4, 1024 tokens on the same sizes 123 + 71 -> 99 + 56.
 //
 // Roles are warp-specialised and synchronise through mbarriers only; the kernel is persistent.
 // Every barrier wait is bounded: on a time-out the CTA raises a status word, stops issuing work,

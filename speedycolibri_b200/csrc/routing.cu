@@ -219,9 +219,10 @@ __global__ void __launch_bounds__(C::NT) k_router_pair(RouteParams p) {
 // the issue slots otherwise: for 8 k a thread issues 8 TM TN FMAs, 8 (TM + TN) operations that widen
 // bf16 to f32 (at half the FMA rate) and TM + TN shared loads.  A small tile spreads few outputs over
 // all SMs, a large one spends fewer slots per FMA: pick_router_tile weighs the two.
-// Measured with the top-k behind it, against a kernel of 16 to 128 tokens x 64 experts per CTA: 48 tokens x 128 experts x 2048 63.8 -> 19.7 us, 24 x 256 x 7168 202 -> 47, 512 x 128 x 2048
-// 65 -> 30, 709 x 256 x 7168 320 -> 151, 2048 x 256 x 7168 320 -> 277.  Staging the operands as f32 by
-// warps of their own was built and is slower from 200 tokens on (shared-memory reads).
+// Measured with the top-k behind it, against a kernel of 16 to 128 tokens x 64 experts per CTA: 48 tokens x
+// 128 experts x 2048 64 -> 15 us, 24 x 256 x 7168 202 -> 33, 512 x 128 x 2048 65 -> 25, 709 x 256 x 7168
+// 320 -> 135, 2048 x 256 x 7168 320 -> 264.  (The top-k's own mending is 5 to 12 us of each.)  Staging the
+// operands as f32 by warps of their own was built and is slower from 200 tokens on (shared-memory reads).
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16u : 0u) : "memory");
 }
