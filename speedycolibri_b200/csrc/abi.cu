@@ -589,6 +589,9 @@ extern "C" int coli_b200_moe_create(ColiMoe **out, const ColiMoeLayer *L, int ma
         }
     }
   }
+  m->segs_in_expert_order = true;
+  for (int e = 0; e < E; ++e)
+    if (m->h_seg_expert[e] != e) m->segs_in_expert_order = false;
   // weight tables
   std::vector<WeightRef> tg(E + 1), tu(E + 1), td(E + 1);
   auto ref = [&](ColiCudaTensor *t, int wantI, int wantO, WeightRef &r, const char *name, int e) -> bool {
@@ -797,6 +800,9 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
   const bool tc = use_tc_path(m->L.fmt, rows, m->nseg, m->L.I) && m->xg != nullptr;
   const int rpi = tc ? tct_tile_tokens(rows, m->nseg) : rows_per_item_for(m->L, rows, m->nseg);
   const int max_items = max_work_items(rows, m->nseg, rpi);
+  // Segments are in (owner, expert id) order, also when every expert is resident: only where that is the
+  // expert order do the kernels index the weight tables by segment and save the dependent load.
+  const int32_t *seg_expert = m->segs_in_expert_order ? nullptr : m->seg_expert;
   const bool prof = m->profiling;
 #define COLI_MARK(i)                                                         \
   do {                                                                       \
@@ -824,7 +830,7 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
     tp.gate = m->gate;
     tp.up = m->up;
     tp.down = m->down;
-    tp.seg_expert = nullptr;  // every expert is resident: segment order is expert order, the shared expert last
+    tp.seg_expert = seg_expert;
     tp.item_seg = m->item_seg;
     tp.item_row0 = m->item_row0;
     tp.item_nrows = m->item_nrows;
@@ -846,7 +852,7 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
     fp.gate = m->gate;
     fp.up = m->up;
     fp.down = m->down;
-    fp.seg_expert = nullptr;  // every expert is resident: segment order is expert order, the shared expert last
+    fp.seg_expert = seg_expert;
     fp.item_seg = m->item_seg;
     fp.item_row0 = m->item_row0;
     fp.item_nrows = m->item_nrows;

@@ -42,6 +42,7 @@ struct ColiMoe {
   bool all_resident;
   std::vector<int32_t> h_expert_slot;  // expert -> segment position in (owner, id) order
   std::vector<int32_t> h_seg_expert;   // segment position -> weight-table index
+  bool segs_in_expert_order;           // h_seg_expert is the identity (one rank, or owners that ascend)
   std::vector<int32_t> h_owner;        // expert -> owning rank
   int first_local_seg, n_local_seg;
   // device tables
