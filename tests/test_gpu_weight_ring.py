@@ -48,3 +48,26 @@ def test_six_rows_per_segment_on_a_layer_of_many_tiles(gpu_backend, orc):
         want = L.expert_ffn(e, x[part])
         err = np.linalg.norm(y[part] - want, axis=1) / np.linalg.norm(want, axis=1)
         assert err.max() <= 5e-3, (e, err.max())
+
+
+@pytest.mark.parametrize("fmt", [FMT_NVFP4, FMT_FP8_B128, FMT_E4M3_ROW], ids=["nvfp4", "fp8_b128", "e4m3_row"])
+def test_rows_past_the_end_of_a_tile_do_not_reach_the_results(gpu_backend, orc, fmt):
+    """A partial weight tile leaves in the ring what the slot held before.  Every other expert of the group is
+    all NaN, and a CTA's second tile is another expert's, one tile further: 3 tiles an expert, 240 in all."""
+    rows_each, pairs = 9, 40
+    shape = MoeShape("past_the_end", H=264, E=2, k=1, I=304, T=4, fmt=fmt, shared=False)
+    L, packed = host_layer(shape)
+    codes_or_scales = 1 if fmt == FMT_NVFP4 else 0
+    for matrix in packed["experts"][0]:
+        matrix[codes_or_scales][...] = 0x7F  # the NaN of e4m3
+    nan, good = upload_layer(shape, packed).experts
+    es = [nan, good] * pairs
+    rng = np.random.default_rng(3)
+    x = synth.bf16_bits_to_f32(synth.f32_to_bf16_bits(rng.standard_normal((2 * pairs * rows_each, shape.H)).astype(np.float32)))
+    y = gpu_backend.expert_group([e.gate for e in es], [e.up for e in es], [e.down for e in es], [rows_each] * len(es), x)
+    y, x = (a.reshape(pairs, 2, rows_each, shape.H) for a in (y, x))
+    assert np.isnan(y[:, 0]).all()
+    want = L.expert_ffn(1, x[:, 1].reshape(-1, shape.H))
+    got = y[:, 1].reshape(-1, shape.H)
+    err = np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)
+    assert err.max() <= 5e-3, err.max()  # the bound of the test above
