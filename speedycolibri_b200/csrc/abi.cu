@@ -505,11 +505,14 @@ int coli_tct_tile_tokens(int rows, int nseg) {
 // rows, as long as the tcgen05 kernel's tiles (128 features of an expert) divide well over the SMs.
 // Measured (register-level / tcgen05, us a call): H 7168, I 2048, 256 experts at 4.5 rows 1443 / 1452,
 // 7.0 2300 / 1496; H 2048, I 768, 128 experts at 6.7 136 / 147, 8.0 150 / 148, FP8 6.7 167 / 179, 8.0
-// 182 / 180.  A pure function of shapes, so that kernel selection never depends on data or addresses.
+// 182 / 180.  FP8 128x128 stays at 8 rows: the register-level kernel applies its scales in f32, the
+// tcgen05 kernel as f16 multipliers (error against 64 bits 2.864e-3 and 2.896e-3 at 7.5 rows, H 2048,
+// I 1024, 256 experts).  A pure function of shapes, so that kernel selection never depends on data or
+// addresses.
 static bool tc_format(int fmt) { return fmt == COLI_FMT_NVFP4 || fmt == COLI_FMT_FP8_B128 || fmt == COLI_FMT_E4M3_ROW; }
 bool coli_use_tc_path(int fmt, int rows, int nseg, int I) {
   if (!tc_format(fmt) || nseg <= 0) return false;
-  const bool many_tiles = (long)nseg * ((I + 127) / 128) >= 148L * 12;
+  const bool many_tiles = fmt != COLI_FMT_FP8_B128 && (long)nseg * ((I + 127) / 128) >= 148L * 12;
   return (long)rows >= (many_tiles ? 6L : 8L) * nseg;
 }
 
