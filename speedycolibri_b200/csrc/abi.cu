@@ -1218,6 +1218,17 @@ extern "C" void coli_cuda_group_stats(uint64_t *calls, uint64_t *experts, uint64
   if (d2h_ms) *d2h_ms = g_group_d2h_ms;
 }
 
+namespace {
+struct StreamWait {
+  cudaStream_t st;
+  bool pending = true;
+  explicit StreamWait(cudaStream_t s) : st(s) {}
+  ~StreamWait() {
+    if (pending) cudaStreamSynchronize(st);
+  }
+};
+}  // namespace
+
 static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups, ColiCudaTensor *const *downs,
                           const int *rows, int count, float *y, const float *x, int want_fmt_a, int want_fmt_b,
                           const char *who) {
@@ -1277,20 +1288,18 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
   int32_t *d_inr = d_irow + max_items;
   int32_t *d_nit = d_inr + max_items;
   int32_t *d_status = d_nit + 1;
+  int32_t kst = 0;
+  // Whatever fails below, the call waits for its stream before it returns: copies may be reading x, rows and
+  // tbl, or writing y and kst.  (A wait between the copies and the kernels as well took 10 us a call.)
+  StreamWait wait(st);
   CK(cudaEventRecord(ctx->ev[0], st), "phase event");
   CK(cudaMemcpyAsync(ctx->buf[0], x, xb * sizeof(float), cudaMemcpyHostToDevice, st), "expert input upload");
   CK(cudaMemcpyAsync(d_tbl, tbl.data(), sizeof(WeightRef) * tbl.size(), cudaMemcpyHostToDevice, st), "expert table upload");
   CK(cudaMemcpyAsync(d_cnt, rows, sizeof(int32_t) * count, cudaMemcpyHostToDevice, st), "row count upload");
   CK(cudaMemsetAsync(d_status, 0, sizeof(int32_t), st), "status clear");
   CK(cudaEventRecord(ctx->ev[1], st), "phase event");
-  // The call waits for the stream before it returns, on every path: the copies above may still be reading
-  // tbl, rows and x.  (Waiting here as well put 10 us between the copies and the kernels.)
-  const auto fail = [&]() {
-    cudaStreamSynchronize(st);
-    return 0;
-  };
-  if (!colib::launch_f32_to_f16((const float *)ctx->buf[0], (__half *)ctx->buf[1], xb, st)) return fail();
-  if (!colib::launch_items_from_counts(d_cnt, count, rpi, d_off, d_iseg, d_irow, d_inr, d_nit, st)) return fail();
+  if (!colib::launch_f32_to_f16((const float *)ctx->buf[0], (__half *)ctx->buf[1], xb, st)) return 0;
+  if (!colib::launch_items_from_counts(d_cnt, count, rpi, d_off, d_iseg, d_irow, d_inr, d_nit, st)) return 0;
   if (tc) {
     colib::TcParams tp;
     tp.fmt = kfmt;
@@ -1312,7 +1321,7 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
     tp.act = current_activation();
     const int sms = ctx->sm_count;
     const int ok = colib::launch_gate_up_tct(tp, ctx->buf[1], (int)total, sms, st) && colib::launch_down_tct(tp, (int)total, sms, st);
-    if (!ok || !colib::launch_bf16_to_f32((const __nv_bfloat16 *)ctx->buf[4], (float *)ctx->buf[0], xb, st)) return fail();
+    if (!ok || !colib::launch_bf16_to_f32((const __nv_bfloat16 *)ctx->buf[4], (float *)ctx->buf[0], xb, st)) return 0;
   } else {
     colib::FfnParams fp;
     fp.fmt = kfmt;
@@ -1336,14 +1345,14 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
     fp.y32 = (float *)ctx->buf[0];  // x f32 is dead once converted
     fp.relu2_out = nullptr;
     fp.act = current_activation();
-    if (!colib::launch_ffn_small(fp, st)) return fail();
+    if (!colib::launch_ffn_small(fp, st)) return 0;
   }
   CK(cudaEventRecord(ctx->ev[2], st), "phase event");
-  int32_t kst = 0;
   CK(cudaMemcpyAsync(y, ctx->buf[0], xb * sizeof(float), cudaMemcpyDeviceToHost, st), "expert output download");
   if (tc) CK(cudaMemcpyAsync(&kst, d_status, sizeof(int32_t), cudaMemcpyDeviceToHost, st), "status read");
   CK(cudaEventRecord(ctx->ev[3], st), "phase event");
   CK(cudaStreamSynchronize(st), "expert call sync");
+  wait.pending = false;
   if (kst != 0) {
     coli_set_error("%s: a tcgen05 expert kernel abandoned a bounded wait (code %d); the output is invalid", who, (int)kst);
     return 0;
