@@ -228,12 +228,14 @@ size_t coli_b200_moe_workspace_bytes(const ColiMoe *moe);
 int coli_b200_moe_block(ColiMoe *moe, const void *x, void *out, int T, int32_t *topk_idx, float *topk_w);
 /* Same with DEVICE pointers, asynchronous on `stream` (a cudaStream_t; NULL is CUDA's default
  * stream, coli_b200_moe_stream() gives the handle's own).  One handle's workspace serves one
- * call at a time: calls on different streams must not overlap. */
+ * call at a time: calls on different streams must not overlap.  x_dev and out_dev must be 16-byte
+ * aligned; other pointers are refused. */
 int coli_b200_moe_block_dev(ColiMoe *moe, const void *x_dev, void *out_dev, int T, void *stream);
 /* The layer step around the block (forward.rs:376-393), all on device pointers and asynchronous
  * on `stream`: x = bf16(rmsnorm(resid, post_ln_w, eps)) (math.rs:8-20, mean square in f64), then
  * resid += moe_block(x), the add fused into the combine so the block output is not rounded first.
- * resid_dev: f32 [T,H], updated in place; post_ln_w_dev: f32 [H].  H must be a multiple of 8.
+ * resid_dev: f32 [T,H], updated in place; post_ln_w_dev: f32 [H]; both 16-byte aligned (others are
+ * refused).  H must be a multiple of 8.
  * No reference C symbol corresponds to it: the reference runs these steps on the host. */
 int coli_b200_moe_layer_step_dev(ColiMoe *moe, float *resid_dev, const float *post_ln_w_dev, float eps, int T, void *stream);
 /* Synchronise the device and return 1 if every kernel launched through this handle since the
@@ -259,7 +261,8 @@ int coli_b200_moe_topk_dev(ColiMoe *moe, const void *x_dev, int T, int32_t *topk
  * expert is resident here into rows_dev (2 bytes per element, capacity T*k rows; the encoding is
  * the library's own -- the bf16 values held as f16 -- and only experts_dev reads it), expert-contiguous in ascending
  * expert id, tokens ascending inside an expert (moe.rs:1373-1387).  seg_count_dev[n_local]
- * receives the rows per resident expert, slot_dev[T*k] the row of each pair or -1. */
+ * receives the rows per resident expert, slot_dev[T*k] the row of each pair or -1.  x_dev and rows_dev
+ * must be 16-byte aligned; other pointers are refused. */
 int coli_b200_moe_gather_local_dev(ColiMoe *moe, const void *x_dev, const int32_t *topk_idx_dev, int T, void *rows_dev,
                                    int32_t *seg_count_dev, int32_t *slot_dev, void *stream);
 /* Grouped SwiGLU FFN of the resident experts over those rows -> y_dev (bf16 [rows, H]); the

@@ -727,6 +727,13 @@ bool coli_check_T(ColiMoe *m, int T, const char *who) {
   return select_ctx(m->ctx);
 }
 
+// Rows are read and written 16 bytes at a time.
+static bool rows_aligned(const void *a, const void *b, const char *who, const char *names) {
+  if (!((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15)) return true;
+  coli_set_error("%s: %s must be 16-byte aligned", who, names);
+  return false;
+}
+
 static colib::RouteParams route_params(ColiMoe *m, const void *x_dev, int T) { return coli_route_params(m, x_dev, T); }
 colib::RouteParams coli_route_params(ColiMoe *m, const void *x_dev, int T) {
   colib::RouteParams rp;
@@ -798,6 +805,7 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
     return 0;
   }
   if (T == 0) return 1;
+  if (!rows_aligned(x_dev, out_dev, "moe_block_dev", "x_dev and out_dev")) return 0;
   cudaStream_t st = pick_stream(m, stream);
   const int k = m->L.k;
   const int rows = T * k + (m->has_shared ? T : 0);
@@ -927,6 +935,7 @@ extern "C" int coli_b200_moe_layer_step_dev(ColiMoe *m, float *resid_dev, const 
     return 0;
   }
   if (T == 0) return 1;
+  if (!rows_aligned(resid_dev, post_ln_w_dev, "moe_layer_step_dev", "resid_dev and post_ln_w_dev")) return 0;
   cudaStream_t st = pick_stream(m, stream);
   if (!colib::launch_rmsnorm_bf16(resid_dev, post_ln_w_dev, eps, m->x_stage, T, m->L.H, st)) return 0;
   return moe_block_impl(m, m->x_stage, nullptr, resid_dev, T, stream);
@@ -1012,6 +1021,7 @@ extern "C" int coli_b200_moe_gather_local_dev(ColiMoe *m, const void *x_dev, con
   }
   cudaStream_t st = pick_stream(m, stream);
   if (T == 0) return coli_cuda_check(cudaMemsetAsync(seg_count_dev, 0, sizeof(int32_t) * m->n_local_seg, st), "count clear") ? 1 : 0;
+  if (!rows_aligned(x_dev, rows_dev, "moe_gather_local_dev", "x_dev and rows_dev")) return 0;
   colib::PermuteParams pp = permute_params(m, x_dev, T, false, colib::TCT_MAX_TOKENS, rows_dev, seg_count_dev, slot_dev);
   pp.topk_idx = topk_idx_dev;
   pp.expert_slot = m->local_slot;

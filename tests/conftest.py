@@ -33,3 +33,11 @@ def gpu_backend():
 
     backend.init([0])
     return backend
+
+
+@pytest.fixture(scope="session")
+def fake_cuda(tmp_path_factory):
+    """The library's host side over a fake of the CUDA runtime (tests/fake_cuda.py)."""
+    from tests.fake_cuda import load
+
+    return load(tmp_path_factory.mktemp("fake_cuda"))

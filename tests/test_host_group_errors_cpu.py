@@ -1,92 +1,31 @@
-"""The host expert call when one of its CUDA calls fails: abi.cu linked against a fake of the CUDA runtime
-and of the kernel launchers.  Copies from or to the caller's buffers and the call's own tables may be queued
-when a later call fails, so on every path the last thing the call does to its stream is to wait for it."""
+"""The host expert call when one of its CUDA calls fails.  Copies from or to the caller's buffers and the
+call's own tables may be queued by then, so on every path the last thing the call does to its stream is to
+wait for it."""
 import ctypes as C
-import os
-import shutil
-import subprocess
 
 import numpy as np
 import pytest
 
-from speedycolibri_b200 import _lib
-
-# What a case needs from the runtime: handles and memory that look real, a log of the calls that put work on
-# a stream, and the n-th of them refused.
-SHIM = r"""
-#include <driver_types.h>
-#include <stdlib.h>
-#include <string.h>
-static int log_n, fail_at;
-static char last;
-void fake_reset(int fail) { log_n = 0; fail_at = fail; last = 0; }
-int fake_queued(void) { return log_n; }
-int fake_waited(void) { return last == 'w'; }
-static int queue(void) { if (++log_n == fail_at) return 1; last = 'q'; return 0; }
-int cudaMalloc(void **p, size_t n) { *p = malloc(n ? n : 1); return 0; }
-int cudaFree(void *p) { free(p); return 0; }
-int cudaGetDeviceCount(int *n) { *n = 1; return 0; }
-int cudaDeviceGetAttribute(int *v) { *v = 148; return 0; }
-int cudaGetDeviceProperties_v2(struct cudaDeviceProp *p) {
-  memset(p, 0, sizeof(*p));
-  p->major = 10;
-  p->multiProcessorCount = 148;
-  return 0;
-}
-int cudaStreamCreateWithFlags(void **s) { *s = malloc(1); return 0; }
-int cudaEventCreate(void **e) { *e = malloc(1); return 0; }
-const char *cudaGetErrorString(int e) { (void)e; return "refused by the test"; }
-int cudaMemcpyAsync(void) { return queue(); }
-int cudaMemsetAsync(void) { return queue(); }
-int cudaEventRecord(void) { return queue(); }
-int cudaStreamSynchronize(void) { last = 'w'; return 0; }
-"""
-
-
-@pytest.fixture(scope="module")
-def fake(tmp_path_factory):
-    """libcoli_b200's host side over the fake: launchers and whatever else it links to return 1 or 0 at once."""
-    d = tmp_path_factory.mktemp("fake_cuda")
-    obj, shim, lib = str(d / "abi.o"), str(d / "shim.c"), str(d / "libfake.so")
-    flags = [f for f in _lib.NVCC_FLAGS if f != "-shared"]
-    subprocess.run(["nvcc", *flags, "-c", "-o", obj, "abi.cu"], cwd=_lib._CSRC, check=True, capture_output=True)
-    undefined = [line.split()[-1] for line in subprocess.run(["nm", "-u", obj], check=True, capture_output=True, text=True).stdout.splitlines()]
-    src = SHIM
-    for s in undefined:
-        if s.startswith("_ZN5colib"):
-            src += f"int {s}(void) {{ return !queue(); }}\n"  # a launcher answers 1 on success
-        elif (s.startswith(("cuda", "__cuda")) or "coli_ep_" in s) and f" {s}(" not in src and f"*{s}(" not in src:
-            src += f"int {s}(void) {{ return 0; }}\n"
-    cuda_include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(shutil.which("nvcc")))), "include")
-    open(shim, "w").write(src)
-    subprocess.run(["gcc", "-w", "-fPIC", "-I", cuda_include, "-c", "-o", shim + ".o", shim], check=True)
-    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-Wl,-z,defs", "-o", lib, obj, shim + ".o", "-lpthread"], check=True)
-    fake = C.CDLL(lib, mode=os.RTLD_LOCAL)
-    assert fake.coli_cuda_init((C.c_int * 1)(0), 1)
-    return fake
+from tests.fake_cuda import wrap_nvfp4
 
 
 @pytest.mark.parametrize("rows", [3, 40], ids=["register_level", "tcgen05"])
-def test_a_host_group_call_that_fails_leaves_nothing_in_flight(fake, rows):
+def test_a_host_group_call_that_fails_leaves_nothing_in_flight(fake_cuda, rows):
     H, I, count = 32, 16, 2
     tensors = [(C.c_void_p * count)() for _ in range(3)]
     for which, (o, i) in enumerate([(I, H), (I, H), (H, I)]):
         for c in range(count):
-            h = C.c_void_p()
-            q, s = np.zeros((o, i // 2), np.uint8), np.zeros((o, (i + 15) // 16), np.uint8)
-            fake.fake_reset(0)
-            assert fake.coli_cuda_tensor_wrap_nvfp4(C.byref(h), q.ctypes.data_as(C.c_void_p), s.ctypes.data_as(C.c_void_p), C.c_float(1.0), i, o, 0)
-            tensors[which][c] = h
+            tensors[which][c] = wrap_nvfp4(fake_cuda, o, i)
     n_rows = (C.c_int * count)(rows, rows)
     x, y = np.zeros((count * rows, H), np.float32), np.zeros((count * rows, H), np.float32)
 
     def call(fail_at):
-        fake.fake_reset(fail_at)
-        return fake.coli_cuda_expert_group_nvfp4(*tensors, n_rows, count, y.ctypes.data_as(C.c_void_p), x.ctypes.data_as(C.c_void_p))
+        fake_cuda.fake_reset(fail_at)
+        return fake_cuda.coli_cuda_expert_group_nvfp4(*tensors, n_rows, count, y.ctypes.data_as(C.c_void_p), x.ctypes.data_as(C.c_void_p))
 
-    assert call(0) == 1 and fake.fake_waited()
-    steps = fake.fake_queued()
+    assert call(0) == 1 and fake_cuda.fake_waited()
+    steps = fake_cuda.fake_queued()
     assert steps >= 10  # four events, three or more copies, three or more launches
     for n in range(1, steps + 1):
         assert call(n) == 0, n
-        assert n == 1 or fake.fake_waited(), f"call {n} of {steps} on the stream failed and the call did not wait for those before it"
+        assert n == 1 or fake_cuda.fake_waited(), f"call {n} of {steps} on the stream failed and the call did not wait for those before it"
