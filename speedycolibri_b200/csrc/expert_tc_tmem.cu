@@ -48,22 +48,6 @@
 
 #include "tc_common.cuh"
 
-#ifdef COLI_TT_TRACE
-// Measurement aid (never compiled into the library as shipped): clock stamps of CTA 0's first stages.
-__device__ long long g_tt_trace[256 * 8];
-extern "C" int coli_debug_tt_trace(long long *host) {
-  return cudaMemcpyFromSymbol(host, g_tt_trace, sizeof(g_tt_trace)) == cudaSuccess ? 1 : 0;
-}
-#define TT_TRACE(it, k)                                                                 \
-  do {                                                                                  \
-    if (GATED && blockIdx.x == 0 && (it) < 256u) g_tt_trace[(it) * 8 + (k)] = clock64(); \
-  } while (0)
-#else
-#define TT_TRACE(it, k) \
-  do {                  \
-  } while (0)
-#endif
-
 namespace colib {
 
 // TMEM budget (512 columns): two accumulators of ACC columns (= the most token rows of a tile) and a
@@ -135,18 +119,13 @@ struct TtPacked {
   uint4 q0, q1;
   uint32_t sc;
 };
-__device__ __forceinline__ uint4 tt_lds128(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-  return v;
-}
 // `codes` = address of the row's chunk 0 (chunks are permuted by XOR, so chunk j is at codes ^ 16 j),
 // `scales` = address of its scale bytes; `half` = which 64 of the k-tile's 128 k.
 __device__ __forceinline__ TtPacked tt_read_packed(uint32_t codes, uint32_t scales, int half) {
   TtPacked r;
   const uint32_t a = codes ^ (uint32_t)(half << 5);
-  r.q0 = tt_lds128(a);
-  r.q1 = tt_lds128(a ^ 16u);
+  r.q0 = lds128(a);
+  r.q1 = lds128(a ^ 16u);
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r.sc) : "r"(scales + half * 4) : "memory");
   return r;
 }
@@ -199,7 +178,7 @@ __device__ __forceinline__ uint32_t tt_f16x2_both(float v) {
 __device__ __forceinline__ TtPacked8 tt_read_packed8(uint32_t codes, int half, uint32_t mult) {
   TtPacked8 r;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) r.q[j] = tt_lds128(codes ^ (uint32_t)((half << 6) | (j << 4)));
+  for (int j = 0; j < 4; ++j) r.q[j] = lds128(codes ^ (uint32_t)((half << 6) | (j << 4)));
   r.mult = mult;
   return r;
 }
@@ -240,15 +219,12 @@ struct TtWeightRing {
   static constexpr int SLOTS = FMT == COLI_FMT_NVFP4 ? (ACC <= 64 ? 9 : 5) : (ACC <= 64 ? 5 : 3);
   static constexpr int BYTES = SLOT * SLOTS;
 };
-__device__ __forceinline__ void tt_cp_async16(uint32_t dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
 
 // Whole-warp wait: the common case, a phase that has completed, costs a test and a vote.  (Kept inline:
 // with the rest behind a call the producers' registers no longer fit and 160-row tiles lost 8 %.)
 __device__ __forceinline__ bool tt_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status, int code) {
   return __all_sync(0xffffffffu, mbar_test_wait(bar, parity)) ||
-         __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code, 1));
+         __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code));
 }
 
 // GATED: the two weight tiles of a stage are gate and up of the same 128 features, result
@@ -317,11 +293,10 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
         const CUtensorMap *tmap = &maps.m[N / TC_BOXN - 1];  // the map whose box is N rows
         for (int kb = 0; kb < KB; ++kb, ++it) {
           const uint32_t s = it % TT_B_STAGES, ph = (it / TT_B_STAGES) & 1u;
-          if (!mbar_wait(empty_s + 8 * s, ph ^ 1u, abort_flag, p.status, TC_ERR_TMA_WAIT, 32)) {
+          if (!mbar_wait(empty_s + 8 * s, ph ^ 1u, abort_flag, p.status, TC_ERR_TMA_WAIT)) {
             alive = false;
             break;
           }
-          TT_TRACE(it, 6);
           const uint32_t dst = smem_u32(smem + s * TT_B_BYTES);
           const uint32_t full = full_s + 8 * (s & ~1u);  // (both rings of stages and k are even)
           if (!(kb & 1)) mbar_expect_tx(full, (uint32_t)N * TC_BK * 4);
@@ -376,10 +351,10 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
           for (int m = 0; m < 2; ++m) {
 #pragma unroll
             for (int i = 0; i < QI; ++i)
-              tt_cp_async16(dst + m * Ring::SLAB + i * TT_LOAD_THREADS * 16, qsrc[m] + i * TT_LOAD_THREADS * 16);
+              cp_async16(dst + m * Ring::SLAB + i * TT_LOAD_THREADS * 16, qsrc[m] + i * TT_LOAD_THREADS * 16);
 #pragma unroll
             for (int i = 0; i < SI; ++i)
-              tt_cp_async16(dst + m * Ring::SLAB + TC_BM * QB + i * TT_LOAD_THREADS * 16, ssrc[m] + i * TT_LOAD_THREADS * 16);
+              cp_async16(dst + m * Ring::SLAB + TC_BM * QB + i * TT_LOAD_THREADS * 16, ssrc[m] + i * TT_LOAD_THREADS * 16);
           }
         } else {
           // Rows past the end keep what the slot held before: a feature is a row of the accumulator of its
@@ -391,11 +366,11 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
           for (int m = 0; m < 2; ++m) {
 #pragma unroll
             for (int i = 0; i < QI; ++i)
-              if (i < qn[m]) tt_cp_async16(dst + m * Ring::SLAB + i * TT_LOAD_THREADS * 16, qsrc[m] + i * TT_LOAD_THREADS * 16);
+              if (i < qn[m]) cp_async16(dst + m * Ring::SLAB + i * TT_LOAD_THREADS * 16, qsrc[m] + i * TT_LOAD_THREADS * 16);
 #pragma unroll
             for (int i = 0; i < SI; ++i)
               if (i < sn[m])
-                tt_cp_async16(dst + m * Ring::SLAB + TC_BM * QB + i * TT_LOAD_THREADS * 16, ssrc[m] + i * TT_LOAD_THREADS * 16);
+                cp_async16(dst + m * Ring::SLAB + TC_BM * QB + i * TT_LOAD_THREADS * 16, ssrc[m] + i * TT_LOAD_THREADS * 16);
           }
         }
 #pragma unroll
@@ -437,10 +412,8 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
       if (!alive) break;
       tc_fence_after();
       for (int kb = 0; kb < KB; kb += 2) {
-        if (lane == 0) TT_TRACE(tix * KB + kb, 0);
         alive = tt_wait(full_s + 8 * sb, phb, abort_flag, p.status, TC_ERR_MMA_WAIT);
         if (!alive) break;
-        if (lane == 0) TT_TRACE(tix * KB + kb, 1);
         tc_fence_after();
         if (elect_one()) {
           // one copy of the code per ring position: every address is then a constant offset
@@ -459,7 +432,6 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
             issue(std::integral_constant<uint32_t, 2>());
         }
         __syncwarp();
-        if (lane == 0) TT_TRACE(tix * KB + kb, 2);
         if ((sb += 2) == TT_B_STAGES) {
           sb = 0;
           phb ^= 1u;
@@ -492,26 +464,16 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
         s1 = f1 < Oout ? __ldg(reinterpret_cast<const float *>(w1.s) + f1) : 0.0f;
       }
       bool ok = true;
-      if (lg == 0 && lane == 0) TT_TRACE(240 + tix, 0);
-      if (lane == 0) ok = mbar_wait(acc_full, tix & 1u, abort_flag, p.status, TC_ERR_EPI_WAIT, 256);
-      if (lg == 0 && lane == 0) TT_TRACE(240 + tix, 1);
+      if (lane == 0) ok = mbar_wait(acc_full, tix & 1u, abort_flag, p.status, TC_ERR_EPI_WAIT);
       ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
       if (!ok) break;
       tc_fence_after();
       const uint32_t tbase = tmem_base + ((uint32_t)(lg * 32) << 16);
       for (int c0 = 0; c0 < N; c0 += 16) {
         uint32_t g[16], u[16];
-#ifdef COLI_TT_TRACE
-        if (GATED && blockIdx.x == 0 && lg == 0 && lane == 0 && tix == 2) g_tt_trace[(200 + c0 / 16) * 8 + 0] = clock64();
-#endif
         tmem_ld16(tbase + c0, g);
         tmem_ld16(tbase + TT_ACC_COLS + c0, u);
         tmem_ld_wait();
-#ifdef COLI_TT_TRACE
-        if (GATED && blockIdx.x == 0 && lg == 0 && lane == 0 && tix == 2) g_tt_trace[(200 + c0 / 16) * 8 + 1] = clock64();
-        if (GATED && blockIdx.x == 0 && lg == 0 && lane == 0 && tix == 2)
-          g_tt_trace[(200 + c0 / 16) * 8 + 3] = clock64() + (long long)(g[0] == 0x12345u) + (long long)(u[15] == 0x12345u) + (long long)(g[7] == 0x12345u);
-#endif
         // all 16 columns are computed first, branch-free, so that their dependent chains (scale,
         // exponential, reciprocal, two roundings) overlap; a branch per column would run them one
         // after the other.  Columns beyond the item's rows hold other rows' sums and are not stored.
@@ -538,7 +500,6 @@ __global__ void __launch_bounds__(TT_THREADS, 1) k_ffn_tct(const __grid_constant
       }
       tc_fence_before();
       __syncwarp();
-      if (lg == 0 && lane == 0) TT_TRACE(240 + tix, 2);
       if (lane == 0) mbar_arrive(acc_empty);
     }
   } else {

@@ -297,6 +297,19 @@ static inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, 
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
+// 16 bytes, global -> shared memory, asynchronously (through L2 only); `valid` = false writes zeros instead
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16u : 0u) : "memory");
+}
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
 // bf16 pair (one 32-bit word) -> f16 pair, saturating at the largest finite f16
 __device__ __forceinline__ uint32_t coli_bf16x2_to_f16x2(uint32_t w) {
   const float lo = fminf(fmaxf(__uint_as_float(w << 16), -65504.0f), 65504.0f);

@@ -223,14 +223,6 @@ __global__ void __launch_bounds__(C::NT) k_router_pair(RouteParams p) {
 // 128 experts x 2048 64 -> 15 us, 24 x 256 x 7168 202 -> 33, 512 x 128 x 2048 65 -> 25, 709 x 256 x 7168
 // 320 -> 135, 2048 x 256 x 7168 320 -> 264.  (The top-k's own mending is 5 to 12 us of each.)  Staging the
 // operands as f32 by warps of their own was built and is slower from 200 tokens on (shared-memory reads).
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool valid) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16u : 0u) : "memory");
-}
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-  return v;
-}
 template <int TM_, int TN_, int WM_, int WN_, int BK_, int STAGES_>
 struct RouterTile {
   static constexpr int TM = TM_, TN = TN_, WM = WM_, WN = WN_, BK = BK_, STAGES = STAGES_;

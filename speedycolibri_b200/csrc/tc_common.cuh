@@ -12,7 +12,7 @@ constexpr int TC_BK = 64;    // k per pipeline stage: one 128-byte swizzle row o
 constexpr int TC_BOXN = 16;  // token rows of a tile are padded to a multiple of this (the granularity of the MMA's N)
 constexpr int TC_EPI_WARPS = 4;
 
-constexpr uint32_t TC_SPIN_LIMIT = 1u << 22;
+constexpr uint32_t TC_POLL_LIMIT = 1u << 18;  // suspended polls of a bounded wait: at most about 0.3 s
 
 enum { TC_OK = 0, TC_ERR_TMA_WAIT = 1, TC_ERR_MMA_WAIT = 2, TC_ERR_PROD_WAIT = 3, TC_ERR_EPI_WAIT = 4 };
 
@@ -47,19 +47,15 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait.  Returns false when the barrier did not flip in time or another role gave up.
-// sleep_ns = 0 polls with test_wait (never suspends); otherwise every poll is a try_wait that the
-// hardware suspends for up to max(sleep_ns, 1000) ns or until the phase completes.  A waiting warp
-// must not spin: the trace of the tensor-memory kernel showed twenty polling warps taking four
-// fifths of the issue slots from the one warp per scheduler that had work (the epilogue ran at a
-// tenth of an instruction per cycle, the MMA-issuing threads lost ~500 cycles per stage).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status, int code,
-                                          uint32_t sleep_ns = 0) {
+// Bounded wait.  Returns false when the barrier did not flip in time or another role gave up.  After the
+// first test every poll is a try_wait that the hardware suspends for about a microsecond or until the phase
+// completes.  A waiting warp must not spin: twenty polling warps took four fifths of the issue slots from the
+// one warp per scheduler that had work (the epilogue ran at a tenth of an instruction per cycle, the
+// MMA-issuing threads lost ~500 cycles per stage).
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status, int code) {
   if (mbar_test_wait(bar, parity)) return true;
-  const uint32_t hint = sleep_ns > 1000u ? sleep_ns : 1000u;
-  const uint32_t limit = sleep_ns ? (TC_SPIN_LIMIT >> 4) : TC_SPIN_LIMIT;  // at most ~0.3 s of suspended polls
-  for (uint32_t i = 0; i < limit; ++i) {
-    if (sleep_ns ? mbar_try_wait_hint(bar, parity, hint) : mbar_test_wait(bar, parity)) return true;
+  for (uint32_t i = 0; i < TC_POLL_LIMIT; ++i) {
+    if (mbar_try_wait_hint(bar, parity, 1000u)) return true;
     if ((i & 7u) == 7u && *abort_flag) return false;
   }
   *abort_flag = 1;
