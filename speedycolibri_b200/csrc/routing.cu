@@ -1027,14 +1027,14 @@ static int permute_max_items(const PermuteParams &p) {
 }
 
 int launch_decode_front(const RouteParams &rp, const PermuteParams &pp, unsigned int *ticket, cudaStream_t st) {
-  const size_t stage = RouterTiny::SMEM;
-  const size_t topk = (size_t)8 * topk_row_floats(rp.E) * sizeof(float);
-  const size_t smem = stage > topk ? stage : topk;
-  if (!(rp.T >= 1 && rp.T <= 8 && rp.H % 8 == 0 && smem <= 180 * 1024 && rp.E <= 32 * kMaxSlots && rp.k <= 32 &&
+  constexpr size_t smem = RouterTiny::SMEM;
+  static_assert((size_t)8 * 32 * kMaxSlots * sizeof(float) <= smem, "the top-k rows of eight warps reuse the staging area");
+  if (!(rp.T >= 1 && rp.T <= 8 && rp.H % 8 == 0 && rp.E <= 32 * kMaxSlots && rp.k <= 32 &&
         rp.n_group <= 32 && (rp.n_group <= 1 || rp.E % rp.n_group == 0) && permute_small_ok(pp) && ticket != nullptr))
     return -1;  // not applicable: the caller runs the separate stages
+  // (with the static lists of the permutation a CTA is above the 48 KB that need no attribute)
   static ColiPerDeviceOnce attr_once;
-  if (!coli_set_smem_limit(attr_once, k_decode_front, 180 * 1024, "decode front shared-memory attribute")) return 0;
+  if (!coli_set_smem_limit(attr_once, k_decode_front, smem, "decode front shared-memory attribute")) return 0;
   coli_count_launch(1);
   return coli_cuda_check(launch_dependent(k_decode_front, dim3((rp.E + 7) / 8), dim3(256), smem, st, rp, pp, permute_max_items(pp), ticket),
                          "decode front launch")
