@@ -512,7 +512,7 @@ int coli_tct_tile_tokens(int rows, int nseg) {
 static bool tc_format(int fmt) { return fmt == COLI_FMT_NVFP4 || fmt == COLI_FMT_FP8_B128 || fmt == COLI_FMT_E4M3_ROW; }
 bool coli_use_tc_path(int fmt, int rows, int nseg, int I) {
   if (!tc_format(fmt) || nseg <= 0) return false;
-  const bool many_tiles = fmt != COLI_FMT_FP8_B128 && (long)nseg * ((I + 127) / 128) >= 148L * 12;
+  const bool many_tiles = fmt != COLI_FMT_FP8_B128 && (long)nseg * ((I + 127) / 128) >= 12L * COLI_SMS;
   return (long)rows >= (many_tiles ? 6L : 8L) * nseg;
 }
 

@@ -397,7 +397,7 @@ static int launch_one(const FfnParams &p, bool gated, cudaStream_t st) {
   const int K = gated ? p.H : p.I, O = gated ? p.I : p.H;
   const int KT = (K + 127) / 128, row_tiles = (O + 15) / 16;
   const long tasks = (long)row_tiles * (p.items_expected > 0 ? p.items_expected : 1);
-  const bool splitk = tasks < 148L * 12;
+  const bool splitk = tasks < 12L * COLI_SMS;
   if (splitk) {
     const int W = pick_w(KT);
     dim3 grid(row_tiles, p.max_items);

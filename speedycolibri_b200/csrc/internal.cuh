@@ -62,6 +62,9 @@ __host__ __device__ static inline int coli_fp4_chunk(int row, int c) { return c 
 __host__ __device__ static inline int coli_fp8_chunk(int row, int c) { return c ^ (row & 7); }
 
 static inline int round_up(int a, int b) { return (a + b - 1) / b * b; }
+// SMs of a B200.  The rules that pick a kernel or a tile count with the constant and not with the device's own
+// figure, so that they are functions of shapes alone, the same on every rank.
+constexpr int COLI_SMS = 148;
 // Upper bound of the work items `rows` rows in at most `nseg` segments cut into: a segment of n
 // rows gives ceil(n / rpi) <= n / rpi + 1 items and at most min(nseg, rows) segments hold a row.
 // Kernel grids are sized from this bound, so a loose one costs idle CTAs on every decode step.

@@ -637,8 +637,8 @@ static bool launch_router_pair(const RouteParams &p, cudaStream_t st) {
 // The time of one k is a function of n, the CTAs of the fullest SM; the figures are nanoseconds measured
 // on B200 between 21 and 16384 tokens (5.3 and 10 are the chain's latency, with its loads and
 // conversions, when an SM has little else).
-static int pick_router_tile(const RouteParams &p) {
-  auto n = [&](int bm, int bn) { return (float)(((long)((p.T + bm - 1) / bm) * ((p.E + bn - 1) / bn) + 147) / 148); };
+static int pick_router_tile(int T, int E) {
+  auto n = [&](int bm, int bn) { return (float)(((long)((T + bm - 1) / bm) * ((E + bn - 1) / bn) + COLI_SMS - 1) / COLI_SMS); };
   const float ns[5] = {fmaxf(5.3f, 1.6f * n(8, 8)), fmaxf(10.0f, 3.0f + 5.6f * n(16, 32)), 3.0f + 33.0f * n(64, 64),
                        5.0f + 46.5f * n(128, 64), 8.0f + 81.0f * n(128, 128)};
   int best = 0;
@@ -665,7 +665,7 @@ int launch_router(const RouteParams &p, cudaStream_t st) {
   const bool rows16 = p.H % 8 == 0 && ((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.router_w)) & 15) == 0;
   if (rows16) {
     bool ok = false;
-    switch (pick_router_tile(p)) {
+    switch (pick_router_tile(p.T, p.E)) {
       case 0: ok = launch_router_chain<RouterTile8x8>(p, st); break;
       case 1: ok = launch_router_chain<RouterTile16x32>(p, st); break;
       case 2: ok = launch_router_chain<RouterTile64x64>(p, st); break;
