@@ -360,6 +360,10 @@ int coli_b200_moe_phase_ms(ColiMoe *moe, float *ms /* [COLI_PHASES] */, int *cal
 void *coli_b200_moe_stream(ColiMoe *moe);
 /* Kernels this library has launched in the calling process since it was loaded. */
 uint64_t coli_b200_launch_count(void);
+/* Which tile (tokens x experts) of the batched router GEMM a batch takes: 0 = 8 x 8, 1 = 16 x 32, 2 = 64 x 64,
+ * 3 = 128 x 64, 4 = 128 x 128; -1 for T < 1 or E < 1.  Needs no device.  (Batches of up to 8 tokens of the block
+ * take the fused decode front instead, and rows off the 16-byte grid a kernel without tiles of this kind.) */
+int coli_b200_router_tile(int T, int E);
 
 /* ---- routing with no allocation (no counterpart in the reference: there the router runs on the
  * CPU, crates/colibri-engine/src/moe.rs:1047-1132, and allocates freely) ------------------------

@@ -1131,6 +1131,8 @@ int launch_items_from_counts(const int32_t *seg_count, int nseg, int rows_per_it
 
 }  // namespace colib
 
+extern "C" int coli_b200_router_tile(int T, int E) { return T < 1 || E < 1 ? -1 : colib::pick_router_tile(T, E); }
+
 // ---------------------------------------------------------------------------------------------
 // Routing without any allocation.
 //

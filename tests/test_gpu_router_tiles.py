@@ -3,25 +3,30 @@ inside a tile on both axes, hidden sizes that end inside a k-block, and rows off
 import numpy as np
 import pytest
 
-from speedycolibri_b200 import synth
+from speedycolibri_b200 import _lib, synth
 from speedycolibri_b200.configs import SCORE_SIGMOID, MoeShape
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("T,E,H,offset", [
-    (1, 9, 8, 0), (9, 130, 136, 0), (8, 128, 2048, 0),      # 8 x 8
-    (610, 140, 200, 0),                                     # 16 x 32
-    (2050, 250, 72, 0),                                     # 64 x 64
-    (4000, 250, 72, 0),                                     # 128 x 64
-    (9500, 380, 72, 0),                                     # 128 x 128
-    (20, 40, 136, 1),                                       # rows that are not 16-byte aligned
+TILES = ["8 x 8", "16 x 32", "64 x 64", "128 x 64", "128 x 128"]  # tokens x experts, by coli_b200_router_tile's number
+
+
+@pytest.mark.parametrize("tile,T,E,H,offset", [
+    ("8 x 8", 1, 9, 8, 0), ("8 x 8", 9, 130, 136, 0), ("8 x 8", 8, 128, 2048, 0),
+    ("16 x 32", 610, 140, 200, 0),
+    ("64 x 64", 2050, 250, 72, 0),
+    ("128 x 64", 4000, 250, 72, 0),
+    ("128 x 128", 9500, 380, 72, 0),
+    (None, 20, 40, 136, 1),                                 # rows that are not 16-byte aligned
 ])
-def test_router_tiles_bit_exact(gpu_backend, orc, T, E, H, offset):
+def test_router_tiles_bit_exact(gpu_backend, orc, tile, T, E, H, offset):
     import torch
 
     from speedycolibri_b200.moe import Config, MoeBlock
 
+    if tile is not None:
+        assert TILES[_lib.load().coli_b200_router_tile(T, E)] == tile  # the case still covers the tile it names
     shape = MoeShape("router_tiles", H=H, E=E, k=4, I=16, T=T, shared=False, norm_topk=True, score=SCORE_SIGMOID,
                      select_bias_std=0.01)
     layer = synth.device_layer(shape)
