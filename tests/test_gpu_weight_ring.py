@@ -6,7 +6,6 @@ import pytest
 
 from speedycolibri_b200 import synth
 from speedycolibri_b200.configs import FMT_E4M3_ROW, FMT_FP8_B128, FMT_NVFP4, MoeShape
-from oracle.layers import oracle_layer_from_device
 from tests.helpers import host_layer, upload_layer
 
 pytestmark = pytest.mark.gpu
@@ -29,25 +28,6 @@ def test_tile_and_ring_edges(gpu_backend, orc, fmt, H, I, rows):
         err = np.linalg.norm(y[off:off + r] - want, axis=1) / np.linalg.norm(want, axis=1)
         assert err.max() <= 5e-3, (e, r, err.max())
         off += r
-
-
-def test_six_rows_per_segment_on_a_layer_of_many_tiles(gpu_backend, orc):
-    """From 6 rows per expert on average (instead of 8) the tcgen05 kernel takes layers of at least 1776
-    tiles of 128 features: 120 experts x 15 tiles, checked on a few experts at both sides of the list."""
-    count, rows_each = 120, 6
-    shape = MoeShape("six_rows", H=64, E=count, k=1, I=1920, T=4, shared=False)
-    layer = synth.device_layer(shape)
-    es = layer.experts
-    rng = np.random.default_rng(6)
-    x = synth.bf16_bits_to_f32(synth.f32_to_bf16_bits(rng.standard_normal((count * rows_each, shape.H)).astype(np.float32)))
-    y = gpu_backend.expert_group([e.gate for e in es], [e.up for e in es], [e.down for e in es], [rows_each] * count, x)
-    needed = [0, 1, 59, 118, 119]
-    L = oracle_layer_from_device(shape, layer, set(needed))
-    for e in needed:
-        part = slice(e * rows_each, (e + 1) * rows_each)
-        want = L.expert_ffn(e, x[part])
-        err = np.linalg.norm(y[part] - want, axis=1) / np.linalg.norm(want, axis=1)
-        assert err.max() <= 5e-3, (e, err.max())
 
 
 @pytest.mark.parametrize("fmt", [FMT_NVFP4, FMT_FP8_B128, FMT_E4M3_ROW], ids=["nvfp4", "fp8_b128", "e4m3_row"])
