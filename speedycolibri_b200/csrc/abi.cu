@@ -503,12 +503,14 @@ int coli_tct_tile_tokens(int rows, int nseg) {
 // kernel re-reads so few token rows per weight tile that it wins.  It cuts segments into items of 8
 // rows there and reads their weights once per item, so on a layer too large for L2 the line lies at 6
 // rows, as long as the tcgen05 kernel's tiles (128 features of an expert) divide well over the SMs.
-// Measured (register-level / tcgen05, us a call): H 7168, I 2048, 256 experts at 4.5 rows 1443 / 1452,
-// 7.0 2300 / 1496; H 2048, I 768, 128 experts at 6.7 136 / 147, 8.0 150 / 148, FP8 6.7 167 / 179, 8.0
-// 182 / 180.  FP8 128x128 stays at 8 rows: the register-level kernel applies its scales in f32, the
-// tcgen05 kernel as f16 multipliers (error against 64 bits 2.864e-3 and 2.896e-3 at 7.5 rows, H 2048,
-// I 1024, 256 experts).  A pure function of shapes, so that kernel selection never depends on data or
-// addresses.
+// Measured (register-level / tcgen05, us a call): H 7168, I 2048, 256 experts (4112 tiles) at 4.5 rows 1443 /
+// 1452, 7.0 2300 / 1496; H 3072, I 1280, 200 experts (2010) at 5.5 354 / 342, 6.3 460 / 344; H 4096, I 1536, 150
+// (1812) at 5.5 408 / 400, 6.3 435 / 400, and 128 (1548) 351 / 345, 378 / 351; H 3072, I 1280, 128 (1290) at 5.4
+// 234 / 238, 6.3 249 / 239; H 2048, I 1024, 128 (1032) at 6.3 146 / 150, 7.2 160 / 150; H 2048, I 768, 128 (774)
+// at 6.7 136 / 147, 8.0 150 / 148, FP8 6.7 167 / 179, 8.0 182 / 180.  So 1776 tiles are on the safe side.
+// FP8 128x128 stays at 8 rows: the register-level kernel applies its scales in f32, the tcgen05 kernel as f16
+// multipliers (error against 64 bits 2.864e-3 and 2.896e-3 at 7.5 rows, H 2048, I 1024, 256 experts).
+// A pure function of shapes, so that kernel selection never depends on data or addresses.
 static bool tc_format(int fmt) { return fmt == COLI_FMT_NVFP4 || fmt == COLI_FMT_FP8_B128 || fmt == COLI_FMT_E4M3_ROW; }
 bool coli_use_tc_path(int fmt, int rows, int nseg, int I) {
   if (!tc_format(fmt) || nseg <= 0) return false;
@@ -520,9 +522,6 @@ int coli_rows_per_item_for(int rows, int nseg) {
   const int avg = (rows + nseg - 1) / (nseg > 0 ? nseg : 1);
   return avg <= 8 ? 8 : avg <= 16 ? 16 : 32;
 }
-static int tct_tile_tokens(int rows, int nseg) { return coli_tct_tile_tokens(rows, nseg); }
-static bool use_tc_path(int fmt, int rows, int nseg, int I) { return coli_use_tc_path(fmt, rows, nseg, I); }
-static int rows_per_item_for(const ColiMoeLayer &, int rows, int nseg) { return coli_rows_per_item_for(rows, nseg); }
 
 extern "C" int coli_b200_moe_create(ColiMoe **out, const ColiMoeLayer *L, int max_tokens) {
   if (!out || !L || max_tokens < 1) {
@@ -665,7 +664,7 @@ extern "C" int coli_b200_moe_create(ColiMoe **out, const ColiMoeLayer *L, int ma
   ok = ok && ws_alloc(m, &m->status, 1) && coli_cuda_check(cudaMemset(m->status, 0, sizeof(int)), "status clear");
   m->ticket = nullptr;
   ok = ok && ws_alloc(m, &m->ticket, 1) && coli_cuda_check(cudaMemset(m->ticket, 0, sizeof(unsigned int)), "ticket clear");
-  if (ok && use_tc_path(coli_kernel_fmt(L->fmt), (int)rows, m->nseg, L->I)) ok = ws_alloc(m, &m->xg, rows * H);
+  if (ok && coli_use_tc_path(coli_kernel_fmt(L->fmt), (int)rows, m->nseg, L->I)) ok = ws_alloc(m, &m->xg, rows * H);
   m->select_bias = nullptr;
   m->logit_bias = nullptr;
   if (ok && L->select_bias) ok = ws_alloc(m, &m->select_bias, E);
@@ -714,7 +713,6 @@ static cudaStream_t pick_stream(ColiMoe *m, void *stream) {
   return (cudaStream_t)stream;
 }
 
-static bool check_T(ColiMoe *m, int T, const char *who) { return coli_check_T(m, T, who); }
 bool coli_check_T(ColiMoe *m, int T, const char *who) {
   if (!m) {
     coli_set_error("%s: null handle", who);
@@ -734,7 +732,6 @@ static bool rows_aligned(const void *a, const void *b, const char *who, const ch
   return false;
 }
 
-static colib::RouteParams route_params(ColiMoe *m, const void *x_dev, int T) { return coli_route_params(m, x_dev, T); }
 colib::RouteParams coli_route_params(ColiMoe *m, const void *x_dev, int T) {
   colib::RouteParams rp;
   rp.T = T;
@@ -756,10 +753,6 @@ colib::RouteParams coli_route_params(ColiMoe *m, const void *x_dev, int T) {
   return rp;
 }
 
-static colib::PermuteParams permute_params(ColiMoe *m, const void *x_dev, int T, bool with_shared, int rpi, void *rows_dev,
-                                           int32_t *seg_count, int32_t *slot) {
-  return coli_permute_params(m, x_dev, T, with_shared, rpi, rows_dev, seg_count, slot);
-}
 colib::PermuteParams coli_permute_params(ColiMoe *m, const void *x_dev, int T, bool with_shared, int rpi, void *rows_dev,
                                          int32_t *seg_count, int32_t *slot) {
   colib::PermuteParams pp;
@@ -795,7 +788,7 @@ colib::PermuteParams coli_permute_params(ColiMoe *m, const void *x_dev, int T, b
 // The block on device pointers.  out_dev: bf16 [T,H] block output; or, when resid_io is given,
 // resid_io[T,H] (f32) += block output without an intermediate rounding (out_dev unused).
 static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *resid_io, int T, void *stream) {
-  if (!check_T(m, T, "moe_block_dev")) return 0;
+  if (!coli_check_T(m, T, "moe_block_dev")) return 0;
   if (!x_dev || (!out_dev && !resid_io)) {
     coli_set_error("moe_block_dev: null pointer");
     return 0;
@@ -809,8 +802,8 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
   cudaStream_t st = pick_stream(m, stream);
   const int k = m->L.k;
   const int rows = T * k + (m->has_shared ? T : 0);
-  const bool tc = use_tc_path(m->L.fmt, rows, m->nseg, m->L.I) && m->xg != nullptr;
-  const int rpi = tc ? tct_tile_tokens(rows, m->nseg) : rows_per_item_for(m->L, rows, m->nseg);
+  const bool tc = coli_use_tc_path(m->L.fmt, rows, m->nseg, m->L.I) && m->xg != nullptr;
+  const int rpi = tc ? coli_tct_tile_tokens(rows, m->nseg) : coli_rows_per_item_for(rows, m->nseg);
   const int max_items = max_work_items(rows, m->nseg, rpi);
   // Segments are in (owner, expert id) order, also when every expert is resident: only where that is the
   // expert order do the kernels index the weight tables by segment and save the dependent load.
@@ -822,14 +815,14 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
   } while (0)
   COLI_MARK(0);
   {
-    colib::PermuteParams pp = permute_params(m, x_dev, T, m->has_shared, rpi, tc ? m->xg : nullptr, m->seg_count, m->slot);
+    colib::PermuteParams pp = coli_permute_params(m, x_dev, T, m->has_shared, rpi, tc ? m->xg : nullptr, m->seg_count, m->slot);
     pp.gather_shared = tc ? 1 : 0;
     pp.x16 = tc ? nullptr : m->x16;
     // decode-sized batches: one launch for router, top-k and permutation (its time is booked
     // under the router phase)
-    const int fused = T <= 8 ? colib::launch_decode_front(route_params(m, x_dev, T), pp, m->ticket, st) : -1;
+    const int fused = T <= 8 ? colib::launch_decode_front(coli_route_params(m, x_dev, T), pp, m->ticket, st) : -1;
     if (fused == 0) return 0;
-    if (fused < 0 && !colib::launch_router(route_params(m, x_dev, T), st)) return 0;
+    if (fused < 0 && !colib::launch_router(coli_route_params(m, x_dev, T), st)) return 0;
     COLI_MARK(1);
     if (fused < 0 && !colib::launch_permute(pp, st)) return 0;
   }
@@ -925,7 +918,7 @@ extern "C" int coli_b200_moe_block_dev(ColiMoe *m, const void *x_dev, void *out_
 // rounded on its way into the stream.
 extern "C" int coli_b200_moe_layer_step_dev(ColiMoe *m, float *resid_dev, const float *post_ln_w_dev, float eps, int T,
                                             void *stream) {
-  if (!check_T(m, T, "moe_layer_step_dev")) return 0;
+  if (!coli_check_T(m, T, "moe_layer_step_dev")) return 0;
   if (!resid_dev || !post_ln_w_dev) {
     coli_set_error("moe_layer_step_dev: null pointer");
     return 0;
@@ -956,7 +949,7 @@ extern "C" int coli_b200_moe_check(ColiMoe *m) {
 }
 
 extern "C" int coli_b200_moe_last_routing(ColiMoe *m, int T, int32_t *topk_idx, float *topk_w) {
-  if (!check_T(m, T, "moe_last_routing")) return 0;
+  if (!coli_check_T(m, T, "moe_last_routing")) return 0;
   if (!coli_cuda_check(cudaDeviceSynchronize(), "routing read sync")) return 0;
   const size_t n = (size_t)T * m->L.k;
   if (topk_idx && !coli_cuda_check(cudaMemcpy(topk_idx, m->topk_idx, n * sizeof(int32_t), cudaMemcpyDeviceToHost), "routing read")) return 0;
@@ -965,7 +958,7 @@ extern "C" int coli_b200_moe_last_routing(ColiMoe *m, int T, int32_t *topk_idx, 
 }
 
 extern "C" int coli_b200_moe_block(ColiMoe *m, const void *x, void *out, int T, int32_t *topk_idx, float *topk_w) {
-  if (!check_T(m, T, "moe_block")) return 0;
+  if (!coli_check_T(m, T, "moe_block")) return 0;
   if (!x || !out) {
     coli_set_error("moe_block: null pointer");
     return 0;
@@ -1000,13 +993,13 @@ extern "C" int coli_b200_moe_local_experts(const ColiMoe *m) { return m ? m->n_l
 
 extern "C" int coli_b200_moe_topk_dev(ColiMoe *m, const void *x_dev, int T, int32_t *topk_idx_dev, float *topk_w_dev,
                                       void *stream) {
-  if (!check_T(m, T, "moe_topk_dev")) return 0;
+  if (!coli_check_T(m, T, "moe_topk_dev")) return 0;
   if (T == 0) return 1;
   if (!x_dev || !topk_idx_dev || !topk_w_dev) {
     coli_set_error("moe_topk_dev: null pointer");
     return 0;
   }
-  colib::RouteParams rp = route_params(m, x_dev, T);
+  colib::RouteParams rp = coli_route_params(m, x_dev, T);
   rp.topk_idx = topk_idx_dev;
   rp.topk_w = topk_w_dev;
   return colib::launch_router(rp, pick_stream(m, stream));
@@ -1014,7 +1007,7 @@ extern "C" int coli_b200_moe_topk_dev(ColiMoe *m, const void *x_dev, int T, int3
 
 extern "C" int coli_b200_moe_gather_local_dev(ColiMoe *m, const void *x_dev, const int32_t *topk_idx_dev, int T,
                                               void *rows_dev, int32_t *seg_count_dev, int32_t *slot_dev, void *stream) {
-  if (!check_T(m, T, "moe_gather_local_dev")) return 0;
+  if (!coli_check_T(m, T, "moe_gather_local_dev")) return 0;
   if (!x_dev || !topk_idx_dev || !rows_dev || !seg_count_dev || !slot_dev) {
     coli_set_error("moe_gather_local_dev: null pointer");
     return 0;
@@ -1022,7 +1015,7 @@ extern "C" int coli_b200_moe_gather_local_dev(ColiMoe *m, const void *x_dev, con
   cudaStream_t st = pick_stream(m, stream);
   if (T == 0) return coli_cuda_check(cudaMemsetAsync(seg_count_dev, 0, sizeof(int32_t) * m->n_local_seg, st), "count clear") ? 1 : 0;
   if (!rows_aligned(x_dev, rows_dev, "moe_gather_local_dev", "x_dev and rows_dev")) return 0;
-  colib::PermuteParams pp = permute_params(m, x_dev, T, false, colib::TCT_MAX_TOKENS, rows_dev, seg_count_dev, slot_dev);
+  colib::PermuteParams pp = coli_permute_params(m, x_dev, T, false, colib::TCT_MAX_TOKENS, rows_dev, seg_count_dev, slot_dev);
   pp.topk_idx = topk_idx_dev;
   pp.expert_slot = m->local_slot;
   pp.nseg_routed = m->n_local_seg;
@@ -1060,8 +1053,8 @@ int coli_run_segments(ColiMoe *m, SegScratch &sc, const WeightRef *g, const Weig
                       const int32_t *seg_expert_dev, const void *rows_dev, const int32_t *seg_count_dev, int n_seg,
                       int rows_cap, int rows_expected, void *y_dev, cudaStream_t st) {
   if (rows_cap == 0 || n_seg == 0) return 1;
-  const bool tc = use_tc_path(m->L.fmt, rows_expected, n_seg, m->L.I);
-  const int rpi = tc ? tct_tile_tokens(rows_expected, n_seg) : rows_per_item_for(m->L, rows_expected, n_seg);
+  const bool tc = coli_use_tc_path(m->L.fmt, rows_expected, n_seg, m->L.I);
+  const int rpi = tc ? coli_tct_tile_tokens(rows_expected, n_seg) : coli_rows_per_item_for(rows_expected, n_seg);
   const int max_items = max_work_items(rows_cap, n_seg, rpi);
   if (!ensure_h(m, sc, (size_t)rows_cap) || !ensure_items(m, sc, max_items, n_seg)) return 0;
   if (!colib::launch_items_from_counts(seg_count_dev, n_seg, rpi, sc.seg_off, sc.item_seg, sc.item_row0, sc.item_nrows,
@@ -1134,7 +1127,7 @@ extern "C" int coli_b200_moe_experts_dev(ColiMoe *m, const void *rows_dev, const
 }
 
 extern "C" int coli_b200_moe_shared_dev(ColiMoe *m, const void *x_dev, int T, void *y_dev, void *stream) {
-  if (!check_T(m, T, "moe_shared_dev")) return 0;
+  if (!coli_check_T(m, T, "moe_shared_dev")) return 0;
   if (!m->has_shared) {
     coli_set_error("moe_shared_dev: the layer has no shared expert");
     return 0;
@@ -1154,7 +1147,7 @@ extern "C" int coli_b200_moe_shared_dev(ColiMoe *m, const void *x_dev, int T, vo
 
 extern "C" int coli_b200_moe_combine_partial_dev(ColiMoe *m, const void *y_rows_dev, const int32_t *slot_dev,
                                                  const float *topk_w_dev, float *partial_dev, int T, void *stream) {
-  if (!check_T(m, T, "moe_combine_partial_dev")) return 0;
+  if (!coli_check_T(m, T, "moe_combine_partial_dev")) return 0;
   if (T == 0) return 1;
   if (!y_rows_dev || !slot_dev || !topk_w_dev || !partial_dev) {
     coli_set_error("moe_combine_partial_dev: null pointer");
@@ -1177,7 +1170,7 @@ extern "C" int coli_b200_moe_combine_partial_dev(ColiMoe *m, const void *y_rows_
 
 extern "C" int coli_b200_moe_finish_dev(ColiMoe *m, const float *partial_dev, const void *shared_y_dev, void *out_dev, int T,
                                         void *stream) {
-  if (!check_T(m, T, "moe_finish_dev")) return 0;
+  if (!coli_check_T(m, T, "moe_finish_dev")) return 0;
   if (T == 0) return 1;
   if (!partial_dev || !out_dev) {
     coli_set_error("moe_finish_dev: null pointer");
@@ -1273,7 +1266,7 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
   const int kfmt = coli_kernel_fmt(fmt);
   const bool tc = tc_format(kfmt) && total >= 8L * count;
   const int avg = (int)((total + count - 1) / count);
-  const int rpi = tc ? tct_tile_tokens((int)total, count) : (avg <= 8 ? 8 : avg <= 16 ? 16 : 32);
+  const int rpi = tc ? coli_tct_tile_tokens((int)total, count) : (avg <= 8 ? 8 : avg <= 16 ? 16 : 32);
   const int max_items = max_work_items((int)total, count, rpi);
   const size_t xb = (size_t)total * D;
   // slots: 0 x f32 / y f32, 1 x f16, 2 h f16, 3 tables + counts + work list + status word, 4 y bf16 (tcgen05 path)

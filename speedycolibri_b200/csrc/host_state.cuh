@@ -87,7 +87,7 @@ static inline bool ws_alloc(ColiMoe *m, T **p, size_t count) {
 }
 
 
-// kernel-family selection: pure functions of (format, rows, segments)
+// kernel-family selection: pure functions of format and shapes (rows, segments, intermediate size)
 int coli_tct_tile_tokens(int rows, int nseg);
 bool coli_use_tc_path(int fmt, int rows, int nseg, int I);
 int coli_rows_per_item_for(int rows, int nseg);
