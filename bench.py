@@ -55,16 +55,16 @@ def measured_peaks():
 # a different share of the experts active than the small case c4s, so the streams do not scale by a
 # constant.  The captures are summarised under profiles/.
 NCU_TRAFFIC = {
-    ("c3s", 512, "gate_up"): (635327232, "profiles/k_ffn_tct_c3s.md", "expert_tc_tmem.cu", "b0773fc4b9a0"),
-    ("c3s", 512, "down"): (331972864, "profiles/k_ffn_tct_c3s.md", "expert_tc_tmem.cu", "b0773fc4b9a0"),
-    ("c3", 4096, "gate_up"): (5082617856, "profiles/k_ffn_tct_c3s.md (c3s capture x 8)", "expert_tc_tmem.cu", "b0773fc4b9a0"),
-    ("c3", 4096, "down"): (2655782912, "profiles/k_ffn_tct_c3s.md (c3s capture x 8)", "expert_tc_tmem.cu", "b0773fc4b9a0"),
-    ("c2", 512, "gate_up"): (433006592, "profiles/k_ffn_tct_c2.md", "expert_tc_tmem.cu", "b0773fc4b9a0"),
-    ("c2", 512, "down"): (218468352, "profiles/k_ffn_tct_c2.md", "expert_tc_tmem.cu", "b0773fc4b9a0"),
-    ("c1", 8, "gate_up"): (93706496, "profiles/k_ffn_mm_c1.md", "expert_small.cu", "9975bf507adc"),
-    ("c1", 8, "down"): (46137600, "profiles/k_ffn_mm_c1.md", "expert_small.cu", "9975bf507adc"),
-    ("c4s", 2048, "gate_up"): (998966016, "profiles/k_ffn_tct_c4s.md", "expert_tc_tmem.cu", "b0773fc4b9a0"),
-    ("c4s", 2048, "down"): (583099136, "profiles/k_ffn_tct_c4s.md", "expert_tc_tmem.cu", "b0773fc4b9a0"),
+    ("c3s", 512, "gate_up"): (633368320, "profiles/k_ffn_tct_c3s.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
+    ("c3s", 512, "down"): (332011264, "profiles/k_ffn_tct_c3s.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
+    ("c3", 4096, "gate_up"): (5066946560, "profiles/k_ffn_tct_c3s.md (c3s capture x 8)", "expert_tc_tmem.cu", "7ee0edfa51e6"),
+    ("c3", 4096, "down"): (2656090112, "profiles/k_ffn_tct_c3s.md (c3s capture x 8)", "expert_tc_tmem.cu", "7ee0edfa51e6"),
+    ("c2", 512, "gate_up"): (432590848, "profiles/k_ffn_tct_c2.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
+    ("c2", 512, "down"): (218450176, "profiles/k_ffn_tct_c2.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
+    ("c1", 8, "gate_up"): (93980928, "profiles/k_ffn_mm_c1.md", "expert_small.cu", "73d73f761ef4"),
+    ("c1", 8, "down"): (46134272, "profiles/k_ffn_mm_c1.md", "expert_small.cu", "73d73f761ef4"),
+    ("c4s", 2048, "gate_up"): (997067264, "profiles/k_ffn_tct_c4s.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
+    ("c4s", 2048, "down"): (585076480, "profiles/k_ffn_tct_c4s.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
 }
 
 
