@@ -815,7 +815,8 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
   } while (0)
   COLI_MARK(0);
   {
-    colib::PermuteParams pp = coli_permute_params(m, x_dev, T, m->has_shared, rpi, tc ? m->xg : nullptr, m->seg_count, m->slot);
+    colib::PermuteParams pp = coli_permute_params(m, x_dev, T, m->has_shared, rpi, tc ? m->xg : nullptr, nullptr, m->slot);
+    if (m->segs_in_expert_order) pp.expert_slot = nullptr;
     pp.gather_shared = tc ? 1 : 0;
     pp.x16 = tc ? nullptr : m->x16;
     // decode-sized batches: one launch for router, top-k and permutation (its time is booked

@@ -148,7 +148,7 @@ struct PermuteParams {
   const int32_t *expert_slot;  // [E] segment position of each expert (null = identity, < 0 = not resident)
   int32_t *local_rank;         // [T*k] scratch
   int32_t *chunk_cnt;          // [nchunk][E] scratch
-  int32_t *seg_count;          // [E] out: rows per segment (segment order)
+  int32_t *seg_count;          // [E] out: rows per segment (segment order), or null when nobody reads them
   int32_t *seg_off;            // [E+2] out: exclusive offsets (+shared)
   int32_t *slot;               // [T*k] out: row position of (t,kk)
   int32_t *row_token;          // [T*k (+T)] out: token of each row

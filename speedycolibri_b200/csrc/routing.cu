@@ -345,22 +345,24 @@ __global__ void __launch_bounds__(C::NT) k_router_chain(RouteParams p) {
 
 // The logits of a decode-sized CTA: one chain per thread of two computing warps, 8 tokens x 8 experts,
 // operands staged as f32.  CW staging warps copy 16-byte chunks of the bf16 rows through a ring of
-// cp.async stages, widen them and store them into one of two f32 buffers of 128 k, while the computing
-// warps read the other three 128-bit loads ahead of the FMAs that use them (5.7 cycles per k).  Rows are
-// padded by 16 bytes (banks).  Against staging all rows first and walking the chain after: the whole
-// front end below 24.4 -> 20.7 us at 1 token, 26 -> 21 at 8 (128 experts x 2048).
+// cp.async stages, widen them and store them into one of two f32 buffers of 256 k, while the computing
+// warps read the other three 128-bit loads ahead of the FMAs that use them.  Rows are padded by 16 bytes
+// (banks).  A k takes 5.4 cycles (an FMA's latency is 4.3): a barrier costs the chain about 115, which is why
+// a block is 256 k long (128: 6.0; 512: 5.3, but its first block is late); loads further ahead or more staging
+// warps change nothing.
 struct RouterTiny {
-  static constexpr int ROWS = 16, BK = 128, LD = BK + 4, CH = BK / 8, STAGES = 6;
+  static constexpr int ROWS = 16, BK = 256, LD = BK + 4, CH = BK / 8, STAGES = 4;
   static constexpr int F32_BYTES = ROWS * LD * 4, RING_BYTES = ROWS * BK * 2;
   static constexpr size_t SMEM = (size_t)2 * F32_BYTES + (size_t)STAGES * RING_BYTES;
 };
-// All threads of a CTA of 2 + CW warps call this; logits of tokens m0.. and experts n0.. are written.
+// The first 2 + CW warps of a CTA call this; logits of tokens m0.. and experts n0.. are written.
 template <int CW>
 __device__ __forceinline__ void router_tiny_block(const RouteParams &p, unsigned char *smem_raw, int m0, int n0) {
   using C = RouterTiny;
   constexpr int LD = C::LD, CH = C::CH, BK = C::BK, CPT = (C::ROWS * CH + 32 * CW - 1) / (32 * CW);
   float *const buf = reinterpret_cast<float *>(smem_raw);  // [2][ROWS][LD]: 8 tokens, then 8 experts
   const int nkb = (p.H + BK - 1) / BK;
+  auto block_barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(64 + 32 * CW) : "memory"); };
   if (threadIdx.x >= 64) {
     const int tid = (int)threadIdx.x - 64;
     unsigned char *const ring = smem_raw + 2 * C::F32_BYTES;
@@ -399,7 +401,7 @@ __device__ __forceinline__ void router_tiny_block(const RouteParams &p, unsigned
     }
     convert(0);
     for (int kb = 0; kb < nkb; ++kb) {
-      __syncthreads();
+      block_barrier();
       if (kb + 1 < nkb) convert(kb + 1);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -408,7 +410,7 @@ __device__ __forceinline__ void router_tiny_block(const RouteParams &p, unsigned
   const int xrow = (int)threadIdx.x >> 3, wrow = (int)threadIdx.x & 7;
   float acc = 0.0f;
   for (int kb = 0; kb < nkb; ++kb) {
-    __syncthreads();  // block kb is staged, and nobody reads its predecessor any more
+    block_barrier();  // block kb is staged, and nobody reads its predecessor any more
     const float4 *xs = reinterpret_cast<const float4 *>(buf + (kb & 1) * (C::ROWS * LD) + xrow * LD);
     const float4 *ws = reinterpret_cast<const float4 *>(buf + (kb & 1) * (C::ROWS * LD) + (8 + wrow) * LD);
     constexpr int D = 4;  // 128-bit operands in flight or in use
@@ -439,11 +441,21 @@ __device__ __forceinline__ void router_tiny_block(const RouteParams &p, unsigned
 // ---------------------------------------------------------------------------------------------
 // Score + top-k: one warp per token.  Expert e lives in lane e % 32, slot e / 32, scores and keys in
 // registers; SLOTS >= E / 32 (<= 16) is a template parameter so that every pass over them unrolls into
-// independent operations.  A pass over shared memory with a load-use step per expert took 21 us for the
-// sigmoid router of 256 experts in 8 groups and 8.5 us for the softmax one of 128, whatever the batch.
+// independent operations.  What bounds it is the length of one token's dependent chain, whatever the batch
+// (clock stamps on a warm SM, 128 experts softmax top-8 / 256 experts sigmoid in 8 groups, cycles):
+//   load + maximum 420, exp 940, ordered sum 560, divide 330, keys 260, selection and weights ...
+// k rounds of two warp reductions and a rescan of the winning lane's slots cost 250 cycles each (2000 / 2500
+// for k = 8), and a group's two best by one lane per group 2750; both are counting steps now (below).
 // ---------------------------------------------------------------------------------------------
 constexpr int kMaxSlots = 16;  // E <= 512
-__host__ __device__ static inline int topk_row_floats(int E) { return (E + 3) & ~3; }  // shared memory per warp
+// Shared memory of one warp: the row of scores (16-byte aligned), and a list of 32 candidates.
+struct TopkCand {
+  uint32_t key;
+  int id;
+  float sc;
+  uint32_t pad;
+};
+__host__ __device__ static constexpr int topk_row_floats(int E) { return ((E + 3) & ~3) + 32 * (int)(sizeof(TopkCand) / 4); }
 
 // order-preserving integer key of a candidate (a value strictly above -inf; NaN is none), 0 otherwise
 __device__ __forceinline__ uint32_t topk_key(float c) {
@@ -451,38 +463,136 @@ __device__ __forceinline__ uint32_t topk_key(float c) {
   const uint32_t bits = __float_as_uint(__fadd_rn(c, 0.0f));  // -0 and +0 tie like the float compare
   return (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
 }
+__device__ __forceinline__ float topk_key_value(uint32_t key) {
+  return key == 0u ? __uint_as_float(0xff800000u) : __uint_as_float((key & 0x80000000u) ? key & 0x7fffffffu : ~key);
+}
+
+// The k best of a warp's keys (largest key, then lowest expert id; key 0 = not a candidate) as list entries
+// 0..k-1 of `cand`, in order; fewer candidates leave expert 0 behind them, which is what the reference's scan
+// returns.  The k-th largest of the lanes' best keys bounds the k-th largest of all from below, so only keys
+// from it upwards can be chosen: a little over k of them as a rule, and each finds its place by counting.
+// More than 32 of them (many equal keys) take the rounds.
+template <int SLOTS>
+__device__ __forceinline__ void topk_select(const uint32_t (&key)[SLOTS], const float (&sc)[SLOTS], int k, TopkCand *cand, int lane) {
+  uint32_t bkey = 0u;
+#pragma unroll
+  for (int s = 0; s < SLOTS; ++s) bkey = max(bkey, key[s]);
+  uint32_t *best = reinterpret_cast<uint32_t *>(cand);
+  best[lane] = bkey;
+  __syncwarp();
+  int above = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint4 q = *reinterpret_cast<const uint4 *>(best + 4 * j);
+    above += (q.x > bkey) + (q.y > bkey) + (q.z > bkey) + (q.w > bkey);
+  }
+  const uint32_t bound = max(1u, __reduce_min_sync(0xffffffffu, above < k ? bkey : 0xffffffffu));
+  uint32_t holders[SLOTS];
+  int n = 0;
+#pragma unroll
+  for (int s = 0; s < SLOTS; ++s) {
+    holders[s] = __ballot_sync(0xffffffffu, key[s] >= bound);
+    n += __popc(holders[s]);
+  }
+  const float sc0 = __shfl_sync(0xffffffffu, sc[0], 0);  // (also: every lane has read `best`)
+  if (n <= 32) {
+    int at = 0;
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      if (key[s] >= bound) {
+        TopkCand c = {key[s], s * 32 + lane, sc[s], 0u};
+        *reinterpret_cast<uint4 *>(cand + at + __popc(holders[s] & ((1u << lane) - 1u))) = *reinterpret_cast<const uint4 *>(&c);
+      }
+      at += __popc(holders[s]);
+    }
+    __syncwarp();
+    const uint4 raw = *reinterpret_cast<const uint4 *>(cand + lane);
+    const TopkCand mine = *reinterpret_cast<const TopkCand *>(&raw);
+    int rank = 0;
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) {  // a slot's candidates precede the next slot's and lanes ascend: j < lane is the lower id
+      const uint32_t other = cand[j].key;
+      rank += other > mine.key || (other == mine.key && j < lane);
+    }
+    __syncwarp();
+    if (lane < n && rank < k) *reinterpret_cast<uint4 *>(cand + rank) = raw;
+    if (lane >= n && lane < k) cand[lane] = TopkCand{0u, 0, sc0, 0u};
+    __syncwarp();
+    return;
+  }
+  uint32_t left[SLOTS];
+#pragma unroll
+  for (int s = 0; s < SLOTS; ++s) left[s] = key[s];
+  TopkCand mine = {0u, 0, sc0, 0u};  // lane kk keeps place kk
+  for (int kk = 0; kk < k; ++kk) {
+    uint32_t bk = 0u, bs = 0u;
+    float bsc = 0.0f;
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s)  // ascending e within the lane: strict > keeps the lowest index
+      if (left[s] > bk) {
+        bk = left[s];
+        bs = (uint32_t)s;
+        bsc = sc[s];
+      }
+    const uint32_t top = __reduce_max_sync(0xffffffffu, bk);
+    if (top == 0u) break;
+    const uint32_t win = __reduce_min_sync(0xffffffffu, bk == top ? bs * 32 + lane : 0xffffffffu);
+    const float wsc = __shfl_sync(0xffffffffu, bsc, win & 31);
+    if (lane == kk) mine = {top, (int)win, wsc, 0u};
+    if (lane == (int)(win & 31)) {
+#pragma unroll
+      for (int s = 0; s < SLOTS; ++s)
+        if (s == (int)bs) left[s] = 0u;
+    }
+  }
+  if (lane < k) cand[lane] = mine;
+  __syncwarp();
+}
 
 // One warp scores token t and selects its experts; `row` is topk_row_floats(E) floats of shared
-// memory, 16-byte aligned and private to the warp.
+// memory, 16-byte aligned and private to the warp.  The experts' ids also go to ids_out[0..k) when given.
 template <int SLOTS>
-__device__ __forceinline__ void route_topk_slots(const RouteParams &p, int t, float *row, int lane) {
+__device__ __forceinline__ void route_topk_slots(const RouteParams &p, int t, float *row, int lane, int *ids_out) {
   const int E = p.E, k = min(p.k, p.E);
   const float *z = p.logits + (size_t)t * E;
   const float NEG_INF = __uint_as_float(0xff800000u);
+  TopkCand *cand = reinterpret_cast<TopkCand *>(row + ((E + 3) & ~3));
+  const bool biased = p.score != COLI_SCORE_SOFTMAX;
 
   float sc[SLOTS];  // score of each of this lane's experts
 #pragma unroll
   for (int s = 0; s < SLOTS; ++s) sc[s] = lane + 32 * s < E ? __ldcg(z + lane + 32 * s) : NEG_INF;
+  float bias[SLOTS];  // requested beside the logits
+#pragma unroll
+  for (int s = 0; s < SLOTS; ++s) bias[s] = (biased && p.select_bias && lane + 32 * s < E) ? p.select_bias[lane + 32 * s] : 0.0f;
   if (p.score == COLI_SCORE_SOFTMAX) {
     float mx = NEG_INF;
 #pragma unroll
     for (int s = 0; s < SLOTS; ++s) mx = fmaxf(mx, sc[s]);  // max is order-independent
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    mx = topk_key_value(__reduce_max_sync(0xffffffffu, topk_key(mx)));
 #pragma unroll
     for (int s = 0; s < SLOTS; ++s) {
       sc[s] = coli_expf(__fsub_rn(sc[s], mx));
       if (lane + 32 * s < E) row[lane + 32 * s] = sc[s];
     }
     __syncwarp();
-    float tot = 0.0f;  // sequential over e, every lane redundantly (moe.rs:1068)
+    float tot = 0.0f;  // sequential over e, every lane redundantly (moe.rs:1068); the next 16 are read ahead
     int e = 0;
+    float4 v[4];
+    if (E >= 16) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float4 *>(row + 4 * i);
+    }
     for (; e + 16 <= E; e += 16) {
-      float4 v[4];
+      float4 u[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float4 *>(row + e + 4 * i);
+      for (int i = 0; i < 4; ++i) u[i] = v[i];
+      if (e + 32 <= E) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) tot = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(tot, v[i].x), v[i].y), v[i].z), v[i].w);
+        for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float4 *>(row + e + 16 + 4 * i);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) tot = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(tot, u[i].x), u[i].y), u[i].z), u[i].w);
     }
     for (; e < E; ++e) tot = __fadd_rn(tot, row[e]);
     if (tot > 0.0f) {
@@ -495,17 +605,16 @@ __device__ __forceinline__ void route_topk_slots(const RouteParams &p, int t, fl
   }
 
   // selection scores as keys
-  const bool biased = p.score != COLI_SCORE_SOFTMAX;
   uint32_t key[SLOTS];
   float ch[SLOTS];
 #pragma unroll
   for (int s = 0; s < SLOTS; ++s) {
-    const int e = lane + 32 * s;
-    ch[s] = biased ? __fadd_rn(sc[s], (p.select_bias && e < E) ? p.select_bias[e] : 0.0f) : sc[s];
-    key[s] = e < E ? topk_key(ch[s]) : 0u;
+    ch[s] = biased ? __fadd_rn(sc[s], bias[s]) : sc[s];
+    key[s] = lane + 32 * s < E ? topk_key(ch[s]) : 0u;
   }
 
-  // group-limited selection: allowed-group bit mask (n_group <= 32)
+  // group-limited selection (n_group <= 32): a group's score is the sum of its two largest, found by as many
+  // lanes as fit (four for 8 groups); the best topk_group groups are those with fewer than topk_group above
   if (p.n_group > 1) {
     const int G = p.n_group, gs = E / G, kg = min(p.topk_group, G);
     __syncwarp();  // the sum above has read the row
@@ -513,92 +622,63 @@ __device__ __forceinline__ void route_topk_slots(const RouteParams &p, int t, fl
     for (int s = 0; s < SLOTS; ++s)
       if (lane + 32 * s < E) row[lane + 32 * s] = ch[s];
     __syncwarp();
-    uint32_t gkey = 0u;
-    if (lane < G) {
-      float m1 = NEG_INF, m2 = NEG_INF;  // the two largest of the lane's group
-      for (int e0 = 0; e0 < gs; e0 += 8) {
-        float c[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) c[i] = e0 + i < gs ? row[lane * gs + e0 + i] : NEG_INF;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const bool first = c[i] > m1;
-          m2 = first ? m1 : (c[i] > m2 ? c[i] : m2);
-          m1 = first ? c[i] : m1;
-        }
+    int per = 1;  // lanes of a group: a power of two
+    while (2 * per * G <= 32) per *= 2;
+    const int g = lane / per;
+    float m1 = NEG_INF, m2 = NEG_INF;
+    if (g < G)
+#pragma unroll 4
+      for (int i = lane % per; i < gs; i += per) {
+        const float c = row[g * gs + i];
+        m2 = c > m1 ? m1 : (c > m2 ? c : m2);
+        m1 = c > m1 ? c : m1;
       }
-      gkey = topk_key(__fadd_rn(m1, m2));
+    for (int o = 1; o < per; o <<= 1) {
+      const float o1 = __shfl_xor_sync(0xffffffffu, m1, o), o2 = __shfl_xor_sync(0xffffffffu, m2, o);
+      m2 = fmaxf(fminf(m1, o1), fmaxf(m2, o2));
+      m1 = fmaxf(m1, o1);
     }
-    uint32_t gmask = 0;
-    for (int j = 0; j < kg; ++j) {
-      const uint32_t top = __reduce_max_sync(0xffffffffu, gkey);
-      const uint32_t win = __reduce_min_sync(0xffffffffu, (top != 0u && gkey == top) ? (uint32_t)lane : 0xffffffffu);
-      const int best = top != 0u ? (int)win : 0;
-      if (lane == best) gkey = 0u;
-      gmask |= 1u << best;
-    }
+    const uint32_t gkey = g < G && lane % per == 0 ? topk_key(__fadd_rn(m1, m2)) : 0u;
+    uint32_t *gk = reinterpret_cast<uint32_t *>(cand);
+    if (lane % per == 0 && g < G) gk[g] = gkey;
+    __syncwarp();
+    int above = 0;
+    for (int j = 0; j < G; ++j) above += gk[j] > gkey || (gk[j] == gkey && j < g);
+    const uint32_t kept = __ballot_sync(0xffffffffu, gkey != 0u && above < kg);  // the first lanes of kept groups
+    uint32_t gmask = __popc(__ballot_sync(0xffffffffu, gkey != 0u)) < kg ? 1u : 0u;  // no candidate: group 0
+    for (int j = 0; j < G; ++j) gmask |= ((kept >> (j * per)) & 1u) << j;
 #pragma unroll
     for (int s = 0; s < SLOTS; ++s)
       if (lane + 32 * s < E && !((gmask >> ((lane + 32 * s) / gs)) & 1u)) key[s] = 0u;
+    __syncwarp();
   }
 
-  // k rounds of arg-max over the allowed, not yet chosen experts.  Every lane keeps the best of
-  // its own remaining experts (key 0 = none left); a round is two warp reductions -- the largest
-  // key, then the lowest expert id among its holders -- and the winning lane drops that expert.
-  uint32_t bkey, bslot;
-  float bsc;
-  auto lane_best = [&]() {
-    bkey = 0u;
-    bslot = 0u;
-    bsc = 0.0f;
-#pragma unroll
-    for (int s = 0; s < SLOTS; ++s)  // ascending e within the lane: strict > keeps the lowest index
-      if (key[s] > bkey) {
-        bkey = key[s];
-        bslot = (uint32_t)s;
-        bsc = sc[s];
-      }
-  };
-  int my_idx = 0;  // lane kk keeps idx[kk]
-  float my_w = 0.0f;
-  const float sc0 = __shfl_sync(0xffffffffu, sc[0], 0);
-  lane_best();
-  for (int kk = 0; kk < k; ++kk) {
-    const uint32_t top = __reduce_max_sync(0xffffffffu, bkey);
-    const uint32_t win = __reduce_min_sync(0xffffffffu, (top != 0u && bkey == top) ? bslot * 32 + lane : 0xffffffffu);
-    const float wsc = __shfl_sync(0xffffffffu, bsc, win & 31);
-    const int best = top != 0u ? (int)win : 0;  // no candidate: expert 0, as the reference's scan returns
-    if (lane == kk) {
-      my_idx = best;
-      my_w = top != 0u ? wsc : sc0;
-    }
-    if (top != 0u && (best & 31) == lane) {
-#pragma unroll
-      for (int s = 0; s < SLOTS; ++s)
-        if (s == (int)bslot) key[s] = 0u;
-      lane_best();
-    }
-  }
-  if (p.norm_topk) {
-    float smv = 0.0f;
-    for (int kk = 0; kk < k; ++kk) smv = __fadd_rn(smv, __shfl_sync(0xffffffffu, my_w, kk));
-    smv = __fadd_rn(smv, 1e-20f);
-    my_w = __fdiv_rn(my_w, smv);
-  }
-  my_w = __fmul_rn(my_w, p.routed_scale);
+  topk_select<SLOTS>(key, sc, k, cand, lane);
   if (lane < k) {
-    p.topk_idx[(size_t)t * k + lane] = my_idx;
-    p.topk_w[(size_t)t * k + lane] = my_w;
+    float w = cand[lane].sc;
+    if (p.norm_topk) {
+      float smv = 0.0f;
+#pragma unroll 8
+      for (int kk = 0; kk < k; ++kk) smv = __fadd_rn(smv, cand[kk].sc);
+      smv = __fadd_rn(smv, 1e-20f);
+      w = __fdiv_rn(w, smv);
+    }
+    const int id = cand[lane].id;
+    if (p.topk_idx) {
+      p.topk_idx[(size_t)t * k + lane] = id;
+      p.topk_w[(size_t)t * k + lane] = __fmul_rn(w, p.routed_scale);
+    }
+    if (ids_out) ids_out[lane] = id;
   }
   __syncwarp();  // the row may be reused for the warp's next token
 }
-__device__ __forceinline__ void route_topk_token(const RouteParams &p, int t, float *row, int lane) {
+__device__ __forceinline__ void route_topk_token(const RouteParams &p, int t, float *row, int lane, int *ids_out = nullptr) {
   if (p.E <= 128)
-    route_topk_slots<4>(p, t, row, lane);
+    route_topk_slots<4>(p, t, row, lane, ids_out);
   else if (p.E <= 256)
-    route_topk_slots<8>(p, t, row, lane);
+    route_topk_slots<8>(p, t, row, lane, ids_out);
   else
-    route_topk_slots<kMaxSlots>(p, t, row, lane);
+    route_topk_slots<kMaxSlots>(p, t, row, lane, ids_out);
 }
 
 __global__ void __launch_bounds__(128) k_route_topk(RouteParams p) {
@@ -845,7 +925,8 @@ __global__ void __launch_bounds__(1024) k_seg_scan(PermuteParams p, int nchunk, 
   }
   build_work_list(p, seg_cnt, nseg, max_items, seg_off, seg_ibase);
   for (int s = threadIdx.x; s <= nseg; s += blockDim.x) p.seg_off[s] = seg_off[s];
-  for (int s = threadIdx.x; s < nrt; s += blockDim.x) p.seg_count[s] = seg_cnt[s];
+  if (p.seg_count)
+    for (int s = threadIdx.x; s < nrt; s += blockDim.x) p.seg_count[s] = seg_cnt[s];
 }
 
 __global__ void __launch_bounds__(256) k_permute(PermuteParams p) {
@@ -940,7 +1021,8 @@ __device__ __forceinline__ void permute_small_body(const PermuteParams &p, int m
   __syncthreads();
   build_work_list(p, cnt, nseg, max_items, off, sm.ibase);
   for (int s = threadIdx.x; s <= nseg; s += blockDim.x) p.seg_off[s] = off[s];
-  for (int s = threadIdx.x; s < nrt; s += blockDim.x) p.seg_count[s] = cnt[s];
+  if (p.seg_count)
+    for (int s = threadIdx.x; s < nrt; s += blockDim.x) p.seg_count[s] = cnt[s];
   for (int i = threadIdx.x; i < npairs; i += blockDim.x) {
     const int s = idx_sm[i];
     if (s < 0) {
@@ -974,9 +1056,89 @@ __device__ __forceinline__ void permute_small_body(const PermuteParams &p, int m
   }
 }
 
+// The same for at most 256 pairs in a block that wants no counts per segment: a thread per pair finds its row --
+// the pairs of lower segments and the earlier ones of its own -- by comparing with every other pair, and the
+// item that a row opens by the rows that open one before it (a bit per row).  Two barriers and no scan over
+// the segments: the steps above take 3300 cycles for 8 pairs of 128 experts on a warm SM, this 500.
+// `seg` holds the pairs' segments (below 0: no row), padded to a multiple of 4 entries with INT_MAX, and `opens`
+// eight zeros; both are visible to the CTA.
+constexpr int kPairwiseMax = 256;
+struct PermutePairsSmem {
+  __align__(16) int seg[kPairwiseMax];
+  int pos[kPairwiseMax];
+  uint32_t opens[kPairwiseMax / 32];
+};
+__device__ __forceinline__ void permute_pairs(const PermuteParams &p, int max_items, PermutePairsSmem &sm) {
+  const int n = p.T * p.k, i = (int)threadIdx.x, rpi = p.rows_per_item;
+  int s = -1, below = 0, before = 0, equal = 0, share = 1;
+  if (i < n) s = sm.seg[i];
+  if (s >= 0) {
+#pragma unroll 2
+    for (int j = 0; j < n; j += 4) {
+      const int4 q = *reinterpret_cast<const int4 *>(sm.seg + j);
+      below += ((unsigned)q.x < (unsigned)s) + ((unsigned)q.y < (unsigned)s) + ((unsigned)q.z < (unsigned)s) + ((unsigned)q.w < (unsigned)s);
+      const int eq = (q.x == s) | (q.y == s) << 1 | (q.z == s) << 2 | (q.w == s) << 3;
+      equal += __popc(eq);
+      before += i <= j ? 0 : __popc(i >= j + 4 ? eq : eq & ((1 << (i - j)) - 1));
+    }
+    share = work_item_rows(equal, rpi);
+  }
+  const int pos = below + before;
+  const bool opens = s >= 0 && before % share == 0;
+  if (i < n) {
+    sm.pos[i] = s >= 0 ? pos : -1;
+    p.slot[i] = s >= 0 ? pos : -1;
+    if (s >= 0) p.row_token[pos] = i / p.k;
+  }
+  if (opens) atomicOr(&sm.opens[pos >> 5], 1u << (pos & 31));
+  const int rows = __syncthreads_count(s >= 0);  // the shared expert's rows follow them
+  int items = 0, item = 0;
+#pragma unroll
+  for (int w = 0; w < kPairwiseMax / 32; ++w) {
+    const uint32_t bits = sm.opens[w];
+    if (w < (pos >> 5)) item += __popc(bits);
+    if (w == (pos >> 5)) item += __popc(bits & ((1u << (pos & 31)) - 1u));
+    items += __popc(bits);
+  }
+  if (opens && item < max_items) {
+    p.item_seg[item] = s;
+    p.item_row0[item] = pos;
+    p.item_nrows[item] = min(share, equal - before);
+  }
+  if (p.has_shared) {
+    const int sshare = work_item_rows(p.T, rpi), nsh = (p.T + sshare - 1) / sshare;
+    if (i < nsh && items + i < max_items) {
+      p.item_seg[items + i] = p.nseg_routed;
+      p.item_row0[items + i] = rows + i * sshare;
+      p.item_nrows[items + i] = min(sshare, p.T - i * sshare);
+    }
+    if (i < p.T) p.row_token[rows + i] = i;
+    items += nsh;
+  }
+  if (i == 0) *p.n_items = min(items, max_items);
+  if (p.xg) {  // gather rows: one warp per row
+    const int total = n + ((p.has_shared && p.gather_shared) ? p.T : 0);
+    const int vec = p.H / 8;
+    for (int r = i >> 5; r < total; r += (int)blockDim.x >> 5) {
+      const int t = r < n ? r / p.k : r - n, to = r < n ? sm.pos[r] : rows + t;
+      if (to < 0) continue;
+      const uint4 *src = reinterpret_cast<const uint4 *>(p.x + (size_t)t * p.H);
+      uint4 *dst = reinterpret_cast<uint4 *>(p.xg + (size_t)to * p.H);
+      for (int c = i & 31; c < vec; c += 32) dst[c] = coli_bf16x8_to_f16x8(src[c]);
+    }
+  }
+}
+// a pair's segment: below 0 for an id that is no expert or lives on another rank
+__device__ __forceinline__ int pair_segment(const PermuteParams &p, int id) {
+  return (id < 0 || id >= p.E) ? -1 : (p.expert_slot ? p.expert_slot[id] : id);
+}
+
 __global__ void __launch_bounds__(1024) k_permute_small(PermuteParams p, int max_items) {
   coli_grid_wait();
-  __shared__ PermuteSmallSmem sm;
+  __shared__ union {
+    PermuteSmallSmem all;
+    PermutePairsSmem pairs;
+  } sm;
   if (blockIdx.x > 0) {  // the extra CTAs only write the token-order f16 copy of x
     const size_t n = (size_t)p.T * p.H / 8;
     const uint4 *src = reinterpret_cast<const uint4 *>(p.x);
@@ -985,40 +1147,85 @@ __global__ void __launch_bounds__(1024) k_permute_small(PermuteParams p, int max
       dst[i] = coli_bf16x8_to_f16x8(src[i]);
     return;
   }
-  permute_small_body(p, max_items, sm);
+  const int n = p.T * p.k;
+  if (p.seg_count || n > kPairwiseMax) {
+    permute_small_body(p, max_items, sm.all);
+    return;
+  }
+  for (int i = threadIdx.x; i < kPairwiseMax; i += blockDim.x) sm.pairs.seg[i] = i < n ? pair_segment(p, p.topk_idx[i]) : 0x7fffffff;
+  if (threadIdx.x < kPairwiseMax / 32) sm.pairs.opens[threadIdx.x] = 0u;
+  __syncthreads();
+  permute_pairs(p, max_items, sm.pairs);
 }
 
 // Decode front end (T <= 8): router logits, top-k and the permutation in ONE launch.  Every CTA
 // computes the logits of 8 experts (and converts its slice of the tokens to f16); the CTA
 // that finishes last -- found with an atomic ticket, nobody waits for anybody -- scores the
 // tokens and builds the segments.  `ticket` must be zero at launch and is left zero.
+// The kernel is latency from end to end, and its CTAs must not share an SM: started early, while the
+// previous call's last kernels still hold most SMs, two or three packed onto each free one and the chains
+// took 14.6 cycles per k instead of 6 (8 tokens, 128 experts x 2048: 30 000 of the kernel's 44 000 cycles).
+// kFrontSmem is therefore more than half of an SM's shared memory.  The last CTA runs its top-k once per call,
+// with instructions that the streamed weights have pushed out of every cache: a warp that has nothing else to do
+// runs the same code beside the chains, on router weights for logits, and drops the result.
+constexpr int kFrontStaging = 4;
+constexpr size_t kFrontSmem = 116 * 1024;
+static_assert(RouterTiny::SMEM <= kFrontSmem && (size_t)9 * topk_row_floats(32 * kMaxSlots) * sizeof(float) <= kFrontSmem - RouterTiny::SMEM,
+              "the top-k rows of eight warps and of the one that warms up lie behind the staging area");
 __global__ void __launch_bounds__(256) k_decode_front(RouteParams rp, PermuteParams pp, int max_items, unsigned int *ticket) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ PermuteSmallSmem psm;
+  __shared__ PermutePairsSmem psm;
+  __shared__ int ids[kPairwiseMax];
   __shared__ int is_last;
   coli_grid_dependency_sync();
-  if (pp.x16 && threadIdx.x >= 64) {  // this CTA's share of the f16 copy, by the staging warps
-    const int n = rp.T * (rp.H / 8);
-    const int per = (n + (int)gridDim.x - 1) / (int)gridDim.x;
-    const int lo = (int)blockIdx.x * per, hi = min(n, lo + per);
-    const uint4 *src = reinterpret_cast<const uint4 *>(rp.x);
-    uint4 *dst = reinterpret_cast<uint4 *>(pp.x16);
-    for (int i = lo + (int)threadIdx.x - 64; i < hi; i += (int)blockDim.x - 64) dst[i] = coli_bf16x8_to_f16x8(src[i]);
-  }
-  router_tiny_block<6>(rp, smem_raw, 0, (int)blockIdx.x * 8);
-  __threadfence();  // this CTA's logits are visible device-wide before its ticket is
-  __syncthreads();
-  if (threadIdx.x == 0) is_last = (atomicAdd(ticket, 1u) == gridDim.x - 1) ? 1 : 0;
-  __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
-    float *sm = reinterpret_cast<float *>(smem_raw);  // the staging area is free now
-    for (int t = warp; t < rp.T; t += nwarp) route_topk_token(rp, t, sm + (size_t)warp * topk_row_floats(rp.E), lane);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float *rows = reinterpret_cast<float *>(smem_raw + RouterTiny::SMEM);
+  RouteParams tp = rp;
+  int first = 0, step = 8, last = 0;  // the tokens that this warp scores
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {  // both passes run one copy of the top-k
+    if (pass == 0) {
+      if (warp < 2 + kFrontStaging) {
+        router_tiny_block<kFrontStaging>(rp, smem_raw, 0, (int)blockIdx.x * 8);
+      } else {
+        if (pp.x16) {  // this CTA's share of the f16 copy
+          const int n = rp.T * (rp.H / 8);
+          const int per = (n + (int)gridDim.x - 1) / (int)gridDim.x;
+          const int lo = (int)blockIdx.x * per, hi = min(n, lo + per);
+          const uint4 *src = reinterpret_cast<const uint4 *>(rp.x);
+          uint4 *dst = reinterpret_cast<uint4 *>(pp.x16);
+          for (int i = lo + (int)threadIdx.x - 32 * (2 + kFrontStaging); i < hi; i += 256 - 32 * (2 + kFrontStaging))
+            dst[i] = coli_bf16x8_to_f16x8(src[i]);
+        }
+        if (warp == 7) {
+          tp.logits = const_cast<float *>(reinterpret_cast<const float *>(rp.router_w));  // E * H bf16 hold E floats (H >= 8)
+          tp.topk_idx = nullptr;
+          last = 1;
+        }
+      }
+    } else {
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        __threadfence();  // this CTA's logits are visible device-wide before its ticket is
+        is_last = (atomicAdd(ticket, 1u) == gridDim.x - 1) ? 1 : 0;
+        __threadfence();
+      }
+      if (threadIdx.x < kPairwiseMax / 32) psm.opens[threadIdx.x] = 0u;
+      __syncthreads();
+      if (!is_last) return;
+      tp.logits = rp.logits;
+      tp.topk_idx = rp.topk_idx;
+      first = warp;
+      last = rp.T;
+    }
+    for (int t = first; t < last; t += step)
+      route_topk_token(tp, t, rows + (size_t)(pass ? warp : 8) * topk_row_floats(rp.E), lane, pass ? ids + t * rp.k : nullptr);
   }
   __syncthreads();  // the routing this CTA wrote is read back below
-  permute_small_body(pp, max_items, psm);
+  const int i = (int)threadIdx.x;
+  psm.seg[i] = i < rp.T * rp.k ? pair_segment(pp, ids[i]) : 0x7fffffff;
+  __syncthreads();
+  permute_pairs(pp, max_items, psm);
   if (threadIdx.x == 0) *ticket = 0u;
 }
 
@@ -1028,16 +1235,14 @@ static int permute_max_items(const PermuteParams &p) {
 }
 
 int launch_decode_front(const RouteParams &rp, const PermuteParams &pp, unsigned int *ticket, cudaStream_t st) {
-  constexpr size_t smem = RouterTiny::SMEM;
-  static_assert((size_t)8 * 32 * kMaxSlots * sizeof(float) <= smem, "the top-k rows of eight warps reuse the staging area");
-  if (!(rp.T >= 1 && rp.T <= 8 && rp.H % 8 == 0 && rp.E <= 32 * kMaxSlots && rp.k <= 32 &&
-        rp.n_group <= 32 && (rp.n_group <= 1 || rp.E % rp.n_group == 0) && permute_small_ok(pp) && ticket != nullptr))
+  if (!(rp.T >= 1 && rp.T <= 8 && rp.H % 8 == 0 && rp.E <= 32 * kMaxSlots && rp.k <= 32 && rp.k <= rp.E &&
+        rp.n_group <= 32 && (rp.n_group <= 1 || rp.E % rp.n_group == 0) && pp.seg_count == nullptr && ticket != nullptr))
     return -1;  // not applicable: the caller runs the separate stages
-  // (with the static lists of the permutation a CTA is above the 48 KB that need no attribute)
+  static_assert(8 * 32 <= kPairwiseMax, "a thread per pair");
   static ColiPerDeviceOnce attr_once;
-  if (!coli_set_smem_limit(attr_once, k_decode_front, smem, "decode front shared-memory attribute")) return 0;
+  if (!coli_set_smem_limit(attr_once, k_decode_front, kFrontSmem, "decode front shared-memory attribute")) return 0;
   coli_count_launch(1);
-  return coli_cuda_check(launch_dependent(k_decode_front, dim3((rp.E + 7) / 8), dim3(256), smem, st, rp, pp, permute_max_items(pp), ticket),
+  return coli_cuda_check(launch_dependent(k_decode_front, dim3((rp.E + 7) / 8), dim3(256), kFrontSmem, st, rp, pp, permute_max_items(pp), ticket),
                          "decode front launch")
              ? 1
              : 0;

@@ -1,0 +1,39 @@
+"""Top-k and permutation at the edges of their short paths: the decode front (up to 8 tokens), the pairwise
+permutation (up to 256 pairs), and the selection by counting with more candidates than a warp has lanes."""
+import numpy as np
+import pytest
+
+from speedycolibri_b200 import synth
+from speedycolibri_b200.configs import SCORE_SIGMOID, SCORE_SOFTMAX, MoeShape
+from oracle.layers import oracle_layer_from_device, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,E,k,H,score,groups,shared", [
+    (1, 32, 1, 24, SCORE_SOFTMAX, 1, False), (1, 128, 8, 520, SCORE_SOFTMAX, 1, True), (8, 40, 32, 264, SCORE_SOFTMAX, 1, True),
+    (7, 257, 8, 256, SCORE_SIGMOID, 1, True), (8, 512, 8, 1032, SCORE_SOFTMAX, 1, False), (3, 256, 8, 248, SCORE_SIGMOID, 8, True),
+    (8, 96, 6, 136, SCORE_SIGMOID, 3, True), (2, 64, 4, 512, SCORE_SIGMOID, 32, False),                    # decode front
+    (9, 70, 5, 64, SCORE_SIGMOID, 7, True), (32, 64, 8, 64, SCORE_SOFTMAX, 1, True), (33, 64, 8, 64, SCORE_SOFTMAX, 1, True),
+    (256, 300, 1, 64, SCORE_SOFTMAX, 1, True),                                                              # 256 | 264 pairs
+])
+@pytest.mark.parametrize("equal", [0, 40], ids=["distinct", "ties"])
+def test_routing_and_block_at_the_edges(gpu_backend, orc, T, E, k, H, score, groups, shared, equal):
+    from speedycolibri_b200.moe import Config, MoeBlock
+
+    shape = MoeShape("front_edges", H=H, E=E, k=k, I=16, T=T, shared=shared, norm_topk=True, score=score, n_group=groups,
+                     topk_group=max(1, (groups + 1) // 2), select_bias_std=0.0 if equal else 0.01)
+    layer = synth.device_layer(shape)
+    if equal:  # equal rows of the router give equal logits: ties go to the lowest id
+        layer.router[:equal] = layer.router[0]
+    blk = MoeBlock(Config.from_shape(shape), layer, max(T, 8))
+    x = synth.host_tokens(shape)
+    x[T // 2] = 0  # all logits of this token are equal
+    out, idx, w = blk.moe(x, want_routing=True)
+    L = oracle_layer_from_device(shape, layer, set(range(E)))
+    want = L.moe_block(x)
+    assert np.array_equal(idx, want["idx"])
+    assert np.array_equal(w.view(np.uint32), want["w"].view(np.uint32))
+    # h and y are rounded to bf16, 2^-9 relative each
+    assert rel_l2(out, want["out"]) <= 5e-3
+    blk.close()
