@@ -875,7 +875,7 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
     fp.act = m->act;
     if (!colib::launch_gate_up_small(fp, st)) return 0;
     COLI_MARK(3);
-    if (!colib::launch_down_small(fp, st)) return 0;
+    if (!colib::launch_down_small(fp, !prof, st)) return 0;  // (profiling records an event between the two)
   }
   COLI_MARK(4);
   colib::CombineParams cp;
@@ -1484,7 +1484,7 @@ static int run_host_group_relu2(ColiCudaTensor *const *ups, ColiCudaTensor *cons
   fp.h = (__half *)ctx->buf[1];
   fp.y32 = nullptr;
   fp.relu2_out = (__half *)ctx->buf[2];
-  if (!colib::launch_down_small(fp, st)) return 0;
+  if (!colib::launch_down_small(fp, false, st)) return 0;
   // down: h [total, I] -> y [total, D]
   fp.H = D;
   fp.I = I;
@@ -1492,7 +1492,7 @@ static int run_host_group_relu2(ColiCudaTensor *const *ups, ColiCudaTensor *cons
   fp.h = (__half *)ctx->buf[2];
   fp.y32 = (float *)ctx->buf[0];  // x f32 is dead once converted
   fp.relu2_out = nullptr;
-  if (!colib::launch_down_small(fp, st)) return 0;
+  if (!colib::launch_down_small(fp, false, st)) return 0;
   CK(cudaMemcpyAsync(y, ctx->buf[0], xb * sizeof(float), cudaMemcpyDeviceToHost, st), "expert output download");
   CK(cudaStreamSynchronize(st), "expert call sync");
   return 1;
@@ -1594,7 +1594,7 @@ static int run_host_matmul(ColiCudaTensor *w, float *y, const float *x, int S, c
   fp.y32 = (float *)ctx->buf[2];
   fp.relu2_out = nullptr;
   fp.act = current_activation();
-  if (!colib::launch_down_small(fp, st)) return 0;
+  if (!colib::launch_down_small(fp, false, st)) return 0;
   CK(cudaMemcpyAsync(y, ctx->buf[2], yb * sizeof(float), cudaMemcpyDeviceToHost, st), "matmul output download");
   CK(cudaStreamSynchronize(st), "matmul sync");
   return 1;

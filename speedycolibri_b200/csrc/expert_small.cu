@@ -18,10 +18,12 @@
 // per-tensor scale is applied once per output, as the reference does.  The intermediate
 // h = silu(g)*u is rounded to bf16 (then held in f16) before the down projection.
 //
-// Work decomposition: grid = (row tiles of 16 outputs, work items); an item is at most 8*NB
+// Two kernels: k_ffn_stream for items of at most eight rows (every decode call), and k_ffn_mm for the host calls
+// that hand over up to 32 rows of one matrix.
+//
+// Work decomposition of k_ffn_mm: grid = (row tiles of 16 outputs, work items); an item is at most 8*NB
 // consecutive rows of one expert segment.  The W warps of a CTA split the K axis (k-tile kt
-// goes to warp kt % W) so that even a single-token decode exposes thousands of warps, and
-// reduce through shared memory.
+// goes to warp kt % W) where there are few tasks, and reduce through shared memory.
 #include "internal.cuh"
 
 namespace colib {
@@ -31,11 +33,6 @@ __device__ __forceinline__ void mma_f16_16816(float (&d)[4], const uint32_t (&a)
       "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint32_t hmul2_f16(uint32_t a, uint32_t b) {
-  uint32_t d;
-  asm("mul.rn.f16x2 %0, %1, %2;\n" : "=r"(d) : "r"(a), "r"(b));
-  return d;
 }
 __device__ __forceinline__ uint4 ldg_nc_v4(const void *p) {
   uint4 v;
@@ -104,25 +101,25 @@ __device__ __forceinline__ void load_a(AFrag<FMT> &f, const WeightRef &w, int Op
   }
 }
 
-// Per k-tile: the lane's four block scales (rows g and g+8, two 16-k blocks each) as f16x2
-// with the scale in both halves.
+// Per k-tile: the lane's four block scales (rows g and g+8, two 16-k blocks each) as f16; the multiply takes
+// either half of a pair as its operand.
 struct AScale {
-  uint32_t lo[2], hi[2];
+  __half2 lo, hi;
 };
 template <int FMT>
 __device__ __forceinline__ AScale decode_scales(const AFrag<FMT> &f) {
-  AScale r;
+  AScale r = {};
   if (FMT == COLI_FMT_NVFP4) {
     uint32_t sl, sh;
     cvt_e4m3x4(f.sc, sl, sh);  // (s_blk0, s_blk1) of row g; of row g+8
-    r.lo[0] = __byte_perm(sl, sl, 0x1010);
-    r.lo[1] = __byte_perm(sl, sl, 0x3232);
-    r.hi[0] = __byte_perm(sh, sh, 0x1010);
-    r.hi[1] = __byte_perm(sh, sh, 0x3232);
-  } else {
-    r.lo[0] = r.lo[1] = r.hi[0] = r.hi[1] = 0;
+    r.lo = *reinterpret_cast<const __half2 *>(&sl);
+    r.hi = *reinterpret_cast<const __half2 *>(&sh);
   }
   return r;
+}
+__device__ __forceinline__ uint32_t scaled_by(uint32_t v, __half2 pair, bool high) {
+  const __half2 z = __hmul2_rn(*reinterpret_cast<const __half2 *>(&v), high ? __high2half2(pair) : __low2half2(pair));
+  return *reinterpret_cast<const uint32_t *>(&z);
 }
 
 // Decode the fragment of MMA step m (0..7) of a k-tile: a[0],a[2] = row g pairs, a[1],a[3] = row g+8.
@@ -138,11 +135,10 @@ __device__ __forceinline__ void decode_a(const AFrag<FMT> &f, const AScale &sc, 
       cvt_e2m1x4<false>(wl, l0, l1);
       cvt_e2m1x4<false>(wh, h0, h1);
     }
-    const uint32_t ml = sc.lo[m >> 2], mh = sc.hi[m >> 2];
-    a[0] = hmul2_f16(l0, ml);
-    a[2] = hmul2_f16(l1, ml);
-    a[1] = hmul2_f16(h0, mh);
-    a[3] = hmul2_f16(h1, mh);
+    a[0] = scaled_by(l0, sc.lo, m >= 4);
+    a[2] = scaled_by(l1, sc.lo, m >= 4);
+    a[1] = scaled_by(h0, sc.hi, m >= 4);
+    a[3] = scaled_by(h1, sc.hi, m >= 4);
   } else {
     const uint32_t wl = (&f.lo[m >> 2].x)[m & 3], wh = (&f.hi[m >> 2].x)[m & 3];
     cvt_e4m3x4(wl, a[0], a[2]);
@@ -388,6 +384,422 @@ __global__ void __launch_bounds__(SPLITK ? 256 : 64, SPLITK                  ? 1
 }
 
 
+// ---- items of at most eight rows: the decode kernel -----------------------------------------------------
+// A warp's task is a pair of weight slabs of 16 R rows over all of K -- gate and up of the same features, or two
+// adjacent slabs of down -- and its packed k-tiles come through a shared-memory ring of its own, filled by cp.async
+// STAGES - 1 k-tiles ahead, across the ends of tasks: no barrier between warps, and the loads never drain.
+// Two CTAs of eight warps fill an SM.  Full rounds of tasks are dealt to the warps as they are; what is left
+// (all of it when a call has few tasks) is spread over the CTAs and split over K among 2, 4 or 8 warps of a CTA,
+// as far as there are warps, so that the last round is short and a single token still loads on every SM.
+// Tasks of the down projection are known before its input is: launched behind the gate/up launch of this
+// kernel (which lets it start only when the work list is complete), its warps fill their rings first.
+//
+// What bounds it: instruction issue (0.57 of the slots; with the weight loads taken out the launches take 0.87 of
+// their time, with the token loads out 0.95, with the MMAs out 0.92), and on a large layer the power limit: packed
+// weights read at 7 TB/s and nothing else already hold this GPU at 1000 W and 1.44 GHz, so every instruction left out
+// comes back as clock.  Per 2304 bytes of weights it executes 210 warp instructions with 32-row slabs and 249 with
+// 16-row ones, 144 of them conversions, scale multiplies and MMAs; a kernel with the weights in a register ring
+// two k-tiles deep took 257, had half of a warp's time behind its loads, and needed a second wave of CTAs for a
+// single token.  Launches, before and now (us, each between events): 1 token on H 2048, I 768, 128 experts 15.0 + 10.6 ->
+// 12.5 + 10.2; 8 tokens 27.1 + 16.5 -> 23.1 + 18.5 (in a call 21.9 + 12.5 -> 18.7 + 10.0); 48 tokens 54.4 + 32.8 -> 53.3 +
+// 32.6; FP8, 21 tokens 65.1 + 34.9 -> 54.0 + 32.8; 24 tokens on H 7168, I 2048, 256 experts 448 + 239 -> 414 + 207.  Built and no
+// better: six ring stages instead of five, one CTA of 16 warps, ring slots of two k-tiles (more instructions).
+template <int FMT, int R>
+struct StreamTile {
+  static constexpr int WARPS = 8, CTAS = 2;
+  static constexpr int QB = FMT == COLI_FMT_NVFP4 ? 64 : 128;  // code bytes of a row and k-tile
+  static constexpr int SB = FMT == COLI_FMT_NVFP4 ? 8 : 0;     // scale bytes
+  static constexpr int Q = 16 * R * QB;                        // codes of one slab and k-tile
+  static constexpr int SLOT = 2 * 16 * R * (QB + SB);          // both slabs' codes, then their scales
+  static constexpr int STAGES = FMT == COLI_FMT_NVFP4 && R == 1 ? 5 : 3;
+  static constexpr int UNITS = 8 / R;                          // tasks a warp's loads may be ahead, and more
+  static_assert(UNITS > STAGES && 2 * R * 4 * 32 * 4 <= STAGES * SLOT, "task queue; partial sums reuse the ring");
+};
+struct __align__(16) StreamUnit {  // what the multiplying side of a warp needs of a task
+  int row0, nrows, r0, pad;
+  const float *sc0, *sc1;          // FP8: scales of the two slabs' matrices
+  float g0, g1;
+  int tok[8];                      // source row of each token column (columns past nrows repeat the last)
+};
+template <int FMT, int R>
+constexpr size_t stream_smem() {
+  using C = StreamTile<FMT, R>;
+  return (size_t)C::WARPS * (C::STAGES * C::SLOT + C::UNITS * sizeof(StreamUnit));
+}
+template <int FMT, bool GATED, int R>
+__global__ void __launch_bounds__(256, 2) k_ffn_stream(FfnParams p, int items_known) {
+  using C = StreamTile<FMT, R>;
+  constexpr int QB = C::QB, SB = C::SB, STAGES = C::STAGES, ROWS = GATED ? 16 * R : 32 * R;
+  constexpr bool FP4 = FMT == COLI_FMT_NVFP4;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);  // (known to be the same in all lanes)
+  const int K = GATED ? p.H : p.I, Oout = GATED ? p.I : p.H;
+  const int KT = (K + 127) >> 7, Op = (Oout + 15) & ~15;
+  const int tiles = (Op + ROWS - 1) / ROWS;  // tasks of an item
+  const __half *src = GATED ? p.x : p.h;
+  unsigned char *ring = smem_raw + warp * (STAGES * C::SLOT);
+  const uint32_t ring_u = (uint32_t)__cvta_generic_to_shared(ring), ring_end = ring_u + STAGES * C::SLOT;
+  StreamUnit *queue = reinterpret_cast<StreamUnit *>(smem_raw + C::WARPS * STAGES * C::SLOT) + warp * C::UNITS;
+
+  if (!items_known) coli_grid_wait();
+  if (GATED) coli_grid_trigger();  // behind the wait: the successor may read the work list at once
+  const int n_tasks = __ldcg(p.n_items) * tiles;
+  const int warps = (int)gridDim.x * C::WARPS;
+  const int full = n_tasks / warps, rest = n_tasks - full * warps;
+  int ks = 1;  // warps that share a task of the last round
+  while (ks < 8 && 2 * ks <= KT && rest * 2 * ks <= warps) ks *= 2;
+  const int my_rest = (warp / ks) * (int)gridDim.x + (int)blockIdx.x, piece = warp % ks;
+  const int n_units = full + (rest > 0 && my_rest < rest ? 1 : 0);
+
+  // ---- loading side ----
+  struct Item {
+    int seg, row0, nrows, tile;
+  };
+  const int dq = warps / tiles, dr = warps - dq * tiles;  // from one round's task to the next's
+  int fi, ft;
+  {
+    const int first = (int)blockIdx.x * C::WARPS + warp;
+    fi = first / tiles;
+    ft = first - fi * tiles;
+  }
+  auto fetch_item = [&](int v) {  // called for v = 0, 1, 2, ...
+    Item it = {0, 0, 1, 0};
+    if (v < n_units) {
+      if (v == full) {
+        const int task = full * warps + my_rest;
+        fi = task / tiles;
+        ft = task - fi * tiles;
+      }
+      it = {__ldcg(p.item_seg + fi), __ldcg(p.item_row0 + fi), __ldcg(p.item_nrows + fi), ft};
+      fi += dq;
+      ft += dr;
+      if (ft >= tiles) {
+        ft -= tiles;
+        ++fi;
+      }
+    }
+    return it;
+  };
+  const uint8_t *rq0 = nullptr, *rq1 = nullptr, *rs0 = nullptr, *rs1 = nullptr;  // the next unit's matrices
+  float rg0 = 0.0f, rg1 = 0.0f;
+  int rtok = 0;
+  auto fetch_ref = [&](int v, const Item &it) {
+    if (v >= n_units) return;
+    const int ex = p.seg_expert ? p.seg_expert[it.seg] : it.seg;
+    const WeightRef *a = (GATED ? p.gate : p.down) + ex;
+    rq0 = a->q, rs0 = a->s, rg0 = a->g;
+    if (GATED) {
+      const WeightRef *b = p.up + ex;
+      rq1 = b->q, rs1 = b->s, rg1 = b->g;
+    } else {
+      rq1 = rq0, rs1 = rs0, rg1 = rg0;
+    }
+    const int row = it.row0 + min(g, it.nrows - 1);
+    rtok = GATED && p.row_token ? __ldcg(p.row_token + row) : row;
+  };
+  int lv = 0, left = 0;  // unit and k-tiles that the loads are at
+  const uint8_t *q0 = nullptr, *q1 = nullptr, *sp = nullptr;
+  size_t qstep = 0, sstep = 0;
+  Item it_next = fetch_item(0), it_after = fetch_item(1);
+  fetch_ref(0, it_next);
+  auto enter_unit = [&]() {  // unit lv: its matrices have been fetched; the next one's follow
+    const int r0 = it_next.tile * ROWS;
+    const int k0 = lv < full ? 0 : piece, step = lv < full ? 1 : ks;
+    // (a missing second slab, R = 1 only: the first one again, and nothing of it is stored)
+    const int r1 = GATED ? r0 : (r0 + 16 * R < Op ? r0 + 16 * R : r0);
+    const size_t krow = (size_t)k0 * Op;
+    q0 = rq0 + (krow + r0) * QB + lane * 16;
+    q1 = rq1 + (krow + r1) * QB + lane * 16;
+    if (FP4) sp = (lane < 8 * R ? rs0 + (krow + r0) * SB : rs1 + (krow + r1) * SB) + (lane & (8 * R - 1)) * 16;
+    qstep = (size_t)step * Op * QB;
+    sstep = (size_t)step * Op * SB;
+    left = lv < full ? KT : (KT - k0 + step - 1) / step;
+    StreamUnit &u = queue[lv % C::UNITS];
+    if (lane == 0) {
+      u.row0 = it_next.row0;
+      u.nrows = it_next.nrows;
+      u.r0 = r0;
+      u.sc0 = reinterpret_cast<const float *>(rs0);
+      u.sc1 = reinterpret_cast<const float *>(rs1);
+      u.g0 = rg0;
+      u.g1 = rg1;
+    }
+    if (t == 0) u.tok[g] = rtok;
+    it_next = it_after;
+    fetch_ref(lv + 1, it_next);
+    it_after = fetch_item(lv + 2);
+  };
+  uint32_t fill = ring_u;  // the slot that is filled next
+  auto issue = [&]() {
+    if (left > 0) {
+      const uint32_t d = fill + lane * 16;
+#pragma unroll
+      for (int i = 0; i < C::Q / 512; ++i) {
+        cp_async16(d + i * 512, q0 + i * 512);
+        cp_async16(d + C::Q + i * 512, q1 + i * 512);
+      }
+      if (FP4 && lane < 16 * R) cp_async16(d + 2 * C::Q, sp);
+      q0 += qstep;
+      q1 += qstep;
+      if (FP4) sp += sstep;
+      fill += C::SLOT;
+      if (fill == ring_end) fill = ring_u;
+      if (--left == 0 && ++lv < n_units) enter_unit();
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if (n_units > 0) enter_unit();
+#pragma unroll 1
+  for (int i = 0; i < STAGES - 1; ++i) issue();
+  if (items_known) coli_grid_wait();  // the input rows
+  if (!GATED) coli_grid_trigger();
+  __syncwarp();
+
+  // ---- multiplying side ----
+  // token fragments: lane (g, t) reads x[token g][kt*128 + 32t + 8c .. +7] (16 bytes, two MMA steps), a k-tile ahead
+  const __half *xp = src;  // this lane's fragments of the k-tile loaded last
+  bool column = false;
+  const bool ragged = (K & 127) != 0;
+  auto load_x = [&](uint4 (&x)[4], int kt) {
+    if (!ragged || kt + 1 < KT) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (column) x[c] = *reinterpret_cast<const uint4 *>(xp + 8 * c);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        x[c] = make_uint4(0, 0, 0, 0);
+        if (column && kt * 128 + t * 32 + 8 * c + 8 <= K) x[c] = *reinterpret_cast<const uint4 *>(xp + 8 * c);
+      }
+    }
+  };
+  // A lane whose column is no row of the item keeps zeros: multiplied by copies of a row instead, the empty
+  // columns drew power, and on a large layer the launch runs against the power limit.
+  uint4 xa[4], xb[4];
+  auto enter_x = [&](uint4 (&x)[4], int v) {
+    const StreamUnit &e = queue[v % C::UNITS];
+    const int kt = v < full ? 0 : piece;
+    column = g < e.nrows;
+    xp = src + (size_t)e.tok[g] * K + kt * 128 + t * 32;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) x[c] = make_uint4(0, 0, 0, 0);
+    load_x(x, kt);
+  };
+  if (n_units > 0) enter_x(xa, 0);
+  // With one tile of 16 rows a slab, the steps of a k-tile add into two sets of sums in turn: eight dependent MMAs one
+  // behind the other are longer than what four warps of a scheduler hide.
+  constexpr int SETS = R == 1 ? 2 : 1, NT = 2 * R;  // tile j: rows 16 (j % R) of slab j / R
+  float acc[SETS][NT][4];
+  // where this lane reads its codes: chunk t (FP8: 2t) of row g
+  const uint32_t code_off = FP4 ? g * 64 + coli_fp4_chunk(g, t) * 16 : g * 128 + coli_fp8_chunk(g, 2 * t) * 16;
+  uint32_t base = ring_u;  // the slot in use
+  int row0 = 0, nrows = 0, r0 = 0;
+  const StreamUnit *u = queue;
+
+  // element c of the sums of slab 0 and slab 1 at row tile r
+  auto emit = [&](int c, int r, float v0, float v1) {
+    const int col = 2 * t + (c & 1), o0 = r0 + 16 * r + g + ((c & 2) ? 8 : 0), o1 = GATED ? o0 : o0 + 16 * R;
+    if (col >= nrows) return;
+    float s0 = 1.0f, s1 = 1.0f;
+    if (FP4) {
+      s0 = u->g0;
+      s1 = u->g1;
+    } else if (FMT == COLI_FMT_E4M3_ROW) {
+      s0 = o0 < Oout ? u->sc0[o0] : 0.0f;
+      s1 = o1 < Oout ? u->sc1[o1] : 0.0f;
+    }
+    const size_t row = (size_t)(row0 + col);
+    if (GATED) {
+      if (o0 < Oout) p.h[row * p.I + o0] = coli_f32_to_f16_via_bf16(coli_act_fast(v0 * s0, v1 * s1, p.act));
+      return;
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const int o = m ? o1 : o0;
+      const float v = m ? v1 * s1 : v0 * s0;
+      if (o >= Oout) continue;
+      if (p.relu2_out) {
+        const float f = fmaxf(v, 0.0f);
+        p.relu2_out[row * p.H + o] = coli_f32_to_f16_via_bf16(f * f);
+      } else if (p.y32) {
+        p.y32[row * p.H + o] = v;
+      } else {
+        p.y[row * p.H + o] = __float2bfloat16_rn(v);
+      }
+    }
+  };
+
+  // one k-tile: its token fragments are in x; `more`: the task goes on at k-tile `next`, whose fragments go to xnext,
+  // otherwise those of the next task's first k-tile do
+  auto k_tile = [&](const uint4 (&x)[4], uint4 (&xnext)[4], int v, int kt, bool more, int next) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncwarp();  // this k-tile has arrived for every lane, and the slot before it has been read by all
+    issue();
+    if (more) {
+      xp += (next - kt) * 128;
+      load_x(xnext, next);
+    } else if (v + 1 < n_units) {
+      enter_x(xnext, v + 1);
+    }
+    float kscale[2] = {1.0f, 1.0f};
+    if (FMT == COLI_FMT_FP8_B128) {  // one f32 scale per (128-row block, k-tile): convert.rs:731-741
+      const int rb = (r0 >> 7) * KT + kt;
+      kscale[0] = __ldg(u->sc0 + rb);
+      kscale[1] = GATED ? __ldg(u->sc1 + rb) : kscale[0];  // (both down slabs are in one block of 128 rows)
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      AFrag<FMT> f[2];
+      AScale asc[2];
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const uint32_t q = base + m * C::Q + r * 16 * QB;
+        if constexpr (FP4) {
+          const uint32_t sc = base + 2 * C::Q + (m * R + r) * 128 + lane * 2;
+          f[m].lo[0] = lds128(q + code_off);
+          f[m].hi[0] = lds128(q + 512 + code_off);
+          uint16_t a, b;
+          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(a) : "r"(sc) : "memory");
+          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(b) : "r"(sc + 64) : "memory");
+          f[m].sc = (uint32_t)a | ((uint32_t)b << 16);
+        } else {
+          f[m].lo[0] = lds128(q + code_off);
+          f[m].lo[1] = lds128(q + (code_off ^ 16));
+          f[m].hi[0] = lds128(q + 1024 + code_off);
+          f[m].hi[1] = lds128(q + 1024 + (code_off ^ 16));
+          f[m].sc = 0;
+        }
+        asc[m] = decode_scales<FMT>(f[m]);
+      }
+      float part[2][2][4];
+      if (FMT == COLI_FMT_FP8_B128) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) part[q][m][c] = 0.0f;
+      }
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const uint4 &xv = x[s >> 1];
+        const uint32_t b0 = (s & 1) ? xv.z : xv.x, b1 = (s & 1) ? xv.w : xv.y;
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          uint32_t a[4];
+          decode_a<FMT>(f[m], asc[m], s, a);
+          if (FMT == COLI_FMT_FP8_B128)
+            mma_f16_16816(part[s & 1][m], a, b0, b1);
+          else
+            mma_f16_16816(acc[s % SETS][m * R + r], a, b0, b1);
+        }
+      }
+      if (FMT == COLI_FMT_FP8_B128) {
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            acc[0][m * R + r][c] = fmaf(kscale[m], part[0][m][c] + part[1][m][c], acc[0][m * R + r][c]);
+      }
+    }
+    base += C::SLOT;
+    if (base == ring_end) base = ring_u;
+  };
+
+  for (int v = 0; v < n_units; ++v) {
+    u = queue + v % C::UNITS;
+    row0 = u->row0;
+    nrows = u->nrows;
+    r0 = u->r0;
+    const int step = v < full ? 1 : ks;
+#pragma unroll
+    for (int q = 0; q < SETS; ++q)
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[q][j][c] = 0.0f;
+    if (!column) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) xb[c] = make_uint4(0, 0, 0, 0);
+    }
+    int kt = v < full ? 0 : piece;
+#pragma unroll 1
+    for (; kt + step < KT; kt += 2 * step) {  // two buffers of fragments in turn: no copies between them
+      k_tile(xa, xb, v, kt, true, kt + step);
+      k_tile(xb, xa, v, kt + step, kt + 2 * step < KT, kt + 2 * step);
+    }
+    if (kt < KT) {
+      k_tile(xa, xb, v, kt, false, 0);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) xa[c] = xb[c];
+    }
+    if (SETS == 2) {
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[0][j][c] += acc[SETS - 1][j][c];
+    }
+    if (v < full || ks == 1) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) emit(c, r, acc[0][r][c], acc[0][R + r][c]);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  if (rest == 0 || ks == 1) return;
+  // partial sums of the split round, added in the order of the pieces
+  float *own = reinterpret_cast<float *>(ring);
+  __syncwarp();
+  if (n_units > full) {
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) own[(j * 4 + c) * 32 + lane] = acc[0][j][c];
+  }
+  __syncthreads();
+  if (n_units > full) {
+    const unsigned char *first = ring - (size_t)piece * (STAGES * C::SLOT);
+    for (int e = piece; e < 4 * R; e += ks) {  // element e % 4 of row tile e / 4
+      float v0 = 0.0f, v1 = 0.0f;
+      for (int w = 0; w < ks; ++w) {
+        const float *part = reinterpret_cast<const float *>(first + (size_t)w * (STAGES * C::SLOT));
+        v0 += part[e * 32 + lane];
+        v1 += part[(4 * R + e) * 32 + lane];
+      }
+      emit(e & 3, e >> 2, v0, v1);
+    }
+  }
+}
+
+template <int FMT, int R>
+static int launch_stream(const FfnParams &p, bool gated, bool items_known, cudaStream_t st) {
+  using C = StreamTile<FMT, R>;
+  constexpr size_t smem = stream_smem<FMT, R>();
+  static ColiPerDeviceOnce once[2];
+  if (!(gated ? coli_set_smem_limit(once[0], k_ffn_stream<FMT, true, R>, smem, "expert ffn shared-memory attribute")
+              : coli_set_smem_limit(once[1], k_ffn_stream<FMT, false, R>, smem, "expert ffn shared-memory attribute")))
+    return 0;
+  const dim3 grid(C::CTAS * COLI_SMS);
+  const cudaError_t e = gated ? launch_dependent(k_ffn_stream<FMT, true, R>, grid, dim3(32 * C::WARPS), smem, st, p, 0)
+                              : launch_dependent(k_ffn_stream<FMT, false, R>, grid, dim3(32 * C::WARPS), smem, st, p, items_known ? 1 : 0);
+  coli_count_launch(1);
+  return coli_cuda_check(e, "expert ffn launch") ? 1 : 0;
+}
+// Slabs of 32 rows from two rounds of such tasks on: the instructions around a k-tile are then spent on twice the
+// weights, and the tasks still divide over the warps.  24 tokens on H 7168, I 2048, 256 experts 675 -> 627 us a call; at
+// 1.3 rounds (48 tokens, H 2048, I 768, 128 experts) 108.7 -> 110.7, at 0.5 (8 tokens) 49.3 and 49.8: 16 rows there.
+// FP8 k-tiles are twice as long: two CTAs of such rings do not fit an SM.
+template <int FMT>
+static int launch_stream_rows(const FfnParams &p, bool gated, bool items_known, cudaStream_t st) {
+  if constexpr (FMT == COLI_FMT_NVFP4) {
+    const int O = gated ? p.I : p.H, rows = gated ? 32 : 64;
+    if (O % rows == 0 && (long)p.items_expected * (O / rows) >= 2L * 16 * COLI_SMS)
+      return launch_stream<FMT, 2>(p, gated, items_known, st);
+  }
+  return launch_stream<FMT, 1>(p, gated, items_known, st);
+}
 static int pick_w(int KT) { return KT >= 8 ? 8 : KT >= 4 ? 4 : KT >= 2 ? 2 : 1; }
 
 // Split K across the warps of a CTA only when there are too few (item, row tile) tasks to fill
@@ -434,7 +846,8 @@ static int launch_one(const FfnParams &p, bool gated, cudaStream_t st) {
 }
 
 // rows_per_item the caller cut the work list with selects NB (8 * NB >= rows per item).
-static int launch_ffn_stage(const FfnParams &p, bool gated, cudaStream_t st) {
+// items_known: a gate/up launch of the streaming kernel stands between the work list and this one.
+static int launch_ffn_stage(const FfnParams &p, bool gated, bool items_known, cudaStream_t st) {
   if (p.max_items <= 0) return 1;
   if (p.H % 8 || p.I % 8) {
     coli_set_error("expert ffn: H=%d and I=%d must be multiples of 8", p.H, p.I);
@@ -446,7 +859,7 @@ static int launch_ffn_stage(const FfnParams &p, bool gated, cudaStream_t st) {
   }
   const int nb = p.rows_per_item <= 8 ? 1 : p.rows_per_item <= 16 ? 2 : 4;
 #define COLI_DISPATCH(F) \
-  (nb == 1 ? launch_one<F, 1>(p, gated, st) : nb == 2 ? launch_one<F, 2>(p, gated, st) : launch_one<F, 4>(p, gated, st))
+  (nb == 1 ? launch_stream_rows<F>(p, gated, items_known, st) : nb == 2 ? launch_one<F, 2>(p, gated, st) : launch_one<F, 4>(p, gated, st))
   switch (p.fmt) {
     case COLI_FMT_NVFP4:
       return COLI_DISPATCH(COLI_FMT_NVFP4);
@@ -461,10 +874,10 @@ static int launch_ffn_stage(const FfnParams &p, bool gated, cudaStream_t st) {
 #undef COLI_DISPATCH
 }
 
-int launch_gate_up_small(const FfnParams &p, cudaStream_t st) { return launch_ffn_stage(p, true, st); }
-int launch_down_small(const FfnParams &p, cudaStream_t st) { return launch_ffn_stage(p, false, st); }
+int launch_gate_up_small(const FfnParams &p, cudaStream_t st) { return launch_ffn_stage(p, true, false, st); }
+int launch_down_small(const FfnParams &p, bool behind_gate_up, cudaStream_t st) { return launch_ffn_stage(p, false, behind_gate_up, st); }
 int launch_ffn_small(const FfnParams &p, cudaStream_t st) {
-  return launch_gate_up_small(p, st) && launch_down_small(p, st);
+  return launch_gate_up_small(p, st) && launch_down_small(p, true, st);
 }
 
 }  // namespace colib

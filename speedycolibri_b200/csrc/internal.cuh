@@ -213,7 +213,8 @@ struct FfnParams {
   ActParams act;
 };
 int launch_gate_up_small(const FfnParams &p, cudaStream_t st);  // h = silu(gate x) * (up x)
-int launch_down_small(const FfnParams &p, cudaStream_t st);     // y = down h
+// y = down h; `behind_gate_up`: launch_gate_up_small with the same work list is the launch before it in the stream
+int launch_down_small(const FfnParams &p, bool behind_gate_up, cudaStream_t st);
 int launch_ffn_small(const FfnParams &p, cudaStream_t st);      // both
 
 // expert_tc_tmem.cu — tcgen05 path for prefill-sized segments.  Token rows per work item = per tile:
