@@ -637,7 +637,7 @@ extern "C" int coli_b200_moe_create(ColiMoe **out, const ColiMoeLayer *L, int ma
   ok = ok && ws_alloc(m, &m->router_w, (size_t)E * H) && ws_alloc(m, &m->gate, E + 1) && ws_alloc(m, &m->up, E + 1) &&
        ws_alloc(m, &m->down, E + 1) && ws_alloc(m, &m->expert_slot, E) && ws_alloc(m, &m->seg_expert, E + 1) && ws_alloc(m, &m->local_slot, E) &&
        ws_alloc(m, &m->logits, T * E) && ws_alloc(m, &m->topk_w, T * k) && ws_alloc(m, &m->topk_idx, T * k) &&
-       ws_alloc(m, &m->local_rank, T * k) && ws_alloc(m, &m->chunk_cnt, (size_t)nchunk * E) &&
+       ws_alloc(m, &m->local_rank, T * k) && ws_alloc(m, &m->expert_rows, E) && ws_alloc(m, &m->chunk_cnt, (size_t)nchunk * E) &&
        ws_alloc(m, &m->seg_count, E + 1) && ws_alloc(m, &m->seg_off, E + 2) && ws_alloc(m, &m->slot, T * k) &&
        ws_alloc(m, &m->row_token, rows) && ws_alloc(m, &m->item_seg, m->item_cap) &&
        ws_alloc(m, &m->item_row0, m->item_cap) && ws_alloc(m, &m->item_nrows, m->item_cap) && ws_alloc(m, &m->n_items, 1) &&
@@ -767,6 +767,7 @@ colib::PermuteParams coli_permute_params(ColiMoe *m, const void *x_dev, int T, b
   pp.expert_slot = m->expert_slot;
   pp.local_rank = m->local_rank;
   pp.chunk_cnt = m->chunk_cnt;
+  pp.expert_rows = nullptr;
   pp.seg_count = seg_count;
   pp.seg_off = m->seg_off;
   pp.slot = slot;
@@ -821,11 +822,17 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
     pp.x16 = tc ? nullptr : m->x16;
     // decode-sized batches: one launch for router, top-k and permutation (its time is booked
     // under the router phase)
-    const int fused = T <= 8 ? colib::launch_decode_front(coli_route_params(m, x_dev, T), pp, m->ticket, st) : -1;
+    colib::RouteParams rp = coli_route_params(m, x_dev, T);
+    const int fused = T <= 8 ? colib::launch_decode_front(rp, pp, m->ticket, st) : -1;
     if (fused == 0) return 0;
-    if (fused < 0 && !colib::launch_router(coli_route_params(m, x_dev, T), st)) return 0;
+    const bool place = fused < 0 && colib::place_rows_ok(pp);
+    if (place) {
+      pp.expert_rows = rp.expert_rows = m->expert_rows;
+      rp.local_rank = m->local_rank;
+    }
+    if (fused < 0 && !colib::launch_router(rp, st)) return 0;
     COLI_MARK(1);
-    if (fused < 0 && !colib::launch_permute(pp, st)) return 0;
+    if (fused < 0 && !(place ? colib::launch_place_rows(pp, st) : colib::launch_permute(pp, st))) return 0;
   }
   COLI_MARK(2);
   if (tc) {

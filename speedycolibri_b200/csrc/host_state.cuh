@@ -53,7 +53,7 @@ struct ColiMoe {
   int32_t *local_slot;  // expert -> position among this rank's experts, or -1
   // workspace
   float *logits, *topk_w;
-  int32_t *topk_idx, *local_rank, *chunk_cnt, *seg_count, *seg_off, *slot, *row_token;
+  int32_t *topk_idx, *local_rank, *expert_rows, *chunk_cnt, *seg_count, *seg_off, *slot, *row_token;
   int32_t *item_seg, *item_row0, *item_nrows, *n_items;
   int item_cap;
   SegScratch seg_main;  // views of h / the work list / seg_off above, for run_segments

@@ -136,6 +136,8 @@ struct RouteParams {
   float *logits;                  // [T,E] scratch
   int32_t *topk_idx;              // [T,k]
   float *topk_w;                  // [T,k]
+  int32_t *expert_rows = nullptr; // [E] pairs of each expert, counted by the top-k, or null; then also
+  int32_t *local_rank = nullptr;  // [T,k] how many of its expert's pairs were counted before a pair
 };
 int launch_router(const RouteParams &p, cudaStream_t st);
 
@@ -147,6 +149,7 @@ struct PermuteParams {
   const int32_t *topk_idx;     // [T,k]
   const int32_t *expert_slot;  // [E] segment position of each expert (null = identity, < 0 = not resident)
   int32_t *local_rank;         // [T*k] scratch
+  const int32_t *expert_rows;  // [E] pairs of each expert (launch_place_rows)
   int32_t *chunk_cnt;          // [nchunk][E] scratch
   int32_t *seg_count;          // [E] out: rows per segment (segment order), or null when nobody reads them
   int32_t *seg_off;            // [E+2] out: exclusive offsets (+shared)
@@ -183,6 +186,10 @@ int launch_permute(const PermuteParams &p, cudaStream_t st);
 // success, 0 on error, -1 when the shapes do not qualify (run launch_router + launch_permute).
 // `ticket` is a device word that is zero between launches.
 int launch_decode_front(const RouteParams &rp, const PermuteParams &pp, unsigned int *ticket, cudaStream_t st);
+// The permutation of a batch whose top-k was given expert_rows and local_rank, where place_rows_ok says so: one launch.
+// Rows of an expert come in the order in which the top-k counted them.
+bool place_rows_ok(const PermuteParams &p);
+int launch_place_rows(const PermuteParams &p, cudaStream_t st);
 // Work list for rows that are already expert-contiguous (counts on the device).
 int launch_items_from_counts(const int32_t *seg_count, int nseg, int rows_per_item, int32_t *seg_off,
                              int32_t *item_seg, int32_t *item_row0, int32_t *item_nrows, int32_t *n_items,

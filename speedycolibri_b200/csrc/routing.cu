@@ -20,6 +20,12 @@
 
 namespace colib {
 
+// The counts that the top-k behind a router launch adds to (RouteParams::expert_rows) are cleared by that launch.
+__device__ __forceinline__ void clear_expert_rows(const RouteParams &p) {
+  if (p.expert_rows && blockIdx.x + blockIdx.y == 0)
+    for (int e = threadIdx.x; e < p.E; e += blockDim.x) p.expert_rows[e] = 0;
+}
+
 // ---------------------------------------------------------------------------------------------
 // Router GEMM, general shape.  Block = 16x16 threads, thread tile TM x TN, k-chunk 32 staged in
 // shared memory as f32 (transposed so the inner loop reads broadcast / consecutive words).
@@ -27,6 +33,7 @@ namespace colib {
 template <int TM, int TN>
 __global__ void __launch_bounds__(256) k_router_gemm(RouteParams p) {
   coli_grid_trigger();  // the top-k may be scheduled; it waits for this grid
+  clear_expert_rows(p);
   constexpr int BM = 16 * TM, BN = 16 * TN, BK = 32;
   __shared__ float xs[BK][BM + 4];
   __shared__ float ws[BK][BN + 4];
@@ -117,6 +124,7 @@ struct RouterPairTile {
 template <class C>
 __global__ void __launch_bounds__(C::NT) k_router_pair(RouteParams p) {
   coli_grid_trigger();  // the top-k may be scheduled; it waits for this grid
+  clear_expert_rows(p);
   constexpr int TM = C::TM, TN = C::TN, BK = C::BK, LD = C::LD, BM = C::BM;
   extern __shared__ __align__(16) float rsm[];
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * C::BN;
@@ -236,6 +244,7 @@ struct RouterTile {
 template <class C>
 __global__ void __launch_bounds__(C::NT) k_router_chain(RouteParams p) {
   coli_grid_trigger();  // the top-k may be scheduled; it waits for this grid
+  clear_expert_rows(p);
   constexpr int TM = C::TM, TN = C::TN, RS = C::RS, CH = C::CH, BM = C::BM, BN = C::BN;
   constexpr bool SMALL = TM * TN <= 8;  // the next chunk's operands are loaded ahead of this one's FMAs
   constexpr bool PAIRED = TM % 2 == 0;  // two tokens per FMA instruction (3 to 6 % at every tile that can)
@@ -667,6 +676,7 @@ __device__ __forceinline__ void route_topk_slots(const RouteParams &p, int t, fl
     if (p.topk_idx) {
       p.topk_idx[(size_t)t * k + lane] = id;
       p.topk_w[(size_t)t * k + lane] = __fmul_rn(w, p.routed_scale);
+      if (p.expert_rows) p.local_rank[(size_t)t * k + lane] = atomicAdd(p.expert_rows + id, 1);
     }
     if (ids_out) ids_out[lane] = id;
   }
@@ -679,6 +689,16 @@ __device__ __forceinline__ void route_topk_token(const RouteParams &p, int t, fl
     route_topk_slots<8>(p, t, row, lane, ids_out);
   else
     route_topk_slots<kMaxSlots>(p, t, row, lane, ids_out);
+}
+
+// The same chains for batches above 8 tokens whose 8 x 8 tiles have an SM each (its shared memory sees to that).
+constexpr size_t kStagedSmem = 116 * 1024;
+static_assert(RouterTiny::SMEM <= kStagedSmem, "staging area");
+__global__ void __launch_bounds__(192) k_router_staged(RouteParams p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  coli_grid_trigger();  // the top-k may be scheduled; it waits for this grid
+  clear_expert_rows(p);
+  router_tiny_block<4>(p, smem_raw, (int)blockIdx.x * 8, (int)blockIdx.y * 8);
 }
 
 __global__ void __launch_bounds__(128) k_route_topk(RouteParams p) {
@@ -719,7 +739,7 @@ static bool launch_router_pair(const RouteParams &p, cudaStream_t st) {
 // conversions, when an SM has little else).
 static int pick_router_tile(int T, int E) {
   auto n = [&](int bm, int bn) { return (float)(((long)((T + bm - 1) / bm) * ((E + bn - 1) / bn) + COLI_SMS - 1) / COLI_SMS); };
-  const float ns[5] = {fmaxf(5.3f, 1.6f * n(8, 8)), fmaxf(10.0f, 3.0f + 5.6f * n(16, 32)), 3.0f + 33.0f * n(64, 64),
+  const float ns[5] = {n(8, 8) <= 1.0f ? 2.8f : fmaxf(5.3f, 1.6f * n(8, 8)), fmaxf(10.0f, 3.0f + 5.6f * n(16, 32)), 3.0f + 33.0f * n(64, 64),
                        5.0f + 46.5f * n(128, 64), 8.0f + 81.0f * n(128, 128)};
   int best = 0;
   for (int i = 1; i < 5; ++i)
@@ -727,8 +747,18 @@ static int pick_router_tile(int T, int E) {
   return best;
 }
 
-int launch_router(const RouteParams &p, cudaStream_t st) {
-  if (p.T <= 0) return 1;
+// 8 x 8 tiles with an SM to themselves take the staged kernel: 2.8 ns a k against 5.3 of the chain kernel, which holds
+// its rows as bf16 and widens them between the FMAs (launches of 21 tokens x 128 experts x 2048 9 us, 24 x 256 x 7168 24).
+// Two of its CTAs on an SM would be no faster than the chain kernel's.
+static long router_tiles_8x8(int T, int E) { return (long)((T + 7) / 8) * ((E + 7) / 8); }
+static bool launch_router_staged(const RouteParams &p, cudaStream_t st) {
+  static ColiPerDeviceOnce attr_once;
+  if (!coli_set_smem_limit(attr_once, k_router_staged, kStagedSmem, "router shared-memory attribute")) return false;
+  k_router_staged<<<dim3((p.T + 7) / 8, (p.E + 7) / 8), 192, kStagedSmem, st>>>(p);
+  return true;
+}
+
+static int launch_router_logits(const RouteParams &p, cudaStream_t st) {
   if (p.E > 32 * kMaxSlots) {
     coli_set_error("router: E=%d exceeds the supported maximum of %d", p.E, 32 * kMaxSlots);
     return 0;
@@ -746,7 +776,7 @@ int launch_router(const RouteParams &p, cudaStream_t st) {
   if (rows16) {
     bool ok = false;
     switch (pick_router_tile(p.T, p.E)) {
-      case 0: ok = launch_router_chain<RouterTile8x8>(p, st); break;
+      case 0: ok = router_tiles_8x8(p.T, p.E) <= COLI_SMS ? launch_router_staged(p, st) : launch_router_chain<RouterTile8x8>(p, st); break;
       case 1: ok = launch_router_chain<RouterTile16x32>(p, st); break;
       case 2: ok = launch_router_chain<RouterTile64x64>(p, st); break;
       case 3: ok = launch_router_pair<RouterTile128x64>(p, st); break;
@@ -759,8 +789,20 @@ int launch_router(const RouteParams &p, cudaStream_t st) {
     k_router_gemm<1, 1><<<dim3((p.E + 15) / 16, (p.T + 15) / 16), 256, 0, st>>>(p);
   }
   coli_count_launch(1);
-  const size_t sm = (size_t)4 * topk_row_floats(p.E) * sizeof(float);
-  if (!coli_cuda_check(cudaGetLastError(), "router launch")) return 0;
+  return coli_cuda_check(cudaGetLastError(), "router launch") ? 1 : 0;
+}
+
+constexpr int kSmSharedBytes = 228 * 1024;
+int launch_router(const RouteParams &p, cudaStream_t st) {
+  if (p.T <= 0) return 1;
+  if (!launch_router_logits(p, st)) return 0;
+  // Shared memory for no more CTAs on an SM than an even spread puts there: started early they pack onto the SMs that
+  // are free (512 tokens, 128 experts: 6500 cycles a token where one alone takes 3500).
+  const int ctas = (p.T + 3) / 4, per_sm = (ctas + COLI_SMS - 1) / COLI_SMS;
+  size_t sm = (size_t)4 * topk_row_floats(p.E) * sizeof(float);
+  if (per_sm <= 4 && sm < (size_t)kSmSharedBytes / (per_sm + 1)) sm = (size_t)kSmSharedBytes / (per_sm + 1);
+  static ColiPerDeviceOnce attr_once;
+  if (!coli_set_smem_limit(attr_once, k_route_topk, kSmSharedBytes / 2, "top-k shared-memory attribute")) return 0;
   coli_count_launch(1);
   return coli_cuda_check(launch_dependent(k_route_topk, dim3((p.T + 3) / 4), dim3(128), sm, st, p), "top-k launch") ? 1 : 0;
 }
@@ -1059,39 +1101,41 @@ __device__ __forceinline__ void permute_small_body(const PermuteParams &p, int m
 // The same for at most 256 pairs in a block that wants no counts per segment: a thread per pair finds its row --
 // the pairs of lower segments and the earlier ones of its own -- by comparing with every other pair, and the
 // item that a row opens by the rows that open one before it (a bit per row).  Two barriers and no scan over
-// the segments: the steps above take 3300 cycles for 8 pairs of 128 experts on a warm SM, this 500.
+// the segments.  Called by `threads` threads of a CTA, numbered i, that meet at barrier `bar`.
 // `seg` holds the pairs' segments (below 0: no row), padded to a multiple of 4 entries with INT_MAX, and `opens`
-// eight zeros; both are visible to the CTA.
+// eight zeros; both are visible to those threads.  A dry run writes nothing.
 constexpr int kPairwiseMax = 256;
 struct PermutePairsSmem {
   __align__(16) int seg[kPairwiseMax];
   int pos[kPairwiseMax];
   uint32_t opens[kPairwiseMax / 32];
 };
-__device__ __forceinline__ void permute_pairs(const PermuteParams &p, int max_items, PermutePairsSmem &sm) {
-  const int n = p.T * p.k, i = (int)threadIdx.x, rpi = p.rows_per_item;
+__device__ __forceinline__ void permute_pairs(const PermuteParams &p, int max_items, PermutePairsSmem &sm, int i, int threads, int bar, bool dry) {
+  const int n = p.T * p.k, rpi = p.rows_per_item;
   int s = -1, below = 0, before = 0, equal = 0, share = 1;
   if (i < n) s = sm.seg[i];
   if (s >= 0) {
-#pragma unroll 2
     for (int j = 0; j < n; j += 4) {
       const int4 q = *reinterpret_cast<const int4 *>(sm.seg + j);
       below += ((unsigned)q.x < (unsigned)s) + ((unsigned)q.y < (unsigned)s) + ((unsigned)q.z < (unsigned)s) + ((unsigned)q.w < (unsigned)s);
-      const int eq = (q.x == s) | (q.y == s) << 1 | (q.z == s) << 2 | (q.w == s) << 3;
-      equal += __popc(eq);
-      before += i <= j ? 0 : __popc(i >= j + 4 ? eq : eq & ((1 << (i - j)) - 1));
+      equal += (q.x == s) + (q.y == s) + (q.z == s) + (q.w == s);
+      before += (q.x == s && j < i) + (q.y == s && j + 1 < i) + (q.z == s && j + 2 < i) + (q.w == s && j + 3 < i);
     }
     share = work_item_rows(equal, rpi);
   }
   const int pos = below + before;
   const bool opens = s >= 0 && before % share == 0;
-  if (i < n) {
+  if (i < n && !dry) {
     sm.pos[i] = s >= 0 ? pos : -1;
     p.slot[i] = s >= 0 ? pos : -1;
     if (s >= 0) p.row_token[pos] = i / p.k;
   }
   if (opens) atomicOr(&sm.opens[pos >> 5], 1u << (pos & 31));
-  const int rows = __syncthreads_count(s >= 0);  // the shared expert's rows follow them
+  int rows;  // the shared expert's rows follow them
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %3, 0;\nbarrier.cta.red.popc.aligned.u32 %0, %1, %2, p;\n}"
+               : "=r"(rows)
+               : "r"(bar), "r"(threads), "r"(s >= 0 ? 1 : 0)
+               : "memory");
   int items = 0, item = 0;
 #pragma unroll
   for (int w = 0; w < kPairwiseMax / 32; ++w) {
@@ -1100,26 +1144,26 @@ __device__ __forceinline__ void permute_pairs(const PermuteParams &p, int max_it
     if (w == (pos >> 5)) item += __popc(bits & ((1u << (pos & 31)) - 1u));
     items += __popc(bits);
   }
-  if (opens && item < max_items) {
+  if (opens && item < max_items && !dry) {
     p.item_seg[item] = s;
     p.item_row0[item] = pos;
     p.item_nrows[item] = min(share, equal - before);
   }
   if (p.has_shared) {
     const int sshare = work_item_rows(p.T, rpi), nsh = (p.T + sshare - 1) / sshare;
-    if (i < nsh && items + i < max_items) {
+    if (i < nsh && items + i < max_items && !dry) {
       p.item_seg[items + i] = p.nseg_routed;
       p.item_row0[items + i] = rows + i * sshare;
       p.item_nrows[items + i] = min(sshare, p.T - i * sshare);
     }
-    if (i < p.T) p.row_token[rows + i] = i;
+    if (i < p.T && !dry) p.row_token[rows + i] = i;
     items += nsh;
   }
-  if (i == 0) *p.n_items = min(items, max_items);
-  if (p.xg) {  // gather rows: one warp per row
+  if (i == 0 && !dry) *p.n_items = min(items, max_items);
+  if (p.xg && !dry) {  // gather rows: one warp per row
     const int total = n + ((p.has_shared && p.gather_shared) ? p.T : 0);
     const int vec = p.H / 8;
-    for (int r = i >> 5; r < total; r += (int)blockDim.x >> 5) {
+    for (int r = i >> 5; r < total; r += threads >> 5) {
       const int t = r < n ? r / p.k : r - n, to = r < n ? sm.pos[r] : rows + t;
       if (to < 0) continue;
       const uint4 *src = reinterpret_cast<const uint4 *>(p.x + (size_t)t * p.H);
@@ -1135,10 +1179,7 @@ __device__ __forceinline__ int pair_segment(const PermuteParams &p, int id) {
 
 __global__ void __launch_bounds__(1024) k_permute_small(PermuteParams p, int max_items) {
   coli_grid_wait();
-  __shared__ union {
-    PermuteSmallSmem all;
-    PermutePairsSmem pairs;
-  } sm;
+  __shared__ PermuteSmallSmem sm;
   if (blockIdx.x > 0) {  // the extra CTAs only write the token-order f16 copy of x
     const size_t n = (size_t)p.T * p.H / 8;
     const uint4 *src = reinterpret_cast<const uint4 *>(p.x);
@@ -1147,15 +1188,7 @@ __global__ void __launch_bounds__(1024) k_permute_small(PermuteParams p, int max
       dst[i] = coli_bf16x8_to_f16x8(src[i]);
     return;
   }
-  const int n = p.T * p.k;
-  if (p.seg_count || n > kPairwiseMax) {
-    permute_small_body(p, max_items, sm.all);
-    return;
-  }
-  for (int i = threadIdx.x; i < kPairwiseMax; i += blockDim.x) sm.pairs.seg[i] = i < n ? pair_segment(p, p.topk_idx[i]) : 0x7fffffff;
-  if (threadIdx.x < kPairwiseMax / 32) sm.pairs.opens[threadIdx.x] = 0u;
-  __syncthreads();
-  permute_pairs(p, max_items, sm.pairs);
+  permute_small_body(p, max_items, sm);
 }
 
 // Decode front end (T <= 8): router logits, top-k and the permutation in ONE launch.  Every CTA
@@ -1165,44 +1198,44 @@ __global__ void __launch_bounds__(1024) k_permute_small(PermuteParams p, int max
 // The kernel is latency from end to end, and its CTAs must not share an SM: started early, while the
 // previous call's last kernels still hold most SMs, two or three packed onto each free one and the chains
 // took 14.6 cycles per k instead of 6 (8 tokens, 128 experts x 2048: 30 000 of the kernel's 44 000 cycles).
-// kFrontSmem is therefore more than half of an SM's shared memory.  The last CTA runs its top-k once per call,
-// with instructions that the streamed weights have pushed out of every cache: a warp that has nothing else to do
-// runs the same code beside the chains, on router weights for logits, and drops the result.
-constexpr int kFrontStaging = 4;
+// kFrontSmem is therefore more than half of an SM's shared memory.  The last CTA runs top-k and permutation once per
+// call, with instructions that the streamed weights have pushed out of every cache: two warps that have nothing else to
+// do run the same code beside the chains, on router weights for logits, and write nothing (8 tokens, the weights of
+// three layers in turn: top-k 2.4 us, permutation 4.6 -> 1.8; the front 15.9 -> 14.4 us).
+constexpr int kFrontStaging = 4, kFrontDry = 64;  // staging warps; threads of the dry run
 constexpr size_t kFrontSmem = 116 * 1024;
 static_assert(RouterTiny::SMEM <= kFrontSmem && (size_t)9 * topk_row_floats(32 * kMaxSlots) * sizeof(float) <= kFrontSmem - RouterTiny::SMEM,
-              "the top-k rows of eight warps and of the one that warms up lie behind the staging area");
+              "the top-k rows of eight warps and of the dry run lie behind the staging area");
 __global__ void __launch_bounds__(256) k_decode_front(RouteParams rp, PermuteParams pp, int max_items, unsigned int *ticket) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ PermutePairsSmem psm;
   __shared__ int ids[kPairwiseMax];
   __shared__ int is_last;
   coli_grid_dependency_sync();
+  constexpr int first_dry = 256 - kFrontDry;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float *rows = reinterpret_cast<float *>(smem_raw + RouterTiny::SMEM);
   RouteParams tp = rp;
-  int first = 0, step = 8, last = 0;  // the tokens that this warp scores
+  int first = 0, last = 0;  // the tokens that this warp scores
 #pragma unroll 1
-  for (int pass = 0; pass < 2; ++pass) {  // both passes run one copy of the top-k
-    if (pass == 0) {
-      if (warp < 2 + kFrontStaging) {
+  for (int pass = 0; pass < 2; ++pass) {  // both passes run one copy of the code
+    const bool dry = pass == 0;
+    if (dry) {
+      if ((int)threadIdx.x < first_dry) {
         router_tiny_block<kFrontStaging>(rp, smem_raw, 0, (int)blockIdx.x * 8);
-      } else {
-        if (pp.x16) {  // this CTA's share of the f16 copy
-          const int n = rp.T * (rp.H / 8);
-          const int per = (n + (int)gridDim.x - 1) / (int)gridDim.x;
-          const int lo = (int)blockIdx.x * per, hi = min(n, lo + per);
-          const uint4 *src = reinterpret_cast<const uint4 *>(rp.x);
-          uint4 *dst = reinterpret_cast<uint4 *>(pp.x16);
-          for (int i = lo + (int)threadIdx.x - 32 * (2 + kFrontStaging); i < hi; i += 256 - 32 * (2 + kFrontStaging))
-            dst[i] = coli_bf16x8_to_f16x8(src[i]);
-        }
-        if (warp == 7) {
-          tp.logits = const_cast<float *>(reinterpret_cast<const float *>(rp.router_w));  // E * H bf16 hold E floats (H >= 8)
-          tp.topk_idx = nullptr;
-          last = 1;
-        }
+        continue;
       }
+      if (pp.x16) {  // this CTA's share of the f16 copy
+        const int n = rp.T * (rp.H / 8);
+        const int per = (n + (int)gridDim.x - 1) / (int)gridDim.x;
+        const int lo = (int)blockIdx.x * per, hi = min(n, lo + per);
+        const uint4 *src = reinterpret_cast<const uint4 *>(rp.x);
+        uint4 *dst = reinterpret_cast<uint4 *>(pp.x16);
+        for (int i = lo + (int)threadIdx.x - first_dry; i < hi; i += kFrontDry) dst[i] = coli_bf16x8_to_f16x8(src[i]);
+      }
+      tp.logits = const_cast<float *>(reinterpret_cast<const float *>(rp.router_w));  // E * H bf16 hold E floats (H >= 8)
+      tp.topk_idx = nullptr;
+      last = warp == 7 ? 1 : 0;
     } else {
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -1210,7 +1243,6 @@ __global__ void __launch_bounds__(256) k_decode_front(RouteParams rp, PermutePar
         is_last = (atomicAdd(ticket, 1u) == gridDim.x - 1) ? 1 : 0;
         __threadfence();
       }
-      if (threadIdx.x < kPairwiseMax / 32) psm.opens[threadIdx.x] = 0u;
       __syncthreads();
       if (!is_last) return;
       tp.logits = rp.logits;
@@ -1218,15 +1250,85 @@ __global__ void __launch_bounds__(256) k_decode_front(RouteParams rp, PermutePar
       first = warp;
       last = rp.T;
     }
-    for (int t = first; t < last; t += step)
-      route_topk_token(tp, t, rows + (size_t)(pass ? warp : 8) * topk_row_floats(rp.E), lane, pass ? ids + t * rp.k : nullptr);
+    const int i = (int)threadIdx.x - (dry ? first_dry : 0), threads = dry ? kFrontDry : 256, bar = dry ? 2 : 0;
+    for (int t = first; t < last; t += 8)
+      route_topk_token(tp, t, rows + (size_t)(dry ? 8 : warp) * topk_row_floats(rp.E), lane, ids + t * rp.k);
+    if (i < kPairwiseMax / 32) psm.opens[i] = 0u;
+    asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(bar), "r"(threads) : "memory");  // the routing is read back below
+    for (int j = i; j < kPairwiseMax; j += threads) psm.seg[j] = j < (dry ? rp.k : rp.T * rp.k) ? pair_segment(pp, ids[j]) : 0x7fffffff;
+    asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(bar), "r"(threads) : "memory");
+    permute_pairs(pp, max_items, psm, i, threads, bar, dry);
   }
-  __syncthreads();  // the routing this CTA wrote is read back below
-  const int i = (int)threadIdx.x;
-  psm.seg[i] = i < rp.T * rp.k ? pair_segment(pp, ids[i]) : 0x7fffffff;
-  __syncthreads();
-  permute_pairs(pp, max_items, psm);
   if (threadIdx.x == 0) *ticket = 0u;
+}
+
+// Rows of a batch whose top-k has counted them (RouteParams::expert_rows): every pair knows its rank among its
+// expert's, so what is left is a sum over the segments, which each CTA makes for itself, and the rows.  CTA 0 builds the
+// work list while the others write: a warp per (t, kk) row, rows T*k .. T*k+T-1 are the shared expert's, and when
+// a token-order f16 copy of x is wanted, a warp more for each 1024 elements of it.
+// Against launches for counts per 32 tokens, one CTA's scan over them and the rows (up to 1024 pairs: one CTA for all
+// of it), us a call: 333 tokens, H 1024, 32 experts 50.3 -> 44.1; 512 tokens, H 2048, 128 experts 186.9 -> 177.2; 21 tokens
+// 96.7 -> 92.7; 48 tokens 111.8 -> 101.8 (these two with the router above).  The whole permutation by the last CTA of the top-k
+// was built too: its code, cold and run once, took 10 us more than these launches.
+__global__ void __launch_bounds__(256) k_place_rows(PermuteParams p, int max_items) {
+  __shared__ int cnt[32 * kMaxSlots + 1], off[32 * kMaxSlots + 2], ibase[32 * kMaxSlots + 2];
+  coli_grid_dependency_sync();
+  const int nrt = p.nseg_routed, nseg = nrt + (p.has_shared ? 1 : 0), nrouted = p.T * p.k;
+  const int warp = (((int)blockIdx.x - 1) * (int)blockDim.x + (int)threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  // what this warp's row needs of the routing is requested beside the counts
+  int e = -1, rank = 0;
+  if (blockIdx.x > 0 && warp < nrouted) {
+    e = p.topk_idx[warp];
+    rank = p.local_rank[warp];
+  }
+  for (int i = threadIdx.x; i < p.E; i += blockDim.x) {
+    const int s = pair_segment(p, i);
+    if (s >= 0) cnt[s] = p.expert_rows[i];
+  }
+  if (threadIdx.x == 0 && p.has_shared) cnt[nrt] = p.T;
+  __syncthreads();
+  if (blockIdx.x == 0) {
+    build_work_list(p, cnt, nseg, max_items, off, ibase);
+    return;
+  }
+  const int total = nrouted + (p.has_shared ? p.T : 0);
+  const int seg = warp < nrouted ? pair_segment(p, e) : nrt;
+  int first = 0;  // rows of the segments before this warp's
+  if (warp < total)
+    for (int i = lane; i < seg; i += 32) first += cnt[i];
+  first = __reduce_add_sync(0xffffffffu, first);
+  if (warp >= total) {
+    if (p.x16) {
+      const int n = p.T * (p.H / 8), base = (warp - total) * 128 + lane;
+      const uint4 *src = reinterpret_cast<const uint4 *>(p.x);
+      uint4 *dst = reinterpret_cast<uint4 *>(p.x16), v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = base + 32 * u < n ? src[base + 32 * u] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (base + 32 * u < n) dst[base + 32 * u] = coli_bf16x8_to_f16x8(v[u]);
+    }
+    return;
+  }
+  const int t = warp < nrouted ? warp / p.k : warp - nrouted;
+  const int pos = first + (warp < nrouted ? rank : t);
+  if (lane == 0) {
+    if (warp < nrouted) p.slot[warp] = seg < 0 ? -1 : pos;
+    if (seg >= 0) p.row_token[pos] = t;
+  }
+  if (!p.xg || seg < 0 || (warp >= nrouted && !p.gather_shared)) return;
+  const int vec = p.H / 8;
+  const uint4 *src = reinterpret_cast<const uint4 *>(p.x + (size_t)t * p.H);
+  uint4 *dst = reinterpret_cast<uint4 *>(p.xg + (size_t)pos * p.H);
+  int c = lane;
+  for (; c + 96 < vec; c += 128) {  // four loads in flight per lane
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = src[c + 32 * u];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) dst[c + 32 * u] = coli_bf16x8_to_f16x8(v[u]);
+  }
+  for (; c < vec; c += 32) dst[c] = coli_bf16x8_to_f16x8(src[c]);
 }
 
 static bool permute_small_ok(const PermuteParams &p) { return p.T * p.k <= 1024 && p.k <= 32 && p.E <= 1024; }
@@ -1246,6 +1348,20 @@ int launch_decode_front(const RouteParams &rp, const PermuteParams &pp, unsigned
                          "decode front launch")
              ? 1
              : 0;
+}
+
+// Whether a batch's rows are counted by its top-k and placed in one launch.  Gathered rows of up to 1024 pairs that
+// are more than the one-CTA permutation takes (128 KB) keep the separate stages, whose number of launches callers
+// count on; above 65536 pairs the atomic counts of a popular expert queue up.
+bool place_rows_ok(const PermuteParams &p) {
+  const long pairs = (long)p.T * p.k;
+  if (p.virt || p.seg_count || p.rows_cap != 0x7fffffff || p.E > 32 * kMaxSlots || pairs > 65536) return false;
+  return !p.xg || pairs > 1024 || (size_t)p.T * (p.k + 1) * p.H * 2 <= 128 * 1024;
+}
+int launch_place_rows(const PermuteParams &p, cudaStream_t st) {
+  const int warps = p.T * p.k + (p.has_shared ? p.T : 0) + (p.x16 ? (int)(((size_t)p.T * (p.H / 8) + 127) / 128) : 0);
+  coli_count_launch(1);
+  return coli_cuda_check(launch_dependent(k_place_rows, dim3(1 + (warps + 7) / 8), dim3(256), 0, st, p, permute_max_items(p)), "row placement launch") ? 1 : 0;
 }
 
 int launch_permute(const PermuteParams &p, cudaStream_t st) {

@@ -1,5 +1,6 @@
-"""Top-k and permutation at the edges of their short paths: the decode front (up to 8 tokens), the pairwise
-permutation (up to 256 pairs), and the selection by counting with more candidates than a warp has lanes."""
+"""Router, top-k and permutation at the edges of their paths: the decode front (up to 8 tokens), the staged router
+(8 x 8 tiles up to the number of SMs), rows placed by the counts of the top-k (with a copy of x up to and with
+gathered rows above 1024 pairs), and the selection by counting with more candidates than a warp has lanes."""
 import numpy as np
 import pytest
 
@@ -15,7 +16,11 @@ pytestmark = pytest.mark.gpu
     (7, 257, 8, 256, SCORE_SIGMOID, 1, True), (8, 512, 8, 1032, SCORE_SOFTMAX, 1, False), (3, 256, 8, 248, SCORE_SIGMOID, 8, True),
     (8, 96, 6, 136, SCORE_SIGMOID, 3, True), (2, 64, 4, 512, SCORE_SIGMOID, 32, False),                    # decode front
     (9, 70, 5, 64, SCORE_SIGMOID, 7, True), (32, 64, 8, 64, SCORE_SOFTMAX, 1, True), (33, 64, 8, 64, SCORE_SOFTMAX, 1, True),
-    (256, 300, 1, 64, SCORE_SOFTMAX, 1, True),                                                              # 256 | 264 pairs
+    (256, 300, 1, 64, SCORE_SOFTMAX, 1, True), (32, 296, 8, 1032, SCORE_SOFTMAX, 1, False),                 # 148 tiles of the staged router
+    (33, 296, 8, 520, SCORE_SIGMOID, 1, True), (130, 400, 8, 264, SCORE_SOFTMAX, 1, True),                  # ... 185 tiles; 1040 pairs, x copied
+    (12, 4, 4, 264, SCORE_SOFTMAX, 1, True), (170, 20, 6, 264, SCORE_SOFTMAX, 1, True),                     # gathered: 31 KB | 1020 pairs, 628 KB
+    (171, 20, 6, 264, SCORE_SOFTMAX, 1, True), (600, 512, 32, 72, SCORE_SIGMOID, 1, False),                 # 1026 and 19200 pairs
+    (2049, 40, 32, 24, SCORE_SOFTMAX, 1, True),                                                             # above 65536 pairs
 ])
 @pytest.mark.parametrize("equal", [0, 40], ids=["distinct", "ties"])
 def test_routing_and_block_at_the_edges(gpu_backend, orc, T, E, k, H, score, groups, shared, equal):
