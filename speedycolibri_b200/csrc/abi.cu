@@ -36,6 +36,7 @@ namespace {
 std::mutex g_init_mu;
 DeviceContext *g_ctx[COLI_CUDA_MAX_DEVICES];
 int g_ndev = 0;
+colib_host::CopyPool g_copy_pool;
 int g_act_oai = 0;  // process-wide gate/up combine, backend_cuda.cu:339-350
 float g_act_alpha = 1.702f;
 float g_act_limit = 0.0f;
@@ -123,11 +124,13 @@ extern "C" void coli_cuda_shutdown(void) {
       if (c->buf[s]) cudaFree(c->buf[s]);
     for (int s = 0; s < 4; ++s)
       if (c->ev[s]) cudaEventDestroy(c->ev[s]);
+    c->ring.release();
     cudaStreamDestroy(c->stream);
     delete c;
     g_ctx[i] = nullptr;
   }
   g_ndev = 0;
+  g_copy_pool.stop();
 }
 extern "C" int coli_cuda_device_count(void) { return g_ndev; }
 extern "C" int coli_cuda_device_at(int index) { return (index >= 0 && index < g_ndev) ? g_ctx[index]->device : -1; }
@@ -965,6 +968,17 @@ extern "C" int coli_b200_moe_last_routing(ColiMoe *m, int T, int32_t *topk_idx, 
   return 1;
 }
 
+namespace {
+struct StreamWait {
+  cudaStream_t st;
+  bool pending = true;
+  explicit StreamWait(cudaStream_t s) : st(s) {}
+  ~StreamWait() {
+    if (pending) cudaStreamSynchronize(st);
+  }
+};
+}  // namespace
+
 extern "C" int coli_b200_moe_block(ColiMoe *m, const void *x, void *out, int T, int32_t *topk_idx, float *topk_w) {
   if (!coli_check_T(m, T, "moe_block")) return 0;
   if (!x || !out) {
@@ -975,13 +989,22 @@ extern "C" int coli_b200_moe_block(ColiMoe *m, const void *x, void *out, int T, 
   std::lock_guard<std::mutex> lk(m->ctx->mu);
   cudaStream_t st = m->ctx->stream;
   const size_t bytes = (size_t)T * m->L.H * sizeof(__nv_bfloat16);
-  CK(cudaMemcpyAsync(m->x_stage, x, bytes, cudaMemcpyHostToDevice, st), "moe_block input upload");
+  StreamWait wait(st);  // whatever fails below: nothing of the caller's is in use when the call returns
+  colib_host::HostCopies copies(m->ctx->ring, g_copy_pool, st);
+  if (!copies.staged(x, bytes))
+    CK(cudaMemcpyAsync(m->x_stage, x, bytes, cudaMemcpyHostToDevice, st), "moe_block input upload");
+  else if (!copies.upload(m->x_stage, x, bytes, false, "moe_block input upload"))
+    return 0;
   if (!coli_b200_moe_block_dev(m, m->x_stage, m->out_stage, T, st)) return 0;
-  CK(cudaMemcpyAsync(out, m->out_stage, bytes, cudaMemcpyDeviceToHost, st), "moe_block output download");
+  if (!copies.staged(out, bytes))
+    CK(cudaMemcpyAsync(out, m->out_stage, bytes, cudaMemcpyDeviceToHost, st), "moe_block output download");
+  else if (!copies.download(out, m->out_stage, bytes, false, "moe_block output download"))
+    return 0;
   const size_t n = (size_t)T * m->L.k;
   if (topk_idx) CK(cudaMemcpyAsync(topk_idx, m->topk_idx, n * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "routing download");
   if (topk_w) CK(cudaMemcpyAsync(topk_w, m->topk_w, n * sizeof(float), cudaMemcpyDeviceToHost, st), "routing download");
   CK(cudaStreamSynchronize(st), "moe_block sync");
+  wait.pending = false;
   int kst = 0;
   CK(cudaMemcpy(&kst, m->status, sizeof(int), cudaMemcpyDeviceToHost), "status read");
   if (kst != 0) {
@@ -1229,17 +1252,6 @@ extern "C" void coli_cuda_group_stats(uint64_t *calls, uint64_t *experts, uint64
   if (d2h_ms) *d2h_ms = g_group_d2h_ms;
 }
 
-namespace {
-struct StreamWait {
-  cudaStream_t st;
-  bool pending = true;
-  explicit StreamWait(cudaStream_t s) : st(s) {}
-  ~StreamWait() {
-    if (pending) cudaStreamSynchronize(st);
-  }
-};
-}  // namespace
-
 static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups, ColiCudaTensor *const *downs,
                           const int *rows, int count, float *y, const float *x, int want_fmt_a, int want_fmt_b,
                           const char *who) {
@@ -1285,31 +1297,38 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
     return 0;
   if (!ctx->ev[0])
     for (int i = 0; i < 4; ++i) CK(cudaEventCreate(&ctx->ev[i]), "event creation");
-  std::vector<WeightRef> tbl(3 * (size_t)count);
+  // the tables, the row counts and a cleared status word, as they lie on the device
+  const size_t head_bytes = sizeof(WeightRef) * 3 * count + sizeof(int32_t) * ((size_t)count + 1);
+  std::vector<WeightRef> head((head_bytes + sizeof(WeightRef) - 1) / sizeof(WeightRef));
   for (int c = 0; c < count; ++c) {
-    tbl[c] = WeightRef{gates[c]->q, gates[c]->s, gates[c]->gscale, 0};
-    tbl[count + c] = WeightRef{ups[c]->q, ups[c]->s, ups[c]->gscale, 0};
-    tbl[2 * count + c] = WeightRef{downs[c]->q, downs[c]->s, downs[c]->gscale, 0};
+    head[c] = WeightRef{gates[c]->q, gates[c]->s, gates[c]->gscale, 0};
+    head[count + c] = WeightRef{ups[c]->q, ups[c]->s, ups[c]->gscale, 0};
+    head[2 * count + c] = WeightRef{downs[c]->q, downs[c]->s, downs[c]->gscale, 0};
   }
+  memcpy(&head[3 * (size_t)count], rows, sizeof(int32_t) * count);
+  memset((char *)&head[3 * (size_t)count] + sizeof(int32_t) * count, 0, sizeof(int32_t));
   WeightRef *d_tbl = (WeightRef *)ctx->buf[3];
   int32_t *d_cnt = (int32_t *)(d_tbl + 3 * (size_t)count);
-  int32_t *d_off = d_cnt + count;
+  int32_t *d_status = d_cnt + count;
+  int32_t *d_off = d_status + 1;
   int32_t *d_iseg = d_off + count + 1;
   int32_t *d_irow = d_iseg + max_items;
   int32_t *d_inr = d_irow + max_items;
   int32_t *d_nit = d_inr + max_items;
-  int32_t *d_status = d_nit + 1;
   int32_t kst = 0;
-  // Whatever fails below, the call waits for its stream before it returns: copies may be reading x, rows and
-  // tbl, or writing y and kst.  (A wait between the copies and the kernels as well took 10 us a call.)
+  // Whatever fails below, the call waits for its stream before it returns: copies may be reading x and
+  // head, or writing y and kst.  (A wait between the copies and the kernels as well took 10 us a call.)
   StreamWait wait(st);
+  colib_host::HostCopies copies(ctx->ring, g_copy_pool, st);
   CK(cudaEventRecord(ctx->ev[0], st), "phase event");
-  CK(cudaMemcpyAsync(ctx->buf[0], x, xb * sizeof(float), cudaMemcpyHostToDevice, st), "expert input upload");
-  CK(cudaMemcpyAsync(d_tbl, tbl.data(), sizeof(WeightRef) * tbl.size(), cudaMemcpyHostToDevice, st), "expert table upload");
-  CK(cudaMemcpyAsync(d_cnt, rows, sizeof(int32_t) * count, cudaMemcpyHostToDevice, st), "row count upload");
-  CK(cudaMemsetAsync(d_status, 0, sizeof(int32_t), st), "status clear");
+  CK(cudaMemcpyAsync(d_tbl, head.data(), head_bytes, cudaMemcpyHostToDevice, st), "expert table upload");
+  const bool x_staged = copies.staged(x, xb * sizeof(float)), y_staged = copies.staged(y, xb * sizeof(float));
+  if (!x_staged)
+    CK(cudaMemcpyAsync(ctx->buf[0], x, xb * sizeof(float), cudaMemcpyHostToDevice, st), "expert input upload");
+  else if (!copies.upload(ctx->buf[1], x, xb * sizeof(float), true, "expert input upload"))
+    return 0;
   CK(cudaEventRecord(ctx->ev[1], st), "phase event");
-  if (!colib::launch_f32_to_f16((const float *)ctx->buf[0], (__half *)ctx->buf[1], xb, st)) return 0;
+  if (!x_staged && !colib::launch_f32_to_f16((const float *)ctx->buf[0], (__half *)ctx->buf[1], xb, st)) return 0;
   if (!colib::launch_items_from_counts(d_cnt, count, rpi, d_off, d_iseg, d_irow, d_inr, d_nit, st)) return 0;
   if (tc) {
     colib::TcParams tp;
@@ -1332,7 +1351,7 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
     tp.act = current_activation();
     const int sms = ctx->sm_count;
     const int ok = colib::launch_gate_up_tct(tp, ctx->buf[1], (int)total, sms, st) && colib::launch_down_tct(tp, (int)total, sms, st);
-    if (!ok || !colib::launch_bf16_to_f32((const __nv_bfloat16 *)ctx->buf[4], (float *)ctx->buf[0], xb, st)) return 0;
+    if (!ok || (!y_staged && !colib::launch_bf16_to_f32((const __nv_bfloat16 *)ctx->buf[4], (float *)ctx->buf[0], xb, st))) return 0;
   } else {
     colib::FfnParams fp;
     fp.fmt = kfmt;
@@ -1359,7 +1378,10 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
     if (!colib::launch_ffn_small(fp, st)) return 0;
   }
   CK(cudaEventRecord(ctx->ev[2], st), "phase event");
-  CK(cudaMemcpyAsync(y, ctx->buf[0], xb * sizeof(float), cudaMemcpyDeviceToHost, st), "expert output download");
+  if (!y_staged)
+    CK(cudaMemcpyAsync(y, ctx->buf[0], xb * sizeof(float), cudaMemcpyDeviceToHost, st), "expert output download");
+  else if (!copies.download(y, tc ? ctx->buf[4] : ctx->buf[0], xb * sizeof(float), tc, "expert output download"))
+    return 0;
   if (tc) CK(cudaMemcpyAsync(&kst, d_status, sizeof(int32_t), cudaMemcpyDeviceToHost, st), "status read");
   CK(cudaEventRecord(ctx->ev[3], st), "phase event");
   CK(cudaStreamSynchronize(st), "expert call sync");

@@ -238,6 +238,66 @@ int launch_bf16_to_f16(const __nv_bfloat16 *src, __half *dst, size_t n, cudaStre
   return coli_cuda_check(cudaGetLastError(), "bf16->f16 launch") ? 1 : 0;
 }
 
+// Page-locked host memory over the link: 16 bytes a thread and access, whole lines a warp.
+template <bool TO_F16>
+__global__ void __launch_bounds__(256) k_from_host(uint4 *dst, const uint4 *host, size_t n) {  // n 16-byte pieces on the host
+  const size_t step = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
+    const uint4 v = __ldcs(host + i);
+    if (TO_F16) {
+      const float4 f = *reinterpret_cast<const float4 *>(&v);
+      auto clamp = [](float a) { return fminf(fmaxf(a, -65504.0f), 65504.0f); };
+      const __half2 lo = __floats2half2_rn(clamp(f.x), clamp(f.y)), hi = __floats2half2_rn(clamp(f.z), clamp(f.w));
+      reinterpret_cast<uint2 *>(dst)[i] = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+    } else {
+      dst[i] = v;
+    }
+  }
+}
+int launch_from_host(void *dst, const void *host, size_t bytes, bool to_f16, cudaStream_t st) {
+  const size_t n = bytes / 16;
+  if (n == 0) return 1;
+  const size_t blocks = (n + 511) / 512;  // two pieces a thread
+  const unsigned grid = (unsigned)(blocks > 4 * COLI_SMS ? 4 * COLI_SMS : blocks);
+  if (to_f16)
+    k_from_host<true><<<grid, 256, 0, st>>>((uint4 *)dst, (const uint4 *)host, n);
+  else
+    k_from_host<false><<<grid, 256, 0, st>>>((uint4 *)dst, (const uint4 *)host, n);
+  coli_count_launch(1);
+  return coli_cuda_check(cudaGetLastError(), "host read launch") ? 1 : 0;
+}
+// One CTA a chunk: its pieces, made visible to the host, then its mark.
+template <bool FROM_BF16>
+__global__ void __launch_bounds__(512) k_to_host(uint4 *host, const uint4 *src, size_t n, uint32_t *arrived, uint32_t mark) {
+  constexpr int PIECES = (int)(HOST_CHUNK / 16);
+  const size_t base = (size_t)blockIdx.x * PIECES;
+#pragma unroll 8
+  for (int j = (int)threadIdx.x; j < PIECES; j += 512) {
+    const size_t i = base + j;
+    if (i >= n) break;
+    if (FROM_BF16) {
+      const uint2 v = reinterpret_cast<const uint2 *>(src)[i];
+      host[i] = make_uint4(v.x << 16, v.x & 0xffff0000u, v.y << 16, v.y & 0xffff0000u);
+    } else {
+      host[i] = src[i];
+    }
+  }
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(arrived + blockIdx.x), "r"(mark) : "memory");
+}
+int launch_to_host(void *host, const void *src, size_t bytes, bool from_bf16, uint32_t *arrived, uint32_t mark, cudaStream_t st) {
+  const size_t n = bytes / 16;
+  if (n == 0) return 1;
+  const unsigned grid = (unsigned)((bytes + HOST_CHUNK - 1) / HOST_CHUNK);
+  if (from_bf16)
+    k_to_host<true><<<grid, 512, 0, st>>>((uint4 *)host, (const uint4 *)src, n, arrived, mark);
+  else
+    k_to_host<false><<<grid, 512, 0, st>>>((uint4 *)host, (const uint4 *)src, n, arrived, mark);
+  coli_count_launch(1);
+  return coli_cuda_check(cudaGetLastError(), "host write launch") ? 1 : 0;
+}
+
 __global__ void k_matmul_f32_seq(const float *x, const float *w, float *y, int S, int I, int O) {
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)S * O) return;

@@ -4,6 +4,7 @@
 #include <mutex>
 #include <vector>
 
+#include "host_copy.cuh"
 #include "internal.cuh"
 
 struct DeviceContext {
@@ -16,6 +17,7 @@ struct DeviceContext {
   size_t cap[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // phase marks of the host-pointer group calls
   int sm_count = 0;
+  colib_host::HostRing ring;  // page-locked chunks between pageable memory and this device
 };
 DeviceContext *coli_find_ctx(int device);
 bool coli_select_ctx(DeviceContext *c);

@@ -272,6 +272,12 @@ int launch_rmsnorm_bf16(const float *x, const float *w, float eps, __nv_bfloat16
 int launch_bf16_to_f16(const __nv_bfloat16 *src, __half *dst, size_t n, cudaStream_t st);
 int launch_f32_to_f16(const float *src, __half *dst, size_t n, cudaStream_t st);
 int launch_bf16_to_f32(const __nv_bfloat16 *src, float *dst, size_t n, cudaStream_t st);
+// Rows through page-locked host memory, read or written by the kernels themselves; `bytes` (a multiple of 16) are those
+// on the host.  to_f16: f32 there, f16 on the device, as launch_f32_to_f16.  from_bf16: bf16 on the device, f32 on
+// the host.  launch_to_host sets arrived[i] = mark behind chunk i of HOST_CHUNK bytes.
+constexpr size_t HOST_CHUNK = 64 * 1024;
+int launch_from_host(void *dst, const void *host, size_t bytes, bool to_f16, cudaStream_t st);
+int launch_to_host(void *host, const void *src, size_t bytes, bool from_bf16, uint32_t *arrived, uint32_t mark, cudaStream_t st);
 // y[S,O] = x[S,I] @ W[O,I]^T, all f32, one thread per output, multiply then add per k in order
 // (crates/colibri-engine/src/linear.rs:199-220).
 int launch_matmul_f32_seq(const float *x, const float *w, float *y, int S, int I, int O, cudaStream_t st);

@@ -1,0 +1,66 @@
+"""Calls on pageable host memory against the same call on device memory, bit for bit: sizes on both sides of what goes
+as it is, of a chunk of the page-locked ring, of its halves and of the whole of it."""
+import threading
+
+import numpy as np
+import pytest
+
+from speedycolibri_b200 import synth
+from speedycolibri_b200.configs import MoeShape
+
+pytestmark = pytest.mark.gpu
+
+H = 2048  # 4 KB a row
+
+
+@pytest.fixture(scope="module")
+def block(gpu_backend):
+    from speedycolibri_b200.moe import Config, MoeBlock
+
+    shape = MoeShape("host_copies", H=H, E=8, k=2, I=64, T=1, norm_topk=True)
+    blk = MoeBlock(Config.from_shape(shape), synth.device_layer(shape), 1600)
+    yield blk, shape
+    blk.close()
+
+
+def on_device(blk, x):
+    import torch
+
+    return blk.forward(torch.from_numpy(x.view(np.int16)).cuda().view(torch.bfloat16)).view(torch.int16).cpu().numpy().view(np.uint16)
+
+
+@pytest.mark.parametrize("T", [1, 63, 64, 65, 80, 511, 512, 513, 1024, 1025, 1536, 1537, 1600])
+@pytest.mark.parametrize("pinned", [False, True], ids=["pageable", "pinned"])
+def test_host_rows_give_what_device_rows_give(block, T, pinned):
+    import torch
+
+    blk, shape = block
+    x = synth.host_tokens(shape, T)
+    want = on_device(blk, x)
+    if pinned:
+        src = torch.from_numpy(x.view(np.int16)).pin_memory()
+        dst = torch.zeros((T, H), dtype=torch.int16).pin_memory()
+        blk.moe_ptr(src.data_ptr(), dst.data_ptr(), T)
+        got = dst.numpy().view(np.uint16)
+    else:
+        got = blk.moe(x)
+    assert np.array_equal(got, want)
+
+
+def test_host_calls_of_several_threads(block):
+    blk, shape = block
+    xs = [synth.host_tokens(shape, T, index=T) for T in (40, 300, 700, 1100)]
+    want = [on_device(blk, x) for x in xs]
+    bad = []
+
+    def calls(i):
+        for _ in range(5):
+            if not np.array_equal(blk.moe(xs[i]), want[i]):
+                bad.append(i)
+
+    threads = [threading.Thread(target=calls, args=(i,)) for i in range(len(xs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
