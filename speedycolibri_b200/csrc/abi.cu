@@ -826,6 +826,7 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
     // decode-sized batches: one launch for router, top-k and permutation (its time is booked
     // under the router phase)
     colib::RouteParams rp = coli_route_params(m, x_dev, T);
+    rp.in_call = resid_io != nullptr;  // the norm of the layer step
     const int fused = T <= 8 ? colib::launch_decode_front(rp, pp, m->ticket, st) : -1;
     if (fused == 0) return 0;
     const bool place = fused < 0 && colib::place_rows_ok(pp);

@@ -138,6 +138,7 @@ struct RouteParams {
   float *topk_w;                  // [T,k]
   int32_t *expert_rows = nullptr; // [E] pairs of each expert, counted by the top-k, or null; then also
   int32_t *local_rank = nullptr;  // [T,k] how many of its expert's pairs were counted before a pair
+  bool in_call = false;           // the launch before the router's is one of the same call
 };
 int launch_router(const RouteParams &p, cudaStream_t st);
 

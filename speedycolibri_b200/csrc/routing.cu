@@ -32,7 +32,7 @@ __device__ __forceinline__ void clear_expert_rows(const RouteParams &p) {
 // ---------------------------------------------------------------------------------------------
 template <int TM, int TN>
 __global__ void __launch_bounds__(256) k_router_gemm(RouteParams p) {
-  coli_grid_trigger();  // the top-k may be scheduled; it waits for this grid
+  coli_grid_dependency_sync();
   clear_expert_rows(p);
   constexpr int BM = 16 * TM, BN = 16 * TN, BK = 32;
   __shared__ float xs[BK][BM + 4];
@@ -123,7 +123,7 @@ struct RouterPairTile {
 };
 template <class C>
 __global__ void __launch_bounds__(C::NT) k_router_pair(RouteParams p) {
-  coli_grid_trigger();  // the top-k may be scheduled; it waits for this grid
+  coli_grid_dependency_sync();
   clear_expert_rows(p);
   constexpr int TM = C::TM, TN = C::TN, BK = C::BK, LD = C::LD, BM = C::BM;
   extern __shared__ __align__(16) float rsm[];
@@ -243,7 +243,7 @@ struct RouterTile {
 };
 template <class C>
 __global__ void __launch_bounds__(C::NT) k_router_chain(RouteParams p) {
-  coli_grid_trigger();  // the top-k may be scheduled; it waits for this grid
+  coli_grid_dependency_sync();
   clear_expert_rows(p);
   constexpr int TM = C::TM, TN = C::TN, RS = C::RS, CH = C::CH, BM = C::BM, BN = C::BN;
   constexpr bool SMALL = TM * TN <= 8;  // the next chunk's operands are loaded ahead of this one's FMAs
@@ -691,12 +691,10 @@ __device__ __forceinline__ void route_topk_token(const RouteParams &p, int t, fl
     route_topk_slots<kMaxSlots>(p, t, row, lane, ids_out);
 }
 
-// The same chains for batches above 8 tokens whose 8 x 8 tiles have an SM each (its shared memory sees to that).
-constexpr size_t kStagedSmem = 116 * 1024;
-static_assert(RouterTiny::SMEM <= kStagedSmem, "staging area");
+// The same chains for batches above 8 tokens whose 8 x 8 tiles have an SM each.
 __global__ void __launch_bounds__(192) k_router_staged(RouteParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  coli_grid_trigger();  // the top-k may be scheduled; it waits for this grid
+  coli_grid_dependency_sync();
   clear_expert_rows(p);
   router_tiny_block<4>(p, smem_raw, (int)blockIdx.x * 8, (int)blockIdx.y * 8);
 }
@@ -718,20 +716,38 @@ using RouterTile64x64 = RouterTile<8, 4, 2, 2, 64, 6>;
 // ... and of k_router_pair:             TM TN WM WN CW
 using RouterTile128x64 = RouterPairTile<8, 8, 4, 1, 2>;
 using RouterTile128x128 = RouterPairTile<16, 8, 2, 2, 0>;
+// A kernel that starts before its predecessor has ended packs its CTAs onto the SMs that are free by then (router of 4096
+// tokens 445 -> 1183 us; top-k of 512 tokens 6500 cycles a token where one alone takes 3500).  With shared memory for no
+// more CTAs on an SM than an even spread puts there it can start early all the same: `need` raised to that, or
+// `need` itself where an SM gets more than four.
+constexpr int kSmSharedBytes = 228 * 1024, kSpreadMost = 4;
+static int ctas_per_sm(long ctas) { return (int)((ctas + COLI_SMS - 1) / COLI_SMS); }
+static size_t spread_smem(long ctas, size_t need) {
+  const int per_sm = ctas_per_sm(ctas);
+  const size_t alone = (size_t)kSmSharedBytes / (per_sm + 1);
+  return per_sm <= kSpreadMost && need < alone ? alone : need;
+}
+// Launches a router GEMM: early if its CTAs stay spread and the caller gains by it (us a call: 333 tokens, H 1024, 32 experts
+// 44.4 -> 41.6; 512 tokens, H 2048, 128 experts 179.6 -> 173.9; 1024 389.0 -> 387.6).
+template <class K>
+static bool launch_router_kernel(K kernel, ColiPerDeviceOnce &attr_once, dim3 grid, int threads, size_t need, const RouteParams &p, cudaStream_t st,
+                                 bool early = true) {
+  const long ctas = (long)grid.x * grid.y;
+  const size_t smem = spread_smem(ctas, need), most = (size_t)kSmSharedBytes / 2;
+  if (!coli_set_smem_limit(attr_once, kernel, need > most ? need : most, "router shared-memory attribute")) return false;
+  if (early && ctas_per_sm(ctas) <= kSpreadMost) return coli_cuda_check(launch_dependent(kernel, grid, dim3(threads), smem, st, p), "router launch");
+  kernel<<<grid, threads, smem, st>>>(p);
+  return true;
+}
 template <class C>
 static bool launch_router_chain(const RouteParams &p, cudaStream_t st) {
   static ColiPerDeviceOnce attr_once;
-  if (C::SMEM > 48 * 1024 && !coli_set_smem_limit(attr_once, k_router_chain<C>, C::SMEM, "router shared-memory attribute")) return false;
-  const dim3 grid((p.T + C::BM - 1) / C::BM, (p.E + C::BN - 1) / C::BN);
-  k_router_chain<C><<<grid, C::NT, C::SMEM, st>>>(p);
-  return true;
+  return launch_router_kernel(k_router_chain<C>, attr_once, dim3((p.T + C::BM - 1) / C::BM, (p.E + C::BN - 1) / C::BN), C::NT, C::SMEM, p, st);
 }
 template <class C>
 static bool launch_router_pair(const RouteParams &p, cudaStream_t st) {
   static ColiPerDeviceOnce attr_once;
-  if (C::SMEM > 48 * 1024 && !coli_set_smem_limit(attr_once, k_router_pair<C>, C::SMEM, "router shared-memory attribute")) return false;
-  k_router_pair<C><<<dim3((p.T + C::BM - 1) / C::BM, (p.E + C::BN - 1) / C::BN), C::NT, C::SMEM, st>>>(p);
-  return true;
+  return launch_router_kernel(k_router_pair<C>, attr_once, dim3((p.T + C::BM - 1) / C::BM, (p.E + C::BN - 1) / C::BN), C::NT, C::SMEM, p, st);
 }
 // The tile of a batch: 0 = 8 x 8, 1 = 16 x 32, 2 = 64 x 64, 3 = 128 x 64, 4 = 128 x 128 tokens x experts.
 // The time of one k is a function of n, the CTAs of the fullest SM; the figures are nanoseconds measured
@@ -753,9 +769,8 @@ static int pick_router_tile(int T, int E) {
 static long router_tiles_8x8(int T, int E) { return (long)((T + 7) / 8) * ((E + 7) / 8); }
 static bool launch_router_staged(const RouteParams &p, cudaStream_t st) {
   static ColiPerDeviceOnce attr_once;
-  if (!coli_set_smem_limit(attr_once, k_router_staged, kStagedSmem, "router shared-memory attribute")) return false;
-  k_router_staged<<<dim3((p.T + 7) / 8, (p.E + 7) / 8), 192, kStagedSmem, st>>>(p);
-  return true;
+  // (early behind the norm of a layer step, 48 tokens 101.6 -> 100.4 us; not behind another call, 21 tokens 92.8 -> 94.0)
+  return launch_router_kernel(k_router_staged, attr_once, dim3((p.T + 7) / 8, (p.E + 7) / 8), 192, RouterTiny::SMEM, p, st, p.in_call);
 }
 
 static int launch_router_logits(const RouteParams &p, cudaStream_t st) {
@@ -792,15 +807,11 @@ static int launch_router_logits(const RouteParams &p, cudaStream_t st) {
   return coli_cuda_check(cudaGetLastError(), "router launch") ? 1 : 0;
 }
 
-constexpr int kSmSharedBytes = 228 * 1024;
 int launch_router(const RouteParams &p, cudaStream_t st) {
   if (p.T <= 0) return 1;
   if (!launch_router_logits(p, st)) return 0;
-  // Shared memory for no more CTAs on an SM than an even spread puts there: started early they pack onto the SMs that
-  // are free (512 tokens, 128 experts: 6500 cycles a token where one alone takes 3500).
-  const int ctas = (p.T + 3) / 4, per_sm = (ctas + COLI_SMS - 1) / COLI_SMS;
-  size_t sm = (size_t)4 * topk_row_floats(p.E) * sizeof(float);
-  if (per_sm <= 4 && sm < (size_t)kSmSharedBytes / (per_sm + 1)) sm = (size_t)kSmSharedBytes / (per_sm + 1);
+  const int ctas = (p.T + 3) / 4;
+  const size_t sm = spread_smem(ctas, (size_t)4 * topk_row_floats(p.E) * sizeof(float));
   static ColiPerDeviceOnce attr_once;
   if (!coli_set_smem_limit(attr_once, k_route_topk, kSmSharedBytes / 2, "top-k shared-memory attribute")) return 0;
   coli_count_launch(1);
