@@ -839,6 +839,19 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
     if (fused < 0 && !(place ? colib::launch_place_rows(pp, st) : colib::launch_permute(pp, st))) return 0;
   }
   COLI_MARK(2);
+  colib::CombineParams cp;
+  cp.T = T;
+  cp.H = m->L.H;
+  cp.k = k;
+  cp.has_shared = m->has_shared ? 1 : 0;
+  cp.y = m->y;
+  cp.shared_y = m->y + (size_t)T * k * m->L.H;
+  cp.slot = m->slot;
+  cp.topk_w = m->topk_w;
+  cp.out = (__nv_bfloat16 *)out_dev;
+  cp.out32 = resid_io;
+  cp.resid = resid_io;
+  const bool one = T == 1 && !tc && colib::down_combine_one_ok(k + (m->has_shared ? 1 : 0), m->L.H);
   if (tc) {
     colib::TcParams tp;
     tp.fmt = m->L.fmt;
@@ -886,22 +899,11 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
     fp.act = m->act;
     if (!colib::launch_gate_up_small(fp, st)) return 0;
     COLI_MARK(3);
-    if (!colib::launch_down_small(fp, !prof, st)) return 0;  // (profiling records an event between the two)
+    if (!one && !colib::launch_down_small(fp, !prof, st)) return 0;  // (profiling records an event between the two)
+    if (one && !colib::launch_down_combine_one(fp, cp, m->topk_idx, m->L.E, !prof, st)) return 0;
   }
   COLI_MARK(4);
-  colib::CombineParams cp;
-  cp.T = T;
-  cp.H = m->L.H;
-  cp.k = k;
-  cp.has_shared = m->has_shared ? 1 : 0;
-  cp.y = m->y;
-  cp.shared_y = m->y + (size_t)T * k * m->L.H;
-  cp.slot = m->slot;
-  cp.topk_w = m->topk_w;
-  cp.out = (__nv_bfloat16 *)out_dev;
-  cp.out32 = resid_io;
-  cp.resid = resid_io;
-  if (!colib::launch_combine(cp, st)) return 0;
+  if (!one && !colib::launch_combine(cp, st)) return 0;
   COLI_MARK(5);
 #undef COLI_MARK
   if (prof) {
@@ -990,26 +992,32 @@ extern "C" int coli_b200_moe_block(ColiMoe *m, const void *x, void *out, int T, 
   std::lock_guard<std::mutex> lk(m->ctx->mu);
   cudaStream_t st = m->ctx->stream;
   const size_t bytes = (size_t)T * m->L.H * sizeof(__nv_bfloat16);
+  int32_t own = 0;
   StreamWait wait(st);  // whatever fails below: nothing of the caller's is in use when the call returns
   colib_host::HostCopies copies(m->ctx->ring, g_copy_pool, st);
   if (!copies.staged(x, bytes))
     CK(cudaMemcpyAsync(m->x_stage, x, bytes, cudaMemcpyHostToDevice, st), "moe_block input upload");
   else if (!copies.upload(m->x_stage, x, bytes, false, "moe_block input upload"))
     return 0;
-  if (!coli_b200_moe_block_dev(m, m->x_stage, m->out_stage, T, st)) return 0;
-  if (!copies.staged(out, bytes))
+  // page-locked results are written by the last kernel itself, as it makes them (1024 tokens, H 2048: 389 -> 372 us a call)
+  void *mapped = colib_host::mapped_host(out, bytes);
+  if ((reinterpret_cast<uintptr_t>(mapped) & 15) != 0) mapped = nullptr;
+  if (!coli_b200_moe_block_dev(m, m->x_stage, mapped ? mapped : m->out_stage, T, st)) return 0;
+  if (mapped)
+    ;  // done
+  else if (!copies.staged(out, bytes))
     CK(cudaMemcpyAsync(out, m->out_stage, bytes, cudaMemcpyDeviceToHost, st), "moe_block output download");
   else if (!copies.download(out, m->out_stage, bytes, false, "moe_block output download"))
     return 0;
   const size_t n = (size_t)T * m->L.k;
   if (topk_idx) CK(cudaMemcpyAsync(topk_idx, m->topk_idx, n * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "routing download");
   if (topk_w) CK(cudaMemcpyAsync(topk_w, m->topk_w, n * sizeof(float), cudaMemcpyDeviceToHost, st), "routing download");
+  volatile int32_t *kst = m->ctx->ring.ready() ? m->ctx->ring.status : &own;
+  CK(cudaMemcpyAsync((void *)kst, m->status, sizeof(int32_t), cudaMemcpyDeviceToHost, st), "status read");
   CK(cudaStreamSynchronize(st), "moe_block sync");
   wait.pending = false;
-  int kst = 0;
-  CK(cudaMemcpy(&kst, m->status, sizeof(int), cudaMemcpyDeviceToHost), "status read");
-  if (kst != 0) {
-    coli_set_error("a tcgen05 expert kernel abandoned a bounded wait (code %d); the output is invalid", kst);
+  if (*kst != 0) {
+    coli_set_error("a tcgen05 expert kernel abandoned a bounded wait (code %d); the output is invalid", (int)*kst);
     cudaMemset(m->status, 0, sizeof(int));
     return 0;
   }
@@ -1316,9 +1324,9 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
   int32_t *d_irow = d_iseg + max_items;
   int32_t *d_inr = d_irow + max_items;
   int32_t *d_nit = d_inr + max_items;
-  int32_t kst = 0;
+  int32_t own = 0;
   // Whatever fails below, the call waits for its stream before it returns: copies may be reading x and
-  // head, or writing y and kst.  (A wait between the copies and the kernels as well took 10 us a call.)
+  // head, or writing y and own.  (A wait between the copies and the kernels as well took 10 us a call.)
   StreamWait wait(st);
   colib_host::HostCopies copies(ctx->ring, g_copy_pool, st);
   CK(cudaEventRecord(ctx->ev[0], st), "phase event");
@@ -1383,12 +1391,13 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
     CK(cudaMemcpyAsync(y, ctx->buf[0], xb * sizeof(float), cudaMemcpyDeviceToHost, st), "expert output download");
   else if (!copies.download(y, tc ? ctx->buf[4] : ctx->buf[0], xb * sizeof(float), tc, "expert output download"))
     return 0;
-  if (tc) CK(cudaMemcpyAsync(&kst, d_status, sizeof(int32_t), cudaMemcpyDeviceToHost, st), "status read");
+  volatile int32_t *kst = tc && ctx->ring.ready() ? ctx->ring.status : &own;
+  if (tc) CK(cudaMemcpyAsync((void *)kst, d_status, sizeof(int32_t), cudaMemcpyDeviceToHost, st), "status read");
   CK(cudaEventRecord(ctx->ev[3], st), "phase event");
   CK(cudaStreamSynchronize(st), "expert call sync");
   wait.pending = false;
-  if (kst != 0) {
-    coli_set_error("%s: a tcgen05 expert kernel abandoned a bounded wait (code %d); the output is invalid", who, (int)kst);
+  if (*kst != 0) {
+    coli_set_error("%s: a tcgen05 expert kernel abandoned a bounded wait (code %d); the output is invalid", who, (int)*kst);
     return 0;
   }
   float ms[3] = {0.0f, 0.0f, 0.0f};

@@ -800,6 +800,149 @@ static int launch_stream_rows(const FfnParams &p, bool gated, bool items_known, 
   }
   return launch_stream<FMT, 1>(p, gated, items_known, st);
 }
+// ---- one token: down and combine ---------------------------------------------------------------------
+// A CTA makes 16 features of the result: a warp for each of the token's rows (its k experts and the shared one), all
+// of K through a ring of its own, then the weighted sum of k_combine -- the same terms, rounded the same way -- out of
+// shared memory.  The result rows never leave the SM, and a launch and its wait are gone from a chain of four.
+// The rings are filled before the input is there, as those of the kernel above.
+// One token on H 2048, I 768, 128 experts: 26.2 -> 25.2 us a call.  From more features than SMs x 16 on the two kernels are
+// better (H 7168, I 2048, 256 experts: 80.7 and 84.4): there the whole of K by one warp is a long chain.
+constexpr int kOneRows = 17, kOneStages = 6;
+template <int FMT>
+__global__ void __launch_bounds__(32 * kOneRows) k_down_combine_one(FfnParams p, CombineParams c, const int32_t *topk_idx, int shared, int items_known) {
+  constexpr bool FP4 = FMT == COLI_FMT_NVFP4;
+  constexpr int QB = FP4 ? 64 : 128, SB = FP4 ? 8 : 0, Q = 16 * QB, SLOT = 16 * (QB + SB);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), rows = (int)blockDim.x >> 5;
+  const int K = p.I, KT = (K + 127) >> 7, Op = (p.H + 15) & ~15, r0 = (int)blockIdx.x * 16;
+  float *ys = reinterpret_cast<float *>(smem_raw + (size_t)rows * kOneStages * SLOT);  // [rows][16]
+  const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem_raw) + warp * (kOneStages * SLOT);
+  if (!items_known) coli_grid_wait();
+  const int ex = warp < c.k ? __ldcg(topk_idx + warp) : shared;
+  const int row = warp < c.k ? __ldcg(c.slot + warp) : c.k;
+  const WeightRef w = p.down[ex];
+  int kf = 0;  // the k-tile that is fetched next
+  auto issue = [&]() {
+    if (kf < KT) {
+      const uint32_t d = ring + (kf % kOneStages) * SLOT + lane * 16;
+      const uint8_t *q = w.q + ((size_t)kf * Op + r0) * QB + lane * 16;
+#pragma unroll
+      for (int i = 0; i < Q / 512; ++i) cp_async16(d + i * 512, q + i * 512);
+      if (FP4 && lane < 8) cp_async16(d + Q, w.s + ((size_t)kf * Op + r0) * SB + lane * 16);
+      ++kf;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll 1
+  for (int i = 0; i < kOneStages - 1; ++i) issue();
+  if (items_known) coli_grid_wait();
+  coli_grid_trigger();
+  const __half *h = p.h + (size_t)row * K + t * 32;  // column 0, the token, is read by the lanes of g = 0
+  auto load_x = [&](uint4 (&x)[4], int kt) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      x[i] = make_uint4(0, 0, 0, 0);
+      if (g == 0 && kt * 128 + t * 32 + 8 * i + 8 <= K) x[i] = *reinterpret_cast<const uint4 *>(h + kt * 128 + 8 * i);
+    }
+  };
+  uint4 xn[4];
+  load_x(xn, 0);
+  float acc[2][4] = {};  // the steps of a k-tile add into two sets in turn
+  const uint32_t code_off = FP4 ? g * 64 + coli_fp4_chunk(g, t) * 16 : g * 128 + coli_fp8_chunk(g, 2 * t) * 16;
+  for (int kt = 0; kt < KT; ++kt) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kOneStages - 2) : "memory");
+    __syncwarp();  // this k-tile has arrived for every lane, and the slot before it has been read by all
+    issue();
+    uint4 x[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = xn[i];
+    if (kt + 1 < KT) load_x(xn, kt + 1);
+    const uint32_t base = ring + (kt % kOneStages) * SLOT;
+    AFrag<FMT> f;
+    if constexpr (FP4) {
+      f.lo[0] = lds128(base + code_off);
+      f.hi[0] = lds128(base + 512 + code_off);
+      uint16_t a, b;
+      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(a) : "r"(base + Q + lane * 2) : "memory");
+      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(b) : "r"(base + Q + 64 + lane * 2) : "memory");
+      f.sc = (uint32_t)a | ((uint32_t)b << 16);
+    } else {
+      f.lo[0] = lds128(base + code_off);
+      f.lo[1] = lds128(base + (code_off ^ 16));
+      f.hi[0] = lds128(base + 1024 + code_off);
+      f.hi[1] = lds128(base + 1024 + (code_off ^ 16));
+      f.sc = 0;
+    }
+    const AScale asc = decode_scales<FMT>(f);
+    float part[2][4] = {};
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const uint4 &xv = x[s >> 1];
+      uint32_t a[4];
+      decode_a<FMT>(f, asc, s, a);
+      if (FMT == COLI_FMT_FP8_B128)
+        mma_f16_16816(part[s & 1], a, (s & 1) ? xv.z : xv.x, (s & 1) ? xv.w : xv.y);
+      else
+        mma_f16_16816(acc[s & 1], a, (s & 1) ? xv.z : xv.x, (s & 1) ? xv.w : xv.y);
+    }
+    if (FMT == COLI_FMT_FP8_B128) {  // one f32 scale per (128-row block, k-tile): convert.rs:731-741
+      const float sc = __ldg(reinterpret_cast<const float *>(w.s) + (size_t)(r0 >> 7) * KT + kt);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[0][i] = fmaf(sc, part[0][i] + part[1][i], acc[0][i]);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  if (t == 0) {  // column 0: elements 0 (row g) and 2 (row g + 8)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int o = r0 + g + 8 * i;
+      float v = acc[0][2 * i] + acc[1][2 * i];
+      if (FP4) v *= w.g;
+      if (FMT == COLI_FMT_E4M3_ROW) v *= o < p.H ? reinterpret_cast<const float *>(w.s)[o] : 0.0f;
+      ys[warp * 16 + g + 8 * i] = __bfloat162float(__float2bfloat16_rn(v));
+    }
+  }
+  __syncthreads();
+  const int o = r0 + (int)threadIdx.x;
+  if (threadIdx.x >= 16 || o >= p.H) return;
+  float sum = 0.0f;
+  for (int kk = 0; kk < c.k; ++kk) sum = fmaf(c.topk_w[kk], ys[kk * 16 + threadIdx.x], sum);
+  if (rows > c.k) sum += ys[c.k * 16 + threadIdx.x];
+  if (c.resid) sum = c.resid[o] + sum;
+  if (c.out32)
+    c.out32[o] = sum;
+  else
+    c.out[o] = __float2bfloat16_rn(sum);
+}
+bool down_combine_one_ok(int rows, int H) { return rows <= kOneRows && (H + 15) / 16 <= COLI_SMS; }
+template <int FMT>
+static int launch_one_token(const FfnParams &p, const CombineParams &c, const int32_t *topk_idx, int shared, bool items_known, cudaStream_t st) {
+  constexpr int SLOT = FMT == COLI_FMT_NVFP4 ? 16 * 72 : 16 * 128;
+  const int rows = c.k + c.has_shared;
+  const size_t smem = (size_t)rows * (kOneStages * SLOT + 16 * sizeof(float));
+  static ColiPerDeviceOnce once;
+  if (!coli_set_smem_limit(once, k_down_combine_one<FMT>, (size_t)kOneRows * (kOneStages * SLOT + 16 * sizeof(float)), "down of one token: shared-memory attribute"))
+    return 0;
+  coli_count_launch(1);
+  return coli_cuda_check(launch_dependent(k_down_combine_one<FMT>, dim3((p.H + 15) / 16), dim3(32 * rows), smem, st, p, c, topk_idx, shared, items_known ? 1 : 0),
+                         "down of one token")
+             ? 1
+             : 0;
+}
+int launch_down_combine_one(const FfnParams &p, const CombineParams &c, const int32_t *topk_idx, int shared, bool items_known, cudaStream_t st) {
+  switch (p.fmt) {
+    case COLI_FMT_NVFP4:
+      return launch_one_token<COLI_FMT_NVFP4>(p, c, topk_idx, shared, items_known, st);
+    case COLI_FMT_FP8_B128:
+      return launch_one_token<COLI_FMT_FP8_B128>(p, c, topk_idx, shared, items_known, st);
+    case COLI_FMT_E4M3_ROW:
+      return launch_one_token<COLI_FMT_E4M3_ROW>(p, c, topk_idx, shared, items_known, st);
+  }
+  coli_set_error("expert ffn: unsupported weight format %d", p.fmt);
+  return 0;
+}
+
 static int pick_w(int KT) { return KT >= 8 ? 8 : KT >= 4 ? 4 : KT >= 2 ? 2 : 1; }
 
 // Split K across the warps of a CTA only when there are too few (item, row tile) tasks to fill

@@ -129,6 +129,7 @@ class CopyPool {
 struct HostRing {
   char *mem = nullptr;                    // two halves of chunks
   volatile uint32_t *arrived = nullptr;   // behind them: a word a chunk, the batch that it holds
+  volatile int32_t *status = nullptr;     // and one for the status word of a call's kernels
   cudaEvent_t read[2] = {};               // the device has read a half
   uint32_t batch = 0;
   bool tried = false;
@@ -137,7 +138,7 @@ struct HostRing {
     tried = true;
     void *p = nullptr;
     const size_t chunks = 2 * kHalf;
-    if (cudaHostAlloc(&p, chunks * kChunk + chunks * sizeof(uint32_t), cudaHostAllocDefault) != cudaSuccess || !p) {
+    if (cudaHostAlloc(&p, chunks * kChunk + (chunks + 1) * sizeof(uint32_t), cudaHostAllocDefault) != cudaSuccess || !p) {
       cudaGetLastError();
       return false;
     }
@@ -149,8 +150,9 @@ struct HostRing {
         tried = true;
         return false;
       }
-    memset((char *)p + chunks * kChunk, 0, chunks * sizeof(uint32_t));
+    memset((char *)p + chunks * kChunk, 0, (chunks + 1) * sizeof(uint32_t));
     arrived = (volatile uint32_t *)((char *)p + chunks * kChunk);
+    status = (volatile int32_t *)(arrived + chunks);
     mem = (char *)p;
     return true;
   }
@@ -164,6 +166,18 @@ struct HostRing {
     tried = false;
   }
 };
+
+// The device's address of page-locked memory that kernels may write directly, null for any other: both ends of it
+// have to be of one mapping.
+inline void *mapped_host(void *host, size_t bytes) {
+  cudaPointerAttributes a = {}, z = {};
+  if (cudaPointerGetAttributes(&a, host) != cudaSuccess || cudaPointerGetAttributes(&z, (char *)host + bytes - 1) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (a.type != cudaMemoryTypeHost || z.type != cudaMemoryTypeHost || !a.devicePointer || !z.devicePointer) return nullptr;
+  return (char *)a.devicePointer + bytes - 1 == (char *)z.devicePointer ? a.devicePointer : nullptr;
+}
 
 // Of one host-pointer call: its copies to and from the device on stream `st`.  Sizes are multiples of 16 bytes.
 class HostCopies {

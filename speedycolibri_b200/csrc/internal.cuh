@@ -262,6 +262,10 @@ struct CombineParams {
   const float *resid;             // [T,H] f32 residual stream added to the block output (forward.rs:391-393);
                                   // may alias out32 (every element is read and written by one thread)
 };
+// One token: down of its `rows` = k (+ 1 shared) rows and their combine in one launch, behind launch_gate_up_small
+// (`items_known` as for launch_down_small); expert ids in topk_idx, the shared expert is entry `shared` of the tables.
+bool down_combine_one_ok(int rows, int H);
+int launch_down_combine_one(const FfnParams &p, const CombineParams &c, const int32_t *topk_idx, int shared, bool items_known, cudaStream_t st);
 int launch_combine(const CombineParams &p, cudaStream_t st);
 int launch_finish(const float *partial, const __nv_bfloat16 *shared_y, __nv_bfloat16 *out, int T, int H, cudaStream_t st);
 int launch_f32_to_bf16(const float *src, __nv_bfloat16 *dst, size_t n, cudaStream_t st);
