@@ -364,8 +364,10 @@ struct RouterTiny {
   static constexpr int F32_BYTES = ROWS * LD * 4, RING_BYTES = ROWS * BK * 2;
   static constexpr size_t SMEM = (size_t)2 * F32_BYTES + (size_t)STAGES * RING_BYTES;
 };
-// The first 2 + CW warps of a CTA call this; logits of tokens m0.. and experts n0.. are written.
-template <int CW>
+// The first 2 + CW warps of a CTA call this; logits of tokens m0.. and experts n0.. are written.  EARLY: the kernel may
+// still be waiting for its predecessor; the router weights, which are older, are requested first, and the staging warps
+// wait before they touch the tokens (the others get everything from them).
+template <int CW, bool EARLY>
 __device__ __forceinline__ void router_tiny_block(const RouteParams &p, unsigned char *smem_raw, int m0, int n0) {
   using C = RouterTiny;
   constexpr int LD = C::LD, CH = C::CH, BK = C::BK, CPT = (C::ROWS * CH + 32 * CW - 1) / (32 * CW);
@@ -375,11 +377,12 @@ __device__ __forceinline__ void router_tiny_block(const RouteParams &p, unsigned
   if (threadIdx.x >= 64) {
     const int tid = (int)threadIdx.x - 64;
     unsigned char *const ring = smem_raw + 2 * C::F32_BYTES;
-    auto fetch = [&](int kb) {  // rows of k-block kb; beyond T, E or H they are zeros
+    auto fetch = [&](int kb, bool tokens, bool experts) {  // rows of k-block kb; beyond T, E or H they are zeros
 #pragma unroll
       for (int i = 0; i < CPT; ++i) {
         const int idx = i * 32 * CW + tid, r = idx / CH, k = kb * BK + idx % CH * 8;
         if (idx >= C::ROWS * CH) break;
+        if (!(r < 8 ? tokens : experts)) continue;
         const int row = r < 8 ? m0 + r : n0 + r - 8;
         const __nv_bfloat16 *base = r < 8 ? p.x : p.router_w;
         const bool valid = row < (r < 8 ? p.T : p.E) && k < p.H;
@@ -400,12 +403,17 @@ __device__ __forceinline__ void router_tiny_block(const RouteParams &p, unsigned
         reinterpret_cast<uint4 *>(dst)[0] = make_uint4(v.x << 16, v.x & hi, v.y << 16, v.y & hi);
         reinterpret_cast<uint4 *>(dst)[1] = make_uint4(v.z << 16, v.z & hi, v.w << 16, v.w & hi);
       }
-      if (kb + C::STAGES < nkb) fetch(kb + C::STAGES);
+      if (kb + C::STAGES < nkb) fetch(kb + C::STAGES, true, true);
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    if (EARLY) {
+#pragma unroll 1
+      for (int s = 0; s < C::STAGES && s < nkb; ++s) fetch(s, false, true);
+      coli_grid_wait();
+    }
 #pragma unroll 1
     for (int s = 0; s < C::STAGES; ++s) {
-      if (s < nkb) fetch(s);
+      if (s < nkb) fetch(s, true, !EARLY);
       asm volatile("cp.async.commit_group;" ::: "memory");
     }
     convert(0);
@@ -696,7 +704,7 @@ __global__ void __launch_bounds__(192) k_router_staged(RouteParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   coli_grid_dependency_sync();
   clear_expert_rows(p);
-  router_tiny_block<4>(p, smem_raw, (int)blockIdx.x * 8, (int)blockIdx.y * 8);
+  router_tiny_block<4, false>(p, smem_raw, (int)blockIdx.x * 8, (int)blockIdx.y * 8);
 }
 
 __global__ void __launch_bounds__(128) k_route_topk(RouteParams p) {
@@ -1212,7 +1220,8 @@ __global__ void __launch_bounds__(1024) k_permute_small(PermuteParams p, int max
 // kFrontSmem is therefore more than half of an SM's shared memory.  The last CTA runs top-k and permutation once per
 // call, with instructions that the streamed weights have pushed out of every cache: two warps that have nothing else to
 // do run the same code beside the chains, on router weights for logits, and write nothing (8 tokens, the weights of
-// three layers in turn: top-k 2.4 us, permutation 4.6 -> 1.8; the front 15.9 -> 14.4 us).
+// three layers in turn: top-k 2.4 us, permutation 4.6 -> 1.8; the front 15.9 -> 14.4 us).  They and the first router
+// weights do not wait for the predecessor: a call of 8 tokens 54.9 -> 53.0 us, of 1 token 25.1 -> 24.3.
 constexpr int kFrontStaging = 4, kFrontDry = 64;  // staging warps; threads of the dry run
 constexpr size_t kFrontSmem = 116 * 1024;
 static_assert(RouterTiny::SMEM <= kFrontSmem && (size_t)9 * topk_row_floats(32 * kMaxSlots) * sizeof(float) <= kFrontSmem - RouterTiny::SMEM,
@@ -1222,7 +1231,7 @@ __global__ void __launch_bounds__(256) k_decode_front(RouteParams rp, PermutePar
   __shared__ PermutePairsSmem psm;
   __shared__ int ids[kPairwiseMax];
   __shared__ int is_last;
-  coli_grid_dependency_sync();
+  coli_grid_trigger();  // (each role waits where it first needs the predecessor)
   constexpr int first_dry = 256 - kFrontDry;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float *rows = reinterpret_cast<float *>(smem_raw + RouterTiny::SMEM);
@@ -1233,17 +1242,10 @@ __global__ void __launch_bounds__(256) k_decode_front(RouteParams rp, PermutePar
     const bool dry = pass == 0;
     if (dry) {
       if ((int)threadIdx.x < first_dry) {
-        router_tiny_block<kFrontStaging>(rp, smem_raw, 0, (int)blockIdx.x * 8);
+        router_tiny_block<kFrontStaging, true>(rp, smem_raw, 0, (int)blockIdx.x * 8);
         continue;
       }
-      if (pp.x16) {  // this CTA's share of the f16 copy
-        const int n = rp.T * (rp.H / 8);
-        const int per = (n + (int)gridDim.x - 1) / (int)gridDim.x;
-        const int lo = (int)blockIdx.x * per, hi = min(n, lo + per);
-        const uint4 *src = reinterpret_cast<const uint4 *>(rp.x);
-        uint4 *dst = reinterpret_cast<uint4 *>(pp.x16);
-        for (int i = lo + (int)threadIdx.x - first_dry; i < hi; i += kFrontDry) dst[i] = coli_bf16x8_to_f16x8(src[i]);
-      }
+      if (rp.H >= 4096) coli_grid_wait();  // beside long chains there is time, and before them other kernels (281 / 283 us, 8 x 7168)
       tp.logits = const_cast<float *>(reinterpret_cast<const float *>(rp.router_w));  // E * H bf16 hold E floats (H >= 8)
       tp.topk_idx = nullptr;
       last = warp == 7 ? 1 : 0;
@@ -1269,6 +1271,17 @@ __global__ void __launch_bounds__(256) k_decode_front(RouteParams rp, PermutePar
     for (int j = i; j < kPairwiseMax; j += threads) psm.seg[j] = j < (dry ? rp.k : rp.T * rp.k) ? pair_segment(pp, ids[j]) : 0x7fffffff;
     asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(bar), "r"(threads) : "memory");
     permute_pairs(pp, max_items, psm, i, threads, bar, dry);
+    if (dry) {
+      coli_grid_wait();
+      if (pp.x16) {  // this CTA's share of the f16 copy
+        const int n = rp.T * (rp.H / 8);
+        const int per = (n + (int)gridDim.x - 1) / (int)gridDim.x;
+        const int lo = (int)blockIdx.x * per, hi = min(n, lo + per);
+        const uint4 *src = reinterpret_cast<const uint4 *>(rp.x);
+        uint4 *dst = reinterpret_cast<uint4 *>(pp.x16);
+        for (int i = lo + (int)threadIdx.x - first_dry; i < hi; i += kFrontDry) dst[i] = coli_bf16x8_to_f16x8(src[i]);
+      }
+    }
   }
   if (threadIdx.x == 0) *ticket = 0u;
 }
