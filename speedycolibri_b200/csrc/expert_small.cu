@@ -787,15 +787,16 @@ static int launch_stream(const FfnParams &p, bool gated, bool items_known, cudaS
   coli_count_launch(1);
   return coli_cuda_check(e, "expert ffn launch") ? 1 : 0;
 }
-// Slabs of 32 rows from two rounds of such tasks on: the instructions around a k-tile are then spent on twice the
-// weights, and the tasks still divide over the warps.  24 tokens on H 7168, I 2048, 256 experts 675 -> 627 us a call; at
-// 1.3 rounds (48 tokens, H 2048, I 768, 128 experts) 108.7 -> 110.7, at 0.5 (8 tokens) 49.3 and 49.8: 16 rows there.
+// Slabs of 32 rows from one and a half rounds of such tasks on (by the host's estimate): the instructions around a k-tile
+// are then spent on twice the weights, and the tasks still divide over the warps.  24 tokens on H 7168, I 2048, 256
+// experts (6.6 rounds) 675 -> 627 us a call; 48 tokens on H 2048, I 768, 128 experts (gate+up 1.9) 100.1 -> 97.5; 8 tokens there
+// (down 1.1 rounds) 52.2 and 52.8, (gate+up 0.8) 52.2 and 53.8: 16 rows.
 // FP8 k-tiles are twice as long: two CTAs of such rings do not fit an SM.
 template <int FMT>
 static int launch_stream_rows(const FfnParams &p, bool gated, bool items_known, cudaStream_t st) {
   if constexpr (FMT == COLI_FMT_NVFP4) {
     const int O = gated ? p.I : p.H, rows = gated ? 32 : 64;
-    if (O % rows == 0 && (long)p.items_expected * (O / rows) >= 2L * 16 * COLI_SMS)
+    if (O % rows == 0 && (long)p.items_expected * (O / rows) >= 3L * 8 * COLI_SMS)
       return launch_stream<FMT, 2>(p, gated, items_known, st);
   }
   return launch_stream<FMT, 1>(p, gated, items_known, st);

@@ -1217,13 +1217,14 @@ __global__ void __launch_bounds__(1024) k_permute_small(PermuteParams p, int max
 // The kernel is latency from end to end, and its CTAs must not share an SM: started early, while the
 // previous call's last kernels still hold most SMs, two or three packed onto each free one and the chains
 // took 14.6 cycles per k instead of 6 (8 tokens, 128 experts x 2048: 30 000 of the kernel's 44 000 cycles).
-// kFrontSmem is therefore more than half of an SM's shared memory.  The last CTA runs top-k and permutation once per
+// kFrontSmem is therefore, with what is static, more than half of an SM's shared memory, and little enough to lie beside one CTA
+// of the decode expert kernel, which may still hold the SM when the front starts.  The last CTA runs top-k and permutation once per
 // call, with instructions that the streamed weights have pushed out of every cache: two warps that have nothing else to
 // do run the same code beside the chains, on router weights for logits, and write nothing (8 tokens, the weights of
 // three layers in turn: top-k 2.4 us, permutation 4.6 -> 1.8; the front 15.9 -> 14.4 us).  They and the first router
 // weights do not wait for the predecessor: a call of 8 tokens 54.9 -> 53.0 us, of 1 token 25.1 -> 24.3.
 constexpr int kFrontStaging = 4, kFrontDry = 64;  // staging warps; threads of the dry run
-constexpr size_t kFrontSmem = 116 * 1024;
+constexpr size_t kFrontSmem = 112 * 1024;
 static_assert(RouterTiny::SMEM <= kFrontSmem && (size_t)9 * topk_row_floats(32 * kMaxSlots) * sizeof(float) <= kFrontSmem - RouterTiny::SMEM,
               "the top-k rows of eight warps and of the dry run lie behind the staging area");
 __global__ void __launch_bounds__(256) k_decode_front(RouteParams rp, PermuteParams pp, int max_items, unsigned int *ticket) {
