@@ -755,7 +755,10 @@ static bool launch_router_chain(const RouteParams &p, cudaStream_t st) {
 template <class C>
 static bool launch_router_pair(const RouteParams &p, cudaStream_t st) {
   static ColiPerDeviceOnce attr_once;
-  return launch_router_kernel(k_router_pair<C>, attr_once, dim3((p.T + C::BM - 1) / C::BM, (p.E + C::BN - 1) / C::BN), C::NT, C::SMEM, p, st);
+  // (never early: thousands of tokens follow a combine of as many rows, whose last CTAs its own then wait beside; us a call,
+  // ordinary / early: 3000 tokens, H 3072, 256 experts 689 / 706; 8192, H 2048, 256 1008 / 1028; 7026, H 1920, 177 572 / 598;
+  // 16384, H 2048, 384 10470 / 10700; 4096, H 7168, 256 3750 / 3750)
+  return launch_router_kernel(k_router_pair<C>, attr_once, dim3((p.T + C::BM - 1) / C::BM, (p.E + C::BN - 1) / C::BN), C::NT, C::SMEM, p, st, false);
 }
 // The tile of a batch: 0 = 8 x 8, 1 = 16 x 32, 2 = 64 x 64, 3 = 128 x 64, 4 = 128 x 128 tokens x experts.
 // The time of one k is a function of n, the CTAs of the fullest SM; the figures are nanoseconds measured
