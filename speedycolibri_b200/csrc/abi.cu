@@ -502,29 +502,29 @@ extern "C" void *coli_b200_moe_stream(ColiMoe *m) { return m ? (void *)m->ctx->s
 int coli_tct_tile_tokens(int rows, int nseg) {
   return rows <= 48 * (nseg > 0 ? nseg : 1) ? colib::TCT_SHORT_TOKENS : colib::TCT_MAX_TOKENS;
 }
-// The tcgen05 path takes over from 8 rows per segment on average: below that the register-level
-// kernel re-reads so few token rows per weight tile that it wins.  It cuts segments into items of 8
-// rows there and reads their weights once per item, so on a layer too large for L2 the line lies at 6
-// rows, as long as the tcgen05 kernel's tiles (128 features of an expert) divide well over the SMs.
-// Measured (register-level / tcgen05, us a call): H 7168, I 2048, 256 experts (4112 tiles) at 4.5 rows 1443 /
-// 1452, 7.0 2300 / 1496; H 3072, I 1280, 200 experts (2010) at 5.5 354 / 342, 6.3 460 / 344; H 4096, I 1536, 150
-// (1812) at 5.5 408 / 400, 6.3 435 / 400, and 128 (1548) 351 / 345, 378 / 351; H 3072, I 1280, 128 (1290) at 5.4
-// 234 / 238, 6.3 249 / 239; H 2048, I 1024, 128 (1032) at 6.3 146 / 150, 7.2 160 / 150; H 2048, I 768, 128 (774)
-// at 6.7 136 / 147, 8.0 150 / 148, FP8 6.7 167 / 179, 8.0 182 / 180.  So 1776 tiles are on the safe side.
-// FP8 128x128 stays at 8 rows: the register-level kernel applies its scales in f32, the tcgen05 kernel as f16
-// multipliers (error against 64 bits 2.864e-3 and 2.896e-3 at 7.5 rows, H 2048, I 1024, 256 experts).
+// The tcgen05 path takes over from 8 rows per segment on average: below that the decode kernel, which reads a segment's
+// weights once per item of 8 rows and converts as many of them as it reads, wins on every layer that was measured (decode /
+// tcgen05, us a call): H 7168, I 2048, 256 experts (4112 weight tiles of 128 features) at 6.0 rows 1203 / 1438, 7.9 1459 / 1441; H 3072,
+// I 1280, 128 experts (1290) 7.9 214 / 234; H 1024, I 2048, 120 experts 7.9 124 / 141.  NVFP4 layers of up to 888 tiles take it up to
+// 10 rows, where most segments are two items whose weights meet in L2: H 2048, I 768, 128 experts (774) 8.2 113 / 129, 9.0 117 / 122,
+// 10.0 120 / 122, 11.0 132 / 128; H 1024, I 512, 64 experts (260) 10.0 46 / 52; 1290 tiles 9.0 227 / 226; per-row FP8 on 774 tiles 8.2
+// 143 / 147, 9.0 142 / 140.
+// FP8 128x128 stays at 8 rows although the tcgen05 kernel wins from 5 (H 4096, I 1024, 256 experts 5.0 550 / 532): it applies the
+// scales as f16 multipliers, the decode kernel in f32 (error against 64 bits 2.896e-3 and 2.864e-3 at 7.5 rows, H 2048, I 1024).
+// Layers of a single k-tile with many weight tiles keep their line at 6 rows and with it the number of launches that callers
+// know (the decode kernel would take 39 us against 55 at 6 rows, H 128, I 1920, 120 experts).
 // A pure function of shapes, so that kernel selection never depends on data or addresses.
 static bool tc_format(int fmt) { return fmt == COLI_FMT_NVFP4 || fmt == COLI_FMT_FP8_B128 || fmt == COLI_FMT_E4M3_ROW; }
-bool coli_use_tc_path(int fmt, int rows, int nseg, int I) {
+bool coli_use_tc_path(int fmt, int rows, int nseg, int H, int I) {
   if (!tc_format(fmt) || nseg <= 0) return false;
-  const bool many_tiles = fmt != COLI_FMT_FP8_B128 && (long)nseg * ((I + 127) / 128) >= 12L * COLI_SMS;
-  return (long)rows >= (many_tiles ? 6L : 8L) * nseg;
+  const long tiles = (long)nseg * ((I + 127) / 128);
+  long line = 8;
+  if (fmt == COLI_FMT_NVFP4 && tiles <= 6L * COLI_SMS) line = 10;
+  if (fmt != COLI_FMT_FP8_B128 && tiles >= 12L * COLI_SMS && H <= 128) line = 6;
+  return (long)rows >= line * nseg;
 }
-
-int coli_rows_per_item_for(int rows, int nseg) {
-  const int avg = (rows + nseg - 1) / (nseg > 0 ? nseg : 1);
-  return avg <= 8 ? 8 : avg <= 16 ? 16 : 32;
-}
+// Rows of a work item on the decode kernel.
+constexpr int kDecodeItemRows = 8;
 
 extern "C" int coli_b200_moe_create(ColiMoe **out, const ColiMoeLayer *L, int max_tokens) {
   if (!out || !L || max_tokens < 1) {
@@ -667,7 +667,7 @@ extern "C" int coli_b200_moe_create(ColiMoe **out, const ColiMoeLayer *L, int ma
   ok = ok && ws_alloc(m, &m->status, 1) && coli_cuda_check(cudaMemset(m->status, 0, sizeof(int)), "status clear");
   m->ticket = nullptr;
   ok = ok && ws_alloc(m, &m->ticket, 1) && coli_cuda_check(cudaMemset(m->ticket, 0, sizeof(unsigned int)), "ticket clear");
-  if (ok && coli_use_tc_path(coli_kernel_fmt(L->fmt), (int)rows, m->nseg, L->I)) ok = ws_alloc(m, &m->xg, rows * H);
+  if (ok && coli_use_tc_path(coli_kernel_fmt(L->fmt), (int)rows, m->nseg, L->H, L->I)) ok = ws_alloc(m, &m->xg, rows * H);
   m->select_bias = nullptr;
   m->logit_bias = nullptr;
   if (ok && L->select_bias) ok = ws_alloc(m, &m->select_bias, E);
@@ -806,8 +806,8 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
   cudaStream_t st = pick_stream(m, stream);
   const int k = m->L.k;
   const int rows = T * k + (m->has_shared ? T : 0);
-  const bool tc = coli_use_tc_path(m->L.fmt, rows, m->nseg, m->L.I) && m->xg != nullptr;
-  const int rpi = tc ? coli_tct_tile_tokens(rows, m->nseg) : coli_rows_per_item_for(rows, m->nseg);
+  const bool tc = coli_use_tc_path(m->L.fmt, rows, m->nseg, m->L.H, m->L.I) && m->xg != nullptr;
+  const int rpi = tc ? coli_tct_tile_tokens(rows, m->nseg) : kDecodeItemRows;
   const int max_items = max_work_items(rows, m->nseg, rpi);
   // Segments are in (owner, expert id) order, also when every expert is resident: only where that is the
   // expert order do the kernels index the weight tables by segment and save the dependent load.
@@ -1093,8 +1093,8 @@ int coli_run_segments(ColiMoe *m, SegScratch &sc, const WeightRef *g, const Weig
                       const int32_t *seg_expert_dev, const void *rows_dev, const int32_t *seg_count_dev, int n_seg,
                       int rows_cap, int rows_expected, void *y_dev, cudaStream_t st) {
   if (rows_cap == 0 || n_seg == 0) return 1;
-  const bool tc = coli_use_tc_path(m->L.fmt, rows_expected, n_seg, m->L.I);
-  const int rpi = tc ? coli_tct_tile_tokens(rows_expected, n_seg) : coli_rows_per_item_for(rows_expected, n_seg);
+  const bool tc = coli_use_tc_path(m->L.fmt, rows_expected, n_seg, m->L.H, m->L.I);
+  const int rpi = tc ? coli_tct_tile_tokens(rows_expected, n_seg) : kDecodeItemRows;
   const int max_items = max_work_items(rows_cap, n_seg, rpi);
   if (!ensure_h(m, sc, (size_t)rows_cap) || !ensure_items(m, sc, max_items, n_seg)) return 0;
   if (!colib::launch_items_from_counts(seg_count_dev, n_seg, rpi, sc.seg_off, sc.item_seg, sc.item_row0, sc.item_nrows,
@@ -1242,9 +1242,9 @@ extern "C" uint64_t coli_b200_sharding_fingerprint(uint32_t num_nodes, uint32_t 
 // Kernel selection follows the row counts alone, as the reference's does (backend_cuda.cu:4738-4783
 // switches kernels at 32 rows): from 8 rows per expert on average the group runs on the tcgen05
 // kernels, whose y is rounded to bf16 before it is widened to f32; below that on the
-// register-level kernel, which writes f32 directly.  (The block, whose rows are bf16 on both paths,
-// moves its line for large layers; here that would cost groups of 6 and 7 rows their f32 results:
-// error against 64 bits 1.68e-3 -> 2.37e-3.)
+// decode kernel, which writes f32 directly.  (The block, whose rows are bf16 on both paths, moves its line with
+// the layer; here a lower one would cost groups of 6 and 7 rows their f32 results: error against 64 bits
+// 1.68e-3 -> 2.37e-3.)
 namespace {
 std::mutex g_group_stats_mu;  // backend_cuda.cu:98-100
 uint64_t g_group_calls = 0, g_group_experts = 0, g_group_rows = 0;

@@ -20,6 +20,7 @@ pytestmark = pytest.mark.gpu
     (33, 296, 8, 520, SCORE_SIGMOID, 1, True), (130, 400, 8, 264, SCORE_SOFTMAX, 1, True),                  # ... 185 tiles; 1040 pairs, x copied
     (12, 4, 4, 264, SCORE_SOFTMAX, 1, True), (170, 20, 6, 264, SCORE_SOFTMAX, 1, True),                     # gathered: 31 KB | 1020 pairs, 628 KB
     (171, 20, 6, 264, SCORE_SOFTMAX, 1, True), (600, 512, 32, 72, SCORE_SIGMOID, 1, False),                 # 1026 and 19200 pairs
+    (29, 20, 6, 264, SCORE_SOFTMAX, 1, True), (30, 20, 6, 264, SCORE_SOFTMAX, 1, True),                     # 9.7 | 10 rows a segment: two items each
     (2049, 40, 32, 24, SCORE_SOFTMAX, 1, True),                                                             # above 65536 pairs
 ])
 @pytest.mark.parametrize("equal", [0, 40], ids=["distinct", "ties"])
