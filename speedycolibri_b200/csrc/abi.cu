@@ -1294,8 +1294,7 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
   cudaStream_t st = ctx->stream;
   const int kfmt = coli_kernel_fmt(fmt);
   const bool tc = tc_format(kfmt) && total >= 8L * count;
-  const int avg = (int)((total + count - 1) / count);
-  const int rpi = tc ? coli_tct_tile_tokens((int)total, count) : (avg <= 8 ? 8 : avg <= 16 ? 16 : 32);
+  const int rpi = tc ? coli_tct_tile_tokens((int)total, count) : kDecodeItemRows;
   const int max_items = max_work_items((int)total, count, rpi);
   const size_t xb = (size_t)total * D;
   // slots: 0 x f32 / y f32, 1 x f16, 2 h f16, 3 tables + counts + work list + status word, 4 y bf16 (tcgen05 path)

@@ -1,7 +1,7 @@
 // Expert FFN for decode-sized segments: a weight-streaming dequant-GEMV/GEMM in which every
 // weight byte is read from HBM exactly once per work item with 128-bit loads, converted to
 // f16 in registers (one hardware cvt per pair of FP4 or FP8 codes, one half2 multiply by the
-// block scale for NVFP4), and contracted against up to 32 token rows with warp-level f16 MMA
+// block scale for NVFP4), and contracted against eight token rows at a time with warp-level f16 MMA
 // (m16n8k16, f32 accumulate).  The path is HBM-bound: the MMA only takes the multiply-adds
 // off the CUDA cores so that the decode arithmetic (about one operation per FP4 weight) is
 // all the SM has to issue per byte streamed.
@@ -146,36 +146,31 @@ __device__ __forceinline__ void decode_a(const AFrag<FMT> &f, const AScale &sc, 
   }
 }
 
-// GATED: two matrices (gate, up) -> h = silu(g)*u;  otherwise one matrix (down) -> y.
+// One matrix over items of 9 to 32 rows: the f32 matmul and ReLU^2 calls on host buffers.
 // SPLITK: grid = (row tiles, work items); the W warps of a CTA share one 16-row tile and split
-// the k-tiles (few work items: a single-token decode).  Otherwise the grid is one-dimensional
-// and sized to what is resident at once; every warp walks (item, row tile) tasks with a stride,
-// owns its tile over all of K and needs no cross-warp reduction.
-template <int FMT, int NB, bool GATED, bool SPLITK>
+// the k-tiles (few work items).  Otherwise the grid is one-dimensional and sized to what is resident at
+// once; every warp walks (item, row tile) tasks with a stride, owns its tile over all of K and needs no
+// cross-warp reduction.
+template <int FMT, int NB, bool SPLITK>
 __global__ void __launch_bounds__(SPLITK ? 256 : 64, SPLITK                  ? 1
-                                                      : FMT == COLI_FMT_NVFP4 ? (NB == 1 ? 10 : NB == 2 ? 8 : 4)
-                                                                              : (NB == 1 ? 7 : NB == 2 ? 5 : 4))
+                                                      : FMT == COLI_FMT_NVFP4 ? (NB == 2 ? 8 : 4)
+                                                                              : (NB == 2 ? 5 : 4))
     k_ffn_mm(FfnParams p) {
-  constexpr int MATS = GATED ? 2 : 1;
   // weight ring depth (k-tiles) and token-fragment ring depth (quarter k-tiles)
   constexpr int D = 2;
   constexpr int R = NB <= 2 ? 4 : 2;
   constexpr int PF = R - 1;
-  extern __shared__ __align__(16) float red[];  // [W][MATS*NB*4][32]
+  extern __shared__ __align__(16) float red[];  // [W][NB*4][32]
   coli_grid_dependency_sync();
   const int n_items = *p.n_items;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int K = GATED ? p.H : p.I;     // contraction length
-  const int Oout = GATED ? p.I : p.H;  // output features
+  const int K = p.I, Oout = p.H;  // contraction length, output features
   const int Kp = (K + 127) & ~127, KT = Kp >> 7, Op = (Oout + 15) & ~15;
   const int row_tiles = Op >> 4;
-  const __half *src = GATED ? p.x : p.h;
 
   // Tasks are (item, row tile) pairs, one per warp and round (per CTA when K is split).  The entry of a
-  // task is requested a task ahead, the first one beside the item count: at one token the chain of
-  // dependent loads in front of the weights was a fifth of the two launches (16.8 + 11.4 -> 14.8 + 10.8 us).
-  // (Splitting a last, mostly empty round over K was built too: its run-time k step cost every round 8 %.)
+  // task is requested a task ahead, the first one beside the item count.
   const int n_warps = (int)gridDim.x * W;
   const int n_tasks = n_items * row_tiles;
   struct ItemInfo {
@@ -196,30 +191,21 @@ __global__ void __launch_bounds__(SPLITK ? 256 : 64, SPLITK                  ? 1
     const int seg = next.seg, row0 = next.row0, nrows = next.nrows;
     if (!SPLITK) next = item_of(task + n_warps);
     const int ex = p.seg_expert ? p.seg_expert[seg] : seg;
-    const WeightRef w0 = GATED ? p.gate[ex] : p.down[ex];
-    const WeightRef w1 = GATED ? p.up[ex] : w0;
+    const WeightRef w0 = p.down[ex];
 
     // source row of token column g of each 8-token block (nullptr = column beyond the item)
     const __half *xrow[NB];
 #pragma unroll
     for (int j = 0; j < NB; ++j) {
       const int r = 8 * j + g;
-      if (r < nrows) {
-        const int row = row0 + r;
-        const size_t sidx = (GATED && p.row_token) ? (size_t)p.row_token[row] : (size_t)row;
-        xrow[j] = src + sidx * K;
-      } else {
-        xrow[j] = nullptr;
-      }
+      xrow[j] = r < nrows ? p.h + (size_t)(row0 + r) * K : nullptr;
     }
 
-    float acc[MATS][NB][4];
+    float acc[NB][4];
 #pragma unroll
-    for (int mtx = 0; mtx < MATS; ++mtx)
+    for (int j = 0; j < NB; ++j)
 #pragma unroll
-      for (int j = 0; j < NB; ++j)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[mtx][j][c] = 0.0f;
+      for (int c = 0; c < 4; ++c) acc[j][c] = 0.0f;
 
     const int kstep = SPLITK ? W : 1;
     const int kt_first = SPLITK ? warp : 0;
@@ -238,15 +224,12 @@ __global__ void __launch_bounds__(SPLITK ? 256 : 64, SPLITK                  ? 1
     // Register rings, both unrolled so that every slot is a fixed set of registers (rotating
     // slots with copies would make each iteration wait for the youngest load): packed weight
     // fragments D k-tiles deep, token fragments R quarter-k-tiles deep.
-    AFrag<FMT> ring[D][MATS];
+    AFrag<FMT> ring[D];
     uint4 xq[R][NB];
 #pragma unroll
     for (int j = 0; j < D - 1; ++j) {
       const int ktl = kt_first + j * kstep;
-      if (ktl < KT) {
-        load_a<FMT>(ring[j][0], w0, Op, r0, ktl, lane);
-        if (GATED) load_a<FMT>(ring[j][MATS - 1], w1, Op, r0, ktl, lane);
-      }
+      if (ktl < KT) load_a<FMT>(ring[j], w0, Op, r0, ktl, lane);
     }
 #pragma unroll
     for (int f = 0; f < PF; ++f) load_x(xq[f % R], kt_first + (f / 4) * kstep, f % 4);
@@ -257,21 +240,14 @@ __global__ void __launch_bounds__(SPLITK ? 256 : 64, SPLITK                  ? 1
         const int kt = kt0 + slot * kstep;
         if (kt >= KT) break;
         const int ktn = kt + (D - 1) * kstep;
-        if (ktn < KT) {
-          load_a<FMT>(ring[(slot + D - 1) % D][0], w0, Op, r0, ktn, lane);
-          if (GATED) load_a<FMT>(ring[(slot + D - 1) % D][MATS - 1], w1, Op, r0, ktn, lane);
-        }
-        AScale asc[MATS];
-#pragma unroll
-        for (int mtx = 0; mtx < MATS; ++mtx) asc[mtx] = decode_scales<FMT>(ring[slot][mtx]);
-        float part[MATS][NB][4];
+        if (ktn < KT) load_a<FMT>(ring[(slot + D - 1) % D], w0, Op, r0, ktn, lane);
+        const AScale asc = decode_scales<FMT>(ring[slot]);
+        float part[NB][4];
         if (FMT == COLI_FMT_FP8_B128) {
 #pragma unroll
-          for (int mtx = 0; mtx < MATS; ++mtx)
+          for (int j = 0; j < NB; ++j)
 #pragma unroll
-            for (int j = 0; j < NB; ++j)
-#pragma unroll
-              for (int c = 0; c < 4; ++c) part[mtx][j][c] = 0.0f;
+            for (int c = 0; c < 4; ++c) part[j][c] = 0.0f;
         }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -281,102 +257,66 @@ __global__ void __launch_bounds__(SPLITK ? 256 : 64, SPLITK                  ? 1
 #pragma unroll
           for (int mm = 0; mm < 2; ++mm) {
             const int m = 2 * c + mm;
+            uint32_t a[4];
+            decode_a<FMT>(ring[slot], asc, m, a);
 #pragma unroll
-            for (int mtx = 0; mtx < MATS; ++mtx) {
-              uint32_t a[4];
-              decode_a<FMT>(ring[slot][mtx], asc[mtx], m, a);
-#pragma unroll
-              for (int j = 0; j < NB; ++j) {
-                const uint32_t b0 = mm ? xb[j].z : xb[j].x, b1 = mm ? xb[j].w : xb[j].y;
-                if (FMT == COLI_FMT_FP8_B128)
-                  mma_f16_16816(part[mtx][j], a, b0, b1);
-                else
-                  mma_f16_16816(acc[mtx][j], a, b0, b1);
-              }
+            for (int j = 0; j < NB; ++j) {
+              const uint32_t b0 = mm ? xb[j].z : xb[j].x, b1 = mm ? xb[j].w : xb[j].y;
+              mma_f16_16816(FMT == COLI_FMT_FP8_B128 ? part[j] : acc[j], a, b0, b1);
             }
           }
         }
         if (FMT == COLI_FMT_FP8_B128) {
           // one f32 scale per (128-row block, k-tile): convert.rs:731-741
+          const float s = reinterpret_cast<const float *>(w0.s)[(size_t)(r0 >> 7) * KT + kt];
 #pragma unroll
-          for (int mtx = 0; mtx < MATS; ++mtx) {
-            const float *sc = reinterpret_cast<const float *>(mtx == 0 ? w0.s : w1.s);
-            const float s = sc[(size_t)(r0 >> 7) * KT + kt];
+          for (int j = 0; j < NB; ++j)
 #pragma unroll
-            for (int j = 0; j < NB; ++j)
-#pragma unroll
-              for (int c = 0; c < 4; ++c) acc[mtx][j][c] = fmaf(s, part[mtx][j][c], acc[mtx][j][c]);
-          }
+            for (int c = 0; c < 4; ++c) acc[j][c] = fmaf(s, part[j][c], acc[j][c]);
         }
       }
     }
 
     // epilogue of one 8-token block given its reduced accumulators
-    auto emit = [&](int j, const float(&v)[MATS][4]) {
+    auto emit = [&](int j, const float(&v)[4]) {
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int orow = r0 + g + ((c & 2) ? 8 : 0);  // output feature
         const int col = 8 * j + 2 * t + (c & 1);      // token within the item
         if (orow >= Oout || col >= nrows) continue;
-        float s0 = 1.0f, s1 = 1.0f;
-        if (FMT == COLI_FMT_NVFP4) {
-          s0 = w0.g;
-          s1 = w1.g;
-        } else if (FMT == COLI_FMT_E4M3_ROW) {
-          s0 = reinterpret_cast<const float *>(w0.s)[orow];
-          s1 = reinterpret_cast<const float *>(w1.s)[orow];
-        }
+        const float s0 = FMT == COLI_FMT_NVFP4 ? w0.g : FMT == COLI_FMT_E4M3_ROW ? reinterpret_cast<const float *>(w0.s)[orow] : 1.0f;
         const size_t row = (size_t)(row0 + col);
-        if (GATED) {
-          const float gv = v[0][c] * s0, uv = v[MATS - 1][c] * s1;
-          const float hv = coli_act_fast(gv, uv, p.act);
-          p.h[row * p.I + orow] = coli_f32_to_f16_via_bf16(hv);
+        if (p.relu2_out) {
+          const float r = fmaxf(v[c] * s0, 0.0f);
+          p.relu2_out[row * p.H + orow] = coli_f32_to_f16_via_bf16(r * r);
         } else {
-          if (p.relu2_out) {
-            const float r = fmaxf(v[0][c] * s0, 0.0f);
-            p.relu2_out[row * p.H + orow] = coli_f32_to_f16_via_bf16(r * r);
-          } else if (p.y32) {
-            p.y32[row * p.H + orow] = v[0][c] * s0;
-          } else {
-            p.y[row * p.H + orow] = __float2bfloat16_rn(v[0][c] * s0);
-          }
+          p.y32[row * p.H + orow] = v[c] * s0;
         }
       }
     };
 
     if (!SPLITK) {
 #pragma unroll
-      for (int j = 0; j < NB; ++j) {
-        float v[MATS][4];
-#pragma unroll
-        for (int mtx = 0; mtx < MATS; ++mtx)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) v[mtx][c] = acc[mtx][j][c];
-        emit(j, v);
-      }
+      for (int j = 0; j < NB; ++j) emit(j, acc[j]);
       continue;
     }
 
     // cross-warp (split-K) reduction; every warp of the CTA is on the same task
-    constexpr int NV = MATS * NB * 4;
+    constexpr int NV = NB * 4;
 #pragma unroll
-    for (int mtx = 0; mtx < MATS; ++mtx)
+    for (int j = 0; j < NB; ++j)
 #pragma unroll
-      for (int j = 0; j < NB; ++j)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) red[((size_t)warp * NV + (mtx * NB + j) * 4 + c) * 32 + lane] = acc[mtx][j][c];
+      for (int c = 0; c < 4; ++c) red[((size_t)warp * NV + j * 4 + c) * 32 + lane] = acc[j][c];
     __syncthreads();
 
     for (int j = warp; j < NB; j += W) {
-      float v[MATS][4];
+      float v[4];
 #pragma unroll
-      for (int mtx = 0; mtx < MATS; ++mtx)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          float s = 0.0f;
-          for (int w = 0; w < W; ++w) s += red[((size_t)w * NV + (mtx * NB + j) * 4 + c) * 32 + lane];
-          v[mtx][c] = s;
-        }
+      for (int c = 0; c < 4; ++c) {
+        float s = 0.0f;
+        for (int w = 0; w < W; ++w) s += red[((size_t)w * NV + j * 4 + c) * 32 + lane];
+        v[c] = s;
+      }
       emit(j, v);
     }
     break;  // the CTA's only task
@@ -949,41 +889,38 @@ static int pick_w(int KT) { return KT >= 8 ? 8 : KT >= 4 ? 4 : KT >= 2 ? 2 : 1; 
 // Split K across the warps of a CTA only when there are too few (item, row tile) tasks to fill
 // the SMs with one warp each; `p.items_expected` is a host-side estimate from shapes alone.
 template <int FMT, int NB>
-static int launch_one(const FfnParams &p, bool gated, cudaStream_t st) {
-  const int K = gated ? p.H : p.I, O = gated ? p.I : p.H;
+static int launch_one(const FfnParams &p, cudaStream_t st) {
+  const int K = p.I, O = p.H;
   const int KT = (K + 127) / 128, row_tiles = (O + 15) / 16;
   const long tasks = (long)row_tiles * (p.items_expected > 0 ? p.items_expected : 1);
   const bool splitk = tasks < 12L * COLI_SMS;
   if (splitk) {
     const int W = pick_w(KT);
     dim3 grid(row_tiles, p.max_items);
-    const size_t sm = (size_t)W * (gated ? 2 : 1) * NB * 4 * 32 * sizeof(float);
-    const cudaError_t e = gated ? launch_dependent(k_ffn_mm<FMT, NB, true, true>, grid, dim3(W * 32), sm, st, p)
-                                : launch_dependent(k_ffn_mm<FMT, NB, false, true>, grid, dim3(W * 32), sm, st, p);
+    const size_t sm = (size_t)W * NB * 4 * 32 * sizeof(float);
+    const cudaError_t e = launch_dependent(k_ffn_mm<FMT, NB, true>, grid, dim3(W * 32), sm, st, p);
     coli_count_launch(1);
     return coli_cuda_check(e, "expert ffn launch") ? 1 : 0;
   } else {
     // two warps per CTA keep the per-SM share of tasks even; the grid covers what fits at once
     constexpr int W = 2;
     // resident CTAs per kernel variant and device ordinal (an occupancy figure belongs to one device)
-    static int resident_tab[2][32];
+    static int resident_tab[32];
     int dev = 0;
     if (!coli_cuda_check(cudaGetDevice(&dev), "device query")) return 0;
     int uncached = 0;
-    int &resident_slot = (dev >= 0 && dev < 32) ? resident_tab[gated ? 1 : 0][dev] : uncached;
+    int &resident_slot = (dev >= 0 && dev < 32) ? resident_tab[dev] : uncached;
     if (resident_slot == 0) {
       int sms = 0, per_sm = 0;
       if (!coli_cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device query")) return 0;
-      const cudaError_t e = gated ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ffn_mm<FMT, NB, true, false>, W * 32, 0)
-                                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ffn_mm<FMT, NB, false, false>, W * 32, 0);
+      const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ffn_mm<FMT, NB, false>, W * 32, 0);
       if (!coli_cuda_check(e, "occupancy query")) return 0;
       resident_slot = sms * (per_sm > 0 ? per_sm : 1);
     }
     const int resident_ctas = resident_slot;
     const long max_ctas = ((long)row_tiles * p.max_items + W - 1) / W;
     const int grid = (int)(max_ctas < resident_ctas ? max_ctas : resident_ctas);
-    const cudaError_t e = gated ? launch_dependent(k_ffn_mm<FMT, NB, true, false>, dim3(grid), dim3(W * 32), 0, st, p)
-                                : launch_dependent(k_ffn_mm<FMT, NB, false, false>, dim3(grid), dim3(W * 32), 0, st, p);
+    const cudaError_t e = launch_dependent(k_ffn_mm<FMT, NB, false>, dim3(grid), dim3(W * 32), 0, st, p);
     coli_count_launch(1);
     return coli_cuda_check(e, "expert ffn launch") ? 1 : 0;
   }
@@ -997,13 +934,13 @@ static int launch_ffn_stage(const FfnParams &p, bool gated, bool items_known, cu
     coli_set_error("expert ffn: H=%d and I=%d must be multiples of 8", p.H, p.I);
     return 0;
   }
-  if (p.rows_per_item > 32) {
-    coli_set_error("expert ffn: rows_per_item=%d exceeds 32", p.rows_per_item);
+  if (p.rows_per_item > (gated ? 8 : 32)) {
+    coli_set_error("expert ffn: rows_per_item=%d exceeds %d", p.rows_per_item, gated ? 8 : 32);
     return 0;
   }
   const int nb = p.rows_per_item <= 8 ? 1 : p.rows_per_item <= 16 ? 2 : 4;
 #define COLI_DISPATCH(F) \
-  (nb == 1 ? launch_stream_rows<F>(p, gated, items_known, st) : nb == 2 ? launch_one<F, 2>(p, gated, st) : launch_one<F, 4>(p, gated, st))
+  (nb == 1 ? launch_stream_rows<F>(p, gated, items_known, st) : nb == 2 ? launch_one<F, 2>(p, st) : launch_one<F, 4>(p, st))
   switch (p.fmt) {
     case COLI_FMT_NVFP4:
       return COLI_DISPATCH(COLI_FMT_NVFP4);

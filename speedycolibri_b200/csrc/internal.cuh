@@ -209,7 +209,7 @@ struct FfnParams {
   const int32_t *seg_expert;          // [nseg] weight-table index of each segment (null = identity)
   const int32_t *item_seg, *item_row0, *item_nrows, *n_items;
   int max_items;
-  int rows_per_item;         // rows per work item the list was cut with (<= 32)
+  int rows_per_item;         // rows per work item the list was cut with (<= 8; the down form alone <= 32)
   int items_expected;        // host estimate of the work items (selects split-K vs tile-per-warp)
   const __half *x;           // source rows (f16)
   const int32_t *row_token;  // row -> source row index (null = identity)
@@ -295,10 +295,11 @@ int launch_matmul_f32_seq(const float *x, const float *w, float *y, int S, int I
 // event between kernels) the device calls are no-ops.
 // Where it is not used, or not early: a kernel whose CTAs must spread evenly over the SMs, several
 // fitting on one, packs onto the SMs that happen to be free while its predecessor still runs (the
-// router of 4096 tokens took 1180 us instead of 445 that way).  The router GEMMs, first in a call, are
-// therefore launched the ordinary way, and a permutation that is followed by the register-level expert
-// kernel lets it start only when it is done (FP8, 130 tokens, H 4096, I 1024, 256 experts: 1030 us a call
-// when the three-launch permutation did not, 558 since; NVFP4 535 and 453).
+// router of 4096 tokens took 1180 us instead of 445 that way).  The top-k and the router GEMMs of up to a few hundred
+// tokens keep their spread by the shared memory they ask for (launch_router_kernel in routing.cu); larger router GEMMs are
+// launched the ordinary way.  The decode expert kernel is two CTAs on every SM wherever it starts.  Behind the
+// three-launch permutation the expert kernel of the time packed (FP8, 130 tokens, H 4096, I 1024, 256 experts: 1030 us a
+// call, 558 when the permutation let it start only when it was done), so k_permute triggers early only for gathered rows.
 __device__ __forceinline__ void coli_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void coli_grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void coli_grid_dependency_sync() {

@@ -994,7 +994,7 @@ __global__ void __launch_bounds__(1024) k_seg_scan(PermuteParams p, int nchunk, 
 }
 
 __global__ void __launch_bounds__(256) k_permute(PermuteParams p) {
-  if (p.xg) coli_grid_trigger();  // (without gathered rows the register-level expert kernel follows: launch_dependent)
+  if (p.xg) coli_grid_trigger();  // (without gathered rows the decode expert kernel follows: launch_dependent)
   coli_grid_wait();
   // one warp per (t, kk) row; rows T*k .. T*k+T-1 are the shared expert's identity rows; when a
   // token-order f16 copy of x is wanted, T more warps write it
