@@ -7,6 +7,8 @@
 // with a copy command and an event for each chunk the same ring was no faster than the driver (90 + 95 us).
 // Memory that is page-locked already, and less than kDirectBytes, goes as it is.
 #pragma once
+#include <cuda.h>
+
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
@@ -167,16 +169,35 @@ struct HostRing {
   }
 };
 
-// The device's address of page-locked memory that kernels may write directly, null for any other: both ends of it
-// have to be of one mapping.
+// Whether all of `bytes` at `host`, whose attributes are `a`, is of one page-locked allocation or registration.
+inline bool page_locked(const cudaPointerAttributes &a, size_t bytes) {
+  using Fn = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+  static const Fn attribute = [] {
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &found) == cudaSuccess && found == cudaDriverEntryPointSuccess)
+      return reinterpret_cast<Fn>(fn);
+    cudaGetLastError();
+    return Fn(nullptr);
+  }();
+  if (!attribute || a.type != cudaMemoryTypeHost || !a.devicePointer) return false;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(a.devicePointer);
+  if (attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS || attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS)
+    return false;
+  return at >= start && at - start <= size && bytes <= size - (at - start);
+}
+
+// The device's address of page-locked memory that kernels may write directly, null for any other (also for a buffer of
+// which only some pages are registered).
 inline void *mapped_host(void *host, size_t bytes) {
-  cudaPointerAttributes a = {}, z = {};
-  if (cudaPointerGetAttributes(&a, host) != cudaSuccess || cudaPointerGetAttributes(&z, (char *)host + bytes - 1) != cudaSuccess) {
+  cudaPointerAttributes a = {};
+  if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  if (a.type != cudaMemoryTypeHost || z.type != cudaMemoryTypeHost || !a.devicePointer || !z.devicePointer) return nullptr;
-  return (char *)a.devicePointer + bytes - 1 == (char *)z.devicePointer ? a.devicePointer : nullptr;
+  return page_locked(a, bytes) ? a.devicePointer : nullptr;
 }
 
 // Of one host-pointer call: its copies to and from the device on stream `st`.  Sizes are multiples of 16 bytes.
@@ -192,7 +213,7 @@ class HostCopies {
     cudaPointerAttributes a = {};
     if (cudaPointerGetAttributes(&a, host) != cudaSuccess)
       cudaGetLastError();
-    else if (a.type != cudaMemoryTypeUnregistered)
+    else if (a.type != cudaMemoryTypeUnregistered && (a.type != cudaMemoryTypeHost || page_locked(a, bytes)))
       return false;
     if (!helped_) helped_ = pool_.begin();
     return true;

@@ -1,5 +1,7 @@
 """Calls on pageable host memory against the same call on device memory, bit for bit: sizes on both sides of what goes
 as it is, of a chunk of the page-locked ring, of its halves and of the whole of it."""
+import ctypes
+import mmap
 import threading
 
 import numpy as np
@@ -64,3 +66,26 @@ def test_host_calls_of_several_threads(block):
     for t in threads:
         t.join()
     assert not bad
+
+
+def test_results_in_a_buffer_registered_in_parts(block):
+    """Its first and last pages are page-locked, those between are not: it is copied to like any other."""
+    from speedycolibri_b200 import _lib
+
+    blk, shape = block
+    x = synth.host_tokens(shape, 300)
+    want = on_device(blk, x)
+    page = mmap.PAGESIZE
+    size = want.nbytes // page * page + 3 * page
+    mem = mmap.mmap(-1, size)  # starts on a page
+    out = np.frombuffer(mem, dtype=np.uint16, count=want.size)
+    base = out.ctypes.data
+    lib = _lib.load()
+    parts = [base, base + (want.nbytes - 1) // page * page]
+    assert all(lib.coli_cuda_host_register(ctypes.c_void_p(p), ctypes.c_size_t(page)) for p in parts)
+    try:
+        blk.moe_ptr(x.ctypes.data, base, 300)
+        assert np.array_equal(out.reshape(want.shape), want)
+    finally:
+        for p in parts:
+            lib.coli_cuda_host_unregister(ctypes.c_void_p(p))
