@@ -1,6 +1,7 @@
 // Host side of libcoli_b200.so: the extern "C" entry points declared in include/coli_b200.h.
 // Lifecycle, resident-weight handles, the whole-block call and its stages, and the reference's
 // host-pointer expert calls expressed through the same kernels.
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -525,6 +526,22 @@ bool coli_use_tc_path(int fmt, int rows, int nseg, int H, int I) {
 }
 // Rows of a work item on the decode kernel.
 constexpr int kDecodeItemRows = 8;
+// Its items when `rows` rows fall on `nseg` segments independently and evenly: sum over j of P(a segment has more than 8 j rows).
+static int likely_items(int rows, int nseg) {
+  const double mean = (double)rows / nseg;
+  double p = exp(-mean), above = 1.0, items = 0.0;  // P(n rows), P(n rows and more)
+  for (int n = 0; n < 32 * kDecodeItemRows && above > 1e-4; ++n) {
+    above -= p;
+    if (n % kDecodeItemRows == 0) items += above;
+    p *= mean / (n + 1);
+  }
+  return (int)(nseg * items + 0.5);
+}
+static int counted_items(const int *rows, int count, int rpi) {
+  int items = 0;
+  for (int c = 0; c < count; ++c) items += (rows[c] + rpi - 1) / rpi;
+  return items;
+}
 
 extern "C" int coli_b200_moe_create(ColiMoe **out, const ColiMoeLayer *L, int max_tokens) {
   if (!out || !L || max_tokens < 1) {
@@ -890,6 +907,7 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
     fp.max_items = max_items;
     fp.rows_per_item = rpi;
     fp.items_expected = (rows < m->nseg ? rows : m->nseg) + rows / rpi;
+    fp.items_likely = m->has_shared ? likely_items(T * k, m->nseg - 1) + (T + rpi - 1) / rpi : likely_items(rows, m->nseg);
     fp.x = m->x16;
     fp.row_token = m->row_token;
     fp.h = m->h;
@@ -1136,6 +1154,7 @@ int coli_run_segments(ColiMoe *m, SegScratch &sc, const WeightRef *g, const Weig
   fp.max_items = max_items;
   fp.rows_per_item = rpi;
   fp.items_expected = (rows_expected < n_seg ? rows_expected : n_seg) + rows_expected / rpi;
+  fp.items_likely = likely_items(rows_expected, n_seg);
   fp.x = (const __half *)rows_dev;
   fp.row_token = nullptr;
   fp.h = sc.h;
@@ -1376,6 +1395,7 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
     fp.max_items = max_items;
     fp.rows_per_item = rpi;
     fp.items_expected = max_items;
+    fp.items_likely = counted_items(rows, count, rpi);
     fp.x = (const __half *)ctx->buf[1];
     fp.row_token = nullptr;
     fp.h = (__half *)ctx->buf[2];
@@ -1511,6 +1531,7 @@ static int run_host_group_relu2(ColiCudaTensor *const *ups, ColiCudaTensor *cons
   fp.max_items = max_items;
   fp.rows_per_item = rpi;
   fp.items_expected = max_items;
+  fp.items_likely = counted_items(rows, count, rpi);
   fp.x = nullptr;
   fp.row_token = nullptr;
   fp.y = nullptr;
@@ -1625,6 +1646,7 @@ static int run_host_matmul(ColiCudaTensor *w, float *y, const float *x, int S, c
   fp.max_items = max_items;
   fp.rows_per_item = rpi;
   fp.items_expected = max_items;
+  fp.items_likely = max_items;
   fp.x = nullptr;
   fp.row_token = nullptr;
   fp.h = (__half *)ctx->buf[1];

@@ -328,9 +328,12 @@ __global__ void __launch_bounds__(SPLITK ? 256 : 64, SPLITK                  ? 1
 // A warp's task is a pair of weight slabs of 16 R rows over all of K -- gate and up of the same features, or two
 // adjacent slabs of down -- and its packed k-tiles come through a shared-memory ring of its own, filled by cp.async
 // STAGES - 1 k-tiles ahead, across the ends of tasks: no barrier between warps, and the loads never drain.
-// Two CTAs of eight warps fill an SM.  Full rounds of tasks are dealt to the warps as they are; what is left
-// (all of it when a call has few tasks) is spread over the CTAs and split over K among 2, 4 or 8 warps of a CTA,
-// as far as there are warps, so that the last round is short and a single token still loads on every SM.
+// Two CTAs of eight or nine warps fill an SM; of every CTA as many warps work as make the rounds of tasks come out even.
+// Calls with few tasks split the K of each among 2, 4 or 8 warps of a CTA, so that a single token still loads on every SM.
+// An output's products are added in one order, k ascending, or where K is split in as many sums as split_of_k says: by the
+// shapes of the call alone, whatever the routing and wherever in the work list a row lies.  (With only the tasks of the last round split,
+// by how many there turned out to be, the launches were shorter -- 8 tokens 52.8 us a call against 54.9, 24 tokens 76.2 against
+// 81.5 -- and a row's bits changed with its place and with the other tokens' routing.)
 // Tasks of the down projection are known before its input is: launched behind the gate/up launch of this
 // kernel (which lets it start only when the work list is complete), its warps fill their rings first.
 //
@@ -340,20 +343,22 @@ __global__ void __launch_bounds__(SPLITK ? 256 : 64, SPLITK                  ? 1
 // comes back as clock.  Per 2304 bytes of weights it executes 210 warp instructions with 32-row slabs and 249 with
 // 16-row ones, 144 of them conversions, scale multiplies and MMAs; a kernel with the weights in a register ring
 // two k-tiles deep took 257, had half of a warp's time behind its loads, and needed a second wave of CTAs for a
-// single token.  Launches, before and now (us, each between events): 1 token on H 2048, I 768, 128 experts 15.0 + 10.6 ->
-// 12.5 + 10.2; 8 tokens 27.1 + 16.5 -> 23.1 + 18.5 (in a call 21.9 + 12.5 -> 18.7 + 10.0); 48 tokens 54.4 + 32.8 -> 53.3 +
-// 32.6; FP8, 21 tokens 65.1 + 34.9 -> 54.0 + 32.8; 24 tokens on H 7168, I 2048, 256 experts 448 + 239 -> 414 + 207.  Built and no
-// better: six ring stages instead of five, one CTA of 16 warps, ring slots of two k-tiles (more instructions).
-template <int FMT, int R>
+// single token.  Calls, with that kernel and with this one (us): H 2048, I 768, 128 experts 1 token 35.0 -> 24.8, 8 tokens
+// 58.7 -> 54.9, 24 tokens 90.8 -> 81.5, 48 tokens 117 -> 99.5; FP8, 21 tokens 99.6 -> 94.5; 24 tokens on H 7168, I 2048, 256 experts
+// 769 -> 630.  Nine warps for eight: one round instead of two at 8 tokens, 57.4 -> 54.9.  A lone warp needs half a microsecond a
+// k-tile, so a round that few warps work on is long; its two slabs in two warps were no faster (61.3 -> 64.0).
+// Built and no better: six ring stages instead of five, one CTA of 16 warps, ring slots of two k-tiles (more instructions).
+template <int FMT, int R, int SETS>  // SETS: 0, or of a split K how many of its sums a warp makes
 struct StreamTile {
-  static constexpr int WARPS = 8, CTAS = 2;
+  static constexpr int WARPS = FMT == COLI_FMT_NVFP4 && R == 1 && SETS == 0 ? 9 : 8, CTAS = 2;
   static constexpr int QB = FMT == COLI_FMT_NVFP4 ? 64 : 128;  // code bytes of a row and k-tile
   static constexpr int SB = FMT == COLI_FMT_NVFP4 ? 8 : 0;     // scale bytes
   static constexpr int Q = 16 * R * QB;                        // codes of one slab and k-tile
   static constexpr int SLOT = 2 * 16 * R * (QB + SB);          // both slabs' codes, then their scales
   static constexpr int STAGES = FMT == COLI_FMT_NVFP4 && R == 1 ? 5 : 3;
   static constexpr int UNITS = 8 / R;                          // tasks a warp's loads may be ahead, and more
-  static_assert(UNITS > STAGES && 2 * R * 4 * 32 * 4 <= STAGES * SLOT, "task queue; partial sums reuse the ring");
+  static constexpr int SUMS = SETS * 2 * R * 4 * 32;           // floats of a warp's sums of a split task
+  static_assert(UNITS > STAGES, "task queue");
 };
 struct __align__(16) StreamUnit {  // what the multiplying side of a warp needs of a task
   int row0, nrows, r0, pad;
@@ -361,16 +366,16 @@ struct __align__(16) StreamUnit {  // what the multiplying side of a warp needs 
   float g0, g1;
   int tok[8];                      // source row of each token column (columns past nrows repeat the last)
 };
-template <int FMT, int R>
+template <int FMT, int R, int SETS>
 constexpr size_t stream_smem() {
-  using C = StreamTile<FMT, R>;
-  return (size_t)C::WARPS * (C::STAGES * C::SLOT + C::UNITS * sizeof(StreamUnit));
+  using C = StreamTile<FMT, R, SETS>;
+  return (size_t)C::WARPS * (C::STAGES * C::SLOT + C::UNITS * sizeof(StreamUnit) + C::SUMS * sizeof(float));
 }
-template <int FMT, bool GATED, int R>
-__global__ void __launch_bounds__(256, 2) k_ffn_stream(FfnParams p, int items_known) {
-  using C = StreamTile<FMT, R>;
+template <int FMT, bool GATED, int R, int SETS>
+__global__ void __launch_bounds__(R == 1 && SETS == 0 ? 288 : 256, 2) k_ffn_stream(FfnParams p, int items_known, int ks) {
+  using C = StreamTile<FMT, R, SETS>;
   constexpr int QB = C::QB, SB = C::SB, STAGES = C::STAGES, ROWS = GATED ? 16 * R : 32 * R;
-  constexpr bool FP4 = FMT == COLI_FMT_NVFP4;
+  constexpr bool FP4 = FMT == COLI_FMT_NVFP4, SPLIT = SETS > 0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);  // (known to be the same in all lanes)
@@ -385,21 +390,24 @@ __global__ void __launch_bounds__(256, 2) k_ffn_stream(FfnParams p, int items_kn
   if (!items_known) coli_grid_wait();
   if (GATED) coli_grid_trigger();  // behind the wait: the successor may read the work list at once
   const int n_tasks = __ldcg(p.n_items) * tiles;
-  const int warps = (int)gridDim.x * C::WARPS;
-  const int full = n_tasks / warps, rest = n_tasks - full * warps;
-  int ks = 1;  // warps that share a task of the last round
-  while (ks < 8 && 2 * ks <= KT && rest * 2 * ks <= warps) ks *= 2;
-  const int my_rest = (warp / ks) * (int)gridDim.x + (int)blockIdx.x, piece = warp % ks;
-  const int n_units = full + (rest > 0 && my_rest < rest ? 1 : 0);
+  // Tasks of a round: one for `step` warps of a CTA (SPLIT: the ks that share its K; otherwise one), with as many warps of
+  // every CTA at work as make the rounds come out even.
+  const int step = SPLIT ? ks : 1, piece = SPLIT ? warp % step : 0;
+  const int grid = (int)gridDim.x, rounds = (n_tasks + grid * C::WARPS - 1) / (grid * C::WARPS);
+  const int busy = SPLIT || rounds == 0 ? C::WARPS : (n_tasks + grid * rounds - 1) / (grid * rounds);
+  const int round = grid * busy / step;
+  const int full = n_tasks / round, rest = n_tasks - full * round;
+  const int spread = (warp / step) * grid + (int)blockIdx.x;  // the last round: over the CTAs
+  const int n_units = warp < busy ? full + (spread < rest ? 1 : 0) : 0;
 
   // ---- loading side ----
   struct Item {
     int seg, row0, nrows, tile;
   };
-  const int dq = warps / tiles, dr = warps - dq * tiles;  // from one round's task to the next's
+  const int dq = round / tiles, dr = round - dq * tiles;  // from one round's task to the next's
   int fi, ft;
   {
-    const int first = (int)blockIdx.x * C::WARPS + warp;
+    const int first = SPLIT ? spread : (int)blockIdx.x * busy + warp;
     fi = first / tiles;
     ft = first - fi * tiles;
   }
@@ -407,7 +415,7 @@ __global__ void __launch_bounds__(256, 2) k_ffn_stream(FfnParams p, int items_kn
     Item it = {0, 0, 1, 0};
     if (v < n_units) {
       if (v == full) {
-        const int task = full * warps + my_rest;
+        const int task = full * round + spread;
         fi = task / tiles;
         ft = task - fi * tiles;
       }
@@ -445,16 +453,15 @@ __global__ void __launch_bounds__(256, 2) k_ffn_stream(FfnParams p, int items_kn
   fetch_ref(0, it_next);
   auto enter_unit = [&]() {  // unit lv: its matrices have been fetched; the next one's follow
     const int r0 = it_next.tile * ROWS;
-    const int k0 = lv < full ? 0 : piece, step = lv < full ? 1 : ks;
     // (a missing second slab, R = 1 only: the first one again, and nothing of it is stored)
     const int r1 = GATED ? r0 : (r0 + 16 * R < Op ? r0 + 16 * R : r0);
-    const size_t krow = (size_t)k0 * Op;
+    const size_t krow = (size_t)piece * Op;
     q0 = rq0 + (krow + r0) * QB + lane * 16;
     q1 = rq1 + (krow + r1) * QB + lane * 16;
     if (FP4) sp = (lane < 8 * R ? rs0 + (krow + r0) * SB : rs1 + (krow + r1) * SB) + (lane & (8 * R - 1)) * 16;
     qstep = (size_t)step * Op * QB;
     sstep = (size_t)step * Op * SB;
-    left = lv < full ? KT : (KT - k0 + step - 1) / step;
+    left = (KT - piece + step - 1) / step;
     StreamUnit &u = queue[lv % C::UNITS];
     if (lane == 0) {
       u.row0 = it_next.row0;
@@ -519,18 +526,15 @@ __global__ void __launch_bounds__(256, 2) k_ffn_stream(FfnParams p, int items_kn
   uint4 xa[4], xb[4];
   auto enter_x = [&](uint4 (&x)[4], int v) {
     const StreamUnit &e = queue[v % C::UNITS];
-    const int kt = v < full ? 0 : piece;
     column = g < e.nrows;
-    xp = src + (size_t)e.tok[g] * K + kt * 128 + t * 32;
+    xp = src + (size_t)e.tok[g] * K + piece * 128 + t * 32;
 #pragma unroll
     for (int c = 0; c < 4; ++c) x[c] = make_uint4(0, 0, 0, 0);
-    load_x(x, kt);
+    load_x(x, piece);
   };
   if (n_units > 0) enter_x(xa, 0);
-  // With one tile of 16 rows a slab, the steps of a k-tile add into two sets of sums in turn: eight dependent MMAs one
-  // behind the other are longer than what four warps of a scheduler hide.
-  constexpr int SETS = R == 1 ? 2 : 1, NT = 2 * R;  // tile j: rows 16 (j % R) of slab j / R
-  float acc[SETS][NT][4];
+  constexpr int NT = 2 * R;  // tile j: rows 16 (j % R) of slab j / R
+  float acc[SETS > 1 ? 2 : 1][NT][4];
   // where this lane reads its codes: chunk t (FP8: 2t) of row g
   const uint32_t code_off = FP4 ? g * 64 + coli_fp4_chunk(g, t) * 16 : g * 128 + coli_fp8_chunk(g, 2 * t) * 16;
   uint32_t base = ring_u;  // the slot in use
@@ -550,29 +554,29 @@ __global__ void __launch_bounds__(256, 2) k_ffn_stream(FfnParams p, int items_kn
       s1 = o1 < Oout ? u->sc1[o1] : 0.0f;
     }
     const size_t row = (size_t)(row0 + col);
-    if (GATED) {
+    if constexpr (GATED) {
       if (o0 < Oout) p.h[row * p.I + o0] = coli_f32_to_f16_via_bf16(coli_act_fast(v0 * s0, v1 * s1, p.act));
-      return;
-    }
+    } else {
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
-      const int o = m ? o1 : o0;
-      const float v = m ? v1 * s1 : v0 * s0;
-      if (o >= Oout) continue;
-      if (p.relu2_out) {
-        const float f = fmaxf(v, 0.0f);
-        p.relu2_out[row * p.H + o] = coli_f32_to_f16_via_bf16(f * f);
-      } else if (p.y32) {
-        p.y32[row * p.H + o] = v;
-      } else {
-        p.y[row * p.H + o] = __float2bfloat16_rn(v);
+      for (int m = 0; m < 2; ++m) {
+        const int o = m ? o1 : o0;
+        const float v = m ? v1 * s1 : v0 * s0;
+        if (o >= Oout) continue;
+        if (p.relu2_out) {
+          const float f = fmaxf(v, 0.0f);
+          p.relu2_out[row * p.H + o] = coli_f32_to_f16_via_bf16(f * f);
+        } else if (p.y32) {
+          p.y32[row * p.H + o] = v;
+        } else {
+          p.y[row * p.H + o] = __float2bfloat16_rn(v);
+        }
       }
     }
   };
 
-  // one k-tile: its token fragments are in x; `more`: the task goes on at k-tile `next`, whose fragments go to xnext,
-  // otherwise those of the next task's first k-tile do
-  auto k_tile = [&](const uint4 (&x)[4], uint4 (&xnext)[4], int v, int kt, bool more, int next) {
+  // one k-tile, added to `acc`: its token fragments are in x; `more`: the task goes on at k-tile `next`, whose fragments go
+  // to xnext, otherwise those of the next task's first k-tile do
+  auto k_tile = [&](float (&acc)[NT][4], const uint4 (&x)[4], uint4 (&xnext)[4], int v, int kt, bool more, int next) {
     asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
     __syncwarp();  // this k-tile has arrived for every lane, and the slot before it has been read by all
     issue();
@@ -612,14 +616,12 @@ __global__ void __launch_bounds__(256, 2) k_ffn_stream(FfnParams p, int items_kn
         }
         asc[m] = decode_scales<FMT>(f[m]);
       }
-      float part[2][2][4];
+      float part[2][4];
       if (FMT == COLI_FMT_FP8_B128) {
 #pragma unroll
-        for (int q = 0; q < 2; ++q)
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-          for (int m = 0; m < 2; ++m)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) part[q][m][c] = 0.0f;
+          for (int c = 0; c < 4; ++c) part[m][c] = 0.0f;
       }
 #pragma unroll
       for (int s = 0; s < 8; ++s) {
@@ -629,58 +631,68 @@ __global__ void __launch_bounds__(256, 2) k_ffn_stream(FfnParams p, int items_kn
         for (int m = 0; m < 2; ++m) {
           uint32_t a[4];
           decode_a<FMT>(f[m], asc[m], s, a);
-          if (FMT == COLI_FMT_FP8_B128)
-            mma_f16_16816(part[s & 1][m], a, b0, b1);
-          else
-            mma_f16_16816(acc[s % SETS][m * R + r], a, b0, b1);
+          mma_f16_16816(FMT == COLI_FMT_FP8_B128 ? part[m] : acc[m * R + r], a, b0, b1);
         }
       }
       if (FMT == COLI_FMT_FP8_B128) {
 #pragma unroll
         for (int m = 0; m < 2; ++m)
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
-            acc[0][m * R + r][c] = fmaf(kscale[m], part[0][m][c] + part[1][m][c], acc[0][m * R + r][c]);
+          for (int c = 0; c < 4; ++c) acc[m * R + r][c] = fmaf(kscale[m], part[m][c], acc[m * R + r][c]);
       }
     }
     base += C::SLOT;
     if (base == ring_end) base = ring_u;
   };
 
+  float *const sums = reinterpret_cast<float *>(smem_raw + C::WARPS * (STAGES * C::SLOT + C::UNITS * sizeof(StreamUnit)));  // SPLIT
   for (int v = 0; v < n_units; ++v) {
     u = queue + v % C::UNITS;
     row0 = u->row0;
     nrows = u->nrows;
     r0 = u->r0;
-    const int step = v < full ? 1 : ks;
 #pragma unroll
-    for (int q = 0; q < SETS; ++q)
+    for (int i = 0; i < (SETS > 1 ? 2 : 1); ++i)
 #pragma unroll
       for (int j = 0; j < NT; ++j)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[q][j][c] = 0.0f;
+        for (int c = 0; c < 4; ++c) acc[i][j][c] = 0.0f;
     if (!column) {
 #pragma unroll
       for (int c = 0; c < 4; ++c) xb[c] = make_uint4(0, 0, 0, 0);
     }
-    int kt = v < full ? 0 : piece;
+    int kt = piece;
 #pragma unroll 1
     for (; kt + step < KT; kt += 2 * step) {  // two buffers of fragments in turn: no copies between them
-      k_tile(xa, xb, v, kt, true, kt + step);
-      k_tile(xb, xa, v, kt + step, kt + 2 * step < KT, kt + 2 * step);
+      k_tile(acc[0], xa, xb, v, kt, true, kt + step);
+      k_tile(acc[SETS > 1 ? 1 : 0], xb, xa, v, kt + step, kt + 2 * step < KT, kt + 2 * step);
     }
     if (kt < KT) {
-      k_tile(xa, xb, v, kt, false, 0);
+      k_tile(acc[0], xa, xb, v, kt, false, 0);
 #pragma unroll
       for (int c = 0; c < 4; ++c) xa[c] = xb[c];
     }
-    if (SETS == 2) {
+    if constexpr (SPLIT) {  // the task's sums, in the order of the k-tiles they start with
+      auto group_barrier = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / step), "r"(32 * step) : "memory"); };
 #pragma unroll
-      for (int j = 0; j < NT; ++j)
+      for (int i = 0; i < SETS; ++i)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[0][j][c] += acc[SETS - 1][j][c];
-    }
-    if (v < full || ks == 1) {
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) sums[warp * C::SUMS + ((i * NT + j) * 4 + c) * 32 + lane] = acc[i][j][c];
+      group_barrier();
+      for (int e = piece; e < 4 * R; e += step) {  // element e % 4 of row tile e / 4
+        float v0 = 0.0f, v1 = 0.0f;
+        for (int i = 0; i < SETS; ++i)
+          for (int w = 0; w < step; ++w) {
+            const float *part = sums + (warp - piece + w) * C::SUMS + (i * NT * 4 + e) * 32 + lane;
+            v0 += part[0];
+            v1 += part[4 * R * 32];
+          }
+        emit(e & 3, e >> 2, v0, v1);
+      }
+      if (v + 1 < n_units) group_barrier();  // before the next task's sums
+    } else {
 #pragma unroll
       for (int r = 0; r < R; ++r)
 #pragma unroll
@@ -688,69 +700,74 @@ __global__ void __launch_bounds__(256, 2) k_ffn_stream(FfnParams p, int items_kn
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  if (rest == 0 || ks == 1) return;
-  // partial sums of the split round, added in the order of the pieces
-  float *own = reinterpret_cast<float *>(ring);
-  __syncwarp();
-  if (n_units > full) {
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) own[(j * 4 + c) * 32 + lane] = acc[0][j][c];
-  }
-  __syncthreads();
-  if (n_units > full) {
-    const unsigned char *first = ring - (size_t)piece * (STAGES * C::SLOT);
-    for (int e = piece; e < 4 * R; e += ks) {  // element e % 4 of row tile e / 4
-      float v0 = 0.0f, v1 = 0.0f;
-      for (int w = 0; w < ks; ++w) {
-        const float *part = reinterpret_cast<const float *>(first + (size_t)w * (STAGES * C::SLOT));
-        v0 += part[e * 32 + lane];
-        v1 += part[(4 * R + e) * 32 + lane];
-      }
-      emit(e & 3, e >> 2, v0, v1);
-    }
-  }
 }
 
-template <int FMT, int R>
-static int launch_stream(const FfnParams &p, bool gated, bool items_known, cudaStream_t st) {
-  using C = StreamTile<FMT, R>;
-  constexpr size_t smem = stream_smem<FMT, R>();
+// Warps that share a task, each with every ks-th k-tile, where there are too few (item, 16 rows) tasks to fill the SMs
+// with one warp each.  A pure function of the shapes, and the same for every task of a launch: the order in which
+// an output's products are added depends on neither the routing, the item's place in the list nor the other rows.
+static int split_of_k(int items_expected, int O, int K) {
+  const int KT = (K + 127) / 128;
+  if ((long)(items_expected > 0 ? items_expected : 1) * ((O + 15) / 16) >= 12L * COLI_SMS) return 1;
+  return KT >= 8 ? 8 : KT >= 4 ? 4 : KT >= 2 ? 2 : 1;
+}
+template <int FMT, int R, int SETS>
+static int launch_stream(const FfnParams &p, bool gated, bool items_known, int ks, cudaStream_t st) {
+  using C = StreamTile<FMT, R, SETS>;
+  constexpr size_t smem = stream_smem<FMT, R, SETS>();
   static ColiPerDeviceOnce once[2];
-  if (!(gated ? coli_set_smem_limit(once[0], k_ffn_stream<FMT, true, R>, smem, "expert ffn shared-memory attribute")
-              : coli_set_smem_limit(once[1], k_ffn_stream<FMT, false, R>, smem, "expert ffn shared-memory attribute")))
+  if (!(gated ? coli_set_smem_limit(once[0], k_ffn_stream<FMT, true, R, SETS>, smem, "expert ffn shared-memory attribute")
+              : coli_set_smem_limit(once[1], k_ffn_stream<FMT, false, R, SETS>, smem, "expert ffn shared-memory attribute")))
     return 0;
   const dim3 grid(C::CTAS * COLI_SMS);
-  const cudaError_t e = gated ? launch_dependent(k_ffn_stream<FMT, true, R>, grid, dim3(32 * C::WARPS), smem, st, p, 0)
-                              : launch_dependent(k_ffn_stream<FMT, false, R>, grid, dim3(32 * C::WARPS), smem, st, p, items_known ? 1 : 0);
+  const cudaError_t e = gated ? launch_dependent(k_ffn_stream<FMT, true, R, SETS>, grid, dim3(32 * C::WARPS), smem, st, p, 0, ks)
+                              : launch_dependent(k_ffn_stream<FMT, false, R, SETS>, grid, dim3(32 * C::WARPS), smem, st, p, items_known ? 1 : 0, ks);
   coli_count_launch(1);
   return coli_cuda_check(e, "expert ffn launch") ? 1 : 0;
 }
-// Slabs of 32 rows from one and a half rounds of such tasks on (by the host's estimate): the instructions around a k-tile
-// are then spent on twice the weights, and the tasks still divide over the warps.  24 tokens on H 7168, I 2048, 256
-// experts (6.6 rounds) 675 -> 627 us a call; 48 tokens on H 2048, I 768, 128 experts (gate+up 1.9) 100.1 -> 97.5; 8 tokens there
-// (down 1.1 rounds) 52.2 and 52.8, (gate+up 0.8) 52.2 and 53.8: 16 rows.
-// FP8 k-tiles are twice as long: two CTAs of such rings do not fit an SM.
+// Slabs of 16 or of 32 rows (NVFP4; of FP8's k-tiles, twice as long, two CTAs of 32-row rings do not fit an SM): the
+// instructions around a k-tile are then spent on twice the weights (210 a 2304 bytes against 249), but there are half as many
+// tasks, and with fewer than six of eight warps at work an SM waits for its loads.  Weighed as rounds x warps at work x
+// instructions, with the tasks that independent, even routing gives.  Us a call, 16 / 32 rows, H 2048, I 768, 128 experts
+// (gate+up): 4 tokens 41.8 / 46.3, 8 tokens 55.5 / 55.5, 12 tokens 67.4 / 64.3, 16 tokens 73.3 / 70.0, 24 tokens (one round of 32 rows and a
+// little) 79.1 / 82.8, 48 tokens 104.4 / 99.1; H 7168, I 2048, 256 experts, 8 tokens 318 / 301, 24 tokens 713 / 630.
 template <int FMT>
 static int launch_stream_rows(const FfnParams &p, bool gated, bool items_known, cudaStream_t st) {
-  if constexpr (FMT == COLI_FMT_NVFP4) {
-    const int O = gated ? p.I : p.H, rows = gated ? 32 : 64;
-    if (O % rows == 0 && (long)p.items_expected * (O / rows) >= 3L * 8 * COLI_SMS)
-      return launch_stream<FMT, 2>(p, gated, items_known, st);
+  const int O = gated ? p.I : p.H, K = gated ? p.H : p.I, KT = (K + 127) / 128, rows = gated ? 16 : 32, ctas = 2 * COLI_SMS;
+  const long tasks = (long)p.items_likely * ((O + rows - 1) / rows);
+  const int ks = split_of_k(p.items_expected, O, K);
+  if (ks > 1) {
+    // a sum a warp, or (NVFP4: FP8 leaves no room) two, which takes half as many warps: whichever has fewer k-tiles in a row,
+    // the end of a task counted as two (us a call, 8 warps a task with one sum / 4 with two: H 2048, I 768, 2 tokens 35.1 / 33.8, 3 tokens 40.2 / 38.4)
+    auto in_a_row = [&](int step) { return (tasks * step + ctas * 8 - 1) / (ctas * 8) * ((KT + step - 1) / step + 2); };
+    if (FMT == COLI_FMT_NVFP4 && in_a_row(ks / 2) <= in_a_row(ks)) return launch_stream<FMT, 1, FMT == COLI_FMT_NVFP4 ? 2 : 1>(p, gated, items_known, ks / 2, st);
+    return launch_stream<FMT, 1, 1>(p, gated, items_known, ks, st);
   }
-  return launch_stream<FMT, 1>(p, gated, items_known, st);
+  if constexpr (FMT == COLI_FMT_NVFP4) {
+    auto cost = [&](long n, int warps, int least, int instructions) {
+      const long rounds = (n + ctas * warps - 1) / (ctas * warps), busy = rounds ? (n + ctas * rounds - 1) / (ctas * rounds) : 0;
+      return rounds * (busy > least ? busy : least) * instructions;
+    };
+    if (O % (2 * rows) == 0 && cost(tasks / 2, StreamTile<FMT, 2, 0>::WARPS, 6, 2 * 210) < cost(tasks, StreamTile<FMT, 1, 0>::WARPS, 1, 249))
+      return launch_stream<FMT, 2, 0>(p, gated, items_known, 1, st);
+  }
+  return launch_stream<FMT, 1, 0>(p, gated, items_known, 1, st);
 }
 // ---- one token: down and combine ---------------------------------------------------------------------
 // A CTA makes 16 features of the result: a warp for each of the token's rows (its k experts and the shared one), all
 // of K through a ring of its own, then the weighted sum of k_combine -- the same terms, rounded the same way -- out of
 // shared memory.  The result rows never leave the SM, and a launch and its wait are gone from a chain of four.
 // The rings are filled before the input is there, as those of the kernel above.
-// One token on H 2048, I 768, 128 experts: 26.2 -> 25.2 us a call.  From more features than SMs x 16 on the two kernels are
+// One token on H 2048, I 768, 128 experts: 25.9 -> 24.7 us a call.  From more features than SMs x 16 on the two kernels are
 // better (H 7168, I 2048, 256 experts: 80.7 and 84.4): there the whole of K by one warp is a long chain.
 constexpr int kOneRows = 17, kOneStages = 6;
 template <int FMT>
-__global__ void __launch_bounds__(32 * kOneRows) k_down_combine_one(FfnParams p, CombineParams c, const int32_t *topk_idx, int shared, int items_known) {
+constexpr size_t one_smem(int rows) {  // a warp's ring, its row of the result, its sums
+  return (size_t)rows * (kOneStages * 16 * (FMT == COLI_FMT_NVFP4 ? 72 : 128) + (16 + 8 * 16) * sizeof(float));
+}
+// CHAIN: all of K is one sum.  Otherwise k-tile kt adds into sum kt % ks and the sums are added in order, as the ks warps of a
+// split task do it; two k-tiles, of different sums, are multiplied side by side.
+template <int FMT, bool CHAIN>
+__global__ void __launch_bounds__(32 * kOneRows) k_down_combine_one(FfnParams p, CombineParams c, const int32_t *topk_idx, int shared, int items_known, int ks) {
   constexpr bool FP4 = FMT == COLI_FMT_NVFP4;
   constexpr int QB = FP4 ? 64 : 128, SB = FP4 ? 8 : 0, Q = 16 * QB, SLOT = 16 * (QB + SB);
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -758,6 +775,7 @@ __global__ void __launch_bounds__(32 * kOneRows) k_down_combine_one(FfnParams p,
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), rows = (int)blockDim.x >> 5;
   const int K = p.I, KT = (K + 127) >> 7, Op = (p.H + 15) & ~15, r0 = (int)blockIdx.x * 16;
   float *ys = reinterpret_cast<float *>(smem_raw + (size_t)rows * kOneStages * SLOT);  // [rows][16]
+  float *sums = ys + rows * 16 + warp * (8 * 16);                                      // [8][16]
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem_raw) + warp * (kOneStages * SLOT);
   if (!items_known) coli_grid_wait();
   const int ex = warp < c.k ? __ldcg(topk_idx + warp) : shared;
@@ -776,69 +794,115 @@ __global__ void __launch_bounds__(32 * kOneRows) k_down_combine_one(FfnParams p,
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 #pragma unroll 1
-  for (int i = 0; i < kOneStages - 1; ++i) issue();
+  for (int i = 0; i < kOneStages; ++i) issue();
   if (items_known) coli_grid_wait();
   coli_grid_trigger();
   const __half *h = p.h + (size_t)row * K + t * 32;  // column 0, the token, is read by the lanes of g = 0
-  auto load_x = [&](uint4 (&x)[4], int kt) {
+  auto load_x = [&](uint4 (&x)[2][4], int kt) {      // of k-tiles kt and kt + 1
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      x[i] = make_uint4(0, 0, 0, 0);
-      if (g == 0 && kt * 128 + t * 32 + 8 * i + 8 <= K) x[i] = *reinterpret_cast<const uint4 *>(h + kt * 128 + 8 * i);
-    }
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = (kt + j) * 128 + 8 * i;
+        x[j][i] = make_uint4(0, 0, 0, 0);
+        if (g == 0 && k + t * 32 + 8 <= K) x[j][i] = *reinterpret_cast<const uint4 *>(h + k);
+      }
   };
-  uint4 xn[4];
+  uint4 xn[2][4];
   load_x(xn, 0);
-  float acc[2][4] = {};  // the steps of a k-tile add into two sets in turn
+  float acc[2][4] = {};
   const uint32_t code_off = FP4 ? g * 64 + coli_fp4_chunk(g, t) * 16 : g * 128 + coli_fp8_chunk(g, 2 * t) * 16;
-  for (int kt = 0; kt < KT; ++kt) {
+#pragma unroll 1
+  for (int kt = 0; kt < KT; kt += 2) {  // (behind an odd last k-tile the other half of the pair is not used)
     asm volatile("cp.async.wait_group %0;" ::"n"(kOneStages - 2) : "memory");
-    __syncwarp();  // this k-tile has arrived for every lane, and the slot before it has been read by all
-    issue();
-    uint4 x[4];
+    __syncwarp();  // these k-tiles have arrived for every lane
+    uint4 x[2][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = xn[i];
-    if (kt + 1 < KT) load_x(xn, kt + 1);
-    const uint32_t base = ring + (kt % kOneStages) * SLOT;
-    AFrag<FMT> f;
-    if constexpr (FP4) {
-      f.lo[0] = lds128(base + code_off);
-      f.hi[0] = lds128(base + 512 + code_off);
-      uint16_t a, b;
-      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(a) : "r"(base + Q + lane * 2) : "memory");
-      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(b) : "r"(base + Q + 64 + lane * 2) : "memory");
-      f.sc = (uint32_t)a | ((uint32_t)b << 16);
-    } else {
-      f.lo[0] = lds128(base + code_off);
-      f.lo[1] = lds128(base + (code_off ^ 16));
-      f.hi[0] = lds128(base + 1024 + code_off);
-      f.hi[1] = lds128(base + 1024 + (code_off ^ 16));
-      f.sc = 0;
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[j][i] = xn[j][i];
+    if (kt + 2 < KT) load_x(xn, kt + 2);
+    AFrag<FMT> f[2];
+    AScale asc[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const uint32_t base = ring + ((kt + j) % kOneStages) * SLOT;
+      if constexpr (FP4) {
+        f[j].lo[0] = lds128(base + code_off);
+        f[j].hi[0] = lds128(base + 512 + code_off);
+        uint16_t a, b;
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(a) : "r"(base + Q + lane * 2) : "memory");
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(b) : "r"(base + Q + 64 + lane * 2) : "memory");
+        f[j].sc = (uint32_t)a | ((uint32_t)b << 16);
+      } else {
+        f[j].lo[0] = lds128(base + code_off);
+        f[j].lo[1] = lds128(base + (code_off ^ 16));
+        f[j].hi[0] = lds128(base + 1024 + code_off);
+        f[j].hi[1] = lds128(base + 1024 + (code_off ^ 16));
+        f[j].sc = 0;
+      }
+      asc[j] = decode_scales<FMT>(f[j]);
     }
-    const AScale asc = decode_scales<FMT>(f);
-    float part[2][4] = {};
+    float *sum[2];  // (of lanes with t = 0: column 0, elements 0 and 2, is the token)
 #pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      const uint4 &xv = x[s >> 1];
+    for (int j = 0; j < 2; ++j) {
+      sum[j] = sums + ((kt + j) & (ks - 1)) * 16 + g;
+      if (!CHAIN || FMT == COLI_FMT_FP8_B128) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[j][i] = 0.0f;
+      }
+      if (!CHAIN && FMT != COLI_FMT_FP8_B128 && kt + j >= ks && t == 0) {
+        acc[j][0] = sum[j][0];
+        acc[j][2] = sum[j][8];
+      }
+    }
+    auto mma = [&](int j, int to, int s) {
+      const uint4 &xv = x[j][s >> 1];
       uint32_t a[4];
-      decode_a<FMT>(f, asc, s, a);
-      if (FMT == COLI_FMT_FP8_B128)
-        mma_f16_16816(part[s & 1], a, (s & 1) ? xv.z : xv.x, (s & 1) ? xv.w : xv.y);
-      else
-        mma_f16_16816(acc[s & 1], a, (s & 1) ? xv.z : xv.x, (s & 1) ? xv.w : xv.y);
-    }
-    if (FMT == COLI_FMT_FP8_B128) {  // one f32 scale per (128-row block, k-tile): convert.rs:731-741
-      const float sc = __ldg(reinterpret_cast<const float *>(w.s) + (size_t)(r0 >> 7) * KT + kt);
+      decode_a<FMT>(f[j], asc[j], s, a);
+      mma_f16_16816(acc[to], a, (s & 1) ? xv.z : xv.x, (s & 1) ? xv.w : xv.y);
+    };
+    if constexpr (CHAIN && FMT != COLI_FMT_FP8_B128) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[0][i] = fmaf(sc, part[0][i] + part[1][i], acc[0][i]);
+      for (int s = 0; s < 8; ++s) mma(0, 0, s);
+      if (kt + 1 < KT) {
+#pragma unroll
+        for (int s = 0; s < 8; ++s) mma(1, 0, s);
+      }
+    } else {
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        mma(0, 0, s);
+        mma(1, 1, s);
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (t != 0 || kt + j >= KT) continue;
+        if (FMT == COLI_FMT_FP8_B128) {  // one f32 scale per (128-row block, k-tile): convert.rs:731-741
+          const float sc = __ldg(reinterpret_cast<const float *>(w.s) + (size_t)(r0 >> 7) * KT + kt + j);
+          const bool first = kt + j < ks;
+          sum[j][0] = fmaf(sc, acc[j][0], first ? 0.0f : sum[j][0]);
+          sum[j][8] = fmaf(sc, acc[j][2], first ? 0.0f : sum[j][8]);
+        } else {
+          sum[j][0] = acc[j][0];
+          sum[j][8] = acc[j][2];
+        }
+      }
     }
+    __syncwarp();  // these slots have been read by all
+    issue();
+    issue();
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  if (t == 0) {  // column 0: elements 0 (row g) and 2 (row g + 8)
+  if (t == 0) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int o = r0 + g + 8 * i;
-      float v = acc[0][2 * i] + acc[1][2 * i];
+      float v = 0.0f;
+      if (CHAIN && FMT != COLI_FMT_FP8_B128)
+        v = acc[0][2 * i];
+      else
+        for (int j = 0; j < ks; ++j) v += sums[j * 16 + g + 8 * i];
       if (FP4) v *= w.g;
       if (FMT == COLI_FMT_E4M3_ROW) v *= o < p.H ? reinterpret_cast<const float *>(w.s)[o] : 0.0f;
       ys[warp * 16 + g + 8 * i] = __bfloat162float(__float2bfloat16_rn(v));
@@ -857,19 +921,23 @@ __global__ void __launch_bounds__(32 * kOneRows) k_down_combine_one(FfnParams p,
     c.out[o] = __float2bfloat16_rn(sum);
 }
 bool down_combine_one_ok(int rows, int H) { return rows <= kOneRows && (H + 15) / 16 <= COLI_SMS; }
-template <int FMT>
-static int launch_one_token(const FfnParams &p, const CombineParams &c, const int32_t *topk_idx, int shared, bool items_known, cudaStream_t st) {
-  constexpr int SLOT = FMT == COLI_FMT_NVFP4 ? 16 * 72 : 16 * 128;
+template <int FMT, bool CHAIN>
+static int launch_one_token_as(const FfnParams &p, const CombineParams &c, const int32_t *topk_idx, int shared, bool items_known, int ks, cudaStream_t st) {
   const int rows = c.k + c.has_shared;
-  const size_t smem = (size_t)rows * (kOneStages * SLOT + 16 * sizeof(float));
   static ColiPerDeviceOnce once;
-  if (!coli_set_smem_limit(once, k_down_combine_one<FMT>, (size_t)kOneRows * (kOneStages * SLOT + 16 * sizeof(float)), "down of one token: shared-memory attribute"))
-    return 0;
+  if (!coli_set_smem_limit(once, k_down_combine_one<FMT, CHAIN>, one_smem<FMT>(kOneRows), "down of one token: shared-memory attribute")) return 0;
   coli_count_launch(1);
-  return coli_cuda_check(launch_dependent(k_down_combine_one<FMT>, dim3((p.H + 15) / 16), dim3(32 * rows), smem, st, p, c, topk_idx, shared, items_known ? 1 : 0),
+  return coli_cuda_check(launch_dependent(k_down_combine_one<FMT, CHAIN>, dim3((p.H + 15) / 16), dim3(32 * rows), one_smem<FMT>(rows), st, p, c, topk_idx, shared,
+                                          items_known ? 1 : 0, ks),
                          "down of one token")
              ? 1
              : 0;
+}
+template <int FMT>
+static int launch_one_token(const FfnParams &p, const CombineParams &c, const int32_t *topk_idx, int shared, bool items_known, cudaStream_t st) {
+  const int ks = split_of_k(p.items_expected, p.H, p.I);
+  return ks > 1 ? launch_one_token_as<FMT, false>(p, c, topk_idx, shared, items_known, ks, st)
+                : launch_one_token_as<FMT, true>(p, c, topk_idx, shared, items_known, 1, st);
 }
 int launch_down_combine_one(const FfnParams &p, const CombineParams &c, const int32_t *topk_idx, int shared, bool items_known, cudaStream_t st) {
   switch (p.fmt) {
@@ -884,18 +952,11 @@ int launch_down_combine_one(const FfnParams &p, const CombineParams &c, const in
   return 0;
 }
 
-static int pick_w(int KT) { return KT >= 8 ? 8 : KT >= 4 ? 4 : KT >= 2 ? 2 : 1; }
-
-// Split K across the warps of a CTA only when there are too few (item, row tile) tasks to fill
-// the SMs with one warp each; `p.items_expected` is a host-side estimate from shapes alone.
 template <int FMT, int NB>
 static int launch_one(const FfnParams &p, cudaStream_t st) {
-  const int K = p.I, O = p.H;
-  const int KT = (K + 127) / 128, row_tiles = (O + 15) / 16;
-  const long tasks = (long)row_tiles * (p.items_expected > 0 ? p.items_expected : 1);
-  const bool splitk = tasks < 12L * COLI_SMS;
-  if (splitk) {
-    const int W = pick_w(KT);
+  const int row_tiles = (p.H + 15) / 16;
+  const int W = split_of_k(p.items_expected, p.H, p.I);
+  if (W > 1) {
     dim3 grid(row_tiles, p.max_items);
     const size_t sm = (size_t)W * NB * 4 * 32 * sizeof(float);
     const cudaError_t e = launch_dependent(k_ffn_mm<FMT, NB, true>, grid, dim3(W * 32), sm, st, p);

@@ -210,7 +210,8 @@ struct FfnParams {
   const int32_t *item_seg, *item_row0, *item_nrows, *n_items;
   int max_items;
   int rows_per_item;         // rows per work item the list was cut with (<= 8; the down form alone <= 32)
-  int items_expected;        // host estimate of the work items (selects split-K vs tile-per-warp)
+  int items_expected;        // host bound of the work items: says whether warps share a K, and with it the order of the sums
+  int items_likely;          // host estimate of them, for what changes no result
   const __half *x;           // source rows (f16)
   const int32_t *row_token;  // row -> source row index (null = identity)
   __half *h;                 // [rows, I] scratch
