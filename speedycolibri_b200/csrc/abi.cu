@@ -37,7 +37,7 @@ namespace {
 std::mutex g_init_mu;
 DeviceContext *g_ctx[COLI_CUDA_MAX_DEVICES];
 int g_ndev = 0;
-colib_host::CopyPool g_copy_pool;
+colib_host::LibraryPool g_copy;
 int g_act_oai = 0;  // process-wide gate/up combine, backend_cuda.cu:339-350
 float g_act_alpha = 1.702f;
 float g_act_limit = 0.0f;
@@ -131,7 +131,7 @@ extern "C" void coli_cuda_shutdown(void) {
     g_ctx[i] = nullptr;
   }
   g_ndev = 0;
-  g_copy_pool.stop();
+  g_copy.pool->stop();
 }
 extern "C" int coli_cuda_device_count(void) { return g_ndev; }
 extern "C" int coli_cuda_device_at(int index) { return (index >= 0 && index < g_ndev) ? g_ctx[index]->device : -1; }
@@ -1012,7 +1012,7 @@ extern "C" int coli_b200_moe_block(ColiMoe *m, const void *x, void *out, int T, 
   const size_t bytes = (size_t)T * m->L.H * sizeof(__nv_bfloat16);
   int32_t own = 0;
   StreamWait wait(st);  // whatever fails below: nothing of the caller's is in use when the call returns
-  colib_host::HostCopies copies(m->ctx->ring, g_copy_pool, st);
+  colib_host::HostCopies copies(m->ctx->ring, *g_copy.pool, st);
   if (!copies.staged(x, bytes))
     CK(cudaMemcpyAsync(m->x_stage, x, bytes, cudaMemcpyHostToDevice, st), "moe_block input upload");
   else if (!copies.upload(m->x_stage, x, bytes, false, "moe_block input upload"))
@@ -1346,7 +1346,7 @@ static int run_host_group(ColiCudaTensor *const *gates, ColiCudaTensor *const *u
   // Whatever fails below, the call waits for its stream before it returns: copies may be reading x and
   // head, or writing y and own.  (A wait between the copies and the kernels as well took 10 us a call.)
   StreamWait wait(st);
-  colib_host::HostCopies copies(ctx->ring, g_copy_pool, st);
+  colib_host::HostCopies copies(ctx->ring, *g_copy.pool, st);
   CK(cudaEventRecord(ctx->ev[0], st), "phase event");
   CK(cudaMemcpyAsync(d_tbl, head.data(), head_bytes, cudaMemcpyHostToDevice, st), "expert table upload");
   const bool x_staged = copies.staged(x, xb * sizeof(float)), y_staged = copies.staged(y, xb * sizeof(float));

@@ -8,6 +8,7 @@
 // Memory that is page-locked already, and less than kDirectBytes, goes as it is.
 #pragma once
 #include <cuda.h>
+#include <unistd.h>
 
 #include <atomic>
 #include <condition_variable>
@@ -49,13 +50,14 @@ struct CopyBatch {
 
 // The helping threads of the process: started by the first call that can use them, asleep between calls, joined
 // by the library's shutdown or the end of the process.  One call has them at a time; another works alone.
+// A forked child has this object, in whatever state, and none of the threads: there it is not touched.
 class CopyPool {
  public:
-  ~CopyPool() { stop(); }
   bool begin() {
-    if (!owner_.try_lock()) return false;
+    if (forked() || !owner_.try_lock()) return false;
     std::lock_guard<std::mutex> lk(mu_);
     if (threads_.empty()) {
+      pid_.store(getpid());
       const unsigned cores = std::thread::hardware_concurrency();
       const int want = cores >= 8 ? 3 : cores >= 4 ? 1 : 0;
       stop_ = false;
@@ -78,7 +80,8 @@ class CopyPool {
     batch_.store(nullptr);
     while (users_.load() != 0) std::this_thread::yield();
   }
-  void stop() {
+  bool stop() {  // false: nothing done, in a forked child
+    if (forked()) return false;
     std::lock_guard<std::mutex> own(owner_);
     {
       std::lock_guard<std::mutex> lk(mu_);
@@ -87,6 +90,7 @@ class CopyPool {
     }
     for (auto &t : threads_) t.join();
     threads_.clear();
+    return true;
   }
   static void pause() {
 #if defined(__x86_64__)
@@ -95,6 +99,10 @@ class CopyPool {
   }
 
  private:
+  bool forked() const {
+    const pid_t p = pid_.load();
+    return p != 0 && p != getpid();
+  }
   void work() {
     uint64_t seen = 0;
     for (;;) {
@@ -117,6 +125,7 @@ class CopyPool {
       }
     }
   }
+  std::atomic<pid_t> pid_{0};  // whose threads they are
   std::mutex owner_, mu_;
   std::condition_variable cv_;
   std::vector<std::thread> threads_;
@@ -125,6 +134,14 @@ class CopyPool {
   std::atomic<bool> active_{false};
   std::atomic<CopyBatch *> batch_{nullptr};
   std::atomic<int> users_{0};
+};
+// The library's pool.  (Members of a pool whose threads are gone are not destroyed either: the condition variable would
+// wait for its sleepers.)
+struct LibraryPool {
+  CopyPool *const pool = new CopyPool;
+  ~LibraryPool() {
+    if (pool->stop()) delete pool;
+  }
 };
 
 // The ring of one device; used by one call at a time (the device's mutex is held).

@@ -23,6 +23,8 @@ int fake_waited(void) { return last == 'w'; }
 static int queue(void) { if (++log_n == fail_at) return 1; last = 'q'; return 0; }
 int cudaMalloc(void **p, size_t n) { *p = malloc(n ? n : 1); return 0; }
 int cudaFree(void *p) { free(p); return 0; }
+int cudaHostAlloc(void **p, size_t n) { return cudaMalloc(p, n); }
+int cudaFreeHost(void *p) { return cudaFree(p); }
 int cudaGetDeviceCount(int *n) { *n = 1; return 0; }
 int cudaDeviceGetAttribute(int *v) { *v = 148; return 0; }
 int cudaGetDeviceProperties_v2(struct cudaDeviceProp *p) {
