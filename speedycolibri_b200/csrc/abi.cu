@@ -505,23 +505,19 @@ int coli_tct_tile_tokens(int rows, int nseg) {
 }
 // The tcgen05 path takes over from 8 rows per segment on average: below that the decode kernel, which reads a segment's
 // weights once per item of 8 rows and converts as many of them as it reads, wins on every layer that was measured (decode /
-// tcgen05, us a call): H 7168, I 2048, 256 experts (4112 weight tiles of 128 features) at 6.0 rows 1203 / 1438, 7.9 1459 / 1441; H 3072,
-// I 1280, 128 experts (1290) 7.9 214 / 234; H 1024, I 2048, 120 experts 7.9 124 / 141.  NVFP4 layers of up to 888 tiles take it up to
-// 10 rows, where most segments are two items whose weights meet in L2: H 2048, I 768, 128 experts (774) 8.2 113 / 129, 9.0 117 / 122,
-// 10.0 120 / 122, 11.0 132 / 128; H 1024, I 512, 64 experts (260) 10.0 46 / 52; 1290 tiles 9.0 227 / 226; per-row FP8 on 774 tiles 8.2
-// 143 / 147, 9.0 142 / 140.
+// tcgen05, us a call): H 7168, I 2048, 256 experts (4112 weight tiles of 128 features) at 6.1 rows 1393 / 1561, 7.0 1469 / 1574, 7.9
+// 1585 / 1580; H 3072, I 1280, 128 experts (1290) 7.1 229 / 242, 7.95 245 / 242; H 1024, I 2048, 128 experts (2064) 7.95 143 / 149;
+// H 128, I 1920, 120 experts (1800) 6.0 39 / 55; per-row FP8 on 774 tiles 7.95 145 / 148.  On small NVFP4 layers it wins a
+// little longer, most segments being two items whose weights meet in L2: up to 9 rows at 774 tiles (H 2048, I 768, 128
+// experts 8.2 118 / 130, 9.0 123 / 122, 9.5 130 / 122), past 10 at 132 and 260 (H 1024, I 512, 32 experts 8.0 33 / 42, 9.85 35 / 42).
 // FP8 128x128 stays at 8 rows although the tcgen05 kernel wins from 5 (H 4096, I 1024, 256 experts 5.0 550 / 532): it applies the
 // scales as f16 multipliers, the decode kernel in f32 (error against 64 bits 2.896e-3 and 2.864e-3 at 7.5 rows, H 2048, I 1024).
-// Layers of a single k-tile with many weight tiles keep their line at 6 rows and with it the number of launches that callers
-// know (the decode kernel would take 39 us against 55 at 6 rows, H 128, I 1920, 120 experts).
 // A pure function of shapes, so that kernel selection never depends on data or addresses.
 static bool tc_format(int fmt) { return fmt == COLI_FMT_NVFP4 || fmt == COLI_FMT_FP8_B128 || fmt == COLI_FMT_E4M3_ROW; }
-bool coli_use_tc_path(int fmt, int rows, int nseg, int H, int I) {
+bool coli_use_tc_path(int fmt, int rows, int nseg, int I) {
   if (!tc_format(fmt) || nseg <= 0) return false;
   const long tiles = (long)nseg * ((I + 127) / 128);
-  long line = 8;
-  if (fmt == COLI_FMT_NVFP4 && tiles <= 6L * COLI_SMS) line = 10;
-  if (fmt != COLI_FMT_FP8_B128 && tiles >= 12L * COLI_SMS && H <= 128) line = 6;
+  const long line = fmt != COLI_FMT_NVFP4 || tiles > 6L * COLI_SMS ? 8 : tiles > 3L * COLI_SMS ? 9 : 10;
   return (long)rows >= line * nseg;
 }
 // Rows of a work item on the decode kernel.
@@ -684,7 +680,7 @@ extern "C" int coli_b200_moe_create(ColiMoe **out, const ColiMoeLayer *L, int ma
   ok = ok && ws_alloc(m, &m->status, 1) && coli_cuda_check(cudaMemset(m->status, 0, sizeof(int)), "status clear");
   m->ticket = nullptr;
   ok = ok && ws_alloc(m, &m->ticket, 1) && coli_cuda_check(cudaMemset(m->ticket, 0, sizeof(unsigned int)), "ticket clear");
-  if (ok && coli_use_tc_path(coli_kernel_fmt(L->fmt), (int)rows, m->nseg, L->H, L->I)) ok = ws_alloc(m, &m->xg, rows * H);
+  if (ok && coli_use_tc_path(coli_kernel_fmt(L->fmt), (int)rows, m->nseg, L->I)) ok = ws_alloc(m, &m->xg, rows * H);
   m->select_bias = nullptr;
   m->logit_bias = nullptr;
   if (ok && L->select_bias) ok = ws_alloc(m, &m->select_bias, E);
@@ -823,7 +819,7 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
   cudaStream_t st = pick_stream(m, stream);
   const int k = m->L.k;
   const int rows = T * k + (m->has_shared ? T : 0);
-  const bool tc = coli_use_tc_path(m->L.fmt, rows, m->nseg, m->L.H, m->L.I) && m->xg != nullptr;
+  const bool tc = coli_use_tc_path(m->L.fmt, rows, m->nseg, m->L.I) && m->xg != nullptr;
   const int rpi = tc ? coli_tct_tile_tokens(rows, m->nseg) : kDecodeItemRows;
   const int max_items = max_work_items(rows, m->nseg, rpi);
   // Segments are in (owner, expert id) order, also when every expert is resident: only where that is the
@@ -1111,7 +1107,7 @@ int coli_run_segments(ColiMoe *m, SegScratch &sc, const WeightRef *g, const Weig
                       const int32_t *seg_expert_dev, const void *rows_dev, const int32_t *seg_count_dev, int n_seg,
                       int rows_cap, int rows_expected, void *y_dev, cudaStream_t st) {
   if (rows_cap == 0 || n_seg == 0) return 1;
-  const bool tc = coli_use_tc_path(m->L.fmt, rows_expected, n_seg, m->L.H, m->L.I);
+  const bool tc = coli_use_tc_path(m->L.fmt, rows_expected, n_seg, m->L.I);
   const int rpi = tc ? coli_tct_tile_tokens(rows_expected, n_seg) : kDecodeItemRows;
   const int max_items = max_work_items(rows_cap, n_seg, rpi);
   if (!ensure_h(m, sc, (size_t)rows_cap) || !ensure_items(m, sc, max_items, n_seg)) return 0;

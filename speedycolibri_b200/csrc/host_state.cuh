@@ -89,9 +89,9 @@ static inline bool ws_alloc(ColiMoe *m, T **p, size_t count) {
 }
 
 
-// kernel-family selection: pure functions of format and shapes (rows, segments, sizes)
+// kernel-family selection: pure functions of format and shapes (rows, segments, intermediate size)
 int coli_tct_tile_tokens(int rows, int nseg);
-bool coli_use_tc_path(int fmt, int rows, int nseg, int H, int I);
+bool coli_use_tc_path(int fmt, int rows, int nseg, int I);
 
 bool coli_check_T(ColiMoe *m, int T, const char *who);
 colib::RouteParams coli_route_params(ColiMoe *m, const void *x_dev, int T);

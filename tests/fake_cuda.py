@@ -16,10 +16,14 @@ SHIM = r"""
 #include <stdlib.h>
 #include <string.h>
 static int log_n, fail_at;
-static char last;
-void fake_reset(int fail) { log_n = 0; fail_at = fail; last = 0; }
+static char last, launched[1 << 16];
+void fake_reset(int fail) { log_n = 0; fail_at = fail; last = 0; launched[0] = 0; }
 int fake_queued(void) { return log_n; }
 int fake_waited(void) { return last == 'w'; }
+const char *fake_launches(void) { return launched; }  /* the launchers called since the reset, by their linker names */
+static void note(const char *name) {
+  if (strlen(launched) + strlen(name) + 2 < sizeof launched) strcat(strcat(launched, name), " ");
+}
 static int queue(void) { if (++log_n == fail_at) return 1; last = 'q'; return 0; }
 int cudaMalloc(void **p, size_t n) { *p = malloc(n ? n : 1); return 0; }
 int cudaFree(void *p) { free(p); return 0; }
@@ -52,7 +56,7 @@ def load(d):
     src = SHIM
     for s in undefined:
         if s.startswith("_ZN5colib"):
-            src += f"int {s}(void) {{ return !queue(); }}\n"  # a launcher answers 1 on success
+            src += f'int {s}(void) {{ note("{s}"); return !queue(); }}\n'  # a launcher answers 1 on success
         elif (s.startswith(("cuda", "__cuda")) or "coli_ep_" in s) and f" {s}(" not in src and f"*{s}(" not in src:
             src += f"int {s}(void) {{ return 0; }}\n"
     cuda_include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(shutil.which("nvcc")))), "include")
@@ -60,6 +64,7 @@ def load(d):
     subprocess.run(["gcc", "-w", "-fPIC", "-I", cuda_include, "-c", "-o", shim + ".o", shim], check=True)
     subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-Wl,-z,defs", "-o", lib, obj, shim + ".o", "-lpthread"], check=True)
     fake = C.CDLL(lib, mode=os.RTLD_LOCAL)
+    fake.fake_launches.restype = C.c_char_p
     assert fake.coli_cuda_init((C.c_int * 1)(0), 1)
     return fake
 
