@@ -1,6 +1,6 @@
 """Router, top-k and permutation at the edges of their paths: the decode front (up to 8 tokens), the staged router
-(8 x 8 tiles up to the number of SMs), rows placed by the counts of the top-k (with a copy of x up to and with
-gathered rows above 1024 pairs), and the selection by counting with more candidates than a warp has lanes."""
+(8 x 8 tiles up to the number of SMs), rows placed by the counts of the top-k (with a copy of x and with gathered
+rows, around 1024 pairs), and the selection by counting with more candidates than a warp has lanes."""
 import numpy as np
 import pytest
 
@@ -42,4 +42,22 @@ def test_routing_and_block_at_the_edges(gpu_backend, orc, T, E, k, H, score, gro
     assert np.array_equal(w.view(np.uint32), want["w"].view(np.uint32))
     # h and y are rounded to bf16, 2^-9 relative each
     assert rel_l2(out, want["out"]) <= 5e-3
+    blk.close()
+
+
+@pytest.mark.parametrize("T", [12, 60, 170, 171])
+def test_gathered_rows_are_placed_in_one_launch(gpu_backend, T):
+    """72 to 1026 pairs, 44 KB to 632 KB of rows: router, top-k, placement, gate+up, down, combine."""
+    import torch
+
+    from speedycolibri_b200 import _lib
+    from speedycolibri_b200.moe import Config, MoeBlock
+
+    shape = MoeShape("front_launches", H=264, E=4 if T == 12 else 20 if T > 60 else 6, k=4 if T == 12 else 6, I=16, T=T)
+    blk = MoeBlock(Config.from_shape(shape), synth.device_layer(shape), T)
+    x = torch.randn((T, shape.H), device="cuda").to(torch.bfloat16)
+    before = _lib.load().coli_b200_launch_count()
+    blk.forward(x)
+    assert _lib.load().coli_b200_launch_count() - before == 6
+    torch.cuda.synchronize()
     blk.close()
