@@ -794,7 +794,6 @@ colib::PermuteParams coli_permute_params(ColiMoe *m, const void *x_dev, int T, b
   pp.n_items = m->n_items;
   pp.x = (const __nv_bfloat16 *)x_dev;
   pp.xg = (__half *)rows_dev;
-  pp.gather_shared = 0;
   pp.x16 = nullptr;
   pp.virt = nullptr;
   pp.rows_cap = 0x7fffffff;
@@ -834,7 +833,6 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
   {
     colib::PermuteParams pp = coli_permute_params(m, x_dev, T, m->has_shared, rpi, tc ? m->xg : nullptr, nullptr, m->slot);
     if (m->segs_in_expert_order) pp.expert_slot = nullptr;
-    pp.gather_shared = tc ? 1 : 0;
     pp.x16 = tc ? nullptr : m->x16;
     // decode-sized batches: one launch for router, top-k and permutation (its time is booked
     // under the router phase)

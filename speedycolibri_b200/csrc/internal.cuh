@@ -160,10 +160,9 @@ struct PermuteParams {
   int32_t *item_row0;          //                first row
   int32_t *item_nrows;         //                rows (<= rows_per_item)
   int32_t *n_items;            // [1]
-  const __nv_bfloat16 *x;      // [T,H]  (null = do not materialise rows)
-  __half *xg;                  // [T*k (+T),H] gathered rows as f16 (null = skip)
-  int gather_shared;           // also copy the shared expert's T identity rows into xg
-  __half *x16;                 // [T,H] f16 copy of x in token order (null = skip)
+  const __nv_bfloat16 *x;      // [T,H]
+  __half *xg;                  // [T*k (+T),H] gathered rows as f16, or (not for launch_permute) null and
+  __half *x16;                 // [T,H] f16 copy of x in token order
   // Virtual batch (expert parallelism): the tokens are the concatenation of up to 8 segments that
   // sit at fixed places of a larger buffer, with their lengths known on the device only.  When
   // `virt` is set, T above is an upper bound used for grid sizes, the token count is virt->total, and
@@ -182,7 +181,7 @@ __device__ __forceinline__ int coli_virt_row(const VirtualBatch *v, int j) {
   while (s + 1 < v->nseg && j >= v->off[s + 1]) ++s;
   return v->phys[s] * v->stride + (j - v->off[s]);
 }
-int launch_permute(const PermuteParams &p, cudaStream_t st);
+int launch_permute(const PermuteParams &p, cudaStream_t st);  // positions, work list and gathered rows
 // Router + top-k + permutation of a decode-sized batch (T <= 8) in one launch.  Returns 1 on
 // success, 0 on error, -1 when the shapes do not qualify (run launch_router + launch_permute).
 // `ticket` is a device word that is zero between launches.
@@ -298,9 +297,7 @@ int launch_matmul_f32_seq(const float *x, const float *w, float *y, int S, int I
 // fitting on one, packs onto the SMs that happen to be free while its predecessor still runs (the
 // router of 4096 tokens took 1180 us instead of 445 that way).  The top-k and the router GEMMs of up to a few hundred
 // tokens keep their spread by the shared memory they ask for (launch_router_kernel in routing.cu); larger router GEMMs are
-// launched the ordinary way.  The decode expert kernel is two CTAs on every SM wherever it starts.  Behind the
-// three-launch permutation the expert kernel of the time packed (FP8, 130 tokens, H 4096, I 1024, 256 experts: 1030 us a
-// call, 558 when the permutation let it start only when it was done), so k_permute triggers early only for gathered rows.
+// launched the ordinary way.  The decode expert kernel is two CTAs on every SM wherever it starts.
 __device__ __forceinline__ void coli_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void coli_grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void coli_grid_dependency_sync() {

@@ -994,24 +994,13 @@ __global__ void __launch_bounds__(1024) k_seg_scan(PermuteParams p, int nchunk, 
 }
 
 __global__ void __launch_bounds__(256) k_permute(PermuteParams p) {
-  if (p.xg) coli_grid_trigger();  // (without gathered rows the decode expert kernel follows: launch_dependent)
-  coli_grid_wait();
-  // one warp per (t, kk) row; rows T*k .. T*k+T-1 are the shared expert's identity rows; when a
-  // token-order f16 copy of x is wanted, T more warps write it
+  coli_grid_dependency_sync();
+  // one warp per (t, kk) row; rows T*k .. T*k+T-1 are the shared expert's identity rows
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int T = p.virt ? p.virt->total : p.T;
   const int nrouted = T * p.k;
   const int total = nrouted + (p.has_shared ? T : 0);
-  if (warp >= total) {
-    const int t = warp - total;
-    if (p.x16 && t < T) {
-      const int vec = p.H / 8;
-      const uint4 *src = reinterpret_cast<const uint4 *>(p.x + (size_t)t * p.H);
-      uint4 *dst = reinterpret_cast<uint4 *>(p.x16 + (size_t)t * p.H);
-      for (int c = lane; c < vec; c += 32) dst[c] = coli_bf16x8_to_f16x8(src[c]);
-    }
-    return;
-  }
+  if (warp >= total) return;
   int t, pos;
   int trow;  // row of the token in x / topk_idx
   if (warp < nrouted) {
@@ -1038,25 +1027,22 @@ __global__ void __launch_bounds__(256) k_permute(PermuteParams p) {
     pos = p.seg_off[p.nseg_routed] + t;
   }
   if (lane == 0) p.row_token[pos] = t;
-  if (p.xg && (warp < nrouted || p.gather_shared)) {
-    const int vec = p.H / 8;
-    const uint4 *src = reinterpret_cast<const uint4 *>(p.x + (size_t)trow * p.H);
-    uint4 *dst = reinterpret_cast<uint4 *>(p.xg + (size_t)pos * p.H);
-    int c = lane;
-    for (; c + 96 < vec; c += 128) {  // four loads in flight per lane
-      uint4 v[4];
+  const int vec = p.H / 8;
+  const uint4 *src = reinterpret_cast<const uint4 *>(p.x + (size_t)trow * p.H);
+  uint4 *dst = reinterpret_cast<uint4 *>(p.xg + (size_t)pos * p.H);
+  int c = lane;
+  for (; c + 96 < vec; c += 128) {  // four loads in flight per lane
+    uint4 v[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = src[c + 32 * u];
+    for (int u = 0; u < 4; ++u) v[u] = src[c + 32 * u];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) dst[c + 32 * u] = coli_bf16x8_to_f16x8(v[u]);
-    }
-    for (; c < vec; c += 32) dst[c] = coli_bf16x8_to_f16x8(src[c]);
+    for (int u = 0; u < 4; ++u) dst[c + 32 * u] = coli_bf16x8_to_f16x8(v[u]);
   }
+  for (; c < vec; c += 32) dst[c] = coli_bf16x8_to_f16x8(src[c]);
 }
 
-// Decode-sized batches (T*k <= 1024 pairs): count, scan, work list and row positions by ONE CTA
-// instead of three launches (each launch costs about as much as the whole decode GEMV).
-// Same stable order as the three-kernel path: positions ascend with the token inside an expert.
+// The same for the gather of at most 1024 pairs and 128 KB of rows: count, scan, work list, row positions and rows by ONE
+// CTA instead of three launches.  Same stable order: positions ascend with the token inside an expert.
 struct PermuteSmallSmem {
   __align__(16) int idx[1024];
   int cnt[1024 + 1];
@@ -1064,10 +1050,11 @@ struct PermuteSmallSmem {
   int rank[1024];
   int ibase[1024 + 2];
 };
-__device__ __forceinline__ void permute_small_body(const PermuteParams &p, int max_items, PermuteSmallSmem &sm) {
+__global__ void __launch_bounds__(1024) k_permute_small(PermuteParams p, int max_items) {
+  coli_grid_wait();
+  __shared__ PermuteSmallSmem sm;
   int *cnt = sm.cnt, *off = sm.off, *rank_sm = sm.rank, *idx_sm = sm.idx;
-  const int E = p.E, nrt = p.nseg_routed, nseg = nrt + (p.has_shared ? 1 : 0);
-  const int npairs = p.T * p.k;
+  const int E = p.E, nseg = p.nseg_routed, npairs = p.T * p.k;
   for (int e = threadIdx.x; e <= E; e += blockDim.x) cnt[e] = 0;
   // segment of every pair, fetched with independent loads before the ordered walk below
   for (int i = threadIdx.x; i < npairs; i += blockDim.x) {
@@ -1081,42 +1068,24 @@ __device__ __forceinline__ void permute_small_body(const PermuteParams &p, int m
     rank_sm[i] = rank_before(idx_sm, i);
     atomicAdd(cnt + s, 1);
   }
-  if (threadIdx.x == 0 && p.has_shared) cnt[nrt] = p.T;
   __syncthreads();
   build_work_list(p, cnt, nseg, max_items, off, sm.ibase);
   for (int s = threadIdx.x; s <= nseg; s += blockDim.x) p.seg_off[s] = off[s];
   if (p.seg_count)
-    for (int s = threadIdx.x; s < nrt; s += blockDim.x) p.seg_count[s] = cnt[s];
+    for (int s = threadIdx.x; s < nseg; s += blockDim.x) p.seg_count[s] = cnt[s];
   for (int i = threadIdx.x; i < npairs; i += blockDim.x) {
     const int s = idx_sm[i];
-    if (s < 0) {
-      p.slot[i] = -1;
-      continue;
-    }
-    const int pos = off[s] + rank_sm[i];
+    const int pos = s < 0 ? -1 : off[s] + rank_sm[i];
     p.slot[i] = pos;
-    p.row_token[pos] = i / p.k;
+    if (s >= 0) p.row_token[pos] = i / p.k;
   }
-  if (p.has_shared)
-    for (int t = threadIdx.x; t < p.T; t += blockDim.x) p.row_token[off[nrt] + t] = t;
-  if (p.xg) {  // gather rows: one warp per row
-    const int total = npairs + ((p.has_shared && p.gather_shared) ? p.T : 0);
-    const int vec = p.H / 8;
-    for (int r = threadIdx.x >> 5; r < total; r += blockDim.x >> 5) {
-      int t, pos;
-      if (r < npairs) {
-        const int s = idx_sm[r];
-        if (s < 0) continue;
-        t = r / p.k;
-        pos = off[s] + rank_sm[r];
-      } else {
-        t = r - npairs;
-        pos = off[nrt] + t;
-      }
-      const uint4 *src = reinterpret_cast<const uint4 *>(p.x + (size_t)t * p.H);
-      uint4 *dst = reinterpret_cast<uint4 *>(p.xg + (size_t)pos * p.H);
-      for (int c = threadIdx.x & 31; c < vec; c += 32) dst[c] = coli_bf16x8_to_f16x8(src[c]);
-    }
+  const int vec = p.H / 8;
+  for (int r = threadIdx.x >> 5; r < npairs; r += blockDim.x >> 5) {  // one warp per row
+    const int s = idx_sm[r];
+    if (s < 0) continue;
+    const uint4 *src = reinterpret_cast<const uint4 *>(p.x + (size_t)(r / p.k) * p.H);
+    uint4 *dst = reinterpret_cast<uint4 *>(p.xg + (size_t)(off[s] + rank_sm[r]) * p.H);
+    for (int c = threadIdx.x & 31; c < vec; c += 32) dst[c] = coli_bf16x8_to_f16x8(src[c]);
   }
 }
 
@@ -1183,7 +1152,7 @@ __device__ __forceinline__ void permute_pairs(const PermuteParams &p, int max_it
   }
   if (i == 0 && !dry) *p.n_items = min(items, max_items);
   if (p.xg && !dry) {  // gather rows: one warp per row
-    const int total = n + ((p.has_shared && p.gather_shared) ? p.T : 0);
+    const int total = n + (p.has_shared ? p.T : 0);
     const int vec = p.H / 8;
     for (int r = i >> 5; r < total; r += threads >> 5) {
       const int t = r < n ? r / p.k : r - n, to = r < n ? sm.pos[r] : rows + t;
@@ -1197,20 +1166,6 @@ __device__ __forceinline__ void permute_pairs(const PermuteParams &p, int max_it
 // a pair's segment: below 0 for an id that is no expert or lives on another rank
 __device__ __forceinline__ int pair_segment(const PermuteParams &p, int id) {
   return (id < 0 || id >= p.E) ? -1 : (p.expert_slot ? p.expert_slot[id] : id);
-}
-
-__global__ void __launch_bounds__(1024) k_permute_small(PermuteParams p, int max_items) {
-  coli_grid_wait();
-  __shared__ PermuteSmallSmem sm;
-  if (blockIdx.x > 0) {  // the extra CTAs only write the token-order f16 copy of x
-    const size_t n = (size_t)p.T * p.H / 8;
-    const uint4 *src = reinterpret_cast<const uint4 *>(p.x);
-    uint4 *dst = reinterpret_cast<uint4 *>(p.x16);
-    for (size_t i = (size_t)(blockIdx.x - 1) * blockDim.x + threadIdx.x; i < n; i += (size_t)(gridDim.x - 1) * blockDim.x)
-      dst[i] = coli_bf16x8_to_f16x8(src[i]);
-    return;
-  }
-  permute_small_body(p, max_items, sm);
 }
 
 // Decode front end (T <= 8): router logits, top-k and the permutation in ONE launch.  Every CTA
@@ -1344,7 +1299,7 @@ __global__ void __launch_bounds__(256) k_place_rows(PermuteParams p, int max_ite
     if (warp < nrouted) p.slot[warp] = seg < 0 ? -1 : pos;
     if (seg >= 0) p.row_token[pos] = t;
   }
-  if (!p.xg || seg < 0 || (warp >= nrouted && !p.gather_shared)) return;
+  if (!p.xg || seg < 0) return;
   const int vec = p.H / 8;
   const uint4 *src = reinterpret_cast<const uint4 *>(p.x + (size_t)t * p.H);
   uint4 *dst = reinterpret_cast<uint4 *>(p.xg + (size_t)pos * p.H);
@@ -1359,7 +1314,6 @@ __global__ void __launch_bounds__(256) k_place_rows(PermuteParams p, int max_ite
   for (; c < vec; c += 32) dst[c] = coli_bf16x8_to_f16x8(src[c]);
 }
 
-static bool permute_small_ok(const PermuteParams &p) { return p.T * p.k <= 1024 && p.k <= 32 && p.E <= 1024; }
 static int permute_max_items(const PermuteParams &p) {
   return max_work_items(p.T * p.k + (p.has_shared ? p.T : 0), p.nseg_routed + (p.has_shared ? 1 : 0), p.rows_per_item);
 }
@@ -1396,20 +1350,18 @@ int launch_permute(const PermuteParams &p, cudaStream_t st) {
     coli_set_error("permute: E=%d exceeds 1024", p.E);
     return 0;
   }
+  if (!p.xg) {
+    coli_set_error("permute: no buffer for the gathered rows");
+    return 0;
+  }
   const int nchunk = (p.T + 31) / 32;
   const int max_items = permute_max_items(p);
-  // the one-CTA form also gathers the rows: fine up to ~128 KB of them, far too slow for a megabyte
-  if (!p.virt && permute_small_ok(p) && (!p.xg || (size_t)p.T * (p.k + 1) * p.H * 2 <= 128 * 1024)) {
-    int conv = 0;
-    if (p.x16) {
-      const size_t n = (size_t)p.T * p.H / 8;
-      conv = (int)((n + 1023) / 1024);
-      if (conv > 64) conv = 64;
-    }
+  // one CTA gathers 128 KB of rows in time, a megabyte far too slowly
+  if (!p.virt && !p.has_shared && p.T * p.k <= 1024 && (size_t)p.T * (p.k + 1) * p.H * 2 <= 128 * 1024) {
     coli_count_launch(1);
-    return coli_cuda_check(launch_dependent(k_permute_small, dim3(1 + conv), dim3(1024), 0, st, p, max_items), "permute launch") ? 1 : 0;
+    return coli_cuda_check(launch_dependent(k_permute_small, dim3(1), dim3(1024), 0, st, p, max_items), "permute launch") ? 1 : 0;
   }
-  const int total = p.T * p.k + (p.has_shared ? p.T : 0) + (p.x16 ? p.T : 0);
+  const int total = p.T * p.k + (p.has_shared ? p.T : 0);
   coli_count_launch(3);
   return coli_cuda_check(launch_dependent(k_seg_count, dim3(nchunk), dim3(256), (size_t)(32 * p.k + p.E) * sizeof(int), st, p, nchunk), "permute launch") &&
                  coli_cuda_check(launch_dependent(k_seg_scan, dim3(1), dim3(1024), 0, st, p, nchunk, max_items), "permute launch") &&

@@ -2,23 +2,22 @@
 import pytest
 
 from speedycolibri_b200 import synth
-from speedycolibri_b200.configs import FMT_E4M3_ROW, MoeShape
+from speedycolibri_b200.configs import FMT_NVFP4, MoeShape
 
 pytestmark = pytest.mark.gpu
 
 
 def test_the_three_launch_permutation_does_not_slow_the_expert_kernel(gpu_backend):
-    """From 1024 (token, expert) pairs on the permutation takes three launches, whose last once let the
-    register-level expert kernel start early: its CTAs packed onto the SMs that were free, and a call of 130
-    tokens took 1.8 times one of 126.  Three per cent more tokens and two more launches stay within 1.3."""
+    """Above 65536 (token, expert) pairs rows are permuted in three launches instead of placed in one, and the expert kernel
+    may start while the last of them runs.  Thirty tokens more on the other side of that line stay within 1.2."""
     import torch
 
     from speedycolibri_b200.moe import Config, MoeBlock
 
-    shape = MoeShape("overlap", H=2048, E=256, k=8, I=768, T=130, fmt=FMT_E4M3_ROW)
-    blk = MoeBlock(Config.from_shape(shape), synth.device_layer(shape), 256)
+    shape = MoeShape("overlap", H=512, E=64, k=16, I=512, T=4130, fmt=FMT_NVFP4)
+    blk = MoeBlock(Config.from_shape(shape), synth.device_layer(shape), 4130)
 
-    def best_of(T, rounds=5, calls=20):
+    def best_of(T, rounds=5, calls=10):
         x = torch.randn((T, shape.H), device="cuda").to(torch.bfloat16)
         out = torch.empty_like(x)
         times = []
@@ -33,5 +32,5 @@ def test_the_three_launch_permutation_does_not_slow_the_expert_kernel(gpu_backen
             times.append(begin.elapsed_time(end))
         return min(times)
 
-    assert best_of(130) <= 1.3 * best_of(126)
+    assert best_of(4126) <= 1.2 * best_of(4096)
     blk.close()
