@@ -1011,7 +1011,9 @@ extern "C" int coli_b200_moe_block(ColiMoe *m, const void *x, void *out, int T, 
     CK(cudaMemcpyAsync(m->x_stage, x, bytes, cudaMemcpyHostToDevice, st), "moe_block input upload");
   else if (!copies.upload(m->x_stage, x, bytes, false, "moe_block input upload"))
     return 0;
-  // page-locked results are written by the last kernel itself, as it makes them (1024 tokens, H 2048: 389 -> 372 us a call)
+  // Page-locked results are written by the last kernel itself, as it makes them, whatever their size (us a call, copied behind
+  // the kernels / written by the last: 4 KB 48.4 / 46.0, 64 KB 94.6 / 92.6, 1 MB 194 / 194, 4 MB 374.5 / 371.4, 16 MB 1125 / 1110,
+  // 32 MB 2135 / 2104, 59 MB 5603 / 5559).
   void *mapped = colib_host::mapped_host(out, bytes);
   if ((reinterpret_cast<uintptr_t>(mapped) & 15) != 0) mapped = nullptr;
   if (!coli_b200_moe_block_dev(m, m->x_stage, mapped ? mapped : m->out_stage, T, st)) return 0;

@@ -2,7 +2,7 @@
 //
 // The driver copies pageable memory through staging buffers of its own, one thread, before and after the transfer:
 // 1.3 MB took 92 us to the device and 103 back where the link needs 24.  Here a ring of page-locked chunks
-// (4 MB a device) stands between: up to four threads copy chunks while kernels move others over the link, which
+// (4 MB a device) stands between: the calling thread and up to three helpers copy chunks while kernels move others over the link, which
 // also convert what has to be converted.  A chunk that has arrived is announced by a word in the same memory:
 // with a copy command and an event for each chunk the same ring was no faster than the driver (90 + 95 us).
 // Memory that is page-locked already, and less than kDirectBytes, goes as it is.
@@ -23,10 +23,10 @@ namespace colib_host {
 
 constexpr size_t kChunk = colib::HOST_CHUNK;
 constexpr int kHalf = 32;                    // chunks of one half of the ring; a batch fills a half
-// Expert group calls of 8 experts, H 2048, us with the driver's copies and with the ring: 128 KB of rows 94 / 85, 256 KB 109 / 95,
-// 512 KB 169 / 128, 1 MB 250 / 168, 4 MB 580 / 367, 16 MB 1900 / 1010, 256 MB 79 400 / 35 400.  Less than 256 KB gains little, and
-// a group there keeps the number of launches that its callers know (rows that are not converted need one more).
-constexpr size_t kDirectBytes = 256 * 1024;
+// Expert group calls of 8 experts, H 2048, us with the driver's copies and with the ring: 64 KB of rows 82 / 78, 96 KB 91 / 84, 128 KB
+// 94 / 87, 192 KB 103 / 92, 256 KB 113 / 97, 1 MB 250 / 168, 4 MB 580 / 367, 16 MB 1900 / 1010, 256 MB 79 400 / 35 400; block calls
+// with 32 KB of rows 63 / 62, 64 KB 67 / 66, 96 KB 94 / 85.
+constexpr size_t kDirectBytes = 64 * 1024;
 
 // One batch of chunks: chunk i may be copied once i < ready, and is when done[i].
 struct CopyBatch {

@@ -31,7 +31,7 @@ def on_device(blk, x):
     return blk.forward(torch.from_numpy(x.view(np.int16)).cuda().view(torch.bfloat16)).view(torch.int16).cpu().numpy().view(np.uint16)
 
 
-@pytest.mark.parametrize("T", [1, 63, 64, 65, 80, 511, 512, 513, 1024, 1025, 1536, 1537, 1600])
+@pytest.mark.parametrize("T", [1, 15, 16, 17, 63, 64, 65, 80, 511, 512, 513, 1024, 1025, 1536, 1537, 1600])
 @pytest.mark.parametrize("pinned", [False, True], ids=["pageable", "pinned"])
 def test_host_rows_give_what_device_rows_give(block, T, pinned):
     import torch
@@ -89,3 +89,17 @@ def test_results_in_a_buffer_registered_in_parts(block):
     finally:
         for p in parts:
             lib.coli_cuda_host_unregister(ctypes.c_void_p(p))
+
+
+@pytest.mark.parametrize("rows", [[1, 2, 4], [3, 4, 1], [2, 4, 3], [8, 8, 16], [9, 8, 16]])
+def test_host_groups_on_both_sides_of_what_goes_as_it_is(gpu_backend, rows):
+    """7, 8 and 9 rows of 8 KB below 8 an expert, 32 and 33 above: the rows of a call are those of calls with one row each."""
+    shape = MoeShape("host_groups", H=H, E=3, k=1, I=64, T=1)
+    es = synth.device_layer(shape).experts
+    x = np.random.default_rng(sum(rows)).standard_normal((sum(rows), H)).astype(np.float32)
+    y = gpu_backend.expert_group([e.gate for e in es], [e.up for e in es], [e.down for e in es], rows, x)
+    of = np.repeat(np.arange(3), rows)
+    for i in range(len(x)):
+        want = gpu_backend.expert_group([es[of[i]].gate], [es[of[i]].up], [es[of[i]].down], [1], x[i:i + 1])[0]
+        # h in bf16 on both sides, from 8 rows an expert on also y (2^-9 relative each)
+        assert np.linalg.norm(y[i] - want) <= 5e-3 * np.linalg.norm(want)
