@@ -61,8 +61,8 @@ NCU_TRAFFIC = {
     ("c3", 4096, "down"): (2656090112, "profiles/k_ffn_tct_c3s.md (c3s capture x 8)", "expert_tc_tmem.cu", "7ee0edfa51e6"),
     ("c2", 512, "gate_up"): (432590848, "profiles/k_ffn_tct_c2.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
     ("c2", 512, "down"): (218450176, "profiles/k_ffn_tct_c2.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
-    ("c1", 8, "gate_up"): (94130000, "profiles/k_ffn_stream_c1.md", "expert_small.cu", "807e7ad6ca3f"),
-    ("c1", 8, "down"): (46180000, "profiles/k_ffn_stream_c1.md", "expert_small.cu", "807e7ad6ca3f"),
+    ("c1", 8, "gate_up"): (94094080, "profiles/k_ffn_stream_c1.md", "expert_small.cu", "f21ec26168b6"),
+    ("c1", 8, "down"): (46182656, "profiles/k_ffn_stream_c1.md", "expert_small.cu", "f21ec26168b6"),
     ("c4s", 2048, "gate_up"): (997067264, "profiles/k_ffn_tct_c4s.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
     ("c4s", 2048, "down"): (585076480, "profiles/k_ffn_tct_c4s.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
 }

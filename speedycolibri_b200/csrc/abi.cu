@@ -862,7 +862,7 @@ static int moe_block_impl(ColiMoe *m, const void *x_dev, void *out_dev, float *r
   cp.out = (__nv_bfloat16 *)out_dev;
   cp.out32 = resid_io;
   cp.resid = resid_io;
-  const bool one = T == 1 && !tc && colib::down_combine_one_ok(k + (m->has_shared ? 1 : 0), m->L.H);
+  const bool one = T == 1 && !tc && colib::down_combine_one_ok(k + (m->has_shared ? 1 : 0), m->L.H, m->L.I);
   if (tc) {
     colib::TcParams tp;
     tp.fmt = m->L.fmt;

@@ -757,12 +757,14 @@ static int launch_stream_rows(const FfnParams &p, bool gated, bool items_known, 
 // of K through a ring of its own, then the weighted sum of k_combine -- the same terms, rounded the same way -- out of
 // shared memory.  The result rows never leave the SM, and a launch and its wait are gone from a chain of four.
 // The rings are filled before the input is there, as those of the kernel above.
-// One token on H 2048, I 768, 128 experts: 25.9 -> 24.7 us a call.  From more features than SMs x 16 on the two kernels are
-// better (H 7168, I 2048, 256 experts: 80.7 and 84.4): there the whole of K by one warp is a long chain.
-constexpr int kOneRows = 17, kOneStages = 6;
+// Two kernels / this one, us a call: H 2048, I 768, 128 experts 25.9 / 24.7, FP8 28.3 / 27.5; H 1024, I 512 18.8 / 17.4, I 768 20.8 / 19.6.
+// Not from more features than SMs x 16 on (H 7168, I 2048, 256 experts 80.7 / 84.4), nor from eight k-tiles on, where one warp's
+// chain is as long as that of eight warps that share the K: I 1024 20.8 / 21.5 (H 1024), 24.5 / 24.5 (1536), 27.6 / 27.6 (2048), 30.9 /
+// 30.3 (2304); I 1408 32.8 / 34.6 (2048); I 2048 25.4 / 31.8 (1024), 37.0 / 40.8 (2048).
+constexpr int kOneRows = 17, kOneStages = 6, kOneTiles = 7;
 template <int FMT>
 constexpr size_t one_smem(int rows) {  // a warp's ring, its row of the result, its sums
-  return (size_t)rows * (kOneStages * 16 * (FMT == COLI_FMT_NVFP4 ? 72 : 128) + (16 + 8 * 16) * sizeof(float));
+  return (size_t)rows * (kOneStages * 16 * (FMT == COLI_FMT_NVFP4 ? 72 : 128) + (16 + 4 * 16) * sizeof(float));
 }
 // CHAIN: all of K is one sum.  Otherwise k-tile kt adds into sum kt % ks and the sums are added in order, as the ks warps of a
 // split task do it; two k-tiles, of different sums, are multiplied side by side.
@@ -775,7 +777,7 @@ __global__ void __launch_bounds__(32 * kOneRows) k_down_combine_one(FfnParams p,
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), rows = (int)blockDim.x >> 5;
   const int K = p.I, KT = (K + 127) >> 7, Op = (p.H + 15) & ~15, r0 = (int)blockIdx.x * 16;
   float *ys = reinterpret_cast<float *>(smem_raw + (size_t)rows * kOneStages * SLOT);  // [rows][16]
-  float *sums = ys + rows * 16 + warp * (8 * 16);                                      // [8][16]
+  float *sums = ys + rows * 16 + warp * (4 * 16);                                      // [ks][16], ks <= 4 with so few k-tiles
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem_raw) + warp * (kOneStages * SLOT);
   if (!items_known) coli_grid_wait();
   const int ex = warp < c.k ? __ldcg(topk_idx + warp) : shared;
@@ -920,7 +922,7 @@ __global__ void __launch_bounds__(32 * kOneRows) k_down_combine_one(FfnParams p,
   else
     c.out[o] = __float2bfloat16_rn(sum);
 }
-bool down_combine_one_ok(int rows, int H) { return rows <= kOneRows && (H + 15) / 16 <= COLI_SMS; }
+bool down_combine_one_ok(int rows, int H, int I) { return rows <= kOneRows && (H + 15) / 16 <= COLI_SMS && (I + 127) / 128 <= kOneTiles; }
 template <int FMT, bool CHAIN>
 static int launch_one_token_as(const FfnParams &p, const CombineParams &c, const int32_t *topk_idx, int shared, bool items_known, int ks, cudaStream_t st) {
   const int rows = c.k + c.has_shared;

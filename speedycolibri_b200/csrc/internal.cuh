@@ -264,7 +264,7 @@ struct CombineParams {
 };
 // One token: down of its `rows` = k (+ 1 shared) rows and their combine in one launch, behind launch_gate_up_small
 // (`items_known` as for launch_down_small); expert ids in topk_idx, the shared expert is entry `shared` of the tables.
-bool down_combine_one_ok(int rows, int H);
+bool down_combine_one_ok(int rows, int H, int I);
 int launch_down_combine_one(const FfnParams &p, const CombineParams &c, const int32_t *topk_idx, int shared, bool items_known, cudaStream_t st);
 int launch_combine(const CombineParams &p, cudaStream_t st);
 int launch_finish(const float *partial, const __nv_bfloat16 *shared_y, __nv_bfloat16 *out, int T, int H, cudaStream_t st);

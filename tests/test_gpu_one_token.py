@@ -1,5 +1,5 @@
 """One token, whose down projection and combine are one launch: formats, rows and K that end inside a tile, as many
-rows as the launch takes and one more, and the residual stream of a layer step."""
+rows and k-tiles as the launch takes and one more, and the residual stream of a layer step."""
 import numpy as np
 import pytest
 
@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("fmt", [FMT_NVFP4, FMT_FP8_B128, FMT_E4M3_ROW, FMT_MXFP4], ids=["nvfp4", "fp8_b128", "e4m3_row", "mxfp4"])
 @pytest.mark.parametrize("H,I,E,k,shared", [(264, 200, 20, 4, True), (128, 128, 20, 16, True), (72, 136, 20, 17, True),
-                                            (128, 1032, 18, 17, False), (64, 8, 16, 1, False), (2368, 64, 8, 2, True), (2376, 64, 8, 2, True)])
+                                            (128, 1032, 18, 17, False), (64, 8, 16, 1, False), (2368, 64, 8, 2, True), (2376, 64, 8, 2, True),
+                                            (128, 896, 18, 4, True), (128, 904, 18, 4, True), (1800, 272, 20, 16, True)])
 def test_one_token(gpu_backend, orc, fmt, H, I, E, k, shared):
     import torch
 
@@ -25,7 +26,7 @@ def test_one_token(gpu_backend, orc, fmt, H, I, E, k, shared):
     x = synth.host_tokens(shape)
     before = _lib.load().coli_b200_launch_count()
     out, idx, w = blk.moe(x, want_routing=True)
-    assert _lib.load().coli_b200_launch_count() - before == (3 if k + shared <= 17 and H <= 16 * 148 else 4)
+    assert _lib.load().coli_b200_launch_count() - before == (3 if k + shared <= 17 and H <= 16 * 148 and I <= 7 * 128 else 4)
     want = L.moe_block(x)
     assert np.array_equal(idx, want["idx"]) and np.array_equal(w.view(np.uint32), want["w"].view(np.uint32))
     # h and y are rounded to bf16, 2^-9 relative each
