@@ -55,16 +55,16 @@ def measured_peaks():
 # a different share of the experts active than the small case c4s, so the streams do not scale by a
 # constant.  The captures are summarised under profiles/.
 NCU_TRAFFIC = {
-    ("c3s", 512, "gate_up"): (633368320, "profiles/k_ffn_tct_c3s.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
-    ("c3s", 512, "down"): (332011264, "profiles/k_ffn_tct_c3s.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
-    ("c3", 4096, "gate_up"): (5066946560, "profiles/k_ffn_tct_c3s.md (c3s capture x 8)", "expert_tc_tmem.cu", "7ee0edfa51e6"),
-    ("c3", 4096, "down"): (2656090112, "profiles/k_ffn_tct_c3s.md (c3s capture x 8)", "expert_tc_tmem.cu", "7ee0edfa51e6"),
-    ("c2", 512, "gate_up"): (432590848, "profiles/k_ffn_tct_c2.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
-    ("c2", 512, "down"): (218450176, "profiles/k_ffn_tct_c2.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
+    ("c3s", 512, "gate_up"): (633377024, "profiles/k_ffn_tct_c3s.md", "expert_tc_tmem.cu", "ca0af473a932"),
+    ("c3s", 512, "down"): (331731200, "profiles/k_ffn_tct_c3s.md", "expert_tc_tmem.cu", "ca0af473a932"),
+    ("c3", 4096, "gate_up"): (5067016192, "profiles/k_ffn_tct_c3s.md (c3s capture x 8)", "expert_tc_tmem.cu", "ca0af473a932"),
+    ("c3", 4096, "down"): (2653849600, "profiles/k_ffn_tct_c3s.md (c3s capture x 8)", "expert_tc_tmem.cu", "ca0af473a932"),
+    ("c2", 512, "gate_up"): (432870144, "profiles/k_ffn_tct_c2.md", "expert_tc_tmem.cu", "ca0af473a932"),
+    ("c2", 512, "down"): (218431232, "profiles/k_ffn_tct_c2.md", "expert_tc_tmem.cu", "ca0af473a932"),
     ("c1", 8, "gate_up"): (94094080, "profiles/k_ffn_stream_c1.md", "expert_small.cu", "f21ec26168b6"),
     ("c1", 8, "down"): (46182656, "profiles/k_ffn_stream_c1.md", "expert_small.cu", "f21ec26168b6"),
-    ("c4s", 2048, "gate_up"): (997067264, "profiles/k_ffn_tct_c4s.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
-    ("c4s", 2048, "down"): (585076480, "profiles/k_ffn_tct_c4s.md", "expert_tc_tmem.cu", "7ee0edfa51e6"),
+    ("c4s", 2048, "gate_up"): (985859840, "profiles/k_ffn_tct_c4s.md", "expert_tc_tmem.cu", "ca0af473a932"),
+    ("c4s", 2048, "down"): (583711488, "profiles/k_ffn_tct_c4s.md", "expert_tc_tmem.cu", "ca0af473a932"),
 }
 
 

@@ -160,7 +160,7 @@ __device__ __forceinline__ void tt_convert(const TtPacked &pk, uint32_t (&r)[32]
 // FP8 (e4m3 codes, one byte per weight): the 64 codes of one row for one 64-k stage and the
 // multiplier of the stage.  A weight is code x scale[row block][k-tile] (convert.rs:731-741, f32);
 // the accumulator runs over all of K inside tensor memory, so the scale cannot be applied per
-// k-tile to partial sums as the register-level kernel does.  Instead each 128-row tile is
+// k-tile to partial sums as the decode kernel does.  Instead each 128-row tile is
 // normalised by the largest scale of its row block: the stage's codes are multiplied by
 // TT_FP8_HEADROOM x scale / max scale (an f16 in (0, 16], one rounding of 2^-11 relative per weight)
 // and the epilogue multiplies the finished sum by max scale / TT_FP8_HEADROOM in f32.  The
