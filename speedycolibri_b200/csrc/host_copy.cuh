@@ -186,8 +186,7 @@ struct HostRing {
   }
 };
 
-// Whether all of `bytes` at `host`, whose attributes are `a`, is of one page-locked allocation or registration.
-inline bool page_locked(const cudaPointerAttributes &a, size_t bytes) {
+inline bool pointer_attribute(void *value, CUpointer_attribute which, CUdeviceptr at) {
   using Fn = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
   static const Fn attribute = [] {
     void *fn = nullptr;
@@ -197,24 +196,30 @@ inline bool page_locked(const cudaPointerAttributes &a, size_t bytes) {
     cudaGetLastError();
     return Fn(nullptr);
   }();
-  if (!attribute || a.type != cudaMemoryTypeHost || !a.devicePointer) return false;
+  return attribute && attribute(value, which, at) == CUDA_SUCCESS;
+}
+
+// Whether all of `bytes` at `host`, whose attributes are `a`, is of one page-locked allocation or registration.
+inline bool page_locked(const cudaPointerAttributes &a, size_t bytes) {
+  if (a.type != cudaMemoryTypeHost || !a.devicePointer) return false;
   CUdeviceptr start = 0;
   size_t size = 0;
   const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(a.devicePointer);
-  if (attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS || attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS)
-    return false;
+  if (!pointer_attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) || !pointer_attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at)) return false;
   return at >= start && at - start <= size && bytes <= size - (at - start);
 }
 
 // The device's address of page-locked memory that kernels may write directly, null for any other (also for a buffer of
-// which only some pages are registered).
+// which only some pages are registered, and for one that is registered for the device to read only).
 inline void *mapped_host(void *host, size_t bytes) {
   cudaPointerAttributes a = {};
   if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  return page_locked(a, bytes) ? a.devicePointer : nullptr;
+  unsigned long long access = 0;
+  if (!page_locked(a, bytes) || !pointer_attribute(&access, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS, reinterpret_cast<CUdeviceptr>(a.devicePointer))) return nullptr;
+  return (access & CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE) == CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE ? a.devicePointer : nullptr;
 }
 
 // Of one host-pointer call: its copies to and from the device on stream `st`.  Sizes are multiples of 16 bytes.

@@ -12,6 +12,7 @@ from speedycolibri_b200 import _lib
 # What a case needs from the runtime: handles and memory that look real, a log of the calls that put work on
 # a stream, and the n-th of them refused.
 SHIM = r"""
+#include <cuda.h>
 #include <driver_types.h>
 #include <stdlib.h>
 #include <string.h>
@@ -29,6 +30,28 @@ int cudaMalloc(void **p, size_t n) { *p = malloc(n ? n : 1); return 0; }
 int cudaFree(void *p) { free(p); return 0; }
 int cudaHostAlloc(void **p, size_t n) { return cudaMalloc(p, n); }
 int cudaFreeHost(void *p) { return cudaFree(p); }
+static char *pinned;  /* the one page-locked allocation: where, how long, what the device may do with it */
+static size_t pinned_n;
+static unsigned long long pinned_access;
+void fake_pin(char *at, size_t n, int access) { pinned = at; pinned_n = n; pinned_access = access; }
+int cudaPointerGetAttributes(struct cudaPointerAttributes *a, char *p) {
+  memset(a, 0, sizeof(*a));
+  if (p >= pinned && p < pinned + pinned_n) a->type = cudaMemoryTypeHost, a->hostPointer = a->devicePointer = p;
+  return 0;
+}
+static int pointer_attribute(void *value, int which, char *p) {
+  if (p < pinned || p >= pinned + pinned_n) return 1;
+  if (which == CU_POINTER_ATTRIBUTE_RANGE_START_ADDR) *(char **)value = pinned;
+  else if (which == CU_POINTER_ATTRIBUTE_RANGE_SIZE) *(size_t *)value = pinned_n;
+  else if (which == CU_POINTER_ATTRIBUTE_ACCESS_FLAGS) *(unsigned long long *)value = pinned_access;
+  else return 1;
+  return 0;
+}
+int cudaGetDriverEntryPoint(const char *name, void **fn, unsigned long long flags, int *found) {
+  *fn = strcmp(name, "cuPointerGetAttribute") ? 0 : (void *)pointer_attribute;
+  *found = 0;
+  return 0;
+}
 int cudaGetDeviceCount(int *n) { *n = 1; return 0; }
 int cudaDeviceGetAttribute(int *v) { *v = 148; return 0; }
 int cudaGetDeviceProperties_v2(struct cudaDeviceProp *p) {
