@@ -168,15 +168,21 @@ int coli_cuda_matmul_nvfp4(ColiCudaTensor **tensor, float *y, const float *x, co
 /* backend_cuda.h:131-132, 152-160: gateless ReLU^2 NVFP4 experts, y = down(relu(up x)^2)
  * (moe.rs:1189-1199).  x, y: host f32, sum(rows) consecutive rows of up->I values in call order.
  * The three forms differ only in how the reference batches its launches; here all run the whole
- * group in two launches.  `exact` is accepted and has no effect: a row's result never depends on
- * the other rows of a call. */
+ * group in two launches.  `exact` is accepted and has no effect: a row's result depends neither on what the
+ * other rows of a call hold nor on its place among them.  (Their number says whether warps share the K of a
+ * small matrix, and with it in how many sums an output's products are added.) */
 int coli_cuda_expert_mlp_nvfp4_relu2(ColiCudaTensor *up, ColiCudaTensor *down, float *y, const float *x, int S, int exact);
 int coli_cuda_expert_group_nvfp4_relu2(ColiCudaTensor *const *ups, ColiCudaTensor *const *downs, const int *rows, int count,
                                        float *y, const float *x);
 int coli_cuda_expert_seg_nvfp4_relu2(ColiCudaTensor *const *ups, ColiCudaTensor *const *downs, const int *rows, int count,
                                      float *y, const float *x);
 /* backend_cuda.h:134-140 / backend_cuda.cu:4410-4792: packed group of same-shaped experts; x and
- * y hold sum(rows) consecutive [D] HOST f32 rows in call order. */
+ * y hold sum(rows) consecutive [D] HOST f32 rows in call order.
+ * On the host, for the expert calls and coli_b200_moe_block: pageable rows from 64 KB on go through 4 MB of page-locked
+ * memory a device, allocated by the first call of any size that may need it and kept until coli_cuda_shutdown; with 8
+ * cores or more three threads of the library (one from 4 cores on) help to copy them.  The threads are started by the first
+ * such call, spin while a call is copying or its kernels run (a few milliseconds at most), sleep between calls
+ * and are joined by coli_cuda_shutdown or the end of the process; a forked child does not have them. */
 int coli_cuda_expert_group_nvfp4(ColiCudaTensor *const *gates, ColiCudaTensor *const *ups,
                                  ColiCudaTensor *const *downs, const int *rows, int count, float *y,
                                  const float *x);
@@ -224,7 +230,8 @@ size_t coli_b200_moe_workspace_bytes(const ColiMoe *moe);
 
 /* One block call, synchronous, HOST bf16 x[T,H] -> HOST bf16 out[T,H] (host<->device copies
  * inside).  topk_idx [T,k] int32 and topk_w [T,k] f32 are optional HOST outputs.  All experts
- * must be resident (single GPU). */
+ * must be resident (single GPU).  A page-locked `out` (16-byte aligned, one allocation or registration) is written by
+ * the last kernel over the link; after a failed call its contents are undefined. */
 int coli_b200_moe_block(ColiMoe *moe, const void *x, void *out, int T, int32_t *topk_idx, float *topk_w);
 /* Same with DEVICE pointers, asynchronous on `stream` (a cudaStream_t; NULL is CUDA's default
  * stream, coli_b200_moe_stream() gives the handle's own).  One handle's workspace serves one

@@ -97,7 +97,7 @@ CONFIGS = {
     "mid_fp8_ragged": MoeShape("mid_fp8_ragged", H=320, E=6, k=2, I=192, T=333, shared=False, fmt=FMT_FP8_B128,
                                block_spread=1.5),
     "mid_fp8row": MoeShape("mid_fp8row", H=256, E=4, k=2, I=128, T=100, fmt=FMT_E4M3_ROW, block_spread=1.0),
-    # MXFP4 (E8M0 scale per 32): register-level and tcgen05 kernel families
+    # MXFP4 (E8M0 scale per 32): decode and tcgen05 kernel families
     "tiny_mx": MoeShape("tiny_mx", H=128, E=8, k=2, I=64, T=21, fmt=FMT_MXFP4, norm_topk=True),
     "mid_mx": MoeShape("mid_mx", H=512, E=8, k=2, I=256, T=512, fmt=FMT_MXFP4, norm_topk=True, block_spread=1.0),
     "tiny_zipf": MoeShape("tiny_zipf", H=64, E=16, k=4, I=32, T=70, shared=False, zipf_s=1.2),

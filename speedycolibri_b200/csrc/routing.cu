@@ -1175,8 +1175,10 @@ __device__ __forceinline__ int pair_segment(const PermuteParams &p, int id) {
 // The kernel is latency from end to end, and its CTAs must not share an SM: started early, while the
 // previous call's last kernels still hold most SMs, two or three packed onto each free one and the chains
 // took 14.6 cycles per k instead of 6 (8 tokens, 128 experts x 2048: 30 000 of the kernel's 44 000 cycles).
-// kFrontSmem is therefore, with what is static, more than half of an SM's shared memory, and little enough to lie beside one CTA
-// of the decode expert kernel, which may still hold the SM when the front starts.  The last CTA runs top-k and permutation once per
+// kFrontSmem is therefore, with what is static, more than half of an SM's shared memory.  (Beside a CTA of the decode expert
+// kernel, which holds the SM until its tasks are done, the front does not fit: at 213 registers a thread the register file is too
+// small.  Compiled to 96 to 127, by launch bounds or with a kernel for each number of score slots, it does, and no
+// call is shorter by it: 8 tokens 54.9 us a call against 55.1 to 55.6, 1 token 25.2 against 25.2 to 25.5.)  The last CTA runs top-k and permutation once per
 // call, with instructions that the streamed weights have pushed out of every cache: two warps that have nothing else to
 // do run the same code beside the chains, on router weights for logits, and write nothing (8 tokens, the weights of
 // three layers in turn: top-k 2.4 us, permutation 4.6 -> 1.8; the front 15.9 -> 14.4 us).  They and the first router
@@ -1204,7 +1206,9 @@ __global__ void __launch_bounds__(256) k_decode_front(RouteParams rp, PermutePar
         router_tiny_block<kFrontStaging, true>(rp, smem_raw, 0, (int)blockIdx.x * 8);
         continue;
       }
-      if (rp.H >= 4096) coli_grid_wait();  // beside long chains there is time, and before them other kernels (281 / 283 us, 8 x 7168)
+      // beside long chains there is time, and ahead of the wait other kernels run (us a call of 8 tokens, I 512, 128 experts, behind
+      // the wait / ahead of it: H 2048 46.4 / 46.05, 3072 57.4 / 57.2, 4096 72.6 / 73.1, 7168 107.6 / 108.3)
+      if (rp.H >= 4096) coli_grid_wait();
       tp.logits = const_cast<float *>(reinterpret_cast<const float *>(rp.router_w));  // E * H bf16 hold E floats (H >= 8)
       tp.topk_idx = nullptr;
       last = warp == 7 ? 1 : 0;

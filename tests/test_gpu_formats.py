@@ -26,7 +26,7 @@ def bf16_valued(rng, shape):
 # ---- MXFP4 ------------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("name,T", [("tiny_mx", 21), ("tiny_mx", 1), ("mid_mx", 512), ("mid_mx", 77)])
 def test_block_mxfp4(gpu_backend, orc, name, T):
-    """E2M1 nibbles with an E8M0 scale per 32 (linear.rs:134-175): register-level kernel (tiny) and
+    """E2M1 nibbles with an E8M0 scale per 32 (linear.rs:134-175): decode kernel (tiny) and
     tcgen05 kernels (mid, block magnitudes spread over several binades)."""
     shape = CONFIGS[name].with_tokens(T)
     L, packed = host_layer(shape)

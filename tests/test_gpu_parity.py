@@ -278,13 +278,14 @@ def test_block_c4_zipf_full_size(gpu_backend, orc):
 
 def test_row_results_do_not_depend_on_batch(gpu_backend, orc):
     """A token's output must not change with the batch it travels in (the reference's `exact`
-    contract, crates/colibri-engine/src/gpu.rs:122-146)."""
+    contract, crates/colibri-engine/src/gpu.rs:122-146), on a layer of one k-tile.  (On longer ones the decode kernel
+    may share a K among another number of warps in calls of other sizes: test_gpu_sum_order.py.)"""
     shape = CONFIGS["tiny_sig"].with_tokens(200)
     _, packed = host_layer(shape)
     blk = make_block(shape, upload_layer(shape, packed))
     x = synth.host_tokens(shape, 200)
     # kernel family is a function of (rows, segments, format) only: < 8 rows per segment on average
-    # runs the register-level kernel, more the tcgen05 kernel; inside a family rows are bit-stable
+    # runs the decode kernel, more the tcgen05 kernel; inside a family rows are bit-stable
     small = blk.moe(x[:24])
     for n in (1, 7, 16):
         assert np.array_equal(blk.moe(x[:n]), small[:n])

@@ -11,7 +11,7 @@ from tests.helpers import host_layer, rel_l2, upload_layer
 pytestmark = pytest.mark.gpu
 
 
-# 5 tokens: the decode front and the register-level kernel; 37: the same behind the separate router and
+# 5 tokens: the decode front and the decode expert kernel; 37: the same behind the separate router and
 # permutation; 433 and 333: the tcgen05 kernel, with and without a shared expert
 @pytest.mark.parametrize("name,T", [("tiny", 5), ("tiny_sig", 37), ("mid", 433), ("mid_ragged", 333)])
 @pytest.mark.parametrize("rank", [0, 1])

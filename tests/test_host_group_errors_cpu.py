@@ -9,7 +9,7 @@ import pytest
 from tests.fake_cuda import wrap_nvfp4
 
 
-@pytest.mark.parametrize("rows", [3, 40], ids=["register_level", "tcgen05"])
+@pytest.mark.parametrize("rows", [3, 40], ids=["decode", "tcgen05"])
 def test_a_host_group_call_that_fails_leaves_nothing_in_flight(fake_cuda, rows):
     H, I, count = 32, 16, 2
     tensors = [(C.c_void_p * count)() for _ in range(3)]
